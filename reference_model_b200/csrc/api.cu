@@ -17,7 +17,7 @@ namespace tb200
 
 tb200_status raise_smem_limit(tb200_ctx* ctx, int bit, const void* kernel, int bytes)
 {
-    if (ctx->smem_attr_set & (1u << bit))
+    if (ctx->smem_attr_set & (1ull << bit))
         return TB200_OK;
     // a context that knows its device's limit raises the kernel to it once; a bare one (the allocation-free entry
     // point's stack object) asks for what this launch needs, every time
@@ -31,7 +31,7 @@ tb200_status raise_smem_limit(tb200_ctx* ctx, int bit, const void* kernel, int b
     }
     TB200_CUDA_CHECK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, want));
     if (ctx->max_smem_optin > 0)
-        ctx->smem_attr_set |= 1u << bit;
+        ctx->smem_attr_set |= 1ull << bit;
     return TB200_OK;
 }
 
@@ -1292,6 +1292,64 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                 if (!(st == TB200_INTERNAL && ctx->err.find("rejected") != std::string::npos))
                     return st;
             }
+        }
+    }
+
+    // ---- fp32: tiled FFMA kernel (sgemm_f32.cu).  Its row table packs window origins into 16 bits and input offsets into 32.
+    // Padding is a zero-filled tap, which equals the reference's skipped tap only for finite weights: a padded layer whose
+    // weights are not known to be finite takes the kernel below.
+    if (input->dtype == TB200_FP32 && ctx->policy == 0 && input->stride[3] == 1 && IH + pad[0] + pad[1] < 32768 &&
+        IW + pad[2] + pad[3] < 32768 && (int64_t)N * input->stride[0] < (1LL << 31))
+    {
+        const int K             = KH * KW * IC;
+        const size_t flag_off   = (size_t)K * conv_f32_ldb(OC) * sizeof(float);
+        const float* wp         = reinterpret_cast<const float*>(weight->data);
+        auto build = [=](tb200_ctx* c, void* block) -> tb200_status {
+            return conv_f32_weights_launch(c, wp, reinterpret_cast<float*>(block), OC, K,
+                                           reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(block) + flag_off));
+        };
+        Prepared* e = nullptr;
+        if (use_cache && ctx->const_cache_on)
+        {
+            std::string key;
+            key_add(&key, (int)8);
+            key_add(&key, wp); key_add(&key, OC); key_add(&key, K);
+            e = cache_find(ctx, key);
+            if (!e)
+                e = cache_insert(ctx, key, { { reinterpret_cast<const char*>(wp), weight->bytes } }, flag_off + 64, build);
+        }
+        const bool padded = pad[0] || pad[1] || pad[2] || pad[3];
+        void* block       = nullptr;
+        if (e)
+        {
+            st = cache_use(ctx, e);
+            if (st == TB200_OK && padded)
+                st = read_host_flag(ctx, e, flag_off);
+            if (st != TB200_OK)
+                return st;
+            if (!padded || e->host_flag == 1)
+                block = e->block;
+        }
+        else if (!padded)
+        {
+            st = ensure_scratch(ctx, flag_off + 64);
+            if (st == TB200_OK)
+                st = build(ctx, ctx->scratch);
+            if (st != TB200_OK)
+                return st;
+            block = ctx->scratch;
+        }
+        if (block)
+        {
+            ConvF32Problem q;
+            q.in = reinterpret_cast<const float*>(input->data); q.wt = reinterpret_cast<const float*>(block);
+            q.bias = reinterpret_cast<const float*>(bias->data); q.out = reinterpret_cast<float*>(output->data);
+            q.N = N; q.IH = IH; q.IW = IW; q.IC = IC; q.OH = OH; q.OW = OW; q.OC = OC; q.KH = KH; q.KW = KW;
+            q.bias_n = bias->shape[0];
+            q.pad_t = pad[0]; q.pad_l = pad[2]; q.sy = stride[0]; q.sx = stride[1]; q.dy = dilation[0]; q.dx = dilation[1];
+            q.in_sn = input->stride[0]; q.in_sh = input->stride[1]; q.in_sw = input->stride[2];
+            q.has_clamp = epi.has_clamp; q.clamp_lo = epi.clamp_lo_f; q.clamp_hi = epi.clamp_hi_f;
+            return conv_f32_launch(ctx, q);
         }
     }
 

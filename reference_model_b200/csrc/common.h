@@ -96,7 +96,7 @@ struct tb200_ctx
     int join_stream      = 1;    // large table joins through the bulk-copy ring kernel (join_stream.cuh)
     int launch_overlap   = 1;    // launch the kernels that support it with programmatic stream serialization
     int max_pairs[3]     = { 0, 0, 0 };    // resident CTA pairs of the three CTA-pair kernels on this device, 0 = not asked yet
-    uint32_t smem_attr_set = 0;            // bit per kernel whose dynamic shared-memory limit has been raised on this device
+    uint64_t smem_attr_set = 0;            // bit per kernel whose dynamic shared-memory limit has been raised on this device
     // output gather across GPUs (dist.cu): an NCCL communicator created by tb200_comm_init or handed in by the host
     void* comm           = nullptr;
     bool comm_owned      = false;
@@ -362,5 +362,23 @@ tb200_status expand_dw_launch(tb200_ctx* ctx, const ExpandDwProblem& q);
 
 // fp32 SGEMM on CUDA cores (sgemm_f32.cu): out[n] = a[n] x b[n], a [N,H,C], b [N,C,W]
 tb200_status sgemm_f32_launch(tb200_ctx* ctx, const float* a, const float* b, float* out, int N, int H, int C, int W);
+
+// fp32 CONV2D on the same kernel: the input gathered tap by tap as the product's rows, weights re-ordered once to
+// [KH*KW*IC][conv_f32_ldb(OC)] by conv_f32_weights_launch (which leaves 0 in *all_finite when a weight is not finite)
+struct ConvF32Problem
+{
+    const float* in;
+    const float* wt;
+    const float* bias;
+    float* out;
+    int N, IH, IW, IC, OH, OW, OC, KH, KW, bias_n;
+    int pad_t, pad_l, sy, sx, dy, dx;
+    int64_t in_sn, in_sh, in_sw;
+    int has_clamp;
+    float clamp_lo, clamp_hi;
+};
+int conv_f32_ldb(int OC);
+tb200_status conv_f32_weights_launch(tb200_ctx* ctx, const float* w, float* wt, int OC, int K, int* all_finite);
+tb200_status conv_f32_launch(tb200_ctx* ctx, const ConvF32Problem& q);
 
 }    // namespace tb200

@@ -1,0 +1,91 @@
+"""fp32 MATMUL and CONV2D at the edges of the tiled FFMA kernel: row / column / K remainders of every tile size, K split
+over a cluster, unaligned rows, window shapes, strides, dilation, a view, infinite weights under padding; against the
+fp64 oracle under the DOT_PRODUCT rule."""
+import numpy as np
+import pytest
+
+import reference_model_b200 as tb
+from oracle import oracle as orc
+from tests import util
+from tests.test_gpu_parity import _dot_check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = tb.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (3, 17, 15, 33), (2, 129, 33, 129), (1, 64, 2048, 64), (1, 1, 4096, 1000),
+                                   (5, 15, 21, 487), (2, 257, 100, 260), (150, 130, 17, 132), (1, 33, 511, 65)])
+def test_matmul_f32_edges(ctx, shape):
+    N, H, C, W = shape
+    r = util.rng(900 + H + C)
+    a, b = r.standard_normal((N, H, C)).astype(np.float32), r.standard_normal((N, C, W)).astype(np.float32)
+    ta, tbb, to = ctx.from_numpy(a), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, (N, H, W))
+    ctx.matmul(ta, tbb, to)
+    assert ctx.last_kernel() == "sgemm_f32"
+    st, out = to.download()
+    ok, info = _dot_check(out, a.astype(np.float64), b.astype(np.float64), orc.matmul, C, "fp32")
+    assert st == tb.Status.OK and ok, info
+    for t in (ta, tbb, to):
+        t.free()
+
+
+# N, IH, IW, IC, OC, KH, KW, stride, dilation, pad, bias length
+CONV = [(1, 5, 5, 1, 1, 1, 1, [1, 1], [1, 1], [0, 0, 0, 0], 1), (2, 13, 9, 5, 7, 3, 3, [1, 1], [1, 1], [1, 1, 1, 1], 7),
+        (3, 17, 20, 16, 65, 3, 2, [2, 1], [1, 2], [1, 1, 2, 0], 65), (1, 9, 9, 130, 129, 1, 1, [2, 2], [1, 1], [0, 0, 0, 0], 129),
+        (4, 30, 31, 3, 64, 5, 5, [1, 1], [1, 1], [2, 2, 2, 2], 64), (1, 4, 4, 512, 33, 3, 3, [1, 1], [1, 1], [1, 1, 1, 1], 33),
+        (8, 28, 28, 40, 128, 3, 3, [1, 1], [1, 1], [1, 1, 1, 1], 128)]
+
+
+@pytest.mark.parametrize("case", range(len(CONV)))
+def test_conv_f32_edges(ctx, case):
+    N, IH, IW, IC, OC, KH, KW, stride, dil, pad, nb = CONV[case]
+    r = util.rng(950 + case)
+    x, w = r.standard_normal((N, IH, IW, IC)).astype(np.float32), r.standard_normal((OC, KH, KW, IC)).astype(np.float32)
+    b = r.standard_normal(nb).astype(np.float32)
+    OH, OW = orc.conv_out_hw(IH, IW, KH, KW, pad, stride, dil)
+    ref = orc.conv2d(x, w, b, pad, stride, dil, mode="f64")
+    bnd = orc.conv2d(x, w, b, pad, stride, dil, mode="f64", bounds=True)
+    ksb = orc.dot_product_ksb(KH * KW * IC + 1, "fp32", "fp32")
+    tx, tw, tbias, to = ctx.from_numpy(x), ctx.from_numpy(w), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, (N, OH, OW, OC))
+    for cache in (ctx.CACHE_ON, ctx.CACHE_OFF):    # without the cache a padded layer runs the untiled kernel
+        ctx.const_cache_control(cache)
+        ctx.conv2d(tx, tw, tbias, to, pad, stride, dil)
+        assert ctx.last_kernel() == ("conv_f32" if cache or not any(pad) else "conv2d_direct")
+        st, out = to.download()
+        ok, info = orc.verify_dot_product(out, ref, bnd, ksb, out="fp32")
+        assert st == tb.Status.OK and ok, (cache, info)
+    ctx.const_cache_control(ctx.CACHE_ON)
+    ctx.conv2d(tx, tw, tbias, to, pad, stride, dil, epilogue=tb.Epilogue(None, (-0.5, 1.0)))
+    st, clamped = to.download()
+    assert np.array_equal(clamped, np.clip(out, -0.5, 1.0)) or orc.verify_dot_product(
+        clamped, np.clip(ref, -0.5, 1.0), bnd, ksb, out="fp32")[0]
+    for t in (tx, tw, tbias, to):
+        t.free()
+
+
+def test_conv_f32_view_and_infinite_weight(ctx):
+    r = util.rng(970)
+    x, w = r.standard_normal((2, 9, 9, 8)).astype(np.float32), r.standard_normal((5, 3, 3, 8)).astype(np.float32)
+    b = r.standard_normal(5).astype(np.float32)
+    tx, tw, tbias, to = ctx.from_numpy(x), ctx.from_numpy(w), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, (2, 7, 7, 5))
+    view = tx.slice([0, 1, 2, 0], [2, 7, 7, 8])
+    ctx.conv2d(view, tw, tbias, to, [1, 1, 1, 1], [1, 1], [1, 1])
+    assert ctx.last_kernel() == "conv_f32"
+    xv = np.ascontiguousarray(x[:, 1:8, 2:9])
+    args = ([1, 1, 1, 1], [1, 1], [1, 1])
+    ok, info = orc.verify_dot_product(to.download()[1], orc.conv2d(xv, w, b, *args, mode="f64"),
+                                      orc.conv2d(xv, w, b, *args, mode="f64", bounds=True), orc.dot_product_ksb(73, "fp32", "fp32"))
+    assert ok, info
+    # new weights through an upload, one of them infinite: skipped taps stay skipped (the corner has no NaN)
+    w[0, 0, 0, 0] = np.inf
+    tw.upload(w)
+    ctx.conv2d(view, tw, tbias, to, *args)
+    assert ctx.last_kernel() == "conv2d_direct"
+    out = to.download()[1]
+    assert not np.isnan(out).any() and np.isinf(out[:, 1:, 1:, 0]).all() and np.isfinite(out[:, 0, :, 0]).all()
