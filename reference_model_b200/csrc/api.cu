@@ -870,10 +870,11 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
     if (!dry_run)
         cache_note_write(ctx, output->data, output->bytes);
 
+    const bool any_first = ctx->policy == 2;
     // ---- tensor-core path
     const bool tc_rescale_ok = !epi.has_rescale || (epi.rs.scale32 && epi.rs.rounding != TB200_INEXACT_ROUND &&
                                                     !epi.rs.out_unsigned);
-    if (ctx->policy == 0 && (!int_path || weight_zp == 0) && tc_rescale_ok &&
+    if (ctx->policy == 0 && !any_first && (!int_path || weight_zp == 0) && tc_rescale_ok &&
         (int_path || input->dtype != TB200_FP32))
     {
         TcProblem q;
@@ -1292,6 +1293,131 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                 if (!(st == TB200_INTERNAL && ctx->err.find("rejected") != std::string::npos))
                     return st;
             }
+        }
+    }
+
+    // ---- channel runs that are no multiple of 32 bytes: gathering tensor-core kernel (tc_any.cu)
+    if (ctx->policy != 1 && (!int_path || weight_zp == 0) && tc_rescale_ok && input->dtype != TB200_FP32 && input->stride[3] == 1 && IC > 0)
+    {
+        const int es       = (int)dtype_size(input->dtype);
+        const int run      = IC * es, runp = (run + 15) & ~15;    // a tap's channel run, in memory and in the packed weights
+        const int taps     = KH * KW;
+        const bool repack  = run != runp;
+        const int Kp       = taps * runp / es;
+        const int OCpad    = (OC + 255) / 256 * 256;
+        const size_t wr_bytes  = repack ? ((size_t)OC * taps * runp + 255) & ~(size_t)255 : 0;
+        const size_t prefix_elems = ((size_t)4 * OC + 3) & ~(size_t)3;
+        const size_t rec_off   = ((prefix_elems + 2 * (size_t)OCpad) * sizeof(int32_t) + OCpad + 63) & ~(size_t)63;
+        const size_t flag_off  = rec_off + (size_t)OCpad * 8 * sizeof(int32_t);
+        const size_t tab_bytes = int_path ? flag_off + 64 : (size_t)OCpad * sizeof(float);
+        TcProblem q;
+        memset(&q, 0, sizeof(q));
+        q.in_dtype = input->dtype;
+        q.a        = input->data;
+        q.N = N; q.IH = IH; q.IW = IW; q.IC = IC;
+        q.a_stride_w = input->stride[2]; q.a_stride_h = input->stride[1]; q.a_stride_n = input->stride[0];
+        q.OH = OH; q.OW = OW; q.OC = OC; q.KH = KH; q.KW = KW;
+        q.pad_t = pad[0]; q.pad_l = pad[2]; q.stride_y = stride[0]; q.stride_x = stride[1]; q.dil_y = dilation[0]; q.dil_x = dilation[1];
+        q.b      = weight->data;
+        q.out    = output->data;
+        q.epi    = int_path ? TC_EPI_I32 : TC_EPI_FLOAT;
+        q.a_fill = int_path ? input_zp : 0;
+        fill_tc_epilogue(&q, epi, output->dtype);
+        q.rec = epi.has_rescale ? reinterpret_cast<const int32_t*>(weight->data) : nullptr;    // (layout only needs to know there are records)
+        if (tc_any_supported(ctx, q))
+        {
+            const int8_t* wp   = reinterpret_cast<const int8_t*>(weight->data);
+            const void* bp     = bias->data;
+            const int32_t* mp  = epi.has_rescale ? reinterpret_cast<const int32_t*>(epi.rs.mult) : nullptr;
+            const int8_t* sp   = epi.has_rescale ? epi.rs.shift : nullptr;
+            const int bias_n = bias->shape[0], per_ch = epi.rs.per_channel, has_rs = epi.has_rescale ? 1 : 0;
+            const int dr_i   = epi.has_rescale && epi.rs.rounding == TB200_DOUBLE_ROUND ? 1 : 0;
+            const int32_t ozp_i = epi.has_rescale ? (int32_t)epi.rs.out_zp_ext : 0;
+            const bool b16 = bias->dtype == TB200_FP16;
+            auto build = [=](tb200_ctx* c, void* blk) -> tb200_status {
+                int8_t* wr   = reinterpret_cast<int8_t*>(blk);
+                uint8_t* tab = reinterpret_cast<uint8_t*>(blk) + wr_bytes;
+                if (repack)
+                    repack_weights_smallc_kernel<<<(int)(((int64_t)OC * taps * runp + 255) / 256), 256, 0, c->stream>>>(wp, wr, OC, taps, 1, run, runp, runp);
+                if (int_path)
+                {
+                    // every tap of every pixel is in scope (the gather fills the border): one correction row, as for a
+                    // 1x1 kernel over all of K
+                    int32_t* prefix = reinterpret_cast<int32_t*>(tab);
+                    int32_t* corr   = prefix + prefix_elems;
+                    int32_t* mult_pad = corr + OCpad;
+                    int* all_ok     = reinterpret_cast<int*>(tab + flag_off);
+                    TB200_CUDA_CHECK(c, cudaMemsetAsync(all_ok, has_rs ? 1 : 0, sizeof(int), c->stream));
+                    conv_epilogue_tables_kernel<<<(OCpad * 32 + 127) / 128, 128, 0, c->stream>>>(
+                        repack ? wr : wp, reinterpret_cast<const int32_t*>(bp), bias_n, OC, OCpad, 1, 1, Kp, input_zp, 0, mp, sp, per_ch, prefix, corr,
+                        has_rs ? mult_pad : nullptr, reinterpret_cast<int8_t*>(mult_pad + OCpad),
+                        has_rs ? reinterpret_cast<int32_t*>(tab + rec_off) : nullptr, nullptr, dr_i, ozp_i, all_ok);
+                }
+                else if (b16)
+                    bias_to_f32_kernel<__half><<<(OCpad + 127) / 128, 128, 0, c->stream>>>(reinterpret_cast<const __half*>(bp), bias_n, OC,
+                                                                                       reinterpret_cast<float*>(tab), OCpad);
+                else
+                    bias_to_f32_kernel<__nv_bfloat16><<<(OCpad + 127) / 128, 128, 0, c->stream>>>(
+                        reinterpret_cast<const __nv_bfloat16*>(bp), bias_n, OC, reinterpret_cast<float*>(tab), OCpad);
+                return post_launch(c, "conv_gather_tables", repack ? 2 : 1);
+            };
+            Prepared* e = nullptr;
+            if (use_cache && ctx->const_cache_on)
+            {
+                std::string key;
+                key_add(&key, (int)9);
+                key_add(&key, wp); key_add(&key, bp); key_add(&key, mp); key_add(&key, sp); key_add(&key, (int)input->dtype);
+                key_add(&key, (int)bias->dtype);
+                key_add(&key, OC); key_add(&key, taps); key_add(&key, IC); key_add(&key, bias_n);
+                key_add(&key, input_zp); key_add(&key, per_ch); key_add(&key, has_rs); key_add(&key, dr_i); key_add(&key, ozp_i);
+                e = cache_find(ctx, key);
+                if (!e)
+                {
+                    std::vector<std::pair<const char*, size_t>> ops = {
+                        { reinterpret_cast<const char*>(wp), weight->bytes }, { reinterpret_cast<const char*>(bp), bias->bytes } };
+                    if (has_rs)
+                    {
+                        ops.push_back({ reinterpret_cast<const char*>(mp), epilogue->rescale.multiplier->bytes });
+                        ops.push_back({ reinterpret_cast<const char*>(sp), epilogue->rescale.shift->bytes });
+                    }
+                    e = cache_insert(ctx, key, std::move(ops), wr_bytes + tab_bytes, build);
+                }
+            }
+            void* block = nullptr;
+            if (e)
+            {
+                st = cache_use(ctx, e);
+                if (st == TB200_OK && has_rs)
+                    st = read_host_flag(ctx, e, wr_bytes + flag_off);
+                if (st != TB200_OK)
+                    return st;
+                block     = e->block;
+                q.lean_ok = has_rs && e->host_flag == 1 ? 1 : 0;
+            }
+            else
+            {
+                st = ensure_scratch(ctx, wr_bytes + tab_bytes);
+                if (st == TB200_OK)
+                    st = build(ctx, ctx->scratch);
+                if (st != TB200_OK)
+                    return st;
+                block = ctx->scratch;
+            }
+            uint8_t* tab = reinterpret_cast<uint8_t*>(block) + wr_bytes;
+            if (repack)
+                q.b = block;
+            if (int_path)
+            {
+                int32_t* corr = reinterpret_cast<int32_t*>(tab) + prefix_elems;
+                q.corr        = corr;
+                q.corr_stride = OCpad;
+                q.mult_pad    = corr + OCpad;
+                q.shift_pad   = reinterpret_cast<const int8_t*>(q.mult_pad + OCpad);
+                q.rec         = has_rs ? reinterpret_cast<const int32_t*>(tab + rec_off) : nullptr;
+            }
+            else
+                q.bias_f_pad = reinterpret_cast<const float*>(tab);
+            return tc_any_launch(ctx, q);
         }
     }
 
@@ -2338,8 +2464,9 @@ extern "C" tb200_status tb200_matmul(tb200_ctx* ctx, const tb200_tensor* a, cons
             return sgemm_f32_launch(ctx, reinterpret_cast<const float*>(a->data), reinterpret_cast<const float*>(b->data),
                                     reinterpret_cast<float*>(output->data), N, H, C, W);
     }
-    else if (ctx->policy == 0)
+    else if (ctx->policy != 1)
     {
+        const bool any_first = ctx->policy == 2;
         TcProblem q;
         memset(&q, 0, sizeof(q));
         q.in_dtype    = a->dtype;
@@ -2362,6 +2489,19 @@ extern "C" tb200_status tb200_matmul(tb200_ctx* ctx, const tb200_tensor* a, cons
         const size_t padb_bytes = pad_b ? (((size_t)N * C * b_ld * es_in + 255) & ~(size_t)255) : 0;
         q.b_ld = b_ld;
         std::string why;
+        // (the CTA-pair kernel takes K tails the single-CTA kernel does not)
+        if (!tc_gemm_pair_supported(q, ctx->num_sms) && (any_first || pad_b || !tc_gemm_supported(q, &why)))
+        {
+            TcProblem g = q;
+            g.b_ld = 0;
+            if (int_path)
+            {
+                g.a_zp = a_zp;
+                g.b_zp = b_zp;
+            }
+            if (tc_any_supported(ctx, g))
+                return tc_any_launch(ctx, g);
+        }
         // (the CTA-pair kernel takes K tails the single-CTA kernel does not)
         if (tc_gemm_pair_supported(q, ctx->num_sms) || tc_gemm_supported(q, &why))
         {

@@ -302,6 +302,7 @@ struct TcProblem
     // [batch * tiles_m * 2 + batch * tiles_w * 2] words that persist between launches, sum_epoch at a value no flag holds
     int fuse_row_sums;
     int32_t a_zp, b_zp;
+    int32_t a_fill;    // gathering kernel: what a tap outside the image contributes (the input zero point)
     uint32_t* sum_flags;
     uint32_t sum_epoch;
     // per-column additive constants, padded: [classes][corr_stride]; corr_stride must be a multiple of 256 and cover
@@ -335,6 +336,15 @@ bool tc_gemm_lean_supported(const tb200_ctx* ctx, const TcProblem& p);
 tb200_status tc_gemm_launch(tb200_ctx* ctx, const TcProblem& p);
 // Total tile count of a problem and the tiles per row block (per batch for MATMUL); tiles are numbered batch-major.
 bool tc_gemm_tile_counts(const TcProblem& p, int* num_tiles, int* tiles_per_row_block);
+
+// The driver's cuTensorMapEncodeTiled, or null
+void* tensor_map_encode_fn();
+
+// Gathering kernel (tc_any.cu): any channel run, row length and alignment, and problems with few tiles.  CONV2D weights are
+// [OC][taps][run], run = the channels rounded up to whole 16-byte pieces (zero padded); the corrections of q are those of
+// interior pixels (q.a_fill is what taps outside the image read).
+bool tc_any_supported(const tb200_ctx* ctx, const TcProblem& q);
+tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q);
 
 // int8 MATMUL on CTA pairs (tc_gemm_pair.cu): large MN-major-B problems with int32 output; tc_gemm_launch routes to it
 bool tc_gemm_pair_supported(const TcProblem& p, int num_sms);

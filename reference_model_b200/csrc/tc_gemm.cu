@@ -1553,6 +1553,11 @@ bool make_lean_plan(const TcProblem& q, int num_sms, int max_smem_optin, TcPlan*
 
 }    // namespace
 
+void* tensor_map_encode_fn()
+{
+    return reinterpret_cast<void*>(get_encode_fn());
+}
+
 bool tc_gemm_supported(const TcProblem& p, std::string* why)
 {
     TcPlan plan;
