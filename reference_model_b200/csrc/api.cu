@@ -2320,6 +2320,51 @@ extern "C" tb200_status tb200_depthwise_conv2d(tb200_ctx* ctx, const tb200_tenso
     d.in_zp = input_zp; d.w_zp = weight_zp; d.bias_n = bias->shape[0];
     fill_conv_dev(&d, epi);
     const int block = 256;
+    // int8 with RESCALE to int8: the sliding kernel, for outputs of at least 2^14 values (below, its serial walk along x has
+    // too few threads and the kernels below finish first)
+    if (int_path && M == 1 && ctx->policy == 0 && weight_zp == 0 && KH == KW && stride[0] == stride[1] && dilation[0] == 1 && dilation[1] == 1 &&
+        epi.has_rescale && epi.rs.scale32 && epi.rs.rounding != TB200_INEXACT_ROUND && output->dtype == TB200_INT8 && !epi.rs.out_unsigned &&
+        ctx->const_cache_on && numel(output) >= (1 << 14))
+    {
+        DepthwiseI8Problem q;
+        memset(&q, 0, sizeof(q));
+        q.in = reinterpret_cast<const int8_t*>(input->data); q.w = reinterpret_cast<const int8_t*>(weight->data);
+        q.bias = reinterpret_cast<const int32_t*>(bias->data); q.mult = reinterpret_cast<const int32_t*>(epi.rs.mult);
+        q.shift = epi.rs.shift; q.out = reinterpret_cast<int8_t*>(output->data);
+        q.N = N; q.IH = IH; q.IW = IW; q.C = C; q.OH = OH; q.OW = OW; q.K = KH; q.S = stride[0]; q.pad_t = pad[0]; q.pad_l = pad[2];
+        q.bias_n = bias->shape[0]; q.per_channel = epi.rs.per_channel; q.double_round = epi.rs.rounding == TB200_DOUBLE_ROUND;
+        q.in_zp = input_zp; q.out_zp = (int32_t)epi.rs.out_zp_ext;
+        TcProblem t;
+        memset(&t, 0, sizeof(t));
+        fill_tc_epilogue(&t, epi, output->dtype);    // RESCALE's range and CLAMP as one interval
+        q.clamp_lo = t.clamp_lo; q.clamp_hi = t.clamp_hi;
+        if (depthwise_slide_supported(q))
+        {
+            std::string key;
+            key_add(&key, (int)10);
+            key_add(&key, q.w); key_add(&key, q.bias); key_add(&key, q.mult); key_add(&key, q.shift);
+            key_add(&key, C); key_add(&key, q.K); key_add(&key, q.bias_n); key_add(&key, input_zp); key_add(&key, q.per_channel);
+            key_add(&key, q.double_round); key_add(&key, q.out_zp);
+            Prepared* e = cache_find(ctx, key);
+            if (!e)
+                e = cache_insert(ctx, key,
+                                 { { reinterpret_cast<const char*>(q.w), weight->bytes }, { reinterpret_cast<const char*>(q.bias), bias->bytes },
+                                   { reinterpret_cast<const char*>(q.mult), epilogue->rescale.multiplier->bytes },
+                                   { reinterpret_cast<const char*>(q.shift), epilogue->rescale.shift->bytes } },
+                                 depthwise_slide_pack_bytes(C, q.K),
+                                 [=](tb200_ctx* c, void* block) { return depthwise_slide_pack(c, q, block); });
+            if (e)
+            {
+                st = cache_use(ctx, e);
+                if (st == TB200_OK)
+                    st = read_host_flag(ctx, e, depthwise_slide_flag_offset(C, q.K));
+                if (st != TB200_OK)
+                    return st;
+                if (e->host_flag == 1)
+                    return depthwise_slide_launch(ctx, q, e->block, "depthwise_slide_i8");
+            }
+        }
+    }
     if (int_path && M == 1 && C % 16 == 0 && KH == 3 && KW == 3 && dilation[0] == 1 && dilation[1] == 1 && ctx->policy == 0 &&
         ((reinterpret_cast<uintptr_t>(input->data) | reinterpret_cast<uintptr_t>(weight->data) |
           reinterpret_cast<uintptr_t>(output->data)) & 15) == 0)

@@ -370,6 +370,22 @@ struct ExpandDwProblem
 bool expand_dw_supported(const tb200_ctx* ctx, const ExpandDwProblem& q, std::string* why);
 tb200_status expand_dw_launch(tb200_ctx* ctx, const ExpandDwProblem& q);
 
+// int8 DEPTHWISE_CONV2D + RESCALE to int8, K x K window (3, 5), stride S (1, 2), multiplier 1 (depthwise_i8.cu)
+struct DepthwiseI8Problem
+{
+    const int8_t *in, *w;
+    const int32_t *bias, *mult;
+    const int8_t* shift;
+    int8_t* out;
+    int N, IH, IW, C, OH, OW, K, S, pad_t, pad_l, bias_n, per_channel, double_round;
+    int32_t in_zp, out_zp, clamp_lo, clamp_hi;
+};
+bool depthwise_slide_supported(const DepthwiseI8Problem& q);
+size_t depthwise_slide_pack_bytes(int C, int K);
+size_t depthwise_slide_flag_offset(int C, int K);    // of the word that says whether every channel's record is usable
+tb200_status depthwise_slide_pack(tb200_ctx* ctx, const DepthwiseI8Problem& q, void* block);
+tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q, const void* block, const char* name);
+
 // fp32 SGEMM on CUDA cores (sgemm_f32.cu): out[n] = a[n] x b[n], a [N,H,C], b [N,C,W]
 tb200_status sgemm_f32_launch(tb200_ctx* ctx, const float* a, const float* b, float* out, int N, int H, int C, int W);
 

@@ -1,0 +1,323 @@
+// int8 DEPTHWISE_CONV2D + RESCALE (+ CLAMP) to int8, 3 x 3 and 5 x 5 windows, stride 1 or 2.
+//
+// A depthwise layer multiplies each channel with its own few weights: no contraction for the tensor cores, and with int8
+// operands the integer instructions bound it long before memory does.  What a thread does here is chosen to need few of
+// them.  It owns four neighbouring channels (one 32-bit word per pixel) and walks along x:
+//   * the words of the window's rows at one x are transposed (6 to 8 byte permutes) into one word per channel that holds
+//     that channel's column of the window, and a column serves every output that looks at it: one dp4a per output, channel
+//     and column instead of one multiply-add per tap;
+//   * at stride 1 a 3 x 3 thread makes two output rows: four rows fill the column words, and the second row's weights are
+//     the first's shifted by a byte;
+//   * weights, packed by columns, and the lean RESCALE records (rescale_rec_build) are prepared once per layer and sit in
+//     registers for the whole walk; taps outside the image read the input zero point, so that all pixels share them.
+// Channel counts that are no multiple of four read each word as two aligned ones.
+// 32 x 56 x 56 x 144, 3 x 3: the sixteen-channels-per-thread kernel with the general RESCALE took 126 us.
+#include <algorithm>
+#include <cuda_runtime.h>
+
+#include "common.h"
+#include "rescale_math.cuh"
+
+namespace tb200
+{
+namespace
+{
+
+struct DwSlideParams
+{
+    const int8_t* in;
+    const int8_t* in_end;    // one past the input's last byte
+    int8_t* out;
+    const int4* wcol;        // [K][C4 / 4]: per channel the window column's first four rows, one byte each
+    const int4* wrow5;       // [K][C4 / 4]: 5 x 5 only, the fifth row's weight at the channel's own byte
+    const int4* rec;         // [C4][2]
+    int N, IH, IW, C, OH, OW, pad_t, pad_l;
+    int c4, strips, row_groups, len;    // channel words, pieces of a row, groups of rows, outputs of a piece
+    uint32_t fd_c4[2], fd_strips[2], fd_rg[2];
+    int total;               // threads with work
+    uint32_t fill4;
+    int clamp_lo, clamp_hi;
+};
+
+template <int K, int S, bool ALIGNED, bool FIX>
+__global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_constant__ DwSlideParams p)
+{
+    constexpr int R  = (K == 3 && S == 1) ? 2 : 1;    // output rows per thread
+    constexpr int NR = (R - 1) * S + K;               // input rows they look at
+    const int item = (int)(blockIdx.x * 128 + threadIdx.x);
+    if (item >= p.total)
+        return;
+    const int r1 = (int)fastdiv_apply((uint32_t)item, p.fd_c4), cw = item - r1 * p.c4;
+    const int r2 = (int)fastdiv_apply((uint32_t)r1, p.fd_strips), strip = r1 - r2 * p.strips;
+    const int n  = (int)fastdiv_apply((uint32_t)r2, p.fd_rg), oy = (r2 - n * p.row_groups) * R;
+    const int c  = cw * 4;
+    const int ox0 = strip * p.len, ox1 = min(p.OW, ox0 + p.len);
+
+    int wc[K][4], w5[K == 5 ? K : 1][4];
+#pragma unroll
+    for (int k = 0; k < K; k++)
+    {
+        const int4 t = __ldg(p.wcol + k * p.c4 + cw);
+        wc[k][0] = t.x; wc[k][1] = t.y; wc[k][2] = t.z; wc[k][3] = t.w;
+        if (K == 5)
+        {
+            const int4 u = __ldg(p.wrow5 + k * p.c4 + cw);
+            w5[K == 5 ? k : 0][0] = u.x; w5[K == 5 ? k : 0][1] = u.y; w5[K == 5 ? k : 0][2] = u.z; w5[K == 5 ? k : 0][3] = u.w;
+        }
+    }
+    int4 ra[4];
+    int2 rb[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+    {
+        ra[i] = __ldg(p.rec + (c + i) * 2);
+        rb[i] = __ldg(reinterpret_cast<const int2*>(p.rec + (c + i) * 2 + 1));
+    }
+
+    const int8_t* row[NR];
+    bool row_in[NR];
+#pragma unroll
+    for (int r = 0; r < NR; r++)
+    {
+        const int y = oy * S - p.pad_t + r;
+        row_in[r]   = (unsigned)y < (unsigned)p.IH;
+        row[r]      = p.in + ((int64_t)n * p.IH + (row_in[r] ? y : 0)) * p.IW * p.C + c;
+    }
+    auto fetch = [&](int r, int x) -> uint32_t {
+        if (!row_in[r] || (unsigned)x >= (unsigned)p.IW)
+            return p.fill4;
+        const int8_t* a = row[r] + x * p.C;
+        if (ALIGNED)
+            return *reinterpret_cast<const uint32_t*>(a);
+        const int sh      = (int)(reinterpret_cast<uintptr_t>(a) & 3);
+        const int8_t* lo  = a - sh;
+        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(lo);
+        const uint32_t w1 = sh && lo + 4 < p.in_end ? *reinterpret_cast<const uint32_t*>(lo + 4) : 0u;
+        return __funnelshift_r(w0, w1, 8 * sh);
+    };
+    // column x of the window's rows: t[0..3] one word per channel (rows 0..3), t[4] the fifth row's four channels
+    struct Column
+    {
+        uint32_t t[K == 5 ? 5 : 4];
+    };
+    auto column = [&](int x, Column& q) {
+        uint32_t a[NR];
+#pragma unroll
+        for (int r = 0; r < NR; r++)
+            a[r] = fetch(r, x);
+        const uint32_t lo01 = __byte_perm(a[0], a[1], 0x5140), hi01 = __byte_perm(a[0], a[1], 0x7362);
+        if (NR == 3)
+        {
+            // (the fourth byte meets a zero weight)
+            q.t[0] = __byte_perm(lo01, a[2], 0x4410);
+            q.t[1] = __byte_perm(lo01, a[2], 0x5532);
+            q.t[2] = __byte_perm(hi01, a[2], 0x6610);
+            q.t[3] = __byte_perm(hi01, a[2], 0x7732);
+        }
+        else
+        {
+            const uint32_t a3   = a[NR > 3 ? 3 : 0];
+            const uint32_t lo23 = __byte_perm(a[2], a3, 0x5140), hi23 = __byte_perm(a[2], a3, 0x7362);
+            q.t[0] = __byte_perm(lo01, lo23, 0x5410);
+            q.t[1] = __byte_perm(lo01, lo23, 0x7632);
+            q.t[2] = __byte_perm(hi01, hi23, 0x5410);
+            q.t[3] = __byte_perm(hi01, hi23, 0x7632);
+        }
+        if (K == 5)
+            q.t[K == 5 ? 4 : 0] = a[NR > 4 ? 4 : 0];
+    };
+    const bool narrow  = p.clamp_lo > -128 || p.clamp_hi < 127;
+    const uint32_t lo4 = (uint32_t)(p.clamp_lo & 0xff) * 0x01010101u, hi4 = (uint32_t)(p.clamp_hi & 0xff) * 0x01010101u;
+    int8_t* const o0   = p.out + (((int64_t)n * p.OH + oy) * p.OW) * p.C + c;
+    const bool two     = R == 2 && oy + 1 < p.OH;
+    auto emit = [&](int ox, const int (&acc)[4], int rr) {
+        uint32_t w;
+        int z[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            z[i] = rescale_rec_apply(acc[i], ra[i].x, ra[i].y, ra[i].z, ra[i].w, rb[i].x, rb[i].y, FIX);
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(z[3]), "r"(z[2]), "r"(0));
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(z[1]), "r"(z[0]), "r"(w));
+        if (narrow)
+            w = __vmins4(__vmaxs4(w, lo4), hi4);
+        int8_t* o = o0 + (rr * p.OW + ox) * p.C;
+        if (ALIGNED)
+            *reinterpret_cast<uint32_t*>(o) = w;
+        else
+        {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (c + i < p.C)
+                    o[i] = (int8_t)(w >> (8 * i));
+        }
+    };
+
+    // The last K columns, as a ring whose positions are compile-time constants: the loop over x is unrolled K times.
+    Column q[K];
+    int x = ox0 * S - p.pad_l;
+#pragma unroll
+    for (int k = 0; k < K - S; k++)
+        column(x + k, q[k]);
+    x += K - S;
+    for (int ox = ox0; ox < ox1; ox += K)
+    {
+#pragma unroll
+        for (int u = 0; u < K; u++)
+        {
+            if (ox + u < ox1)
+            {
+                // ring position of window column k at output ox + u: (u S + k) mod K
+#pragma unroll
+                for (int s = 0; s < S; s++)
+                    column(x + u * S + s, q[(u * S + K - S + s) % K]);
+                int acc[4], acc2[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    acc[i] = acc2[i] = 0;
+#pragma unroll
+                for (int k = 0; k < K; k++)
+                {
+                    const Column& w = q[(u * S + k) % K];
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                    {
+                        acc[i] = __dp4a((int)w.t[i], wc[k][i], acc[i]);
+                        if (K == 5)
+                            acc[i] = __dp4a((int)w.t[K == 5 ? 4 : 0], w5[K == 5 ? k : 0][i], acc[i]);
+                        if (R == 2)
+                            acc2[i] = __dp4a((int)w.t[i], wc[k][i] << 8, acc2[i]);
+                    }
+                }
+                emit(ox + u, acc, 0);
+                if (two)
+                    emit(ox + u, acc2, 1);
+            }
+        }
+        x += K * S;
+    }
+}
+
+// Weights [K][K][C] packed by window columns, RESCALE records; one thread per channel (of C rounded up to four).
+__global__ void depthwise_pack_kernel(const int8_t* __restrict__ w, const int32_t* __restrict__ bias, int bias_n, int C, int C4, int K, int32_t in_zp,
+                                      const int32_t* __restrict__ mult, const int8_t* __restrict__ shift, int per_channel, int double_round,
+                                      int32_t out_zp, int32_t* __restrict__ wcol, int32_t* __restrict__ wrow5, int32_t* __restrict__ rec, int* all_ok)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= C4)
+        return;
+    int32_t sum = 0;
+    for (int kx = 0; kx < K; kx++)
+    {
+        uint32_t col = 0, five = 0;
+        for (int ky = 0; ky < K && c < C; ky++)
+        {
+            const int v = w[(ky * K + kx) * C + c];
+            sum += v;
+            if (ky < 4)
+                col |= (uint32_t)(v & 0xff) << (8 * ky);
+            else
+                five = (uint32_t)(v & 0xff) << (8 * (c & 3));
+        }
+        wcol[kx * C4 + c] = (int32_t)col;
+        if (K == 5)
+            wrow5[kx * C4 + c] = (int32_t)five;
+    }
+    int32_t r8[8] = { 0, 0, 0, 0, 0, 0, 0, 1 };
+    if (c < C)
+    {
+        const int32_t b    = bias[bias_n == 1 ? 0 : c];
+        const int64_t vmax = (int64_t)K * K * 255 * 128 + (b < 0 ? -(int64_t)b : (int64_t)b);
+        rescale_rec_build(mult[per_channel ? c : 0], (int32_t)shift[per_channel ? c : 0], double_round, out_zp, b - in_zp * sum, vmax, r8);
+        if (r8[7] == 0)
+            *all_ok = 0;
+    }
+    for (int i = 0; i < 8; i++)
+        rec[c * 8 + i] = r8[i];
+}
+
+size_t pack_words(int C, int K)
+{
+    const size_t C4 = (size_t)((C + 3) & ~3);
+    return C4 * (size_t)(K == 5 ? 2 * K : K) + C4 * 8;
+}
+
+}    // namespace
+
+bool depthwise_slide_supported(const DepthwiseI8Problem& q)
+{
+    // 32-bit item numbers and offsets inside a row; two rows of a window never wrap around an image smaller than it
+    return (q.K == 3 || q.K == 5) && (q.S == 1 || q.S == 2) && (int64_t)q.N * q.OH * q.OW * ((q.C + 3) / 4) < (1LL << 31) &&
+           (int64_t)q.OW * 2 * q.C < (1LL << 31) && (int64_t)q.IW * q.C < (1LL << 31);
+}
+
+size_t depthwise_slide_pack_bytes(int C, int K)
+{
+    return pack_words(C, K) * 4 + 64;
+}
+
+size_t depthwise_slide_flag_offset(int C, int K)
+{
+    return pack_words(C, K) * 4;
+}
+
+tb200_status depthwise_slide_pack(tb200_ctx* ctx, const DepthwiseI8Problem& q, void* block)
+{
+    const int C4  = (q.C + 3) & ~3;
+    int32_t* wcol = reinterpret_cast<int32_t*>(block);
+    int32_t* five = wcol + C4 * q.K;
+    int32_t* rec  = five + (q.K == 5 ? C4 * q.K : 0);
+    int* flag     = reinterpret_cast<int*>(rec + C4 * 8);
+    TB200_CUDA_CHECK(ctx, cudaMemsetAsync(flag, 1, sizeof(int), ctx->stream));
+    depthwise_pack_kernel<<<(C4 + 127) / 128, 128, 0, ctx->stream>>>(q.w, q.bias, q.bias_n, q.C, C4, q.K, q.in_zp, q.mult, q.shift, q.per_channel,
+                                                                    q.double_round, q.out_zp, wcol, five, rec, flag);
+    return post_launch(ctx, "depthwise_pack");
+}
+
+tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q, const void* block, const char* name)
+{
+    const int C4 = (q.C + 3) & ~3;
+    DwSlideParams p;
+    memset(&p, 0, sizeof(p));
+    p.in     = q.in;
+    p.in_end = q.in + (int64_t)q.N * q.IH * q.IW * q.C;
+    p.out    = q.out;
+    p.wcol   = reinterpret_cast<const int4*>(block);
+    p.wrow5  = p.wcol + C4 / 4 * q.K;
+    p.rec    = p.wrow5 + (q.K == 5 ? C4 / 4 * q.K : 0);
+    p.N = q.N; p.IH = q.IH; p.IW = q.IW; p.C = q.C; p.OH = q.OH; p.OW = q.OW; p.pad_t = q.pad_t; p.pad_l = q.pad_l;
+    p.c4         = C4 / 4;
+    const int R  = q.K == 3 && q.S == 1 ? 2 : 1;
+    p.row_groups = (q.OH + R - 1) / R;
+    // A piece's first K - S columns are fetched again by its neighbour: long pieces waste less, short ones make more
+    // threads.  The longest that still gives every SM two blocks of 256 threads' worth of work, at most 28.
+    const int64_t lines = (int64_t)q.N * p.row_groups * p.c4;
+    const int64_t want  = (int64_t)ctx->num_sms * 1024;
+    int strips = (int)std::min<int64_t>(std::max<int64_t>((want + lines - 1) / lines, (q.OW + 27) / 28), std::max(1, q.OW / 2));
+    p.len      = (q.OW + strips - 1) / strips;
+    p.strips   = (q.OW + p.len - 1) / p.len;
+    fastdiv_make((uint32_t)p.c4, p.fd_c4);
+    fastdiv_make((uint32_t)p.strips, p.fd_strips);
+    fastdiv_make((uint32_t)p.row_groups, p.fd_rg);
+    p.total    = (int)(lines * p.strips);
+    p.fill4    = (uint32_t)(q.in_zp & 0xff) * 0x01010101u;
+    p.clamp_lo = q.clamp_lo;
+    p.clamp_hi = q.clamp_hi;
+    const bool al = q.C % 4 == 0 && ((reinterpret_cast<uintptr_t>(q.in) | reinterpret_cast<uintptr_t>(q.out)) & 3) == 0;
+    const int grid = (p.total + 127) / 128;
+#define TB200_DW(KK, SS)                                                                                                     \
+    if (q.K == KK && q.S == SS)                                                                                              \
+    {                                                                                                                        \
+        if (al && q.double_round) depthwise_slide_i8_kernel<KK, SS, true, true><<<grid, 128, 0, ctx->stream>>>(p);           \
+        else if (al) depthwise_slide_i8_kernel<KK, SS, true, false><<<grid, 128, 0, ctx->stream>>>(p);                       \
+        else if (q.double_round) depthwise_slide_i8_kernel<KK, SS, false, true><<<grid, 128, 0, ctx->stream>>>(p);           \
+        else depthwise_slide_i8_kernel<KK, SS, false, false><<<grid, 128, 0, ctx->stream>>>(p);                              \
+    }
+    TB200_DW(3, 1)
+    TB200_DW(3, 2)
+    TB200_DW(5, 1)
+    TB200_DW(5, 2)
+#undef TB200_DW
+    return post_launch(ctx, name);
+}
+
+}    // namespace tb200

@@ -1,0 +1,119 @@
+"""The gathering tensor-core kernel at the edges of its tiles: runs, rows and columns of every alignment, K shorter than a
+chunk and split over a cluster, one row, borders, views, both zero points, every element type, outputs that are no whole
+16-byte rows; integers bit for bit against the oracle, floats under the DOT_PRODUCT rule."""
+import numpy as np
+import pytest
+
+import reference_model_b200 as tb
+from oracle import oracle as orc
+from tests import util
+from tests.test_gpu_parity import _fp8_codes, oracle_conv_i8, run_conv_fp, run_conv_i8
+
+pytestmark = pytest.mark.gpu
+F16, BF16, F32 = tb.DType.FP16, tb.DType.BF16, tb.DType.FP32
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = tb.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 129, 17, 33), (3, 128, 100, 257), (1, 5, 3000, 300), (4, 250, 36, 40), (1, 33, 130, 515)])
+@pytest.mark.parametrize("zp", [(0, 0), (3, 0), (0, -2), (-128, 127)])
+def test_matmul_i8(ctx, shape, zp):
+    N, H, C, W = shape
+    r = util.rng(2000 + H + W)
+    a, b = r.integers(-128, 128, size=(N, H, C)).astype(np.int8), r.integers(-128, 128, size=(N, C, W)).astype(np.int8)
+    ta, tbb, to = ctx.from_numpy(a), ctx.from_numpy(b), ctx.empty(tb.DType.INT32, (N, H, W))
+    ctx.matmul(ta, tbb, to, *zp)
+    assert ctx.last_kernel() == "tc_gemm_any_i8_i32"
+    st, out = to.download()
+    assert st == tb.Status.OK and np.array_equal(out, orc.matmul(a, b, *zp, nthreads=8))
+    for t in (ta, tbb, to):
+        t.free()
+
+
+@pytest.mark.parametrize("name", ["fp16", "bf16", "e4m3"])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (3, 130, 26, 31), (2, 197, 64, 197), (1, 7, 2679, 72), (2, 60, 77, 300)])
+def test_matmul_float(ctx, name, shape):
+    N, H, C, W = shape
+    r = util.rng(2100 + H + W)
+    if name == "e4m3":
+        ca, cb = _fp8_codes(r, (N, H, C), name), _fp8_codes(r, (N, C, W), name)
+        a, b = orc.fp8_to_f32(ca, name), orc.fp8_to_f32(cb, name)
+        ta, tbb, outs = ctx.from_numpy(ca, tb.DType.FP8E4M3), ctx.from_numpy(cb, tb.DType.FP8E4M3), ((F16, "fp16"), (F32, "fp32"))
+    else:
+        a, b = (orc.fptrunc(r.standard_normal(s).astype(np.float32), name) for s in ((N, H, C), (N, C, W)))
+        dt = F16 if name == "fp16" else BF16
+        ta, tbb = (ctx.from_numpy(v.astype(np.float16)) if dt == F16 else ctx.from_numpy(util.to_bf16_bits(v), BF16) for v in (a, b))
+        outs = ((dt, name), (F32, "fp32"))
+    ref, bnd = orc.matmul(a, b, mode="f64"), orc.matmul(np.abs(a), np.abs(b), mode="f64")
+    for dt, oname in outs:
+        to = ctx.empty(dt, (N, H, W))
+        ctx.matmul(ta, tbb, to)
+        assert ctx.last_kernel().startswith("tc_gemm_any"), ctx.last_kernel()
+        st, out = to.download()
+        out = util.from_bf16_bits(out) if dt == BF16 else out.astype(np.float32)
+        ok, info = orc.verify_dot_product(out, ref, bnd, orc.dot_product_ksb(C, "fp32", oname), out=oname)
+        assert st == tb.Status.OK and ok, info
+        to.free()
+    ta.free(), tbb.free()
+
+
+# N, IH, IW, IC, OC, K, stride, pad, in_zp
+CONV = [(1, 32, 32, 8, 16, 1, 1, 0, 5), (2, 13, 11, 24, 40, 3, 1, 1, -128), (1, 9, 10, 13, 7, 3, 1, 1, 3), (3, 7, 7, 20, 300, 1, 1, 0, -128),
+        (1, 15, 15, 50, 33, 5, 2, 2, 9), (1, 3, 3, 200, 65, 3, 1, 1, -128), (2, 5, 130, 12, 31, 3, 1, 1, 0), (1, 4, 4, 500, 24, 3, 1, 1, 7)]
+
+
+@pytest.mark.parametrize("case", CONV)
+def test_conv_i8(ctx, case):
+    N, IH, IW, IC, OC, K, s, p, izp = case
+    r = util.rng(2200 + IC + OC)
+    x, w, b = util.conv_int8_case(r, N, IH, IW, IC, OC, K, K, bias_range=1 << 16)
+    args = ([p] * 4, [s, s], [1, 1], izp, 0)
+    _, exp = oracle_conv_i8(x, w, b, *args)
+    st, out, kernel = run_conv_i8(ctx, x, w, b, *args)
+    assert kernel == "tc_gemm_any_i8_i32" and st == tb.Status.OK and np.array_equal(out, exp), kernel
+    mult, shift = util.rescale_params(r, OC)
+    for rounding, clamp in (("DOUBLE_ROUND", (-128, 127)), ("SINGLE_ROUND", (-90, 100))):
+        resc = (mult, shift, -3, rounding)
+        est, exp = oracle_conv_i8(x, w, b, *args, rescale=resc, clamp=clamp)
+        assert est == orc.VALID
+        for cache in (True, False):    # with proven records and with the general arithmetic
+            st, out, kernel = run_conv_i8(ctx, x, w, b, *args, rescale=resc, clamp=clamp, cache=cache)
+            assert kernel == "tc_gemm_any_i8_rescale" and st == tb.Status.OK and np.array_equal(out, exp), (rounding, cache)
+
+
+@pytest.mark.parametrize("dt,name", [(F16, "fp16"), (BF16, "bf16")])
+@pytest.mark.parametrize("case", [(2, 9, 11, 12, 20, 3, 1), (1, 14, 14, 9, 33, 3, 1), (2, 6, 6, 100, 70, 1, 0), (1, 20, 7, 3, 8, 5, 2)])
+def test_conv_float(ctx, dt, name, case):
+    N, IH, IW, IC, OC, K, p = case
+    r = util.rng(2300 + IC)
+    x, w, b = (orc.fptrunc(r.standard_normal(s).astype(np.float32), name) for s in ((N, IH, IW, IC), (OC, K, K, IC), (OC,)))
+    args = ([p] * 4, [1, 1], [1, 1])
+    ref, bnd = (orc.conv2d(x, w, b, *args, mode="f64", bounds=f) for f in (False, True))
+    st, out, kernel = run_conv_fp(ctx, x, w, b, *args, dt)
+    ok, info = orc.verify_dot_product(out, ref, bnd, orc.dot_product_ksb(K * K * IC + 1, "fp32", name), out=name)
+    assert kernel == "tc_gemm_any_f16" and st == tb.Status.OK and ok, (kernel, info)
+
+
+def test_bounded_waits_give_up(ctx):
+    """A wait limit far below the time the first copies take: the kernel reports, frees what it holds, and the same call is
+    exact afterwards (a call that finishes in time is fine as well)."""
+    r = util.rng(2400)
+    a, b = r.integers(-128, 128, size=(4, 300, 1001)).astype(np.int8), r.integers(-128, 128, size=(4, 1001, 300)).astype(np.int8)
+    ta, tbb, to = ctx.from_numpy(a), ctx.from_numpy(b), ctx.empty(tb.DType.INT32, (4, 300, 300))
+    exp = orc.matmul(a, b, 3, -2, nthreads=8)
+    ctx.set_wait_limit(200)
+    try:
+        ctx.matmul(ta, tbb, to, 3, -2)
+        assert ctx.last_kernel() == "tc_gemm_any_i8_i32"
+        st = ctx.sync(check=False)
+        assert st in (tb.Status.INTERNAL, tb.Status.OK)
+    finally:
+        ctx.set_wait_limit(4000000000)
+    ctx.matmul(ta, tbb, to, 3, -2)
+    st, out = to.download()
+    assert st == tb.Status.OK and np.array_equal(out, exp)
