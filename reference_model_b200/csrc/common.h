@@ -406,5 +406,10 @@ struct ConvF32Problem
 int conv_f32_ldb(int OC);
 tb200_status conv_f32_weights_launch(tb200_ctx* ctx, const float* w, float* wt, int OC, int K, int* all_finite);
 tb200_status conv_f32_launch(tb200_ctx* ctx, const ConvF32Problem& q);
+// The same two on the tensor cores, operands taken apart into three bf16 parts (sgemm_split.cu); the launches above choose.
+// Estimated SM cycles, 0 where that kernel does not serve.
+double sgemm_split_cost(const tb200_ctx* ctx, int64_t batches, int64_t M, int64_t N, int64_t K, bool conv);
+tb200_status sgemm_split_launch(tb200_ctx* ctx, const float* a, const float* b, float* out, int N, int H, int C, int W);
+tb200_status conv_f32_split_launch(tb200_ctx* ctx, const ConvF32Problem& q);
 
 }    // namespace tb200

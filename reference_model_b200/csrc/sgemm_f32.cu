@@ -1,4 +1,5 @@
-// fp32 batched MATMUL and CONV2D on CUDA cores: FFMA only, no TF32, so every product and sum is an IEEE fp32 operation
+// fp32 batched MATMUL and CONV2D on CUDA cores (deep and large ones go to sgemm_split.cu where that is estimated to be
+// faster): FFMA only, no TF32, so every product and sum is an IEEE fp32 operation
 // and the result stays inside the reference's dot-product error bound.
 //
 // One tiled kernel for both.  A block owns a BM x BN tile of the output and walks K sixteen elements at a time through a
@@ -362,8 +363,13 @@ tb200_status launch_config(tb200_ctx* ctx, const SgemmParams& p, int splits, int
 
 // Tile size and split of K: the pair with the smallest estimated time, which is the larger of the multiply-adds of the
 // fullest SM and the serial chain of K steps of one CTA, plus what starting a CTA (and meeting the cluster) costs.
-template <bool CONV, bool VEC>
-tb200_status launch_any(tb200_ctx* ctx, SgemmParams p, int batches)
+struct SgemmPlan
+{
+    int config, splits;
+    double cost;    // SM cycles
+};
+
+SgemmPlan choose(const tb200_ctx* ctx, const SgemmParams& p, int batches)
 {
     int best = 0, best_split = 1;
     double best_cost = 0;
@@ -388,14 +394,21 @@ tb200_status launch_any(tb200_ctx* ctx, SgemmParams p, int batches)
             }
         }
     }
-    const SgemmConfig& c = kConfigs[best];
+    return { best, best_split, best_cost };
+}
+
+template <bool CONV, bool VEC>
+tb200_status launch_any(tb200_ctx* ctx, SgemmParams p, int batches, const SgemmPlan& plan)
+{
+    const SgemmConfig& c = kConfigs[plan.config];
+    const int best_split = plan.splits, steps = std::max(1, (p.K + BK - 1) / BK);
     p.tiles_m = (p.M + c.bm - 1) / c.bm;
     p.tiles_n = (p.N + c.bn - 1) / c.bn;
     p.k_per_split = (steps + best_split - 1) / best_split * BK;
     const int64_t tiles = (int64_t)batches * p.tiles_m * p.tiles_n;
     if (tiles * best_split >= (1LL << 31))
         return fail(ctx, TB200_ERROR, "fp32 product with too many tiles");
-    switch (best)
+    switch (plan.config)
     {
         case 0: return launch_config<0, CONV, VEC>(ctx, p, best_split, tiles);
         case 1: return launch_config<1, CONV, VEC>(ctx, p, best_split, tiles);
@@ -439,8 +452,12 @@ tb200_status sgemm_f32_launch(tb200_ctx* ctx, const float* a, const float* b, fl
     p.a = a; p.b = b; p.out = out;
     p.M = H; p.N = W; p.K = C; p.ldb = W;
     p.a_batch = (int64_t)H * C; p.b_batch = (int64_t)C * W; p.o_batch = (int64_t)H * W;
+    const SgemmPlan plan = choose(ctx, p, N);
+    const double split   = sgemm_split_cost(ctx, N, H, W, C, false);
+    if (split > 0 && split < plan.cost)
+        return sgemm_split_launch(ctx, a, b, out, N, H, C, W);
     const bool vec = (W % 4) == 0 && (C % 4) == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
-    const tb200_status st = vec ? launch_any<false, true>(ctx, p, N) : launch_any<false, false>(ctx, p, N);
+    const tb200_status st = vec ? launch_any<false, true>(ctx, p, N, plan) : launch_any<false, false>(ctx, p, N, plan);
     return st != TB200_OK ? st : post_launch(ctx, "sgemm_f32");
 }
 
@@ -468,8 +485,12 @@ tb200_status conv_f32_launch(tb200_ctx* ctx, const ConvF32Problem& q)
     p.in_sn = (int)q.in_sn; p.in_sh = (int)q.in_sh; p.in_sw = (int)q.in_sw;
     p.bias = q.bias; p.bias_n = q.bias_n;
     p.has_clamp = q.has_clamp; p.clamp_lo = q.clamp_lo; p.clamp_hi = q.clamp_hi;
+    const SgemmPlan plan = choose(ctx, p, 1);
+    const double split   = sgemm_split_cost(ctx, 1, p.M, p.N, p.K, true);
+    if (split > 0 && split < plan.cost)
+        return conv_f32_split_launch(ctx, q);
     const bool vec = (q.IC % 4) == 0 && ((q.in_sn | q.in_sh | q.in_sw) & 3) == 0 && (reinterpret_cast<uintptr_t>(q.in) & 15) == 0;
-    const tb200_status st = vec ? launch_any<true, true>(ctx, p, 1) : launch_any<true, false>(ctx, p, 1);
+    const tb200_status st = vec ? launch_any<true, true>(ctx, p, 1, plan) : launch_any<true, false>(ctx, p, 1, plan);
     return st != TB200_OK ? st : post_launch(ctx, "conv_f32");
 }
 

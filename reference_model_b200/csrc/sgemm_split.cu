@@ -1,0 +1,687 @@
+// fp32 batched MATMUL and CONV2D on the tensor cores without giving up fp32: every operand is taken apart into three bf16
+// values whose sum is the operand, exactly (24 significant bits = 8 + 8 + 8, cut off, not rounded), and a product is the six
+// partial products that matter (a0 b0, a0 b1, a1 b0, a0 b2, a1 b1, a2 b0; the three left out come to less than 2^-23 of
+// it, 2^-25 on average).  bf16 has fp32's exponent range, so nothing has to be scaled.
+//
+// Sums.  The tensor core cuts its running sum off instead of rounding it, so it never carries one far: a stage of 64 K
+// elements starts from zero, adds the five small partial products first (their cut-off is 2^-8 of the result's) and then
+// the four K steps of a0 b0; the stage's sum is read back and added to fp32 accumulators in registers, rounded to nearest.
+// Error against 64 bits, relative 2-norm, normal operands, K = 256 / 1024 / 4096: 1.3e-7 / 1.5e-7 / 1.9e-7; multiply-adds
+// in K order: 2.9e-7 / 5.7e-7 / 1.15e-6.  (Positive operands: 1.2e-7 / 1.3e-7 / 1.6e-7 against 2.2e-7 / 4.3e-7 / 8.4e-7.)
+//
+// One persistent CTA per SM, 128 x 128 output tiles, sixteen warps:
+//   warps 0-7   add up stages (32 rows x 64 columns each, 64 accumulators per thread), finish and store the tile; the first
+//               issues the MMAs, 24 of 128 x 128 x 16 per stage;
+//   warps 8-15  load fp32 operands straight into registers (64 K elements ahead), take them apart and store three planes in
+//               the tensor core's swizzled layouts.  A warp's unit is 64 elements, two neighbours per lane, so that one code
+//               path serves any alignment, a gathered convolution window and both operands without bank conflicts.
+// Taking operands apart inside the kernel instead of in a pass before it keeps the planes out of memory (3.2 GB for 64
+// products of 1024 x 4096 x 1024).  32 x 1024 x 4096 x 1024: 1.74 ms, 158 TFLOP/s of fp32 (FFMA kernel 57.6), 3 700 SM cycles
+// per stage.  What bounds it: the MMAs alone take 2 680 (24 of ~107 and the hand-over), taking apart and storing 1 600, the
+// loads 3 300 on their own: 64 KB a stage through the ~28 KB of L1 that two 96 KB stages leave.  Three stages of 32 K
+// elements with more L1 lose more to commits and hand-overs (4 500).
+//
+// Values the split cannot carry are computed again with ordinary multiply-adds, 32 rows x 16 columns at a time: results
+// that are not finite (an infinite operand has no split: its lower parts are NaN, so it always shows) and rows or columns so
+// small that lower parts or products would leave the normal range (largest magnitude of the row or column below 2^-100, or
+// of both together below 2^-60).
+#include <algorithm>
+#include <cuda_runtime.h>
+
+#include "common.h"
+#include "ptx_sm100.cuh"
+
+namespace tb200
+{
+namespace
+{
+
+constexpr int kTile = 128, kHalfK = 32, kStageK = 2 * kHalfK, kStages = 2, kAccs = 4;
+constexpr int kPlane = kTile * kHalfK * 2;       // bytes of one bf16 plane of 32 K elements of an operand
+constexpr int kHalfBytes = 6 * kPlane, kStageBytes = 2 * kHalfBytes;    // A planes, B planes of 32 K elements, twice
+constexpr int kFlushWarps = 8, kSplitWarps = 8;
+constexpr int kSplitThreads = 32 * (kFlushWarps + kSplitWarps);
+constexpr int kStagePitch = 17;                   // staged output: 32 rows x 16 columns per warp
+constexpr int kOutOff  = kStages * kStageBytes;
+constexpr int kRowsOff = kOutOff + kFlushWarps * 32 * kStagePitch * 4;    // int2[128]: window origins of a convolution's rows
+constexpr int kMagOff  = kRowsOff + kTile * 8;    // largest magnitudes, for even and odd tiles: rows, column pairs of each warp
+constexpr int kMagWords = kTile + kSplitWarps * (kTile / 2);
+constexpr int kSplitSmem = kMagOff + 2 * kMagWords * 4 + 1024;
+
+struct SplitParams
+{
+    const float* a;
+    const float* b;
+    float* out;
+    int M, N, K;
+    int64_t a_batch, b_batch, o_batch;
+    int ldb;
+    int tiles_m, tiles_n, tiles, nk;
+    int IH, IW, IC, OH, OW, KW, pad_t, pad_l, sy, sx, dy, dx;
+    int in_sn, in_sh, in_sw;
+    const float* bias;
+    int bias_n;
+    int has_clamp;
+    float clamp_lo, clamp_hi;
+    uint32_t idesc;
+    uint64_t a_desc_hi, b_desc_hi;
+    long long wait_limit;
+    int* status;
+};
+
+// origin of an output row's window: element offset, iy0 | ix0
+__device__ __forceinline__ int2 window_of(const SplitParams& p, int m)
+{
+    const int ox = m % p.OW, q = m / p.OW;
+    const int oy = q % p.OH, n = q / p.OH;
+    const int iy0 = oy * p.sy - p.pad_t, ix0 = ox * p.sx - p.pad_l;
+    return make_int2(n * p.in_sn + iy0 * p.in_sh + ix0 * p.in_sw, (int)(((uint32_t)iy0 << 16) | ((uint32_t)ix0 & 0xffffu)));
+}
+
+__device__ __forceinline__ bool window_has(const SplitParams& p, int2 r, int y, int x)
+{
+    return (unsigned)((r.y >> 16) + y) < (unsigned)p.IH && (unsigned)((int)(short)r.y + x) < (unsigned)p.IW;
+}
+
+// Loads with a predicate and no branch around them: a branch makes the compiler wait for each load where the paths join.
+__device__ __forceinline__ float2 load2_if(const float* src, bool inside)
+{
+    float2 v;
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %3, 0;\nmov.b32 %0, 0;\nmov.b32 %1, 0;\n@p ld.global.nc.v2.f32 {%0, %1}, [%2];\n}\n"
+                 : "=&f"(v.x), "=&f"(v.y)
+                 : "l"(src), "r"((int)inside));
+    return v;
+}
+
+__device__ __forceinline__ float load1_if(const float* src, bool inside)
+{
+    float v;
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %2, 0;\nmov.b32 %0, 0;\n@p ld.global.nc.f32 %0, [%1];\n}\n"
+                 : "=&f"(v)
+                 : "l"(src), "r"((int)inside));
+    return v;
+}
+
+// Two fp32 values as three packed bf16 pairs.
+__device__ __forceinline__ void split3(float2 v, uint32_t (&w)[3])
+{
+    const uint32_t x = __float_as_uint(v.x), y = __float_as_uint(v.y);
+    w[0] = __byte_perm(x, y, 0x7632);
+    const float rx = v.x - __uint_as_float(x & 0xffff0000u), ry = v.y - __uint_as_float(y & 0xffff0000u);
+    const uint32_t x1 = __float_as_uint(rx), y1 = __float_as_uint(ry);
+    w[1] = __byte_perm(x1, y1, 0x7632);
+    const float sx = rx - __uint_as_float(x1 & 0xffff0000u), sy = ry - __uint_as_float(y1 & 0xffff0000u);
+    w[2] = __byte_perm(__float_as_uint(sx), __float_as_uint(sy), 0x7632);
+}
+
+// Sixteen columns of one row with ordinary multiply-adds, K in order.
+template <bool CONV>
+__device__ __noinline__ void plain_row(const SplitParams& p, int batch, int m, int n, float* sum)
+{
+    const float* const A = p.a + batch * p.a_batch;
+    const float* const B = p.b + batch * p.b_batch;
+    for (int j = 0; j < 16; j++)
+        sum[j] = 0.f;
+    if (m >= p.M)
+        return;
+    const int2 r = CONV ? window_of(p, m) : make_int2(0, 0);
+    int ic = 0, ky = 0, kx = 0;
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+        v[j] = 0.f;
+    for (int k = 0; k < p.K; k++)
+    {
+        float x;
+        if (CONV)
+        {
+            const int y = ky * p.dy, xx = kx * p.dx;
+            x = window_has(p, r, y, xx) ? A[r.x + y * p.in_sh + xx * p.in_sw + ic] : 0.f;
+            if (++ic == p.IC)
+            {
+                ic = 0;
+                if (++kx == p.KW)
+                {
+                    kx = 0;
+                    ky++;
+                }
+            }
+        }
+        else
+            x = A[(int64_t)m * p.K + k];
+        const float* b = B + (int64_t)k * p.ldb + n;
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+            if (n + j < p.N)
+                v[j] = fmaf(x, b[j], v[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+        sum[j] = v[j];
+}
+
+// AVEC, BVEC: pairs of neighbouring elements of A along K (CONV: along the channels), of B along its rows, are aligned to
+// eight bytes and never straddle an edge.
+template <bool CONV, bool AVEC, bool BVEC>
+__global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __grid_constant__ SplitParams p)
+{
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bar_full[kStages], bar_acc[kAccs], bar_free[kAccs], bar_done;
+    __shared__ uint32_t tmem_base_holder;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* const sm   = smem_raw + (base - ptx::smem_u32(smem_raw));
+    int2* const rows    = reinterpret_cast<int2*>(sm + kRowsOff);
+    uint32_t* const mags = reinterpret_cast<uint32_t*>(sm + kMagOff);
+
+    if (tid == 0)
+    {
+        for (int s = 0; s < kStages; s++)
+            ptx::mbar_init(ptx::smem_u32(&bar_full[s]), kSplitWarps);
+        for (int s = 0; s < kAccs; s++)
+        {
+            ptx::mbar_init(ptx::smem_u32(&bar_acc[s]), 1);
+            ptx::mbar_init(ptx::smem_u32(&bar_free[s]), kFlushWarps);
+        }
+        ptx::mbar_init(ptx::smem_u32(&bar_done), 1);
+        ptx::fence_barrier_init();
+    }
+    if (warp == kFlushWarps)
+    {
+        ptx::tmem_alloc(ptx::smem_u32(&tmem_base_holder), kAccs * kTile);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    ptx::tc_fence_after_sync();
+    const uint32_t tmem = tmem_base_holder;
+    if (tid == 0)
+        ptx::dep_launch_trigger();
+
+    bool ok = true;
+    const int per = p.tiles_m * p.tiles_n;
+    const int mine  = p.tiles > (int)blockIdx.x ? (p.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int total = mine * p.nk;
+    if (warp < kFlushWarps)
+    {
+        // ------------------------------------------------------------------ sums
+        ptx::dep_launch_wait();    // the predecessor may still read what is written here
+        const int quarter = warp & 3, half = warp >> 2;
+        const int row     = quarter * 32 + lane;
+        const uint32_t t0 = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 64);
+        float* const st   = reinterpret_cast<float*>(sm + kOutOff) + warp * 32 * kStagePitch;
+        const bool v8 = (p.N & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
+        // The stage's MMAs, by the first lane of the first of these warps: issuing takes as long as the MMAs before take to make
+        // room in the unit's short queue, so a splitting warp must not do it (the two then take turns: 5 600 cycles a stage), and a warp of its own, the seventeenth, would leave 96 registers per thread instead of 128.
+        // These warps have time: a stage's sums take a fifth of its MMAs.
+        auto issue = [&](int c) {
+            const int buf = c % kAccs, slot = c % kStages;
+            if (!ptx::mbar_wait_bounded(ptx::smem_u32(&bar_free[buf]), ((uint32_t)(c / kAccs) & 1u) ^ 1u, p.wait_limit) ||
+                !ptx::mbar_wait_bounded(ptx::smem_u32(&bar_full[slot]), (uint32_t)(c / kStages) & 1u, p.wait_limit))
+                return false;
+            ptx::tc_fence_after_sync();
+            const uint32_t s = base + (uint32_t)(slot * kStageBytes);
+            uint32_t accum   = 0;
+            // smallest first: a0 b2, a1 b1, a2 b0, a0 b1, a1 b0, a0 b0
+            constexpr int pa[6] = { 0, 1, 2, 0, 1, 0 }, pb[6] = { 2, 1, 0, 1, 0, 0 };
+#pragma unroll
+            for (int q = 0; q < 6; q++)
+            {
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                {
+                    uint64_t ad = ptx::smem_desc(p.a_desc_hi, s + (uint32_t)(h * kHalfBytes + pa[q] * kPlane));
+                    uint64_t bd = ptx::smem_desc(p.b_desc_hi, s + (uint32_t)(h * kHalfBytes + (3 + pb[q]) * kPlane));
+#pragma unroll
+                    for (int kk = 0; kk < kHalfK / 16; kk++, ad += 2, bd += 128)    // 32 bytes along a row; sixteen K rows
+                    {
+                        ptx::mma_f16_ss(tmem + (uint32_t)(buf * kTile), ad, bd, p.idesc, accum);
+                        accum = 1;
+                    }
+                }
+            }
+            ptx::mma_commit(ptx::smem_u32(&bar_acc[buf]));
+            return true;
+        };
+        if (warp == 0)
+        {
+            if (lane == 0 && total > 0)
+                ok = issue(0);
+            ok = __all_sync(0xffffffffu, ok);
+        }
+        int c = 0;
+        for (int i = 0, tile = (int)blockIdx.x; tile < p.tiles && ok; i++, tile += (int)gridDim.x)
+        {
+            const int batch = tile / per, rem = tile - batch * per, tm = rem / p.tiles_n;
+            const int m0 = tm * kTile, n0 = (rem - tm * p.tiles_n) * kTile + half * 64;
+            float acc[64];
+#pragma unroll
+            for (int j = 0; j < 64; j++)
+                acc[j] = 0.f;
+            for (int k = 0; k < p.nk; k++, c++)
+            {
+                const int buf = c % kAccs;
+                if (warp == 0)
+                {
+                    if (lane == 0 && c + 1 < total)
+                        ok = ok && issue(c + 1);
+                    __syncwarp();
+                }
+                ok = ok && ptx::mbar_wait_bounded(ptx::smem_u32(&bar_acc[buf]), (uint32_t)(c / kAccs) & 1u, p.wait_limit);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok)
+                    break;
+                ptx::tc_fence_after_sync();
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                {
+                    uint32_t v[32];
+                    ptx::tmem_ld_32x32b_x32(t0 + (uint32_t)(buf * kTile + h * 32), v);
+                    ptx::tmem_ld_wait();
+                    if (h == 1)
+                    {
+                        ptx::tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0)
+                            ptx::mbar_arrive(ptx::smem_u32(&bar_free[buf]));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        acc[h * 32 + j] += __uint_as_float(v[j]);
+                }
+            }
+            if (!ok)
+                break;
+            // Magnitudes of this row and of this warp's columns (high halves of fp32 values).  The splitting warps come back to
+            // this half of the table two tiles, at least eight stages, later; they are never more than six stages ahead
+            // (two in shared memory, four in tensor memory).
+            const uint32_t* const mg = mags + (i & 1) * kMagWords;
+            uint32_t pair0 = 0, pair1 = 0;
+#pragma unroll
+            for (int q = 0; q < kSplitWarps; q++)
+            {
+                pair0 = __vmaxu2(pair0, mg[kTile + q * (kTile / 2) + half * 32 + (lane >> 1)]);
+                pair1 = __vmaxu2(pair1, mg[kTile + q * (kTile / 2) + half * 32 + 16 + (lane >> 1)]);
+            }
+            const float rmag  = __uint_as_float(mg[row] << 16);
+            const float cmag0 = __uint_as_float(lane & 1 ? pair0 & 0xffff0000u : pair0 << 16);    // column lane
+            const float cmag1 = __uint_as_float(lane & 1 ? pair1 & 0xffff0000u : pair1 << 16);    // column 32 + lane
+            const int m       = m0 + row;
+            const float tiny  = 7.888609e-31f, tiny2 = 8.673617e-19f;    // 2^-100, 2^-60
+#pragma unroll
+            for (int g = 0; g < 4; g++)
+            {
+                float* const y = acc + g * 16;
+                const int n    = n0 + g * 16;
+                if (n >= p.N)
+                    break;
+                uint32_t flag = 0;
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                {
+                    const float cm = __shfl_sync(0xffffffffu, g < 2 ? cmag0 : cmag1, (g & 1) * 16 + j);
+                    const bool odd = !isfinite(y[j]) || (rmag != 0.f && cm != 0.f && (rmag < tiny || cm < tiny || rmag * cm < tiny2));
+                    flag |= odd ? 1u << j : 0u;
+                }
+                if (__any_sync(0xffffffffu, flag != 0))
+                {
+                    float v[16];
+                    plain_row<CONV>(p, batch, m, n, v);
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        y[j] = flag >> j & 1 ? v[j] : y[j];
+                    __syncwarp();
+                }
+                if (CONV)
+                {
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                    {
+                        y[j] = (p.bias_n == 1 ? __ldg(p.bias) : n + j < p.N ? __ldg(p.bias + n + j) : 0.f) + y[j];
+                        if (p.has_clamp)
+                        {
+                            y[j] = (y[j] < p.clamp_lo) ? p.clamp_lo : y[j];
+                            y[j] = (y[j] > p.clamp_hi) ? p.clamp_hi : y[j];
+                        }
+                    }
+                }
+                float* const o = p.out + batch * p.o_batch + (int64_t)m * p.N + n;
+                if (v8)
+                {
+                    if (m < p.M)
+                    {
+#pragma unroll
+                        for (int j = 0; j < 16; j += 8)
+                            if (n + j < p.N)
+                                ptx::st_global_v8(o + j, __float_as_uint(y[j]), __float_as_uint(y[j + 1]), __float_as_uint(y[j + 2]),
+                                                  __float_as_uint(y[j + 3]), __float_as_uint(y[j + 4]), __float_as_uint(y[j + 5]),
+                                                  __float_as_uint(y[j + 6]), __float_as_uint(y[j + 7]));
+                    }
+                }
+                else
+                {
+                    // rows of any alignment: through shared memory, half a warp per row and store
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        st[lane * kStagePitch + j] = y[j];
+                    __syncwarp();
+                    const int col = lane & 15;
+                    float* const og = p.out + batch * p.o_batch + (int64_t)(m0 + quarter * 32) * p.N + n;
+#pragma unroll 4
+                    for (int r = lane >> 4; r < 32; r += 2)
+                        if (m0 + quarter * 32 + r < p.M && n + col < p.N)
+                            og[(int64_t)r * p.N + col] = st[r * kStagePitch + col];
+                    __syncwarp();
+                }
+            }
+        }
+        if (warp == 0 && lane == 0)
+        {
+            ptx::mma_commit(ptx::smem_u32(&bar_done));
+            ptx::mbar_wait_bounded(ptx::smem_u32(&bar_done), 0u, 40000000LL);    // (nothing to wait for unless a role gave up)
+        }
+        __syncwarp();
+    }
+    else
+    {
+        // ------------------------------------------------------------------ load, take apart, store
+        // A warp's unit is 64 elements: two neighbouring rows x 32 K elements of A (64-byte swizzle), 64 columns of one K row of
+        // B (128-byte swizzle).  Eight units of each per stage, w, w + 8, ...: their places in the swizzle are the same.
+        const int w = warp - kFlushWarps;
+        const int kl = 2 * (lane & 15), odd = lane >> 4;    // this lane's K elements of a unit of A, and which row
+        const uint32_t dst_a = base + (uint32_t)(w * 128 + odd * 64 + ((((lane >> 2) & 3) ^ (w & 3)) << 4) + (lane & 3) * 4);
+        const uint32_t dst_b = base + (uint32_t)(3 * kPlane + w * 128 + (((lane >> 2) ^ w) << 4) + (lane & 3) * 4);
+        ptx::dep_launch_wait();
+        // The loads run two stages ahead of the stage being taken apart, across tiles; past the last tile they load nothing.
+        int tile = (int)blockIdx.x, kstage = 0;
+        const float* A = p.a;    // MATMUL: this lane's elements of its first row; CONV2D: the input
+        const float* B = p.b;    // this lane's elements of K row w
+        int nrows = 0;           // MATMUL: rows of the tile from this lane's first one on
+        int ncols = 0;           // columns of the tile
+        int kleft = 0;           // K elements from the stage's first to the end
+        int ic[2] = {}, ky[2] = {}, kx[2] = {};                // CONV: channels and taps of this lane's elements (one tap for both if AVEC)
+        auto next_tap = [&](int q, int step) {
+            ic[q] += step;
+            while (ic[q] >= p.IC)
+            {
+                ic[q] -= p.IC;
+                if (++kx[q] == p.KW)
+                {
+                    kx[q] = 0;
+                    ky[q]++;
+                }
+            }
+        };
+        auto start_tile = [&]() {
+            kstage = 0;
+            kleft  = tile < p.tiles ? p.K : 0;
+            if (tile >= p.tiles)
+                return;
+            const int batch = tile / per, rem = tile - batch * per, tm = rem / p.tiles_n;
+            const int m0 = tm * kTile, n0 = (rem - tm * p.tiles_n) * kTile;
+            A     = p.a + batch * p.a_batch;
+            B     = p.b + batch * p.b_batch + (int64_t)w * p.ldb + n0 + 2 * lane;
+            ncols = (BVEC ? p.ldb : p.N) - n0;    // (BVEC: the same, or zeros up to an even count)
+            if (CONV)
+            {
+                __syncwarp();
+                if (lane < 16)    // (a warp reads its own rows only)
+                {
+                    const int r = 2 * (w + 8 * (lane >> 1)) + (lane & 1);
+                    rows[r]     = m0 + r < p.M ? window_of(p, m0 + r) : make_int2(0, (int)0x80008000);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                {
+                    ic[q] = ky[q] = kx[q] = 0;
+                    next_tap(q, kl + q);
+                }
+            }
+            else
+            {
+                nrows = p.M - m0 - (2 * w + odd);
+                A += (int64_t)(m0 + 2 * w + odd) * p.K + kl;
+            }
+        };
+        auto load_a = [&](float2 (&v)[8]) {
+            if (CONV)
+            {
+                int off[2], y[2], x[2];
+#pragma unroll
+                for (int q = 0; q < (AVEC ? 1 : 2); q++)
+                {
+                    y[q]   = ky[q] * p.dy;
+                    x[q]   = kx[q] * p.dx;
+                    off[q] = y[q] * p.in_sh + x[q] * p.in_sw + ic[q];
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                {
+                    const int2 o = rows[2 * (w + 8 * i) + odd];
+                    if (AVEC)
+                        v[i] = load2_if(A + (o.x + off[0]), kl < kleft && window_has(p, o, y[0], x[0]));
+                    else
+                        v[i] = make_float2(load1_if(A + (o.x + off[0]), kl < kleft && window_has(p, o, y[0], x[0])),
+                                           load1_if(A + (o.x + off[1]), kl + 1 < kleft && window_has(p, o, y[1], x[1])));
+                }
+            }
+            else
+            {
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                {
+                    const float* s = A + (int64_t)(16 * i) * p.K;
+                    const bool row = 16 * i < nrows;
+                    if (AVEC)
+                        v[i] = load2_if(s, row && kl < kleft);
+                    else
+                        v[i] = make_float2(load1_if(s, row && kl < kleft), load1_if(s + 1, row && kl + 1 < kleft));
+                }
+            }
+        };
+        auto load_b = [&](float2 (&v)[8]) {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+            {
+                const int n    = 2 * lane + (i & 1) * 64;
+                const float* s = B + (int64_t)(8 * (i >> 1)) * p.ldb + (i & 1) * 64;
+                const bool k   = w + 8 * (i >> 1) < kleft;
+                if (BVEC)
+                    v[i] = load2_if(s, k && n < ncols);
+                else
+                    v[i] = make_float2(load1_if(s, k && n < ncols), load1_if(s + 1, k && n + 1 < ncols));
+            }
+        };
+        auto next_half = [&]() {
+            kleft -= kHalfK;
+            if (++kstage == 2 * p.nk)
+            {
+                tile += (int)gridDim.x;
+                start_tile();
+                return;
+            }
+            B += (int64_t)kHalfK * p.ldb;
+            if (CONV)
+            {
+#pragma unroll
+                for (int q = 0; q < (AVEC ? 1 : 2); q++)
+                    next_tap(q, kHalfK);
+            }
+            else
+                A += kHalfK;
+        };
+        uint32_t mag_a[8], mag_b[2];    // high halves of the magnitudes, two per word
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            mag_a[i] = 0;
+        mag_b[0] = mag_b[1] = 0;
+        auto put = [&](float2 v, uint32_t dst, uint32_t& mag) {
+            uint32_t x[3];
+            split3(v, x);
+            mag = __vmaxu2(mag, x[0] & 0x7fff7fffu);
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (uint32_t)(q * kPlane)), "r"(x[q]) : "memory");
+        };
+        int left = p.nk, t = 0;    // stages left of the tile being taken apart, and which of this CTA's tiles it is
+        // One stage: loads of the stage two ahead follow the use of their registers, eight at a time (interleaved with their
+        // uses one by one, loads share the few scoreboards with later ones and every use waits for nearly all of them).
+        auto half = [&](float2 (&va)[8], float2 (&vb)[8], uint32_t s) {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                put(va[i], dst_a + s + (uint32_t)(i * 1024), mag_a[i]);
+            load_a(va);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                put(vb[i], dst_b + s + (uint32_t)((i & 1) * (kPlane / 2) + (i >> 1) * 1024), mag_b[i & 1]);
+            load_b(vb);
+            next_half();
+        };
+        float2 a0[8], b0[8], a1[8], b1[8];
+        auto stage = [&](int c) {
+            // the MMAs that read this stage's planes before
+            if (c >= kStages)
+                ok = ok && ptx::mbar_wait_bounded(ptx::smem_u32(&bar_acc[(c - kStages) % kAccs]), (uint32_t)((c - kStages) / kAccs) & 1u, p.wait_limit);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok)
+                return;
+            const uint32_t s = (uint32_t)(c % kStages * kStageBytes);
+            half(a0, b0, s);
+            half(a1, b1, s + kHalfBytes);
+            if (--left == 0)
+            {
+                // the tile's magnitudes, before its last stage is handed over
+                uint32_t* const mg = mags + (t & 1) * kMagWords;
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                {
+                    uint32_t m = max(mag_a[i] & 0xffffu, mag_a[i] >> 16);
+#pragma unroll
+                    for (int o = 8; o > 0; o >>= 1)
+                        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+                    if ((lane & 15) == 0)
+                        mg[2 * (w + 8 * i) + odd] = m;
+                    mag_a[i] = 0;
+                }
+                mg[kTile + w * (kTile / 2) + lane]      = mag_b[0];
+                mg[kTile + w * (kTile / 2) + lane + 32] = mag_b[1];
+                mag_b[0] = mag_b[1] = 0;
+                left = p.nk;
+                t++;
+            }
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0)
+                ptx::mbar_arrive(ptx::smem_u32(&bar_full[c % kStages]));
+        };
+        start_tile();
+        load_a(a0);
+        load_b(b0);
+        next_half();
+        load_a(a1);
+        load_b(b1);
+        next_half();
+        for (int c = 0; c < total && ok; c++)
+            stage(c);
+    }
+    if (!ok)
+        atomicOr(p.status, TB200_DEV_TIMEOUT);
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kFlushWarps)
+    {
+        ptx::tc_fence_after_sync();
+        ptx::tmem_dealloc(tmem, kAccs * kTile);
+    }
+}
+
+template <bool CONV, bool AVEC, bool BVEC>
+tb200_status launch_split(tb200_ctx* ctx, const SplitParams& p)
+{
+    auto kern = sgemm_split_kernel<CONV, AVEC, BVEC>;
+    const tb200_status st = raise_smem_limit(ctx, 52 + (CONV ? 2 : 0) + (AVEC ? 1 : 0), reinterpret_cast<const void*>(kern), kSplitSmem);
+    if (st != TB200_OK)
+        return st;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim          = dim3((unsigned)std::min(p.tiles, ctx->num_sms));
+    cfg.blockDim         = dim3(kSplitThreads);
+    cfg.dynamicSmemBytes = kSplitSmem;
+    cfg.stream           = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id                                           = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs    = at;
+    cfg.numAttrs = ctx->launch_overlap ? 1 : 0;
+    timer_begin(ctx);
+    cudaLaunchKernelEx(&cfg, kern, p);
+    timer_end(ctx);
+    return TB200_OK;
+}
+
+tb200_status finish_split(tb200_ctx* ctx, SplitParams& p, int batches)
+{
+    p.tiles_m = (p.M + kTile - 1) / kTile;
+    p.tiles_n = (p.N + kTile - 1) / kTile;
+    p.tiles   = batches * p.tiles_m * p.tiles_n;
+    p.nk      = (p.K + kStageK - 1) / kStageK;
+    p.idesc      = ptx::make_idesc(1u, 1u, 1u, 0u, 1u, kTile, kTile);
+    p.a_desc_hi  = ptx::make_smem_desc_hi(16, 512, 4u);
+    p.b_desc_hi  = ptx::make_smem_desc_hi(kPlane / 2, 1024, 2u);
+    p.wait_limit = ctx->wait_limit_cycles;
+    p.status     = ctx->d_status;
+    return TB200_OK;
+}
+
+// Shallow products stay with the FFMA kernel: its chains are short enough there to err no more than a stage's cut-off does
+// (1.4e-7 at K = 64), and the tables of magnitudes rely on tiles of at least four stages.
+constexpr int kMinSplitK = 256;
+
+}    // namespace
+
+// Estimated SM cycles of the split kernel, 0 where it does not serve.
+// A stage measured 3 700 cycles, 4 600 with unaligned pairs, 5 000 - 6 500 where A is gathered (16x28x28x256 3x3 256
+// channels: 187 us, 79 TFLOP/s).
+double sgemm_split_cost(const tb200_ctx* ctx, int64_t batches, int64_t M, int64_t N, int64_t K, bool conv)
+{
+    const int64_t tiles = batches * ((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile);
+    if (K < kMinSplitK || tiles >= (1LL << 30) || (ctx->max_smem_optin > 0 && ctx->max_smem_optin < kSplitSmem + 256) || ctx->d_status == nullptr)
+        return 0.0;
+    const double rounds = (double)((tiles + ctx->num_sms - 1) / ctx->num_sms);
+    const double stage  = conv ? 6200.0 : (K % 2 || N % 2) ? 4600.0 : 3700.0;
+    return rounds * ((double)((K + kStageK - 1) / kStageK) * stage + 1500.0) + 5000.0;
+}
+
+tb200_status sgemm_split_launch(tb200_ctx* ctx, const float* a, const float* b, float* out, int N, int H, int C, int W)
+{
+    SplitParams p;
+    memset(&p, 0, sizeof(p));
+    p.a = a; p.b = b; p.out = out;
+    p.M = H; p.N = W; p.K = C; p.ldb = W;
+    p.a_batch = (int64_t)H * C; p.b_batch = (int64_t)C * W; p.o_batch = (int64_t)H * W;
+    finish_split(ctx, p, N);
+    const bool vec = (W % 2) == 0 && (C % 2) == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 7) == 0;
+    const tb200_status st = vec ? launch_split<false, true, true>(ctx, p) : launch_split<false, false, false>(ctx, p);
+    return st != TB200_OK ? st : post_launch(ctx, "sgemm_f32");
+}
+
+tb200_status conv_f32_split_launch(tb200_ctx* ctx, const ConvF32Problem& q)
+{
+    SplitParams p;
+    memset(&p, 0, sizeof(p));
+    p.a = q.in; p.b = q.wt; p.out = q.out;
+    p.M = q.N * q.OH * q.OW; p.N = q.OC; p.K = q.KH * q.KW * q.IC; p.ldb = conv_f32_ldb(q.OC);
+    p.IH = q.IH; p.IW = q.IW; p.IC = q.IC; p.OH = q.OH; p.OW = q.OW; p.KW = q.KW;
+    p.pad_t = q.pad_t; p.pad_l = q.pad_l; p.sy = q.sy; p.sx = q.sx; p.dy = q.dy; p.dx = q.dx;
+    p.in_sn = (int)q.in_sn; p.in_sh = (int)q.in_sh; p.in_sw = (int)q.in_sw;
+    p.bias = q.bias; p.bias_n = q.bias_n;
+    p.has_clamp = q.has_clamp; p.clamp_lo = q.clamp_lo; p.clamp_hi = q.clamp_hi;
+    finish_split(ctx, p, 1);
+    const bool vec = (q.IC % 2) == 0 && ((q.in_sn | q.in_sh | q.in_sw) & 1) == 0 && (reinterpret_cast<uintptr_t>(q.in) & 7) == 0;
+    const tb200_status st = vec ? launch_split<true, true, true>(ctx, p) : launch_split<true, false, true>(ctx, p);
+    return st != TB200_OK ? st : post_launch(ctx, "conv_f32");
+}
+
+}    // namespace tb200

@@ -89,3 +89,84 @@ def test_conv_f32_view_and_infinite_weight(ctx):
     assert ctx.last_kernel() == "conv2d_direct"
     out = to.download()[1]
     assert not np.isnan(out).any() and np.isinf(out[:, 1:, 1:, 0]).all() and np.isfinite(out[:, 0, :, 0]).all()
+
+
+# Products deep and large enough for the tensor-core kernel (three bf16 parts per operand): whole tiles, row / column / K
+# remainders, rows of any alignment, the smallest depth it takes.
+SPLIT = [(148, 128, 256, 128), (70, 255, 319, 256), (40, 250, 258, 383), (37, 256, 1000, 250), (3, 1000, 515, 777)]
+
+
+@pytest.mark.parametrize("shape", SPLIT)
+def test_matmul_f32_split(ctx, shape):
+    N, H, C, W = shape
+    r = util.rng(990 + H + C)
+    a, b = r.standard_normal((N, H, C)).astype(np.float32), r.standard_normal((N, C, W)).astype(np.float32)
+    ta, tbb, to = ctx.from_numpy(a), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, (N, H, W))
+    ctx.matmul(ta, tbb, to)
+    st, out = to.download()
+    ref = a.astype(np.float64) @ b.astype(np.float64)
+    # 24-bit operands, six partial products, a cut-off sum per 64 K elements: far below 2^-22 of the sum of magnitudes
+    assert st == tb.Status.OK and np.all(np.abs(out - ref) <= 2.0 ** -22 * (np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)))
+    assert np.linalg.norm(out - ref) <= 3e-7 * np.linalg.norm(ref)
+    for t in (ta, tbb, to):
+        t.free()
+
+
+@pytest.mark.parametrize("what", ["special", "tiny_lines", "tiny", "overflow"])
+def test_matmul_f32_split_range(ctx, what):
+    """Operands whose parts leave bf16's or the normal range: same classes and the same accuracy as multiply-adds."""
+    N, H, C, W = 40, 256, 320, 256
+    r = util.rng(77)
+    a, b = r.standard_normal((N, H, C)).astype(np.float32), r.standard_normal((N, C, W)).astype(np.float32)
+    if what == "special":
+        a[0, 3, 5], a[1, 7, 9], b[2, 10, 11], b[3, 5, 6], a[3, :100] = np.inf, np.nan, -np.inf, np.inf, 0.0
+        b[4, 0, 0], a[4, :, 0] = 1e38, 2.0
+    elif what == "tiny_lines":
+        a[:, 17] *= 2.0 ** -118
+        b[:, :, 3] *= 2.0 ** -120
+        b[:, :, 9] *= 2.0 ** 50
+    elif what == "tiny":
+        a *= np.float32(2.0 ** -55)
+        b *= np.float32(2.0 ** -60)
+    else:
+        a *= np.float32(2.0 ** 100)
+        b[:, :, ::2] *= np.float32(2.0 ** 60)
+    ta, tbb, to = ctx.from_numpy(a), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, (N, H, W))
+    ctx.matmul(ta, tbb, to)
+    st, out = to.download()
+    with np.errstate(all="ignore"):
+        ref   = a.astype(np.float64) @ b.astype(np.float64)
+        ref32 = ref.astype(np.float32)
+        bound = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
+        assert st == tb.Status.OK and np.array_equal(np.isnan(out), np.isnan(ref32))
+        sure = np.abs(bound) < 2.0 ** 127    # no partial sum can overflow: finite, within K roundings and the subnormal step
+        assert np.all(np.abs(out[sure] - ref[sure]) <= C * 2.0 ** -24 * bound[sure] + C * 2.0 ** -149)
+        assert what != "overflow" or np.isinf(out[:, :, ::2]).all()    # every product is out of range: the first one's sign stays
+        inf = np.isinf(ref)
+        assert np.array_equal(out[inf], ref32[inf])
+    for t in (ta, tbb, to):
+        t.free()
+
+
+@pytest.mark.parametrize("case", [(32, 28, 28, 64, 128, 3, [1, 1], [1, 1, 1, 1]), (32, 29, 27, 33, 127, 3, [1, 1], [1, 1, 1, 1]),
+                                  (32, 57, 57, 256, 260, 1, [2, 2], [0, 0, 0, 0])])
+def test_conv_f32_split(ctx, case):
+    N, IH, IW, IC, OC, K, stride, pad = case
+    r = util.rng(1010 + IC)
+    x, w = r.standard_normal((N, IH, IW, IC)).astype(np.float32), r.standard_normal((OC, K, K, IC)).astype(np.float32)
+    b = r.standard_normal(OC).astype(np.float32)
+    OH, OW = orc.conv_out_hw(IH, IW, K, K, pad, stride, [1, 1])
+    tx, tw, tbias, to = ctx.from_numpy(x), ctx.from_numpy(w), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, (N, OH, OW, OC))
+    ctx.conv2d(tx, tw, tbias, to, pad, stride, [1, 1], epilogue=tb.Epilogue(None, (-20.0, 30.0)))
+    assert ctx.last_kernel() == "conv_f32"
+    st, out = to.download()
+    xp = np.pad(x.astype(np.float64), ((0, 0), (pad[0], pad[1]), (pad[2], pad[3]), (0, 0)))
+    ref, bound = np.zeros((N, OH, OW, OC)) + b, np.zeros((N, OH, OW, OC)) + np.abs(b)
+    for ky in range(K):
+        for kx in range(K):
+            win = xp[:, ky:ky + (OH - 1) * stride[0] + 1:stride[0], kx:kx + (OW - 1) * stride[1] + 1:stride[1]]
+            wt = w[:, ky, kx].astype(np.float64).T
+            ref, bound = ref + win @ wt, bound + np.abs(win) @ np.abs(wt)
+    assert st == tb.Status.OK and np.all(np.abs(out - np.clip(ref, -20.0, 30.0)) <= 2.0 ** -22 * bound)
+    for t in (tx, tw, tbias, to):
+        t.free()
