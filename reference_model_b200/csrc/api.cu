@@ -1296,8 +1296,11 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
         }
     }
 
-    // ---- channel runs that are no multiple of 32 bytes: gathering tensor-core kernel (tc_any.cu)
-    if (ctx->policy != 1 && (!int_path || weight_zp == 0) && tc_rescale_ok && input->dtype != TB200_FP32 && input->stride[3] == 1 && IC > 0)
+    // ---- channel runs that are no multiple of 32 bytes: gathering tensor-core kernel (tc_any.cu).  Not for up to 2^20
+    // multiply-adds in sums of at most 64: one thread per output finishes within the launch's own time there, and needs no
+    // tables and no tensor map (32x32x8 1x1 16 channels: 7.4 against 7.8 us a call, 19 against 49 us the first).
+    const bool tiny = (int64_t)KH * KW * IC <= 64 && (int64_t)N * OH * OW * OC * KH * KW * IC <= (1 << 20);
+    if (ctx->policy != 1 && !tiny && (!int_path || weight_zp == 0) && tc_rescale_ok && input->dtype != TB200_FP32 && input->stride[3] == 1 && IC > 0)
     {
         const int es       = (int)dtype_size(input->dtype);
         const int run      = IC * es, runp = (run + 15) & ~15;    // a tap's channel run, in memory and in the packed weights

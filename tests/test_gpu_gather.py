@@ -64,7 +64,8 @@ def test_matmul_float(ctx, name, shape):
 
 # N, IH, IW, IC, OC, K, stride, pad, in_zp
 CONV = [(1, 32, 32, 8, 16, 1, 1, 0, 5), (2, 13, 11, 24, 40, 3, 1, 1, -128), (1, 9, 10, 13, 7, 3, 1, 1, 3), (3, 7, 7, 20, 300, 1, 1, 0, -128),
-        (1, 15, 15, 50, 33, 5, 2, 2, 9), (1, 3, 3, 200, 65, 3, 1, 1, -128), (2, 5, 130, 12, 31, 3, 1, 1, 0), (1, 4, 4, 500, 24, 3, 1, 1, 7)]
+        (1, 15, 15, 50, 33, 5, 2, 2, 9), (1, 3, 3, 200, 65, 3, 1, 1, -128), (2, 5, 130, 12, 31, 3, 1, 1, 0), (1, 4, 4, 500, 24, 3, 1, 1, 7),
+        (9, 32, 32, 8, 16, 1, 1, 0, 5), (4, 7, 7, 20, 300, 1, 1, 0, -128)]
 
 
 @pytest.mark.parametrize("case", CONV)
@@ -75,7 +76,8 @@ def test_conv_i8(ctx, case):
     args = ([p] * 4, [s, s], [1, 1], izp, 0)
     _, exp = oracle_conv_i8(x, w, b, *args)
     st, out, kernel = run_conv_i8(ctx, x, w, b, *args)
-    assert kernel == "tc_gemm_any_i8_i32" and st == tb.Status.OK and np.array_equal(out, exp), kernel
+    tiny = K * K * IC <= 64 and exp.size * K * K * IC <= 1 << 20    # one thread per output
+    assert kernel == ("conv2d_direct" if tiny else "tc_gemm_any_i8_i32") and st == tb.Status.OK and np.array_equal(out, exp), kernel
     mult, shift = util.rescale_params(r, OC)
     for rounding, clamp in (("DOUBLE_ROUND", (-128, 127)), ("SINGLE_ROUND", (-90, 100))):
         resc = (mult, shift, -3, rounding)
@@ -83,7 +85,7 @@ def test_conv_i8(ctx, case):
         assert est == orc.VALID
         for cache in (True, False):    # with proven records and with the general arithmetic
             st, out, kernel = run_conv_i8(ctx, x, w, b, *args, rescale=resc, clamp=clamp, cache=cache)
-            assert kernel == "tc_gemm_any_i8_rescale" and st == tb.Status.OK and np.array_equal(out, exp), (rounding, cache)
+            assert kernel == ("conv2d_direct" if tiny else "tc_gemm_any_i8_rescale") and st == tb.Status.OK and np.array_equal(out, exp), (rounding, cache)
 
 
 @pytest.mark.parametrize("dt,name", [(F16, "fp16"), (BF16, "bf16")])
