@@ -2538,7 +2538,12 @@ extern "C" tb200_status tb200_matmul(tb200_ctx* ctx, const tb200_tensor* a, cons
         q.b_ld = b_ld;
         std::string why;
         // (the CTA-pair kernel takes K tails the single-CTA kernel does not)
-        if (!tc_gemm_pair_supported(q, ctx->num_sms) && (any_first || pad_b || !tc_gemm_supported(q, &why)))
+        const bool ragged = !tc_gemm_pair_supported(q, ctx->num_sms) && (any_first || pad_b || !tc_gemm_supported(q, &why));
+        // Ragged products of up to 2^23 multiply-adds in sums of at most 64 stay with one thread per output: most of a 128-byte
+        // chunk of K would be padding, and the call is its launch (bf16 4x338x16x363: 8.7 against 10.7 us, 1x133x47x152: 7.4
+        // against 8.9; beyond, 96x197x64x197 takes 72 us there and 23 us on the tensor cores).
+        const bool tiny = ragged && ctx->policy == 0 && C <= 64 && (int64_t)N * H * W * C <= (1 << 23);
+        if (ragged && !tiny)
         {
             TcProblem g = q;
             g.b_ld = 0;
@@ -2550,8 +2555,7 @@ extern "C" tb200_status tb200_matmul(tb200_ctx* ctx, const tb200_tensor* a, cons
             if (tc_any_supported(ctx, g))
                 return tc_any_launch(ctx, g);
         }
-        // (the CTA-pair kernel takes K tails the single-CTA kernel does not)
-        if (tc_gemm_pair_supported(q, ctx->num_sms) || tc_gemm_supported(q, &why))
+        if (!tiny && (tc_gemm_pair_supported(q, ctx->num_sms) || tc_gemm_supported(q, &why)))
         {
             const bool need_sums = int_path && (a_zp != 0 || b_zp != 0);
             const int Wpad       = (W + 255) / 256 * 256;

@@ -20,7 +20,8 @@ def ctx():
     c.close()
 
 
-@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 129, 17, 33), (3, 128, 100, 257), (1, 5, 3000, 300), (4, 250, 36, 40), (1, 33, 130, 515)])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 129, 17, 33), (3, 128, 100, 257), (1, 5, 3000, 300), (4, 250, 36, 40), (1, 33, 130, 515),
+                                   (1, 1, 65, 1), (2, 129, 81, 33), (4, 250, 100, 40), (40, 129, 60, 33)])
 @pytest.mark.parametrize("zp", [(0, 0), (3, 0), (0, -2), (-128, 127)])
 def test_matmul_i8(ctx, shape, zp):
     N, H, C, W = shape
@@ -28,7 +29,8 @@ def test_matmul_i8(ctx, shape, zp):
     a, b = r.integers(-128, 128, size=(N, H, C)).astype(np.int8), r.integers(-128, 128, size=(N, C, W)).astype(np.int8)
     ta, tbb, to = ctx.from_numpy(a), ctx.from_numpy(b), ctx.empty(tb.DType.INT32, (N, H, W))
     ctx.matmul(ta, tbb, to, *zp)
-    assert ctx.last_kernel() == "tc_gemm_any_i8_i32"
+    tiny = C <= 64 and N * H * C * W <= 1 << 23    # one thread per output
+    assert ctx.last_kernel() == ("matmul_direct" if tiny else "tc_gemm_any_i8_i32")
     st, out = to.download()
     assert st == tb.Status.OK and np.array_equal(out, orc.matmul(a, b, *zp, nthreads=8))
     for t in (ta, tbb, to):
@@ -36,7 +38,8 @@ def test_matmul_i8(ctx, shape, zp):
 
 
 @pytest.mark.parametrize("name", ["fp16", "bf16", "e4m3"])
-@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (3, 130, 26, 31), (2, 197, 64, 197), (1, 7, 2679, 72), (2, 60, 77, 300)])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (3, 130, 26, 31), (2, 197, 64, 197), (1, 7, 2679, 72), (2, 60, 77, 300),
+                                   (1, 1, 65, 1), (3, 130, 90, 31), (5, 197, 64, 197)])
 def test_matmul_float(ctx, name, shape):
     N, H, C, W = shape
     r = util.rng(2100 + H + W)
@@ -53,7 +56,8 @@ def test_matmul_float(ctx, name, shape):
     for dt, oname in outs:
         to = ctx.empty(dt, (N, H, W))
         ctx.matmul(ta, tbb, to)
-        assert ctx.last_kernel().startswith("tc_gemm_any"), ctx.last_kernel()
+        tiny = C <= 64 and N * H * C * W <= 1 << 23
+        assert ctx.last_kernel().startswith("matmul_direct" if tiny else "tc_gemm_any"), ctx.last_kernel()
         st, out = to.download()
         out = util.from_bf16_bits(out) if dt == BF16 else out.astype(np.float32)
         ok, info = orc.verify_dot_product(out, ref, bnd, orc.dot_product_ksb(C, "fp32", oname), out=oname)
