@@ -1427,7 +1427,10 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
     // ---- fp32: tiled FFMA kernel (sgemm_f32.cu).  Its row table packs window origins into 16 bits and input offsets into 32.
     // Padding is a zero-filled tap, which equals the reference's skipped tap only for finite weights: a padded layer whose
     // weights are not known to be finite takes the kernel below.
-    if (input->dtype == TB200_FP32 && ctx->policy == 0 && input->stride[3] == 1 && IH + pad[0] + pad[1] < 32768 &&
+    // Sums of at most 20 products, up to 6 M of them in all, stay with one thread per output (5x109x33x16 1x1 16 channels: 9.3
+    // against 11.5 us; at 8x56x56x64 3x3 64 channels it is 60 times slower).
+    const bool shallow = KH * KW * IC <= 20 && (int64_t)N * OH * OW * OC * KH * KW * IC <= 6000000;
+    if (input->dtype == TB200_FP32 && ctx->policy == 0 && !shallow && input->stride[3] == 1 && IH + pad[0] + pad[1] < 32768 &&
         IW + pad[2] + pad[3] < 32768 && (int64_t)N * input->stride[0] < (1LL << 31))
     {
         const int K             = KH * KW * IC;
@@ -2323,11 +2326,11 @@ extern "C" tb200_status tb200_depthwise_conv2d(tb200_ctx* ctx, const tb200_tenso
     d.in_zp = input_zp; d.w_zp = weight_zp; d.bias_n = bias->shape[0];
     fill_conv_dev(&d, epi);
     const int block = 256;
-    // int8 with RESCALE to int8: the sliding kernel, for outputs of at least 2^14 values (below, its serial walk along x has
-    // too few threads and the kernels below finish first)
+    // int8 with RESCALE to int8: the sliding kernel, for at least 2^20 multiply-adds (below, the kernels after it finish within
+    // the launch's own time and need no tables: 9x42x9x107 3x3 stride 2 7.7 against 8.2 us a call)
     if (int_path && M == 1 && ctx->policy == 0 && weight_zp == 0 && KH == KW && stride[0] == stride[1] && dilation[0] == 1 && dilation[1] == 1 &&
         epi.has_rescale && epi.rs.scale32 && epi.rs.rounding != TB200_INEXACT_ROUND && output->dtype == TB200_INT8 && !epi.rs.out_unsigned &&
-        ctx->const_cache_on && numel(output) >= (1 << 14))
+        ctx->const_cache_on && numel(output) * KH * KW >= (1 << 20))
     {
         DepthwiseI8Problem q;
         memset(&q, 0, sizeof(q));

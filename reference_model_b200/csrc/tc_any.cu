@@ -1019,8 +1019,15 @@ bool tc_any_supported(const tb200_ctx* ctx, const TcProblem& q)
         return false;
     if (q.xpar || q.out_sy || q.tile_end || (reinterpret_cast<uintptr_t>(q.out) & 3))
         return false;
-    AnyPlan plan;
-    return any_choose(q, ctx->num_sms, ctx->max_smem_optin > 0 ? ctx->max_smem_optin - 1024 : 200 * 1024, &plan);
+    // (one layout that fits is enough: the launch then has one to choose)
+    const int max_smem = ctx->max_smem_optin > 0 ? ctx->max_smem_optin - 1024 /* static */ : 200 * 1024;
+    for (int bn = 32; bn <= 256; bn *= 2)
+    {
+        AnyPlan plan;
+        if (any_layout(q, max_smem, bn, 1, &plan) && (int64_t)(q.b_mn_major ? q.OH : 1) * plan.k.tiles_m * plan.k.tiles_n < (1LL << 31))
+            return true;
+    }
+    return false;
 }
 
 tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q)

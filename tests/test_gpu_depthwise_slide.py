@@ -34,6 +34,8 @@ CASES = [(2, 31, 33, 16, 3, 1, [1, 1, 1, 1], -128, "DOUBLE_ROUND", True, (-128, 
 def test_depthwise_slide(ctx, case):
     N, IH, IW, C, K, s, pad, izp, rounding, per_ch, clamp = CASES[case]
     r = util.rng(1900 + case)
+    OH, OW = orc.conv_out_hw(IH, IW, K, K, pad, [s, s], [1, 1])
+    N = max(N, -(-(1 << 20) // (OH * OW * C * K * K)))    # 2^20 multiply-adds: below, other kernels run
     x = r.integers(-128, 128, size=(N, IH, IW, C), dtype=np.int8)
     w = r.integers(-128, 128, size=(K, K, C, 1), dtype=np.int8)
     b = r.integers(-65536, 65536, size=C).astype(np.int32)
