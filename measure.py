@@ -151,7 +151,7 @@ def matmul_f16_config(ctx, timer, name, N, H, C, W, iters, seed):
 
 
 def matmul_f32_config(ctx, timer, name, N, H, C, W, iters, seed):
-    """fp32 x fp32 -> fp32 batched MATMUL (FFMA kernel, no TF32)."""
+    """fp32 x fp32 -> fp32 batched MATMUL (no TF32)."""
     r = np.random.default_rng(seed)
     a = r.standard_normal((N, H, C), dtype=np.float32)
     b = r.standard_normal((N, C, W), dtype=np.float32)
@@ -279,7 +279,7 @@ def main():
                     help="also time one int8 TRANSPOSE_CONV2D+RESCALE+CLAMP layer: N,IH,IW,IC,OC,K,stride,out_pad")
     ap.add_argument("--matmul-fp8", default=None, help="also time one FP8E4M3 MATMUL with FP16 output: N,H,C,W")
     ap.add_argument("--matmul-f16", default=None, help="also time one fp16 MATMUL with fp16 output: N,H,C,W")
-    ap.add_argument("--matmul-f32", default=None, help="also time one fp32 MATMUL (FFMA kernel): N,H,C,W")
+    ap.add_argument("--matmul-f32", default=None, help="also time one fp32 MATMUL: N,H,C,W")
     ap.add_argument("--depthwise-f16", default=None, help="also time one fp16 3x3 stride-2 DEPTHWISE_CONV2D + CLAMP: N,H,W,C")
     ap.add_argument("--conv3d", default=None, help="also time one int8 CONV3D (cubic kernel, stride 1, same padding): N,ID,IH,IW,IC,OC,K")
     ap.add_argument("--fused-head", default=None,
@@ -382,7 +382,7 @@ def main():
                 flops = 2.0 * N * H * C * W
                 clk = torch.cuda.get_device_properties(0).clock_rate / 1e6 if hasattr(torch.cuda.get_device_properties(0), "clock_rate") else 1.965
                 peak = 148 * 128 * 2 * 1.965e9 / 1e12
-                res = {"config": "c2b matmul fp32 64x1024x4096x1024 (FFMA, no TF32)", "kernel": ctx.last_kernel(), "ms": ms,
+                res = {"config": "c2b matmul fp32 64x1024x4096x1024 (no TF32)", "kernel": ctx.last_kernel(), "ms": ms,
                        "TFLOPS": flops / ms / 1e9, "bound": "fp32 CUDA cores", "peak_TFLOPS": peak,
                        "frac": flops / ms / 1e9 / peak, "peak_source": "148 SMs x 128 lanes x 2 x 1.965 GHz (nominal max clock)",
                        "l2": note}

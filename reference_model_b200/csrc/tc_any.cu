@@ -1005,9 +1005,6 @@ bool any_choose(const TcProblem& q, int num_sms, int max_smem, AnyPlan* best)
                 best->ctas = ctas;
             }
         }
-#ifdef TC_ANY_FORCE
-    TC_ANY_FORCE
-#endif
     return best_cost > 0;
 }
 
