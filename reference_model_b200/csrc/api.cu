@@ -870,11 +870,10 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
     if (!dry_run)
         cache_note_write(ctx, output->data, output->bytes);
 
-    const bool any_first = ctx->policy == 2;
     // ---- tensor-core path
     const bool tc_rescale_ok = !epi.has_rescale || (epi.rs.scale32 && epi.rs.rounding != TB200_INEXACT_ROUND &&
                                                     !epi.rs.out_unsigned);
-    if (ctx->policy == 0 && !any_first && (!int_path || weight_zp == 0) && tc_rescale_ok &&
+    if (ctx->policy == 0 && (!int_path || weight_zp == 0) && tc_rescale_ok &&
         (int_path || input->dtype != TB200_FP32))
     {
         TcProblem q;
@@ -1300,7 +1299,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
     // multiply-adds in sums of at most 64: one thread per output finishes within the launch's own time there, and needs no
     // tables and no tensor map (32x32x8 1x1 16 channels: 7.4 against 7.8 us a call, 19 against 49 us the first).
     const bool tiny = (int64_t)KH * KW * IC <= 64 && (int64_t)N * OH * OW * OC * KH * KW * IC <= (1 << 20);
-    if (ctx->policy != 1 && !tiny && (!int_path || weight_zp == 0) && tc_rescale_ok && input->dtype != TB200_FP32 && input->stride[3] == 1 && IC > 0)
+    if (ctx->policy == 0 && !tiny && (!int_path || weight_zp == 0) && tc_rescale_ok && input->dtype != TB200_FP32 && input->stride[3] == 1 && IC > 0)
     {
         const int es       = (int)dtype_size(input->dtype);
         const int run      = IC * es, runp = (run + 15) & ~15;    // a tap's channel run, in memory and in the packed weights
@@ -2515,9 +2514,8 @@ extern "C" tb200_status tb200_matmul(tb200_ctx* ctx, const tb200_tensor* a, cons
             return sgemm_f32_launch(ctx, reinterpret_cast<const float*>(a->data), reinterpret_cast<const float*>(b->data),
                                     reinterpret_cast<float*>(output->data), N, H, C, W);
     }
-    else if (ctx->policy != 1)
+    else if (ctx->policy == 0)
     {
-        const bool any_first = ctx->policy == 2;
         TcProblem q;
         memset(&q, 0, sizeof(q));
         q.in_dtype    = a->dtype;
@@ -2541,11 +2539,11 @@ extern "C" tb200_status tb200_matmul(tb200_ctx* ctx, const tb200_tensor* a, cons
         q.b_ld = b_ld;
         std::string why;
         // (the CTA-pair kernel takes K tails the single-CTA kernel does not)
-        const bool ragged = !tc_gemm_pair_supported(q, ctx->num_sms) && (any_first || pad_b || !tc_gemm_supported(q, &why));
+        const bool ragged = !tc_gemm_pair_supported(q, ctx->num_sms) && (pad_b || !tc_gemm_supported(q, &why));
         // Ragged products of up to 2^23 multiply-adds in sums of at most 64 stay with one thread per output: most of a 128-byte
         // chunk of K would be padding, and the call is its launch (bf16 4x338x16x363: 8.7 against 10.7 us, 1x133x47x152: 7.4
         // against 8.9; beyond, 96x197x64x197 takes 72 us there and 23 us on the tensor cores).
-        const bool tiny = ragged && ctx->policy == 0 && C <= 64 && (int64_t)N * H * W * C <= (1 << 23);
+        const bool tiny = ragged && C <= 64 && (int64_t)N * H * W * C <= (1 << 23);
         if (ragged && !tiny)
         {
             TcProblem g = q;
