@@ -1324,6 +1324,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
         q.out    = output->data;
         q.epi    = int_path ? TC_EPI_I32 : TC_EPI_FLOAT;
         q.a_fill = int_path ? input_zp : 0;
+        q.padded = pad[0] || pad[1] || pad[2] || pad[3];
         fill_tc_epilogue(&q, epi, output->dtype);
         q.rec = epi.has_rescale ? reinterpret_cast<const int32_t*>(weight->data) : nullptr;    // (layout only needs to know there are records)
         if (tc_any_supported(ctx, q))

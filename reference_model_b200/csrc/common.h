@@ -303,6 +303,7 @@ struct TcProblem
     int fuse_row_sums;
     int32_t a_zp, b_zp;
     int32_t a_fill;    // gathering kernel: what a tap outside the image contributes (the input zero point)
+    int padded;        // gathering kernel: some window may leave the image
     uint32_t* sum_flags;
     uint32_t sum_epoch;
     // per-column additive constants, padded: [classes][corr_stride]; corr_stride must be a multiple of 256 and cover

@@ -21,6 +21,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
 #include "common.h"
@@ -50,8 +51,10 @@ struct AnyParams
     uint32_t fd_ow[2], fd_oh[2];    // division by OW, OH (fastdiv_make)
     int64_t a_batch, o_batch, b_batch;    // elements between batches
     // gather of A: row m is the window of output pixel m (MATMUL: one tap, "pixel" stride = row stride)
-    int conv, IH, IW, OH, OW, KW, pad_t, pad_l, sy, sx, dy, dx;
+    int conv, IH, IW, OH, OW, KH, KW, pad_t, pad_l, sy, sx, dy, dx;
     int in_sn, in_sh, in_sw;              // elements
+    int skip_nan;           // float CONV2D with padding: see sum_inside()
+    int b_fmt;              // element type for sum_inside(): 0 fp16, 1 bf16, 2 E4M3, 3 E5M2
     uint32_t fill4;         // the input zero point in all four bytes
     int pieces_per_tap, pieces;           // 16-byte pieces of a run; of the whole K
     int chunks, chunks_per_split;         // 128-byte chunks of K; of one CTA of a cluster
@@ -142,6 +145,42 @@ struct Piece
         st_shared_v4(dst, o[0], o[1], o[2], o[3]);
     }
 };
+
+__device__ __forceinline__ float element(const uint8_t* base, int64_t i, int fmt)
+{
+    switch (fmt)
+    {
+        case 0: return __half2float(reinterpret_cast<const __half*>(base)[i]);
+        case 1: return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(base)[i]);
+        case 2: return static_cast<float>(reinterpret_cast<const __nv_fp8_e4m3*>(base)[i]);
+        default: return static_cast<float>(reinterpret_cast<const __nv_fp8_e5m2*>(base)[i]);
+    }
+}
+
+// A tap outside the image is a zero that is multiplied like any other; the reference skips it.  The two differ where a weight
+// is infinite or NaN: zero times it is NaN, and only then.  So a NaN of a window that leaves the image is summed again here,
+// over the taps inside, in ky, kx, channel order (reference_model/src/ops/tensor_ops.cpp:828-873).
+__device__ __noinline__ float sum_inside(const AnyParams& p, int m, int col)
+{
+    const int q  = (int)fastdiv_apply((uint32_t)m, p.fd_ow), n = (int)fastdiv_apply((uint32_t)q, p.fd_oh);
+    const int y0 = (q - n * p.OH) * p.sy - p.pad_t, x0 = (m - q * p.OW) * p.sx - p.pad_l;
+    if (y0 >= 0 && x0 >= 0 && y0 + (p.KH - 1) * p.dy < p.IH && x0 + (p.KW - 1) * p.dx < p.IW)
+        return __uint_as_float(0x7fffffffu);    // every tap is inside: the NaN stands
+    const uint8_t* const w = p.b + (int64_t)col * p.pieces * 16;
+    float sum = 0.f;
+    for (int ky = 0; ky < p.KH; ky++)
+        for (int kx = 0; kx < p.KW; kx++)
+        {
+            const int y = y0 + ky * p.dy, x = x0 + kx * p.dx;
+            if ((unsigned)y >= (unsigned)p.IH || (unsigned)x >= (unsigned)p.IW)
+                continue;
+            const int64_t at = (int64_t)n * p.in_sn + (int64_t)y * p.in_sh + (int64_t)x * p.in_sw;
+            const uint8_t* const wt = w + (int64_t)(ky * p.KW + kx) * p.pieces_per_tap * 16;
+            for (int c = 0; c < p.run_bytes / p.es; c++)
+                sum = fmaf(element(p.a, at + c, p.b_fmt), element(wt, c, p.b_fmt), sum);
+        }
+    return sum;
+}
 
 // Sixteen neighbouring columns of one row: corrections, RESCALE or bias, CLAMP, packing.  w: the packed output bytes.
 enum : int
@@ -701,7 +740,22 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
     uint8_t* const s0 = sm + p.stage_out_off + (p.tiles_n == 1 ? (reinterpret_cast<uintptr_t>(g0) & 15) : 0);
     const int s_pitch = p.tiles_n == 1 ? ncols * p.out_es : (ncols * p.out_es + 7) & ~3;
     bool bad = false;
-    auto finish = [&](int row, int c, const uint32_t (&v)[16]) {
+    auto finish = [&](int row, int c, uint32_t (&v)[16]) {
+        if (EPI == ANY_FLOAT && p.skip_nan)
+        {
+            uint32_t nans = 0;
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                nans |= (v[i] & 0x7fffffffu) > 0x7f800000u && c * 16 + i < ncols ? 1u << i : 0u;
+            for (; nans; nans &= nans - 1)
+            {
+                const int at       = __ffs((int)nans) - 1;
+                const uint32_t sum = __float_as_uint(sum_inside(p, m0 + row, n0 + c * 16 + at));
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    v[i] = i == at ? sum : v[i];
+            }
+        }
         uint32_t w[16];
         epilogue16<EPI>(p, n0 + c * 16, v, rec ? rec + c * 16 : nullptr, w, bad);
         const int left = min(16, ncols - c * 16);
@@ -906,7 +960,7 @@ bool any_layout(const TcProblem& q, int max_smem, int block_n, int splits, AnyPl
     if ((matmul ? sw * q.OW : sn * q.N) >= (1LL << 31))
         return false;    // offsets inside the input are 32 bits
     k.in_sw = (int)sw; k.in_sh = (int)sh; k.in_sn = (int)sn;
-    k.IH = q.IH; k.IW = q.IW; k.OH = matmul ? 1 : q.OH; k.OW = matmul ? 1 : q.OW; k.KW = q.KW;
+    k.IH = q.IH; k.IW = q.IW; k.OH = matmul ? 1 : q.OH; k.OW = matmul ? 1 : q.OW; k.KH = q.KH; k.KW = q.KW;
     fastdiv_make((uint32_t)k.OW, k.fd_ow);
     fastdiv_make((uint32_t)k.OH, k.fd_oh);
     k.pad_t = q.pad_t; k.pad_l = q.pad_l; k.sy = q.stride_y; k.sx = q.stride_x; k.dy = q.dil_y; k.dx = q.dil_x;
@@ -1039,6 +1093,8 @@ tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q)
     k.b   = reinterpret_cast<const uint8_t*>(q.b);
     k.out = reinterpret_cast<uint8_t*>(q.out);
     k.fill4 = (uint32_t)(q.a_fill & 0xff) * 0x01010101u;
+    k.skip_nan = !matmul && q.epi == TC_EPI_FLOAT && q.padded;
+    k.b_fmt    = q.in_dtype == TB200_FP16 ? 0 : q.in_dtype == TB200_BF16 ? 1 : q.in_dtype == TB200_FP8E4M3 ? 2 : 3;
     const bool is_f8 = dtype_is_fp8(q.in_dtype), is_i8 = q.in_dtype == TB200_INT8;
     k.kind = is_i8 ? 0 : is_f8 ? 2 : 1;
     uint32_t cf = is_i8 ? 2u : 1u, af, bf;

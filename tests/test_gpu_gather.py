@@ -105,6 +105,45 @@ def test_conv_float(ctx, dt, name, case):
     assert kernel == "tc_gemm_any_f16" and st == tb.Status.OK and ok, (kernel, info)
 
 
+@pytest.mark.parametrize("name", ["fp16", "bf16", "e5m2"])
+@pytest.mark.parametrize("case", [(2, 9, 11, 12, 20, 1, 1, 1), (1, 12, 9, 9, 70, 2, 1, 2), (1, 5, 6, 200, 33, 1, 2, 2)])
+def test_conv_nonfinite_weights_under_padding(ctx, name, case):
+    """A tap outside the image is skipped, whatever its weight: infinities and NaNs reach only the pixels whose windows hold
+    them.  (The last case splits K over a cluster.)"""
+    N, IH, IW, IC, OC, s, d, p = case
+    r = util.rng(2350 + IC)
+    shapes = (N, IH, IW, IC), (OC, 3, 3, IC)
+    if name == "e5m2":
+        cx, cw = (_fp8_codes(r, sh, name) for sh in shapes)
+        cw[0, 0, 0, 1], cw[2, 2, 1, 0], cw[OC - 1, 1, 2, IC - 1] = 0x7C, 0x7F, 0xFC    # infinity, NaN, -infinity
+        x, w = orc.fp8_to_f32(cx, name), orc.fp8_to_f32(cw, name)
+    else:
+        x, w = (orc.fptrunc(r.standard_normal(sh).astype(np.float32), name) for sh in shapes)
+        w[0, 0, 0, 1], w[2, 2, 1, 0], w[OC - 1, 1, 2, IC - 1] = np.inf, np.nan, -np.inf
+    b = orc.fptrunc(r.standard_normal(OC).astype(np.float32), "bf16" if name == "bf16" else "fp16")
+    pad = [p, p - 1 if (IH + 2 * p - 1 - 2 * d) % s else p, p, p - 1 if (IW + 2 * p - 1 - 2 * d) % s else p]
+    args = (pad, [s, s], [d, d])
+    ref, bnd = (orc.conv2d(x, w, b, *args, mode="f64", bounds=f) for f in (False, True))
+    if name == "e5m2":
+        dt, odt = tb.DType.FP8E5M2, F16
+        tx, tw, tbias, to = ctx.from_numpy(cx, dt), ctx.from_numpy(cw, dt), ctx.from_numpy(b.astype(np.float16)), ctx.empty(odt, ref.shape)
+        ctx.conv2d(tx, tw, tbias, to, *args)
+        kernel = ctx.last_kernel()
+        st, out = to.download()
+        out = out.astype(np.float32)
+        for t in (tx, tw, tbias, to):
+            t.free()
+    else:
+        st, out, kernel = run_conv_fp(ctx, x, w, b, *args, F16 if name == "fp16" else BF16)
+    assert kernel.startswith("tc_gemm_any") and st == tb.Status.OK
+    assert np.array_equal(np.isnan(out), np.isnan(ref)) and np.array_equal(np.isinf(out), np.isinf(ref))
+    assert np.isnan(out).any() and np.isfinite(out[..., [0, 2, OC - 1]]).any()
+    fin = np.isfinite(ref)
+    oname = "bf16" if name == "bf16" else "fp16"
+    ok, info = orc.verify_dot_product(out[fin], ref[fin], bnd[fin], orc.dot_product_ksb(9 * IC + 1, "fp32", oname), out=oname)
+    assert ok, info
+
+
 def test_bounded_waits_give_up(ctx):
     """A wait limit far below the time the first copies take: the kernel reports, frees what it holds, and the same call is
     exact afterwards (a call that finishes in time is fine as well)."""
