@@ -16,7 +16,9 @@
 // is multiplied with B (column sums, in every lane) and with A (row sums, in every column) beside the product itself.
 // Problems with few tiles split K over the CTAs of a cluster; the partial accumulators are added in rank order through
 // distributed shared memory.
-// Every wait is bounded; a wait that gives up sets TB200_DEV_TIMEOUT and the CTA drains and frees its tensor memory.
+// Every wait on a barrier in memory is bounded; one that gives up sets TB200_DEV_TIMEOUT and the CTA drains and frees its
+// tensor memory.  The allocation of tensor memory and the meetings of a cluster have no limit of their own: no CTA holds
+// columns while it waits for another CTA, so both end once the CTAs that run do.
 #include <algorithm>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -815,8 +817,34 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
             }
         }
     }
+    auto release = [&]() {
+        ptx::tc_fence_before_sync();
+        __syncthreads();
+        if (tid == 0 && abort_flag)
+        {
+            // a role gave up: let copies in flight land and MMAs already issued retire before memory is released
+            if (p.b_mode != 2)
+                for (int s = 0; s < p.stages; s++)
+                {
+                    ptx::mbar_wait_bounded(ptx::smem_u32(&bar_full[s]), 0u, 2000000LL);
+                    ptx::mbar_wait_bounded(ptx::smem_u32(&bar_full[s]), 1u, 2000000LL);
+                }
+            ptx::mbar_wait_bounded(ptx::smem_u32(&bar_acc), 0u, 40000000LL);
+        }
+        __syncthreads();
+        if (warp == 9)
+        {
+            ptx::tc_fence_after_sync();
+            ptx::tmem_dealloc(tmem, (uint32_t)p.tmem_cols);
+        }
+    };
     if (p.splits > 1)
     {
+        // Tensor memory goes back before this CTA waits for its peers.  Its allocation is the one wait of the kernel without a
+        // limit, and another launch's CTAs may hold columns of the same SM: two clusters that each held the columns the
+        // other's CTA waits for would wait for ever.  This way whoever holds columns gives them back without waiting for a CTA
+        // that may still be asking for some.
+        release();
         __syncwarp();
         ptx::cluster_sync();    // every CTA's partial tile is in its shared memory
         if (warp < 8 && ok)
@@ -899,30 +927,11 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
         atomicOr(p.status, TB200_DEV_UNPREDICTABLE);
 
     // ---------------------------------------------------------------------- teardown
-    ptx::tc_fence_before_sync();
+    __syncwarp();
     if (p.splits > 1)
-    {
-        __syncwarp();
         ptx::cluster_sync();    // nobody leaves while another CTA may still read its shared memory
-    }
-    __syncthreads();
-    if (tid == 0 && abort_flag)
-    {
-        // a role gave up: let copies in flight land and MMAs already issued retire before memory is released
-        if (p.b_mode != 2)
-            for (int s = 0; s < p.stages; s++)
-            {
-                ptx::mbar_wait_bounded(ptx::smem_u32(&bar_full[s]), 0u, 2000000LL);
-                ptx::mbar_wait_bounded(ptx::smem_u32(&bar_full[s]), 1u, 2000000LL);
-            }
-        ptx::mbar_wait_bounded(ptx::smem_u32(&bar_acc), 0u, 40000000LL);
-    }
-    __syncthreads();
-    if (warp == 9)
-    {
-        ptx::tc_fence_after_sync();
-        ptx::tmem_dealloc(tmem, (uint32_t)p.tmem_cols);
-    }
+    else
+        release();
 }
 
 struct AnyPlan
@@ -1026,7 +1035,7 @@ bool any_layout(const TcProblem& q, int max_smem, int block_n, int splits, AnyPl
     at += q.epi == TC_EPI_RESCALE && q.rec ? block_n * 32 : 0;
     plan->smem_bytes = at + 1024;
     plan->ctas       = 0;
-    // tensor memory of co-resident CTAs must fit together: one that waits for columns could hold up its cluster
+    // tensor memory of co-resident CTAs of one launch must fit together: one that waits for columns would idle its SM's share
     const int per_sm = std::min(3, (max_smem + 1024) / (plan->smem_bytes + 1024));
     if (per_sm * k.tmem_cols > 512)
         plan->smem_bytes = std::max(plan->smem_bytes, max_smem / 2 + 1024);

@@ -1,6 +1,8 @@
 """The gathering tensor-core kernel at the edges of its tiles: runs, rows and columns of every alignment, K shorter than a
 chunk and split over a cluster, one row, borders, views, both zero points, every element type, outputs that are no whole
 16-byte rows; integers bit for bit against the oracle, floats under the DOT_PRODUCT rule."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -162,3 +164,42 @@ def test_bounded_waits_give_up(ctx):
     ctx.matmul(ta, tbb, to, 3, -2)
     st, out = to.download()
     assert st == tb.Status.OK and np.array_equal(out, exp)
+
+
+def test_two_streams_share_the_chip():
+    """Products whose K is split over clusters, from two contexts (two streams) and two threads at once.  Their plans leave room
+    for both on an SM in shared memory but not in tensor memory (512 and 64 columns and more): CTAs queue for columns, and
+    the clusters still all meet."""
+    errors = []
+
+    def work(kind, shape, zp):
+        try:
+            N, H, C, W = shape
+            r = util.rng(2500 + C)
+            with tb.Context(0) as c:
+                if kind == "i8":
+                    a, b = r.integers(-128, 128, size=(N, H, C)).astype(np.int8), r.integers(-128, 128, size=(N, C, W)).astype(np.int8)
+                    exp, dt = orc.matmul(a, b, *zp, nthreads=8), tb.DType.INT32
+                else:    # small whole numbers: sums are exact in any order
+                    a, b = (r.integers(-3, 4, size=s).astype(np.float16) for s in ((N, H, C), (N, C, W)))
+                    exp, dt = np.matmul(a.astype(np.float32), b.astype(np.float32)).astype(np.float16), F16
+                ta, tbb = c.from_numpy(a), c.from_numpy(b)
+                outs = [c.empty(dt, exp.shape) for _ in range(4)]
+                for i in range(400):
+                    c.matmul(ta, tbb, outs[i % 4], *zp)
+                assert c.last_kernel().startswith("tc_gemm_any")
+                for to in outs:
+                    st, out = to.download()
+                    assert st == tb.Status.OK and np.array_equal(out, exp)
+                for t in [ta, tbb] + outs:
+                    t.free()
+        except BaseException as e:    # reported by the main thread
+            errors.append(e)
+
+    jobs = [("i8", (6, 5, 3000, 300), (3, -2)), ("f16", (24, 64, 4000, 62), (0, 0))]
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
