@@ -66,6 +66,7 @@ struct AnyParams
     int stages, stage_bytes, b_box_bytes, b_nbox;
     int ones_off, part_off, stage_out_off, rec_off;    // shared-memory offsets behind the 1024-byte aligned base
     int tmem_cols, csum_col, rsum_col;                 // accumulator columns of the sums (-1: not needed)
+    int halves;             // ANY_SUM32: accumulators per chunk, 1 or 2
     uint32_t idesc, idesc_rsum;
     uint64_t a_desc_hi, b_desc_hi;
     int b_kstep16, kind;    // 0 i8, 1 f16, 2 f8f6f4
@@ -190,6 +191,7 @@ enum : int
     ANY_I32     = 0,
     ANY_RESCALE = 1,
     ANY_FLOAT   = 2,
+    ANY_SUM32   = 3,    // floating-point operands, fp32 output
 };
 
 template <int EPI>
@@ -367,8 +369,14 @@ __device__ __forceinline__ void stage16(const AnyParams& p, uint8_t* dst, int nc
     }
 }
 
+// ANY_SUM32.  The tensor core cuts its running sum off at every step instead of rounding it, which a 16-bit result hides and
+// an fp32 result shows: with operands of one sign the sum of K = 4001 was 2.6e-6 off where rounded multiply-adds are 9e-7 off.
+// So no sum is carried there for more than one 128-byte chunk of K (64 or 128 elements): each stage has its own accumulator,
+// started from zero, and the gathering warps read a finished chunk back and add it to fp32 registers (64 of them at 128
+// columns: one CTA per SM) while later chunks are in flight.  Sums of up to two chunks of 16-bit operands, which rounded
+// multiply-adds do not get far wrong either, have an accumulator for each half of a chunk (K = 65: 1.6e-7 with one).
 template <int EPI, int ALIGN>
-__global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_constant__ AnyParams p)
+__global__ void __launch_bounds__(kThreads, EPI == ANY_SUM32 ? 1 : 2) tc_any_kernel(const __grid_constant__ AnyParams p)
 {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kMaxStages], bar_empty[kMaxStages], bar_acc;
@@ -448,6 +456,11 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
         ptx::dep_launch_trigger();
 
     bool ok = true;
+    constexpr int kSumGroups = EPI == ANY_SUM32 ? 4 : 1;    // sixteen columns each, of up to 128
+    float acc[kSumGroups * 16];
+#pragma unroll
+    for (int i = 0; i < kSumGroups * 16; i++)
+        acc[i] = 0.f;
     if (warp < 8)
     {
         // ------------------------------------------------------------------ gather
@@ -525,14 +538,50 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
                 }
             }
         };
+        auto wait_empty = [&]() {
+            const bool got = ptx::mbar_wait_bounded(ptx::smem_u32(&bar_empty[stage]), phase ^ 1u, p.wait_limit);
+            return EPI == ANY_SUM32 ? (bool)__all_sync(0xffffffffu, got) : got;    // (what follows there is done by whole warps)
+        };
+        // ANY_SUM32: the next chunk's sums into the registers.  Its accumulator is written again `stages` chunks later, which
+        // this thread hands over only after it has been here.
+        int summed = 0, sum_stage = 0;
+        uint32_t sum_phase = 0;
+        auto sum_chunk = [&]() {
+            ok = __all_sync(0xffffffffu, ok && ptx::mbar_wait_bounded(ptx::smem_u32(&bar_empty[sum_stage]), sum_phase, p.wait_limit));
+            if (!ok)
+                return;
+            ptx::tc_fence_after_sync();
+            const uint32_t t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(sum_stage * p.halves * p.block_n + (warp >> 2) * 16);
+            // (a second half that got no MMA was not written)
+            const int halves = p.halves == 2 && p.pieces - (c_lo + summed) * 8 > 4 ? 2 : 1;
+            for (int h = 0; h < halves; h++)
+#pragma unroll
+                for (int g = 0; g < kSumGroups; g++)
+                    if (g * 32 < p.block_n)
+                    {
+                        uint32_t v[16];
+                        ptx::tmem_ld_32x32b_x16(t + (uint32_t)(h * p.block_n + g * 32), v);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; i++)
+                            acc[g * 16 + i] += __uint_as_float(v[i]);
+                    }
+            ptx::tc_fence_before_sync();
+            summed++;
+            if (++sum_stage == p.stages)
+            {
+                sum_stage = 0;
+                sum_phase ^= 1u;
+            }
+        };
         if (ALIGN == 16)
         {
             // asynchronous copies; a stage is handed over once this thread's copies into it have landed: two stages
             // behind the one being filled
             int done = 0, done_stage = 0;
-            for (int i = 0; i < nk; i++)
+            for (int i = 0; i < nk && ok; i++)
             {
-                if (!ptx::mbar_wait_bounded(ptx::smem_u32(&bar_empty[stage]), phase ^ 1u, p.wait_limit))
+                if (!wait_empty())
                 {
                     ok = false;
                     break;
@@ -570,6 +619,8 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
                     done++;
                     done_stage = done_stage + 1 == p.stages ? 0 : done_stage + 1;
                 }
+                if (EPI == ANY_SUM32 && i >= 3)
+                    sum_chunk();
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
             for (; ok && done < nk; done++)
@@ -605,9 +656,9 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
             };
             Chunk cur;
             fetch(cur);
-            for (int i = 0; i < nk; i++)
+            for (int i = 0; i < nk && ok; i++)
             {
-                if (!ptx::mbar_wait_bounded(ptx::smem_u32(&bar_empty[stage]), phase ^ 1u, p.wait_limit))
+                if (!wait_empty())
                 {
                     ok = false;
                     break;
@@ -634,8 +685,13 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
                     stage = 0;
                     phase ^= 1u;
                 }
+                if (EPI == ANY_SUM32 && i >= 2)
+                    sum_chunk();
             }
         }
+        if (EPI == ANY_SUM32)
+            while (ok && summed < nk)
+                sum_chunk();
         if (EPI == ANY_RESCALE)
         {
             // the records have landed for every gathering warp
@@ -698,10 +754,18 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
                 ptx::tc_fence_after_sync();
                 const uint32_t sA = base + (uint32_t)(stage * p.stage_bytes);
                 uint64_t ad = ptx::smem_desc(p.a_desc_hi, sA), bd = ptx::smem_desc(p.b_desc_hi, sA + kABytes);
+                uint32_t d = tmem + (EPI == ANY_SUM32 ? (uint32_t)(stage * p.halves * p.block_n) : 0u);
+                if (EPI == ANY_SUM32)
+                    accum = 0;
                 const int mmas = min(4, (p.pieces - (c_lo + i) * 8 + 1) >> 1);    // 32 bytes of K each
                 for (int m = 0; m < mmas; m++, ad += 2, bd += (uint64_t)p.b_kstep16)
                 {
-                    if (EPI != ANY_FLOAT)
+                    if (EPI == ANY_SUM32 && m == 2 && p.halves == 2)
+                    {
+                        d += (uint32_t)p.block_n;
+                        accum = 0;
+                    }
+                    if (EPI < ANY_FLOAT)
                     {
                         ptx::mma_i8_ss(tmem, ad, bd, p.idesc, accum);
                         if (p.csum_col >= 0)
@@ -710,9 +774,9 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
                             ptx::mma_i8_ss(tmem + (uint32_t)p.rsum_col, ad, ones_a, p.idesc_rsum, accum);
                     }
                     else if (p.kind == 2)
-                        ptx::mma_f8_ss(tmem, ad, bd, p.idesc, accum);
+                        ptx::mma_f8_ss(d, ad, bd, p.idesc, accum);
                     else
-                        ptx::mma_f16_ss(tmem, ad, bd, p.idesc, accum);
+                        ptx::mma_f16_ss(d, ad, bd, p.idesc, accum);
                     accum = 1;
                 }
                 ptx::mma_commit(ptx::smem_u32(&bar_empty[stage]));
@@ -786,7 +850,31 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
             }
             if (EPI == ANY_I32 && rank == 0)
                 rterm -= (uint32_t)p.zp_const;
-            for (int c = warp >> 2; c < groups && c * 16 < ncols; c += 2)
+            auto emit = [&](int c, uint32_t (&v)[16]) {
+                if (p.splits > 1)
+                {
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        *reinterpret_cast<uint4*>(part + c * 16 + 4 * q) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                }
+                else if (row < rows)
+                    finish(row, c, v);
+            };
+            if (EPI == ANY_SUM32)
+            {
+#pragma unroll
+                for (int g = 0; g < kSumGroups; g++)
+                {
+                    const int c = (warp >> 2) + 2 * g;
+                    uint32_t v[16];
+#pragma unroll
+                    for (int i = 0; i < 16; i++)
+                        v[i] = __float_as_uint(acc[g * 16 + i]);
+                    if (c < groups && c * 16 < ncols)
+                        emit(c, v);
+                }
+            }
+            for (int c = warp >> 2; EPI != ANY_SUM32 && c < groups && c * 16 < ncols; c += 2)
             {
                 uint32_t v[16];
                 ptx::tmem_ld_32x32b_x16(t0 + (uint32_t)(c * 16), v);
@@ -806,14 +894,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
                     for (int i = 0; i < 16; i++)
                         v[i] -= rterm;
                 }
-                if (p.splits > 1)
-                {
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        *reinterpret_cast<uint4*>(part + c * 16 + 4 * q) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                }
-                else if (row < rows)
-                    finish(row, c, v);
+                emit(c, v);
             }
         }
     }
@@ -866,7 +947,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_any_kernel(const __grid_consta
                     {
                         uint32_t x0, x1, x2, x3;
                         asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x0), "=r"(x1), "=r"(x2), "=r"(x3) : "r"(src + 16 * q) : "memory");
-                        if (EPI == ANY_FLOAT)
+                        if (EPI >= ANY_FLOAT)
                         {
                             v[4 * q + 0] = __float_as_uint(__uint_as_float(v[4 * q + 0]) + __uint_as_float(x0));
                             v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + __uint_as_float(x1));
@@ -940,6 +1021,7 @@ struct AnyPlan
     int align;    // of A's channel runs: 16, 8, 4 bytes, 0 = less
     int smem_bytes;
     int64_t ctas;
+    bool sum32;    // ANY_SUM32
 };
 
 int64_t any_align(int64_t a, int64_t b)
@@ -1003,7 +1085,11 @@ bool any_layout(const TcProblem& q, int max_smem, int block_n, int splits, AnyPl
     k.direct      = ((int64_t)k.N * k.out_es) % 16 == 0 && (reinterpret_cast<uintptr_t>(q.out) & 15) == 0;
     k.a_zp = q.a_zp; k.b_zp = q.b_zp;
     k.csum_col = k.rsum_col = -1;
-    int cols = block_n;
+    plan->sum32 = q.epi == TC_EPI_FLOAT && q.out_dtype == TB200_FP32;
+    if (plan->sum32 && block_n > 128)
+        return false;
+    k.halves   = plan->sum32 && k.chunks <= 2 && k.es == 2 ? 2 : 1;
+    int cols   = plan->sum32 ? k.stages * k.halves * block_n : block_n;
     if (matmul && q.in_dtype == TB200_INT8)
     {
         if (q.a_zp != 0)
@@ -1057,7 +1143,7 @@ bool any_choose(const TcProblem& q, int num_sms, int max_smem, AnyPlan* best)
             const int64_t ctas = (int64_t)batches * k.tiles_m * k.tiles_n * s;
             if (ctas >= (1LL << 31))
                 continue;
-            const int per_sm     = std::max(1, std::min(2, (max_smem + 1024) / (plan.smem_bytes + 1024)));
+            const int per_sm     = plan.sum32 ? 1 : std::max(1, std::min(2, (max_smem + 1024) / (plan.smem_bytes + 1024)));
             const double rounds  = (double)((ctas + (int64_t)num_sms * per_sm - 1) / ((int64_t)num_sms * per_sm));
             const double stage_c = 500.0 + 2.0 * bn;
             const double cost    = rounds * (3000.0 + k.chunks_per_split * stage_c + bn * 20.0 / s + (s > 1 ? 2000.0 + 8.0 * bn : 0.0));
@@ -1156,12 +1242,14 @@ tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q)
     k.wait_limit = ctx->wait_limit_cycles;
     k.status     = ctx->d_status;
     const int al = plan.align == 16 ? 0 : plan.align == 8 ? 1 : plan.align == 4 ? 2 : 3;
-    static void (*const kernels[3][4])(const AnyParams) = {
+    const int variant = plan.sum32 ? ANY_SUM32 : q.epi;
+    static void (*const kernels[4][4])(const AnyParams) = {
         { tc_any_kernel<ANY_I32, 16>, tc_any_kernel<ANY_I32, 8>, tc_any_kernel<ANY_I32, 4>, tc_any_kernel<ANY_I32, 0> },
         { tc_any_kernel<ANY_RESCALE, 16>, tc_any_kernel<ANY_RESCALE, 8>, tc_any_kernel<ANY_RESCALE, 4>, tc_any_kernel<ANY_RESCALE, 0> },
-        { tc_any_kernel<ANY_FLOAT, 16>, tc_any_kernel<ANY_FLOAT, 8>, tc_any_kernel<ANY_FLOAT, 4>, tc_any_kernel<ANY_FLOAT, 0> } };
-    void (*const kern)(const AnyParams) = kernels[q.epi][al];
-    const tb200_status st = raise_smem_limit(ctx, 20 + q.epi * 4 + al, reinterpret_cast<const void*>(kern), plan.smem_bytes);
+        { tc_any_kernel<ANY_FLOAT, 16>, tc_any_kernel<ANY_FLOAT, 8>, tc_any_kernel<ANY_FLOAT, 4>, tc_any_kernel<ANY_FLOAT, 0> },
+        { tc_any_kernel<ANY_SUM32, 16>, tc_any_kernel<ANY_SUM32, 8>, tc_any_kernel<ANY_SUM32, 4>, tc_any_kernel<ANY_SUM32, 0> } };
+    void (*const kern)(const AnyParams) = kernels[variant][al];
+    const tb200_status st = raise_smem_limit(ctx, (plan.sum32 ? 56 : 20 + q.epi * 4) + al, reinterpret_cast<const void*>(kern), plan.smem_bytes);
     if (st != TB200_OK)
         return st;
     cudaLaunchConfig_t cfg;

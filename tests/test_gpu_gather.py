@@ -68,6 +68,36 @@ def test_matmul_float(ctx, name, shape):
     ta.free(), tbb.free()
 
 
+@pytest.mark.parametrize("name", ["fp16", "bf16", "e4m3", "e5m2"])
+@pytest.mark.parametrize("shape", [(8, 200, 65, 203), (8, 200, 81, 200), (8, 130, 100, 99), (2, 130, 300, 33), (1, 257, 1003, 203), (4, 100, 1160, 61), (2, 60, 4001, 300), (1, 33, 6007, 40)])
+def test_matmul_fp32_output_sums(ctx, name, shape):
+    """fp32 results of operands of one sign, where a running sum that is cut off at every step drifts: no further from the
+    64-bit product than the kernel that rounds every multiply-add."""
+    N, H, C, W = shape
+    r = util.rng(2600 + C)
+    if name[0] == "e":
+        ca, cb = (r.integers(0x28, 0x40, size=s).astype(np.uint8) for s in ((N, H, C), (N, C, W)))
+        a, b = orc.fp8_to_f32(ca, name), orc.fp8_to_f32(cb, name)
+        dt = tb.DType.FP8E4M3 if name == "e4m3" else tb.DType.FP8E5M2
+        ta, tbb = ctx.from_numpy(ca, dt), ctx.from_numpy(cb, dt)
+    else:
+        a, b = (orc.fptrunc(r.uniform(0.5, 1.0, size=s).astype(np.float32), name) for s in ((N, H, C), (N, C, W)))
+        ta, tbb = (ctx.from_numpy(v.astype(np.float16)) if name == "fp16" else ctx.from_numpy(util.to_bf16_bits(v), BF16) for v in (a, b))
+    ref, err, to = a.astype(np.float64) @ b.astype(np.float64), [], ctx.empty(F32, (N, H, W))
+    for policy in (0, 1):
+        old = ctx.set_kernel_policy(policy)
+        ctx.matmul(ta, tbb, to)
+        assert ctx.last_kernel().startswith("matmul_direct" if policy else "tc_gemm_any"), ctx.last_kernel()
+        ctx.set_kernel_policy(old)
+        st, out = to.download()
+        assert st == tb.Status.OK
+        err.append(np.linalg.norm(out - ref) / np.linalg.norm(ref))
+    print(name, shape, err)
+    assert err[0] <= err[1]
+    for t in (ta, tbb, to):
+        t.free()
+
+
 # N, IH, IW, IC, OC, K, stride, pad, in_zp
 CONV = [(1, 32, 32, 8, 16, 1, 1, 0, 5), (2, 13, 11, 24, 40, 3, 1, 1, -128), (1, 9, 10, 13, 7, 3, 1, 1, 3), (3, 7, 7, 20, 300, 1, 1, 0, -128),
         (1, 15, 15, 50, 33, 5, 2, 2, 9), (1, 3, 3, 200, 65, 3, 1, 1, -128), (2, 5, 130, 12, 31, 3, 1, 1, 0), (1, 4, 4, 500, 24, 3, 1, 1, 7),
