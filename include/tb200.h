@@ -292,7 +292,8 @@ extern "C"
                                                   tb200_tensor* output);
 
     /* MATMUL.  Replaces OpMatMul<A,B,Out>::eval (reference_model/src/ops/tensor_ops.cpp:1423-1492, checks :1347-1420).
-     * a [N,H,C], b [N,C,W], output [N,H,W]; INT8xINT8->INT32, FP16/BF16->same or FP32, FP32->FP32 (no TF32),
+     * a [N,H,C], b [N,C,W], output [N,H,W]; INT8xINT8->INT32, FP16/BF16->same or FP32, FP32->FP32 (no TF32: multiply-adds, or for
+     * large products of C >= 256 three bf16 parts per operand on the tensor cores, which leave out at most 2^-24 of a product),
      * FP8E4M3 / FP8E5M2 in any pairing of a and b -> FP16 or FP32 (:2263-2270; fp32 accumulation on the tensor cores,
      * `kind::f8f6f4`, rounded once to the output type). */
     TB200_API tb200_status tb200_matmul(tb200_ctx* ctx, const tb200_tensor* a, const tb200_tensor* b, int32_t a_zp,

@@ -1,13 +1,15 @@
 // fp32 batched MATMUL and CONV2D on the tensor cores without giving up fp32: every operand is taken apart into three bf16
-// values whose sum is the operand, exactly (24 significant bits = 8 + 8 + 8, cut off, not rounded), and a product is the six
-// partial products that matter (a0 b0, a0 b1, a1 b0, a0 b2, a1 b1, a2 b0; the three left out come to less than 2^-23 of
-// it, 2^-25 on average).  bf16 has fp32's exponent range, so nothing has to be scaled.
+// values whose sum is the operand, exactly (the first two rounded to nearest: what is left has 16, then 7 significant bits),
+// and a product is the six partial products that matter (a0 b0, a0 b1, a1 b0, a0 b2, a1 b1, a2 b0).  The three left out come
+// to at most 2^-24 of it, of either sign: |a1| <= 2^-8, |a2| <= 2^-17 of the operand's power of two.  (Parts that are cut off
+// instead leave out up to 2^-21, always of the product's sign.)  bf16 has fp32's exponent range, so nothing has to be scaled.
 //
-// Sums.  The tensor core cuts its running sum off instead of rounding it, so it never carries one far: a stage of 64 K
-// elements starts from zero, adds the five small partial products first (their cut-off is 2^-8 of the result's) and then
-// the four K steps of a0 b0; the stage's sum is read back and added to fp32 accumulators in registers, rounded to nearest.
-// Error against 64 bits, relative 2-norm, normal operands, K = 256 / 1024 / 4096: 1.3e-7 / 1.5e-7 / 1.9e-7; multiply-adds
-// in K order: 2.9e-7 / 5.7e-7 / 1.15e-6.  (Positive operands: 1.2e-7 / 1.3e-7 / 1.6e-7 against 2.2e-7 / 4.3e-7 / 8.4e-7.)
+// Sums.  The tensor core cuts its running sum off instead of rounding it, so it never carries one far, and the leading
+// products not beside the small ones: per stage of 64 K elements one accumulator takes a0 b0 (products of 16 bits, whose sums
+// mostly fit 24), and another, over four stages, the five others (whose cut-off is 2^-8 of the result's).  Both are read back and
+// added to fp32 accumulators in registers, rounded to nearest.
+// Error against 64 bits, relative 2-norm, K = 320: normal operands 8.5e-8 (multiply-adds in K order 3.2e-7), positive ones
+// 4.1e-8 (2.7e-7), one product per sum 2.52e-8 (2.48e-8).
 //
 // One persistent CTA per SM, 128 x 128 output tiles, sixteen warps:
 //   warps 0-7   add up stages (32 rows x 64 columns each, 64 accumulators per thread), finish and store the tile; the first
@@ -16,16 +18,16 @@
 //               the tensor core's swizzled layouts.  A warp's unit is 64 elements, two neighbours per lane, so that one code
 //               path serves any alignment, a gathered convolution window and both operands without bank conflicts.
 // Taking operands apart inside the kernel instead of in a pass before it keeps the planes out of memory (3.2 GB for 64
-// products of 1024 x 4096 x 1024).  32 x 1024 x 4096 x 1024: 1.74 ms, 158 TFLOP/s of fp32 (FFMA kernel 57.6), 3 700 SM cycles
-// per stage.  What bounds it: the MMAs alone take 2 680 (24 of ~107 and the hand-over), taking apart and storing 1 600, the
-// loads 3 300 on their own: 64 KB a stage through the ~28 KB of L1 that two 96 KB stages leave.  Three stages of 32 K
-// elements with more L1 lose more to commits and hand-overs (4 500).
+// products of 1024 x 4096 x 1024).  4 x 1024 x 4096 x 1024: 259 us (FFMA kernel 828), 3 800 SM cycles per stage.  What bounds it:
+// the MMAs alone take 2 680 (24 of ~107 and the hand-over), the loads 3 300 on their own: 64 KB a stage through the ~28 KB of
+// L1 that two 96 KB stages leave.  Three stages of 32 K elements with more L1 lose more to commits and hand-overs (4 500).
 //
 // Values the split cannot carry are computed again with ordinary multiply-adds, 32 rows x 16 columns at a time: results
 // that are not finite (an infinite operand has no split: its lower parts are NaN, so it always shows) and rows or columns so
 // small that lower parts or products would leave the normal range (largest magnitude of the row or column below 2^-100, or
 // of both together below 2^-60).
 #include <algorithm>
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "common.h"
@@ -36,7 +38,10 @@ namespace tb200
 namespace
 {
 
-constexpr int kTile = 128, kHalfK = 32, kStageK = 2 * kHalfK, kStages = 2, kAccs = 4;
+constexpr int kTile = 128, kHalfK = 32, kStageK = 2 * kHalfK, kStages = 2;
+constexpr int kAccs = 2;           // accumulators of a0 b0, one per stage, and of the five small partial products, one per
+constexpr int kSmallStages = 4;    // so many stages of a tile, behind each other in tensor memory
+constexpr int kBigCol = 2 * kTile, kTmemCols = 4 * kTile;
 constexpr int kPlane = kTile * kHalfK * 2;       // bytes of one bf16 plane of 32 K elements of an operand
 constexpr int kHalfBytes = 6 * kPlane, kStageBytes = 2 * kHalfBytes;    // A planes, B planes of 32 K elements, twice
 constexpr int kFlushWarps = 8, kSplitWarps = 8;
@@ -102,16 +107,20 @@ __device__ __forceinline__ float load1_if(const float* src, bool inside)
     return v;
 }
 
-// Two fp32 values as three packed bf16 pairs.
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// Two fp32 values as three packed bf16 pairs.  (A value that rounds to infinity leaves NaN: its results are computed again.)
 __device__ __forceinline__ void split3(float2 v, uint32_t (&w)[3])
 {
-    const uint32_t x = __float_as_uint(v.x), y = __float_as_uint(v.y);
-    w[0] = __byte_perm(x, y, 0x7632);
-    const float rx = v.x - __uint_as_float(x & 0xffff0000u), ry = v.y - __uint_as_float(y & 0xffff0000u);
-    const uint32_t x1 = __float_as_uint(rx), y1 = __float_as_uint(ry);
-    w[1] = __byte_perm(x1, y1, 0x7632);
-    const float sx = rx - __uint_as_float(x1 & 0xffff0000u), sy = ry - __uint_as_float(y1 & 0xffff0000u);
-    w[2] = __byte_perm(__float_as_uint(sx), __float_as_uint(sy), 0x7632);
+    w[0] = bf16_pair(v.x, v.y);
+    const float rx = v.x - __uint_as_float(w[0] << 16), ry = v.y - __uint_as_float(w[0] & 0xffff0000u);
+    w[1] = bf16_pair(rx, ry);
+    const float sx = rx - __uint_as_float(w[1] << 16), sy = ry - __uint_as_float(w[1] & 0xffff0000u);
+    w[2] = __byte_perm(__float_as_uint(sx), __float_as_uint(sy), 0x7632);    // exact: at most seven bits are left
 }
 
 // Sixteen columns of one row with ordinary multiply-adds, K in order.
@@ -189,7 +198,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
     }
     if (warp == kFlushWarps)
     {
-        ptx::tmem_alloc(ptx::smem_u32(&tmem_base_holder), kAccs * kTile);
+        ptx::tmem_alloc(ptx::smem_u32(&tmem_base_holder), kTmemCols);
         ptx::tmem_relinquish();
     }
     ptx::tc_fence_before_sync();
@@ -214,7 +223,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
         const bool v8 = (p.N & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
         // The stage's MMAs, by the first lane of the first of these warps: issuing takes as long as the MMAs before take to make
         // room in the unit's short queue, so a splitting warp must not do it (the two then take turns: 5 600 cycles a stage), and a warp of its own, the seventeenth, would leave 96 registers per thread instead of 128.
-        // These warps have time: a stage's sums take a fifth of its MMAs.
+        // These warps have time: a stage's sums take about a third of its MMAs.
+        int issue_k = 0, issue_small = 0;    // stage of its tile and small accumulator of the next issue
         auto issue = [&](int c) {
             const int buf = c % kAccs, slot = c % kStages;
             if (!ptx::mbar_wait_bounded(ptx::smem_u32(&bar_free[buf]), ((uint32_t)(c / kAccs) & 1u) ^ 1u, p.wait_limit) ||
@@ -222,12 +232,19 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
                 return false;
             ptx::tc_fence_after_sync();
             const uint32_t s = base + (uint32_t)(slot * kStageBytes);
-            uint32_t accum   = 0;
-            // smallest first: a0 b2, a1 b1, a2 b0, a0 b1, a1 b0, a0 b0
+            uint32_t accum   = issue_k % kSmallStages != 0;
+            const uint32_t small = tmem + (uint32_t)(issue_small * kTile), big = tmem + (uint32_t)(kBigCol + buf * kTile);
+            if (++issue_k == p.nk)
+                issue_k = 0;
+            if (issue_k % kSmallStages == 0)
+                issue_small ^= 1;
+            // smallest first: a0 b2, a1 b1, a2 b0, a0 b1, a1 b0; then a0 b0 into an accumulator of its own
             constexpr int pa[6] = { 0, 1, 2, 0, 1, 0 }, pb[6] = { 2, 1, 0, 1, 0, 0 };
 #pragma unroll
             for (int q = 0; q < 6; q++)
             {
+                if (q == 5)
+                    accum = 0;
 #pragma unroll
                 for (int h = 0; h < 2; h++)
                 {
@@ -236,7 +253,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
 #pragma unroll
                     for (int kk = 0; kk < kHalfK / 16; kk++, ad += 2, bd += 128)    // 32 bytes along a row; sixteen K rows
                     {
-                        ptx::mma_f16_ss(tmem + (uint32_t)(buf * kTile), ad, bd, p.idesc, accum);
+                        ptx::mma_f16_ss(q == 5 ? big : small, ad, bd, p.idesc, accum);
                         accum = 1;
                     }
                 }
@@ -250,7 +267,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
                 ok = issue(0);
             ok = __all_sync(0xffffffffu, ok);
         }
-        int c = 0;
+        int c = 0, small = 0;
         for (int i = 0, tile = (int)blockIdx.x; tile < p.tiles && ok; i++, tile += (int)gridDim.x)
         {
             const int batch = tile / per, rem = tile - batch * per, tm = rem / p.tiles_n;
@@ -273,11 +290,28 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
                 if (!ok)
                     break;
                 ptx::tc_fence_after_sync();
+                // (bar_free of a stage also frees the small accumulator that the stage two later may start: its last use was
+                // read back before)
+                const bool last = (k + 1) % kSmallStages == 0 || k + 1 == p.nk;
+                if (last)
+                {
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+                    {
+                        uint32_t v[32];
+                        ptx::tmem_ld_32x32b_x32(t0 + (uint32_t)(small * kTile + h * 32), v);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            acc[h * 32 + j] += __uint_as_float(v[j]);
+                    }
+                    small ^= 1;
+                }
 #pragma unroll
                 for (int h = 0; h < 2; h++)
                 {
                     uint32_t v[32];
-                    ptx::tmem_ld_32x32b_x32(t0 + (uint32_t)(buf * kTile + h * 32), v);
+                    ptx::tmem_ld_32x32b_x32(t0 + (uint32_t)(kBigCol + buf * kTile + h * 32), v);
                     ptx::tmem_ld_wait();
                     if (h == 1)
                     {
@@ -294,8 +328,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
             if (!ok)
                 break;
             // Magnitudes of this row and of this warp's columns (high halves of fp32 values).  The splitting warps come back to
-            // this half of the table two tiles, at least eight stages, later; they are never more than six stages ahead
-            // (two in shared memory, four in tensor memory).
+            // this half of the table two tiles, at least eight stages, later; they are never more than four stages ahead
+            // (two in shared memory, two in tensor memory).
             const uint32_t* const mg = mags + (i & 1) * kMagWords;
             uint32_t pair0 = 0, pair1 = 0;
 #pragma unroll
@@ -393,7 +427,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
         const uint32_t dst_a = base + (uint32_t)(w * 128 + odd * 64 + ((((lane >> 2) & 3) ^ (w & 3)) << 4) + (lane & 3) * 4);
         const uint32_t dst_b = base + (uint32_t)(3 * kPlane + w * 128 + (((lane >> 2) ^ w) << 4) + (lane & 3) * 4);
         ptx::dep_launch_wait();
-        // The loads run two stages ahead of the stage being taken apart, across tiles; past the last tile they load nothing.
+        // The loads run two halves, one stage, ahead of what is being taken apart, across tiles; past the last tile they load nothing.
         int tile = (int)blockIdx.x, kstage = 0;
         const float* A = p.a;    // MATMUL: this lane's elements of its first row; CONV2D: the input
         const float* B = p.b;    // this lane's elements of K row w
@@ -526,7 +560,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
                 asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (uint32_t)(q * kPlane)), "r"(x[q]) : "memory");
         };
         int left = p.nk, t = 0;    // stages left of the tile being taken apart, and which of this CTA's tiles it is
-        // One stage: loads of the stage two ahead follow the use of their registers, eight at a time (interleaved with their
+        // Half a stage: the loads of the half two ahead follow the use of their registers, eight at a time (interleaved with their
         // uses one by one, loads share the few scoreboards with later ones and every use waits for nearly all of them).
         auto half = [&](float2 (&va)[8], float2 (&vb)[8], uint32_t s) {
 #pragma unroll
@@ -593,7 +627,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
     if (warp == kFlushWarps)
     {
         ptx::tc_fence_after_sync();
-        ptx::tmem_dealloc(tmem, kAccs * kTile);
+        ptx::tmem_dealloc(tmem, kTmemCols);
     }
 }
 

@@ -114,6 +114,43 @@ def test_matmul_f32_split(ctx, shape):
         t.free()
 
 
+@pytest.mark.parametrize("what", ["one_term", "cut", "round", "normal", "positive"])
+def test_matmul_f32_split_accuracy(ctx, what):
+    """Against the kernel that rounds every multiply-add, and where the parts lose most: operands whose lower bits are all ones
+    (parts that were cut off would leave out 2^-21 of every product) and those for which rounded parts leave out most, 2^-24."""
+    N, H, C, W = 40, 256, 320, 256
+    r = util.rng(78)
+    if what in ("cut", "round"):
+        v = np.array([0x3F80FFFF if what == "cut" else 0x3F807FC0], np.uint32).view(np.float32)[0]
+        a, b = np.full((N, H, C), v, np.float32), np.full((N, C, W), v, np.float32)
+    elif what == "one_term":
+        a, b = np.zeros((N, H, C), np.float32), r.uniform(1, 2, (N, C, W)).astype(np.float32)
+        a[:, np.arange(H), (np.arange(H) * 7) % C] = r.uniform(1, 2, (N, H))
+    else:
+        draw = r.standard_normal if what == "normal" else lambda s: r.uniform(0.5, 1.0, s)
+        a, b = draw((N, H, C)).astype(np.float32), draw((N, C, W)).astype(np.float32)
+    ref, err = a.astype(np.float64) @ b.astype(np.float64), []
+    ta, tbb, to = ctx.from_numpy(a), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, (N, H, W))
+    for policy in (0, 1):
+        old = ctx.set_kernel_policy(policy)
+        ctx.matmul(ta, tbb, to)
+        ctx.set_kernel_policy(old)
+        st, out = to.download()
+        assert st == tb.Status.OK
+        err.append((np.linalg.norm(out - ref) / np.linalg.norm(ref), np.abs(out / ref - 1).max()))
+    print(what, err)
+    if what in ("cut", "round"):
+        # left out 2^-24; the stage's sum rounded, 2^-24; the sums of one to five stages rounded, a fifth more of 2^-24 each
+        assert err[0][1] <= 5 * 2.0 ** -24
+    elif what == "one_term":
+        # left out 2^-24, rounded once, and what the small products' sum loses
+        assert err[0][1] <= 1.02 * 2.0 ** -23 and err[0][0] <= 1.05 * err[1][0]
+    else:
+        assert err[0][0] <= err[1][0]
+    for t in (ta, tbb, to):
+        t.free()
+
+
 @pytest.mark.parametrize("what", ["special", "tiny_lines", "tiny", "overflow"])
 def test_matmul_f32_split_range(ctx, what):
     """Operands whose parts leave bf16's or the normal range: same classes and the same accuracy as multiply-adds."""
