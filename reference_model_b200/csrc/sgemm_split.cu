@@ -18,11 +18,11 @@
 //               the tensor core's swizzled layouts.  A warp's unit is 64 elements, two neighbours per lane, so that one code
 //               path serves any alignment, a gathered convolution window and both operands without bank conflicts.
 // Taking operands apart inside the kernel instead of in a pass before it keeps the planes out of memory (3.2 GB for 64
-// products of 1024 x 4096 x 1024).  4 x 1024 x 4096 x 1024: 259 us (FFMA kernel 828), 3 800 SM cycles per stage.  What bounds it:
+// products of 1024 x 4096 x 1024).  4 x 1024 x 4096 x 1024: 262 us (FFMA kernel 828), 3 850 SM cycles per stage.  What bounds it:
 // the MMAs alone take 2 680 (24 of ~107 and the hand-over), the loads 3 300 on their own: 64 KB a stage through the ~28 KB of
 // L1 that two 96 KB stages leave.  Three stages of 32 K elements with more L1 lose more to commits and hand-overs (4 500).
 //
-// Values the split cannot carry are computed again with ordinary multiply-adds, 32 rows x 16 columns at a time: results
+// Values the split cannot carry are computed again with ordinary multiply-adds, 32 rows x 32 columns at a time: results
 // that are not finite (an infinite operand has no split: its lower parts are NaN, so it always shows) and rows or columns so
 // small that lower parts or products would leave the normal range (largest magnitude of the row or column below 2^-100, or
 // of both together below 2^-60).
@@ -49,6 +49,7 @@ constexpr int kSplitThreads = 32 * (kFlushWarps + kSplitWarps);
 constexpr int kStagePitch = 17;                   // staged output: 32 rows x 16 columns per warp
 constexpr int kOutOff  = kStages * kStageBytes;
 constexpr int kRowsOff = kOutOff + kFlushWarps * 32 * kStagePitch * 4;    // int2[128]: window origins of a convolution's rows
+constexpr int kAgainSlots = 128;
 constexpr int kMagOff  = kRowsOff + kTile * 8;    // largest magnitudes, for even and odd tiles: rows, column pairs of each warp
 constexpr int kMagWords = kTile + kSplitWarps * (kTile / 2);
 constexpr int kSplitSmem = kMagOff + 2 * kMagWords * 4 + 1024;
@@ -123,50 +124,110 @@ __device__ __forceinline__ void split3(float2 v, uint32_t (&w)[3])
     w[2] = __byte_perm(__float_as_uint(sx), __float_as_uint(sy), 0x7632);    // exact: at most seven bits are left
 }
 
-// Sixteen columns of one row with ordinary multiply-adds, K in order.
+// A result: bias and CLAMP of a convolution.
 template <bool CONV>
-__device__ __noinline__ void plain_row(const SplitParams& p, int batch, int m, int n, float* sum)
+__device__ __forceinline__ float finish(const SplitParams& p, int n, float y)
 {
+    if (CONV)
+    {
+        y = (p.bias_n == 1 ? __ldg(p.bias) : n < p.N ? __ldg(p.bias + n) : 0.f) + y;
+        if (p.has_clamp)
+        {
+            y = (y < p.clamp_lo) ? p.clamp_lo : y;
+            y = (y > p.clamp_hi) ? p.clamp_hi : y;
+        }
+    }
+    return y;
+}
+
+// 32 rows x 32 columns of the output with ordinary multiply-adds, K in order: a lane's row, column by column.  One warp, eight
+// K elements at a time through `st`: A as 32 rows of nine words (no bank conflicts), then B as eight rows of 32.  Per K element
+// a warp reads one word of A and eight broadcast quads of B for its 32 multiply-adds, as the FFMA kernel does.
+// (40 x 256 x 4096 x 256, every block: 2.3 ms, where a row and sixteen columns at a time inside the pipeline took 25.)
+template <bool CONV>
+__device__ __noinline__ void plain_block(const SplitParams& p, int batch, int m0, int n0, float* st)
+{
+    const int lane = threadIdx.x & 31, kq = lane & 7, rq = lane >> 3;
     const float* const A = p.a + batch * p.a_batch;
     const float* const B = p.b + batch * p.b_batch;
-    for (int j = 0; j < 16; j++)
-        sum[j] = 0.f;
-    if (m >= p.M)
-        return;
-    const int2 r = CONV ? window_of(p, m) : make_int2(0, 0);
-    int ic = 0, ky = 0, kx = 0;
-    float v[16];
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-        v[j] = 0.f;
-    for (int k = 0; k < p.K; k++)
+    const int2 r  = !CONV ? make_int2(0, 0) : m0 + lane < p.M ? window_of(p, m0 + lane) : make_int2(0, (int)0x80008000);
+    const bool in = n0 + lane < p.N;
+    int ic = 0, ky = 0, kx = 0;    // CONV: of K element k + kq
+    if (CONV)
     {
-        float x;
-        if (CONV)
+        const int tap = kq / p.IC;
+        ic = kq - tap * p.IC;
+        ky = tap / p.KW;
+        kx = tap - ky * p.KW;
+    }
+    float ra[8], rb[8];
+    auto load = [&](int k) {
+        const int y = ky * p.dy, x = kx * p.dx;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
         {
-            const int y = ky * p.dy, xx = kx * p.dx;
-            x = window_has(p, r, y, xx) ? A[r.x + y * p.in_sh + xx * p.in_sw + ic] : 0.f;
-            if (++ic == p.IC)
+            const int row = rq + 4 * i;
+            if (CONV)
             {
-                ic = 0;
+                const int2 o = make_int2(__shfl_sync(0xffffffffu, r.x, row), __shfl_sync(0xffffffffu, r.y, row));
+                ra[i]        = load1_if(A + (o.x + y * p.in_sh + x * p.in_sw + ic), k + kq < p.K && window_has(p, o, y, x));
+            }
+            else
+                ra[i] = load1_if(A + (int64_t)(m0 + row) * p.K + k + kq, k + kq < p.K && m0 + row < p.M);
+            rb[i] = load1_if(B + (int64_t)(k + i) * p.ldb + n0 + lane, k + i < p.K && in);
+        }
+        if (CONV)
+            for (ic += 8; ic >= p.IC;)
+            {
+                ic -= p.IC;
                 if (++kx == p.KW)
                 {
                     kx = 0;
                     ky++;
                 }
             }
+    };
+    float v[32];
+#pragma unroll
+    for (int j = 0; j < 32; j++)
+        v[j] = 0.f;
+    float* const as = st;
+    float* const bs = st + 32 * 9;
+    load(0);
+    for (int k = 0; k < p.K; k += 8)
+    {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+        {
+            as[(rq + 4 * i) * 9 + kq] = ra[i];
+            bs[i * 32 + lane]         = rb[i];
         }
-        else
-            x = A[(int64_t)m * p.K + k];
-        const float* b = B + (int64_t)k * p.ldb + n;
+        __syncwarp();
+        if (k + 8 < p.K)
+            load(k + 8);
 #pragma unroll
-        for (int j = 0; j < 16; j++)
-            if (n + j < p.N)
-                v[j] = fmaf(x, b[j], v[j]);
+        for (int i = 0; i < 8; i++)
+        {
+            const float x = as[lane * 9 + i];
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+            {
+                const float4 b = *reinterpret_cast<const float4*>(bs + i * 32 + j);
+                v[j]     = fmaf(x, b.x, v[j]);
+                v[j + 1] = fmaf(x, b.y, v[j + 1]);
+                v[j + 2] = fmaf(x, b.z, v[j + 2]);
+                v[j + 3] = fmaf(x, b.w, v[j + 3]);
+            }
+        }
     }
+    __syncwarp();
+    float* const o = p.out + batch * p.o_batch + (int64_t)(m0 + lane) * p.N + n0;
+    if (m0 + lane < p.M)
 #pragma unroll
-    for (int j = 0; j < 16; j++)
-        sum[j] = v[j];
+        for (int j = 0; j < 32; j++)
+            if (n0 + j < p.N)
+                o[j] = finish<CONV>(p, n0 + j, v[j]);
 }
 
 // AVEC, BVEC: pairs of neighbouring elements of A along K (CONV: along the channels), of B along its rows, are aligned to
@@ -177,6 +238,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kStages], bar_acc[kAccs], bar_free[kAccs], bar_done;
     __shared__ uint32_t tmem_base_holder;
+    __shared__ uint32_t again[kAgainSlots];    // blocks of 32 x 32 to be computed again, a bit each, of tiles slot, slot + kAgainSlots, ...
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -184,6 +246,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
     int2* const rows    = reinterpret_cast<int2*>(sm + kRowsOff);
     uint32_t* const mags = reinterpret_cast<uint32_t*>(sm + kMagOff);
 
+    if (tid < kAgainSlots)
+        again[tid] = 0;
     if (tid == 0)
     {
         for (int s = 0; s < kStages; s++)
@@ -358,28 +422,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
                     const bool odd = !isfinite(y[j]) || (rmag != 0.f && cm != 0.f && (rmag < tiny || cm < tiny || rmag * cm < tiny2));
                     flag |= odd ? 1u << j : 0u;
                 }
-                if (__any_sync(0xffffffffu, flag != 0))
-                {
-                    float v[16];
-                    plain_row<CONV>(p, batch, m, n, v);
+                if (__any_sync(0xffffffffu, flag != 0) && lane == 0)
+                    atomicOr(&again[i % kAgainSlots], 1u << (quarter * 4 + half * 2 + (g >> 1)));
 #pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        y[j] = flag >> j & 1 ? v[j] : y[j];
-                    __syncwarp();
-                }
-                if (CONV)
-                {
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                    {
-                        y[j] = (p.bias_n == 1 ? __ldg(p.bias) : n + j < p.N ? __ldg(p.bias + n + j) : 0.f) + y[j];
-                        if (p.has_clamp)
-                        {
-                            y[j] = (y[j] < p.clamp_lo) ? p.clamp_lo : y[j];
-                            y[j] = (y[j] > p.clamp_hi) ? p.clamp_hi : y[j];
-                        }
-                    }
-                }
+                for (int j = 0; j < 16; j++)
+                    y[j] = finish<CONV>(p, n + j, y[j]);
                 float* const o = p.out + batch * p.o_batch + (int64_t)m * p.N + n;
                 if (v8)
                 {
@@ -623,11 +670,28 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
     if (!ok)
         atomicOr(p.status, TB200_DEV_TIMEOUT);
     ptx::tc_fence_before_sync();
-    __syncthreads();
+    const bool all_ok = __syncthreads_and(ok);
     if (warp == kFlushWarps)
     {
         ptx::tc_fence_after_sync();
         ptx::tmem_dealloc(tmem, kTmemCols);
+    }
+    // Results that the split does not carry, by all warps and after the pipeline: inside it the sums of a tile would have to
+    // stay in registers beside those of the block (measured: 9 % of every product), and the other roles would wait as long as
+    // K is deep.  Whole blocks are replaced; of more tiles than slots, those of a slot together.
+    int turn = 0;
+    for (int slot = 0; all_ok && slot < min(mine, kAgainSlots); slot++)
+    {
+        const uint32_t blocks = again[slot];
+        for (int i = slot; blocks != 0 && i < mine; i += kAgainSlots)
+        {
+            const int tile = (int)blockIdx.x + i * (int)gridDim.x;
+            const int batch = tile / per, rem = tile - batch * per, tm = rem / p.tiles_n;
+            for (int b = 0; b < 16; b++)
+                if (blocks >> b & 1 && turn++ % (kFlushWarps + kSplitWarps) == warp)
+                    plain_block<CONV>(p, batch, tm * kTile + (b >> 2) * 32, (rem - tm * p.tiles_n) * kTile + (b & 3) * 32,
+                                      reinterpret_cast<float*>(sm) + warp * 32 * kStagePitch);
+        }
     }
 }
 

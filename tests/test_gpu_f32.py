@@ -209,3 +209,66 @@ def test_conv_f32_split(ctx, case):
     assert st == tb.Status.OK and np.all(np.abs(out - np.clip(ref, -20.0, 30.0)) <= 2.0 ** -22 * bound)
     for t in (tx, tw, tbias, to):
         t.free()
+
+
+def test_split_results_computed_again_in_time(ctx):
+    """Products whose every result is computed again (too small to split, or a NaN per row): no slower than a few times the
+    multiply-adds, and never a time-out, however short the limit of a wait for the pipeline (K = 8192 takes milliseconds)."""
+    N, H, C, W = 20, 200, 8192, 260
+    r = util.rng(81)
+    a, b = (r.standard_normal(s).astype(np.float32) for s in ((N, H, C), (N, C, W)))
+    small_a, small_b = a * np.float32(2.0 ** -70), b * np.float32(2.0 ** -60)
+    nans = a.copy()
+    nans[:, ::32, 4000] = np.nan
+    tensors = {k: ctx.from_numpy(v) for k, v in dict(a=a, b=b, small_a=small_a, small_b=small_b, nans=nans).items()}
+    to = ctx.empty(tb.DType.FP32, (N, H, W))
+    ref = a.astype(np.float64) @ b.astype(np.float64)
+    mag = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
+    try:
+        ctx.set_wait_limit(200000)    # about 0.1 ms; a stage takes some microseconds
+        for x, y, scale in (("a", "b", 1.0), ("small_a", "small_b", 2.0 ** -130), ("nans", "b", 1.0)):
+            ctx.matmul(tensors[x], tensors[y], to)
+            st, out = to.download(check=False)
+            assert st == tb.Status.OK, x
+            if x == "nans":
+                assert np.isnan(out[:, ::32]).all()
+                keep = np.ones(H, bool)
+                keep[::32] = False
+                assert np.all(np.abs(out[:, keep] - ref[:, keep]) <= 2.0 ** -21 * mag[:, keep])
+            else:
+                assert np.all(np.abs(out - scale * ref) <= C * 2.0 ** -24 * scale * mag + C * 2.0 ** -149)
+    finally:
+        ctx.set_wait_limit(4000000000)
+    for t in list(tensors.values()) + [to]:
+        t.free()
+
+
+@pytest.mark.parametrize("conv", [False, True])
+def test_split_bounded_waits_give_up(ctx, conv):
+    """A wait limit below the time of any stage: the kernel reports it (the multiply-add kernel has no waits and could not), ends,
+    and the same call is right afterwards."""
+    r = util.rng(82)
+    if conv:
+        x, w = r.integers(-3, 4, (32, 28, 28, 64)).astype(np.float32), r.integers(-3, 4, (128, 3, 3, 64)).astype(np.float32)
+        xp = np.pad(x, ((0, 0), (1, 1), (1, 1), (0, 0)))
+        exp = sum(xp[:, ky:ky + 28, kx:kx + 28] @ w[:, ky, kx].T for ky in range(3) for kx in range(3))
+        tensors = [ctx.from_numpy(v) for v in (x, w, np.zeros(128, np.float32))] + [ctx.empty(tb.DType.FP32, exp.shape)]
+        call = lambda: ctx.conv2d(*tensors, [1, 1, 1, 1], [1, 1], [1, 1])
+    else:
+        a, b = (r.integers(-3, 4, s).astype(np.float32) for s in ((40, 256, 320), (40, 320, 256)))
+        exp = a @ b
+        tensors = [ctx.from_numpy(v) for v in (a, b)] + [ctx.empty(tb.DType.FP32, exp.shape)]
+        call = lambda: ctx.matmul(*tensors)
+    call()
+    ctx.sync()
+    ctx.set_wait_limit(1)
+    try:
+        call()
+        assert ctx.sync(check=False) == tb.Status.INTERNAL
+    finally:
+        ctx.set_wait_limit(4000000000)
+    call()
+    st, out = tensors[-1].download()
+    assert st == tb.Status.OK and np.array_equal(out, exp)
+    for t in tensors:
+        t.free()
