@@ -18,14 +18,16 @@
 //               the tensor core's swizzled layouts.  A warp's unit is 64 elements, two neighbours per lane, so that one code
 //               path serves any alignment, a gathered convolution window and both operands without bank conflicts.
 // Taking operands apart inside the kernel instead of in a pass before it keeps the planes out of memory (3.2 GB for 64
-// products of 1024 x 4096 x 1024).  4 x 1024 x 4096 x 1024: 262 us (FFMA kernel 828), 3 850 SM cycles per stage.  What bounds it:
+// products of 1024 x 4096 x 1024).  4 x 1024 x 4096 x 1024: 257 us (FFMA kernel 828), 3 800 SM cycles per stage.  What bounds it:
 // the MMAs alone take 2 680 (24 of ~107 and the hand-over), the loads 3 300 on their own: 64 KB a stage through the ~28 KB of
 // L1 that two 96 KB stages leave.  Three stages of 32 K elements with more L1 lose more to commits and hand-overs (4 500).
 //
-// Values the split cannot carry are computed again with ordinary multiply-adds, 32 rows x 32 columns at a time: results
-// that are not finite (an infinite operand has no split: its lower parts are NaN, so it always shows) and rows or columns so
-// small that lower parts or products would leave the normal range (largest magnitude of the row or column below 2^-100, or
-// of both together below 2^-60).
+// Values the split cannot carry are computed again with ordinary multiply-adds:
+//   * results that are not finite (an infinite operand has no split: its lower parts are NaN, so it always shows);
+//   * results so small that what parts and partial products lose below the normal range, 2^-126, could show in them.  A product
+//     loses at most 2^-126 (|a| + |b| + 6), so a sum of K of them is trusted where half its last place is above K times that
+//     for the largest magnitudes of its row and column: |y| >= K 2^-101 (row + column + 8).  Only a tile with a non-zero
+//     operand below 2^-48 can have lost anything: without one all products are above 2^-96.
 #include <algorithm>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -50,8 +52,8 @@ constexpr int kStagePitch = 17;                   // staged output: 32 rows x 16
 constexpr int kOutOff  = kStages * kStageBytes;
 constexpr int kRowsOff = kOutOff + kFlushWarps * 32 * kStagePitch * 4;    // int2[128]: window origins of a convolution's rows
 constexpr int kAgainSlots = 128;
-constexpr int kMagOff  = kRowsOff + kTile * 8;    // largest magnitudes, for even and odd tiles: rows, column pairs of each warp
-constexpr int kMagWords = kTile + kSplitWarps * (kTile / 2);
+constexpr int kMagOff  = kRowsOff + kTile * 8;    // for even and odd tiles: largest magnitudes of rows, of columns by warp, small_key()s
+constexpr int kMinOff  = kTile + kSplitWarps * kTile, kMagWords = kMinOff + kSplitWarps;
 constexpr int kSplitSmem = kMagOff + 2 * kMagWords * 4 + 1024;
 
 struct SplitParams
@@ -123,6 +125,20 @@ __device__ __forceinline__ void split3(float2 v, uint32_t (&w)[3])
     const float sx = rx - __uint_as_float(w[1] << 16), sy = ry - __uint_as_float(w[1] & 0xffff0000u);
     w[2] = __byte_perm(__float_as_uint(sx), __float_as_uint(sy), 0x7632);    // exact: at most seven bits are left
 }
+
+// Largest magnitude; NaN counts for nothing.
+__device__ __forceinline__ float max_abs(float m, float x, float y)
+{
+    asm("max.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(x), "f"(y));
+    return m;
+}
+
+// A value whose magnitude grows as that of x falls; NaN for zero and NaN.  (2^-48: 127 - 48 is its biased exponent.)
+__device__ __forceinline__ float small_key(float x)
+{
+    return __uint_as_float(0x7f800001u - __float_as_uint(x));
+}
+constexpr uint32_t kSmallKey = 0x7f800001u - (79u << 23);
 
 // A result: bias and CLAMP of a convolution.
 template <bool CONV>
@@ -244,7 +260,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
     const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* const sm   = smem_raw + (base - ptx::smem_u32(smem_raw));
     int2* const rows    = reinterpret_cast<int2*>(sm + kRowsOff);
-    uint32_t* const mags = reinterpret_cast<uint32_t*>(sm + kMagOff);
+    float* const mags   = reinterpret_cast<float*>(sm + kMagOff);
 
     if (tid < kAgainSlots)
         again[tid] = 0;
@@ -391,22 +407,41 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
             }
             if (!ok)
                 break;
-            // Magnitudes of this row and of this warp's columns (high halves of fp32 values).  The splitting warps come back to
-            // this half of the table two tiles, at least eight stages, later; they are never more than four stages ahead
-            // (two in shared memory, two in tensor memory).
-            const uint32_t* const mg = mags + (i & 1) * kMagWords;
-            uint32_t pair0 = 0, pair1 = 0;
+            // Magnitudes of this row and of this warp's columns.  The splitting warps come back to this half of the table two
+            // tiles, at least eight stages, later; they are never more than four stages ahead (two in shared memory, two in
+            // tensor memory).
+            const float* const mg = mags + (i & 1) * kMagWords;
+            const int m           = m0 + row;
+            uint32_t odd[2]       = { 0, 0 };    // columns to be computed again
+#pragma unroll
+            for (int j = 0; j < 64; j++)
+                odd[j >> 5] |= isfinite(acc[j]) ? 0u : 1u << (j & 31);
+            float least = 0.f;
 #pragma unroll
             for (int q = 0; q < kSplitWarps; q++)
+                least = fmaxf(least, mg[kMinOff + q]);
+            if (least > __uint_as_float(kSmallKey))
             {
-                pair0 = __vmaxu2(pair0, mg[kTile + q * (kTile / 2) + half * 32 + (lane >> 1)]);
-                pair1 = __vmaxu2(pair1, mg[kTile + q * (kTile / 2) + half * 32 + 16 + (lane >> 1)]);
+                const float rmag = mg[row], lim = (float)p.K * 3.9443045e-31f;    // 2^-101
+                float cmag0 = 0.f, cmag1 = 0.f;                                   // columns lane, 32 + lane
+#pragma unroll
+                for (int q = 0; q < kSplitWarps; q++)
+                {
+                    cmag0 = fmaxf(cmag0, mg[kTile + q * kTile + half * 64 + lane]);
+                    cmag1 = fmaxf(cmag1, mg[kTile + q * kTile + half * 64 + 32 + lane]);
+                }
+#pragma unroll
+                for (int j = 0; j < 64; j++)
+                {
+                    const float cm = __shfl_sync(0xffffffffu, j < 32 ? cmag0 : cmag1, j & 31);
+                    if (rmag != 0.f && cm != 0.f && fabsf(acc[j]) < fmaf(lim, rmag + cm, 8.f * lim))
+                        odd[j >> 5] |= 1u << (j & 31);
+                }
             }
-            const float rmag  = __uint_as_float(mg[row] << 16);
-            const float cmag0 = __uint_as_float(lane & 1 ? pair0 & 0xffff0000u : pair0 << 16);    // column lane
-            const float cmag1 = __uint_as_float(lane & 1 ? pair1 & 0xffff0000u : pair1 << 16);    // column 32 + lane
-            const int m       = m0 + row;
-            const float tiny  = 7.888609e-31f, tiny2 = 8.673617e-19f;    // 2^-100, 2^-60
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                if (n0 + h * 32 < p.N && __any_sync(0xffffffffu, odd[h] != 0) && lane == 0)
+                    atomicOr(&again[i % kAgainSlots], 1u << (quarter * 4 + half * 2 + h));
 #pragma unroll
             for (int g = 0; g < 4; g++)
             {
@@ -414,16 +449,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
                 const int n    = n0 + g * 16;
                 if (n >= p.N)
                     break;
-                uint32_t flag = 0;
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                {
-                    const float cm = __shfl_sync(0xffffffffu, g < 2 ? cmag0 : cmag1, (g & 1) * 16 + j);
-                    const bool odd = !isfinite(y[j]) || (rmag != 0.f && cm != 0.f && (rmag < tiny || cm < tiny || rmag * cm < tiny2));
-                    flag |= odd ? 1u << j : 0u;
-                }
-                if (__any_sync(0xffffffffu, flag != 0) && lane == 0)
-                    atomicOr(&again[i % kAgainSlots], 1u << (quarter * 4 + half * 2 + (g >> 1)));
 #pragma unroll
                 for (int j = 0; j < 16; j++)
                     y[j] = finish<CONV>(p, n + j, y[j]);
@@ -593,15 +618,19 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
             else
                 A += kHalfK;
         };
-        uint32_t mag_a[8], mag_b[2];    // high halves of the magnitudes, two per word
+        float mag_a[8], mag_b[4];    // largest magnitudes: rows, columns of even and odd units
+        float least = 0.f;           // largest small_key() of both operands
+        auto clear = [&]() {
 #pragma unroll
-        for (int i = 0; i < 8; i++)
-            mag_a[i] = 0;
-        mag_b[0] = mag_b[1] = 0;
-        auto put = [&](float2 v, uint32_t dst, uint32_t& mag) {
+            for (int i = 0; i < 8; i++)
+                mag_a[i] = 0.f;
+            mag_b[0] = mag_b[1] = mag_b[2] = mag_b[3] = least = 0.f;
+        };
+        clear();
+        auto put = [&](float2 v, uint32_t dst) {
             uint32_t x[3];
             split3(v, x);
-            mag = __vmaxu2(mag, x[0] & 0x7fff7fffu);
+            least = max_abs(least, small_key(v.x), small_key(v.y));
 #pragma unroll
             for (int q = 0; q < 3; q++)
                 asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (uint32_t)(q * kPlane)), "r"(x[q]) : "memory");
@@ -612,11 +641,18 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
         auto half = [&](float2 (&va)[8], float2 (&vb)[8], uint32_t s) {
 #pragma unroll
             for (int i = 0; i < 8; i++)
-                put(va[i], dst_a + s + (uint32_t)(i * 1024), mag_a[i]);
+            {
+                mag_a[i] = max_abs(mag_a[i], va[i].x, va[i].y);
+                put(va[i], dst_a + s + (uint32_t)(i * 1024));
+            }
             load_a(va);
 #pragma unroll
             for (int i = 0; i < 8; i++)
-                put(vb[i], dst_b + s + (uint32_t)((i & 1) * (kPlane / 2) + (i >> 1) * 1024), mag_b[i & 1]);
+            {
+                mag_b[2 * (i & 1)]     = fmaxf(mag_b[2 * (i & 1)], fabsf(vb[i].x));
+                mag_b[2 * (i & 1) + 1] = fmaxf(mag_b[2 * (i & 1) + 1], fabsf(vb[i].y));
+                put(vb[i], dst_b + s + (uint32_t)((i & 1) * (kPlane / 2) + (i >> 1) * 1024));
+            }
             load_b(vb);
             next_half();
         };
@@ -634,21 +670,25 @@ __global__ void __launch_bounds__(kSplitThreads, 1) sgemm_split_kernel(const __g
             if (--left == 0)
             {
                 // the tile's magnitudes, before its last stage is handed over
-                uint32_t* const mg = mags + (t & 1) * kMagWords;
+                float* const mg = mags + (t & 1) * kMagWords;
 #pragma unroll
                 for (int i = 0; i < 8; i++)
                 {
-                    uint32_t m = max(mag_a[i] & 0xffffu, mag_a[i] >> 16);
+                    float m = mag_a[i];
 #pragma unroll
                     for (int o = 8; o > 0; o >>= 1)
-                        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+                        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
                     if ((lane & 15) == 0)
                         mg[2 * (w + 8 * i) + odd] = m;
-                    mag_a[i] = 0;
                 }
-                mg[kTile + w * (kTile / 2) + lane]      = mag_b[0];
-                mg[kTile + w * (kTile / 2) + lane + 32] = mag_b[1];
-                mag_b[0] = mag_b[1] = 0;
+                // (columns 2 lane, 2 lane + 1 of the even and of the odd units)
+                float* const mc = mg + kTile + w * kTile + 2 * lane;
+                mc[0] = mag_b[0]; mc[1] = mag_b[1]; mc[64] = mag_b[2]; mc[65] = mag_b[3];
+                // (non-negative floats order like their bits)
+                const uint32_t key = __reduce_max_sync(0xffffffffu, __float_as_uint(least));
+                if (lane == 0)
+                    mg[kMinOff + w] = __uint_as_float(key);
+                clear();
                 left = p.nk;
                 t++;
             }

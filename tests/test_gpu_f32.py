@@ -151,6 +151,39 @@ def test_matmul_f32_split_accuracy(ctx, what):
         t.free()
 
 
+@pytest.mark.parametrize("what", ["rows", "columns", "products", "subnormal", "zeros"])
+def test_matmul_f32_split_mixed_magnitudes(ctx, what):
+    """Lines whose large elements meet zeros, so that the small ones, whose lower parts or products leave the normal range, make
+    the sums."""
+    N, H, C, W = 40, 256, 256, 256
+    r = util.rng(79)
+    a, b = (r.uniform(1, 2, s) * r.choice([-1.0, 1.0], s[-1]) for s in ((N, H, C), (N, C, W)))
+    if what == "rows":
+        a, b = a * 2.0 ** -120, b * 2.0 ** 60
+    elif what == "columns":
+        a, b = a * 2.0 ** 60, b * 2.0 ** -120
+    elif what == "products":
+        a, b = a * 2.0 ** -62, b * 2.0 ** -60
+    elif what == "subnormal":
+        a, b = a * 2.0 ** -140, b * 2.0 ** 100
+    else:    # disjoint: exact zeros beside tiny values
+        a[:, :, ::2] *= 2.0 ** -130
+        b[:, ::2], a[:, 5], b[:, :, 7] = 0.0, 0.0, 0.0
+        a[:, 9, 1::2] = 0.0
+    a, b = a.astype(np.float32), b.astype(np.float32)
+    if what != "zeros":
+        a[:, :, 0], b[:, 0] = 1.0, 0.0
+        a[:, :, 1], b[:, 1] = 0.0, 1.0
+    ref = a.astype(np.float64) @ b.astype(np.float64)
+    bound = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
+    ta, tbb, to = ctx.from_numpy(a), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, (N, H, W))
+    ctx.matmul(ta, tbb, to)
+    st, out = to.download()
+    assert st == tb.Status.OK and np.all(np.abs(out - ref) <= C * 2.0 ** -24 * bound + C * 2.0 ** -149)
+    for t in (ta, tbb, to):
+        t.free()
+
+
 @pytest.mark.parametrize("what", ["special", "tiny_lines", "tiny", "overflow"])
 def test_matmul_f32_split_range(ctx, what):
     """Operands whose parts leave bf16's or the normal range: same classes and the same accuracy as multiply-adds."""
