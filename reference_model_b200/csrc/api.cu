@@ -1390,12 +1390,9 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
             if (e)
             {
                 st = cache_use(ctx, e);
-                if (st == TB200_OK && has_rs)
-                    st = read_host_flag(ctx, e, wr_bytes + flag_off);
                 if (st != TB200_OK)
                     return st;
-                block     = e->block;
-                q.lean_ok = has_rs && e->host_flag == 1 ? 1 : 0;
+                block = e->block;
             }
             else
             {
@@ -1417,6 +1414,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                 q.mult_pad    = corr + OCpad;
                 q.shift_pad   = reinterpret_cast<const int8_t*>(q.mult_pad + OCpad);
                 q.rec         = has_rs ? reinterpret_cast<const int32_t*>(tab + rec_off) : nullptr;
+                q.rec_ok      = reinterpret_cast<const int*>(tab + flag_off);
             }
             else
                 q.bias_f_pad = reinterpret_cast<const float*>(tab);

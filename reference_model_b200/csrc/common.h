@@ -315,6 +315,7 @@ struct TcProblem
     const int32_t* mult_pad;     // TC_EPI_RESCALE: multipliers / shifts expanded per column and padded to corr_stride
     const int8_t* shift_pad;
     const int32_t* rec;          // optional: [corr_stride][8] prepared records of the lean RESCALE form (rescale_rec_build)
+    const int* rec_ok;           // gathering kernel, with rec: device word, whether every record is usable
     const int32_t* delta;        // optional, with corr_classes: [classes][corr_stride] class row minus interior row
     int lean_ok;                 // the host knows every column's record is usable: tc_conv_lean_kernel may run
     // tc_conv_lean_kernel only: the batch dimension is (image, parity of the output column): batch index 2 n + p holds

@@ -74,6 +74,7 @@ struct AnyParams
     // epilogue
     const int32_t* corr;    // [N padded] int32 added to every column, or null
     const int32_t* rec;     // lean RESCALE records, or null: multipliers / shifts below
+    const int* rec_ok;      // whether every record is usable, as the kernel that built them left it
     const int32_t* mult;
     const int8_t* shift;
     const float* bias_f;
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(kThreads, EPI == ANY_SUM32 ? 1 : 2) tc_any_ker
     if (tid == 0)
         ptx::dep_launch_trigger();
 
-    bool ok = true;
+    bool ok = true, lean = false;
     constexpr int kSumGroups = EPI == ANY_SUM32 ? 4 : 1;    // sixteen columns each, of up to 128
     float acc[kSumGroups * 16];
 #pragma unroll
@@ -468,6 +469,10 @@ __global__ void __launch_bounds__(kThreads, EPI == ANY_SUM32 ? 1 : 2) tc_any_ker
         const uint8_t* const a = p.a + (int64_t)batch * p.a_batch * p.es;
         const int esl          = p.es - 1;             // log2 of the element size
         ptx::dep_launch_wait();
+        // The verdict is read here and not by the host: no first call waits for it, and a captured graph follows constants that
+        // are replaced under it.
+        if (EPI == ANY_RESCALE && p.rec != nullptr)
+            lean = *p.rec_ok != 0;
 
         int pk = c_lo * 8 + j;                         // this thread's piece of K, its tap and place in the tap's run
         int cp = pk, kx = 0, ky = 0;
@@ -796,7 +801,7 @@ __global__ void __launch_bounds__(kThreads, EPI == ANY_SUM32 ? 1 : 2) tc_any_ker
     }
 
     // ---------------------------------------------------------------------- epilogue (the gathering warps)
-    const int32_t(*const rec)[8] = EPI == ANY_RESCALE && p.rec != nullptr ? reinterpret_cast<const int32_t(*)[8]>(sm + p.rec_off) : nullptr;
+    const int32_t(*const rec)[8] = lean ? reinterpret_cast<const int32_t(*)[8]>(sm + p.rec_off) : nullptr;
     const int groups = p.block_n >> 4;    // sixteen columns each
     const int row_a  = p.splits > 1 ? rank * (kRows / p.splits) : 0;    // rows of the tile this CTA finishes
     const int row_b  = min(rows, p.splits > 1 ? row_a + kRows / p.splits : kRows);
@@ -1230,7 +1235,8 @@ tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q)
         const int interior = q.corr_classes ? (q.KH * (q.KW + 1)) * (q.KW + 1) + q.KW : 0;
         k.corr = q.corr + (int64_t)interior * q.corr_stride;
     }
-    k.rec    = q.epi == TC_EPI_RESCALE && q.lean_ok && q.out_dtype == TB200_INT8 ? q.rec : nullptr;
+    k.rec    = q.epi == TC_EPI_RESCALE && q.out_dtype == TB200_INT8 ? q.rec : nullptr;
+    k.rec_ok = q.rec_ok;
     k.mult   = q.mult_pad;
     k.shift  = q.shift_pad;
     k.bias_f = q.bias_f_pad;

@@ -124,6 +124,47 @@ def test_conv_i8(ctx, case):
             assert kernel == ("conv2d_direct" if tiny else "tc_gemm_any_i8_rescale") and st == tb.Status.OK and np.array_equal(out, exp), (rounding, cache)
 
 
+def test_conv_i8_constants_replaced(ctx):
+    """RESCALE operands replaced by uploads, eagerly and under a captured graph: from provable records to ones that need the
+    general arithmetic and its range check, and back."""
+    r = util.rng(2280)
+    x, w, b = util.conv_int8_case(r, 2, 21, 19, 24, 40, 3, 3, bias_range=1 << 10)
+    args = ([1] * 4, [1, 1], [1, 1], 3, 0)
+    acc = orc.conv2d(x, w, b, *args, nthreads=8)
+    top = int(np.abs(acc).max())
+    bits = top.bit_length()              # every accumulator fits these bits, which the worst case of the layer does not
+    good, tight, low = (util.rescale_params(r, 40), (np.full(40, 1 << 20, np.int32), np.full(40, bits + 1, np.int8)),
+                        (np.full(40, 1 << 20, np.int32), np.full(40, bits - 1, np.int8)))
+    assert (1 << bits) < 24 * 9 * 255 * 128 and top >= 1 << (bits - 2)    # (low: some accumulator is out of the accepted range)
+    tx, tw, tbias, tm, ts = (ctx.from_numpy(v) for v in (x, w, b, *good))
+    to = ctx.empty(tb.DType.INT8, acc.shape)
+    epi = tb.Epilogue(tb.RescaleAttr(tm, ts, 0, 7, True, "DOUBLE_ROUND", per_channel=True), (-100, 120))
+    call = lambda: ctx.conv2d(tx, tw, tbias, to, *args, epi)
+
+    def check(run):
+        for mult, shift in (good, tight, good, low):
+            tm.upload(mult), ts.upload(shift)
+            run()
+            st, out = to.download(check=False)
+            est, exp = orc.rescale(acc, mult, shift, True, True, "DOUBLE_ROUND", 0, 7, 32, 8)
+            if shift is low[1]:
+                assert est != orc.VALID and st == tb.Status.UNPREDICTABLE
+            else:
+                assert est == orc.VALID and st == tb.Status.OK and np.array_equal(out, np.clip(exp, -100, 120))
+
+    check(call)
+    assert ctx.last_kernel() == "tc_gemm_any_i8_rescale"
+    tm.upload(good[0]), ts.upload(good[1])
+    call()
+    ctx.capture_begin()
+    call()
+    graph = ctx.capture_end()
+    check(lambda: ctx.graph_launch(graph))
+    ctx.graph_destroy(graph)
+    for t in (tx, tw, tbias, tm, ts, to):
+        t.free()
+
+
 @pytest.mark.parametrize("dt,name", [(F16, "fp16"), (BF16, "bf16")])
 @pytest.mark.parametrize("case", [(2, 9, 11, 12, 20, 3, 1), (1, 14, 14, 9, 33, 3, 1), (2, 6, 6, 100, 70, 1, 0), (1, 20, 7, 3, 8, 5, 2)])
 def test_conv_float(ctx, dt, name, case):
