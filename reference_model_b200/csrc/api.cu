@@ -2357,14 +2357,19 @@ extern "C" tb200_status tb200_depthwise_conv2d(tb200_ctx* ctx, const tb200_tenso
                                    { reinterpret_cast<const char*>(q.shift), epilogue->rescale.shift->bytes } },
                                  depthwise_slide_pack_bytes(C, q.K),
                                  [=](tb200_ctx* c, void* block) { return depthwise_slide_pack(c, q, block); });
-            if (e)
+            // (operands that an operator writes would have the block packed again before every call: the kernels below read
+            // them as they are)
+            if (e && !e->unstable)
             {
+                // The kernel reads the verdict on the records itself.  The host looks from the second use on, when a layer has
+                // shown that it is used again: those with unusable records are faster below.
                 st = cache_use(ctx, e);
-                if (st == TB200_OK)
+                if (st == TB200_OK && e->used)
                     st = read_host_flag(ctx, e, depthwise_slide_flag_offset(C, q.K));
                 if (st != TB200_OK)
                     return st;
-                if (e->host_flag == 1)
+                e->used = true;
+                if (e->host_flag != 0)
                     return depthwise_slide_launch(ctx, q, e->block, "depthwise_slide_i8");
             }
         }

@@ -57,6 +57,7 @@ struct Prepared
     bool valid    = false;    // the block holds what the operands' current contents give
     bool unstable = false;    // an operator wrote into an operand: rebuild before every use
     int host_flag = -1;       // a verdict the builder left in the block and the host has read back (-1: not read yet)
+    bool used     = false;    // a kernel that reads the verdict itself has run on the block
     uint64_t last_use = 0;
     // enqueues, on the context's stream, the kernels that fill `block` from the operands
     std::function<tb200_status(tb200_ctx*, void* block)> rebuild;
@@ -384,7 +385,7 @@ struct DepthwiseI8Problem
 };
 bool depthwise_slide_supported(const DepthwiseI8Problem& q);
 size_t depthwise_slide_pack_bytes(int C, int K);
-size_t depthwise_slide_flag_offset(int C, int K);    // of the word that says whether every channel's record is usable
+size_t depthwise_slide_flag_offset(int C, int K);    // of the word that says whether every channel's record is usable (the kernel reads it)
 tb200_status depthwise_slide_pack(tb200_ctx* ctx, const DepthwiseI8Problem& q, void* block);
 tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q, const void* block, const char* name);
 

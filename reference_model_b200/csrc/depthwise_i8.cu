@@ -9,7 +9,10 @@
 //   * at stride 1 a 3 x 3 thread makes two output rows: four rows fill the column words, and the second row's weights are
 //     the first's shifted by a byte;
 //   * weights, packed by columns, and the lean RESCALE records (rescale_rec_build) are prepared once per layer and sit in
-//     registers for the whole walk; taps outside the image read the input zero point, so that all pixels share them.
+//     registers for the whole walk; taps outside the image read the input zero point, so that all pixels share them.  Where a
+//     record is not usable a thread makes its outputs one by one with the general arithmetic (beside the walk, which it would
+//     cost 20 registers).  The kernel reads that verdict itself, so no call waits for it and a captured graph follows
+//     constants that are replaced under it.
 // Channel counts that are no multiple of four read each word as two aligned ones.
 // 32 x 56 x 56 x 144, 3 x 3: the sixteen-channels-per-thread kernel with the general RESCALE took 126 us.
 #include <algorithm>
@@ -31,6 +34,13 @@ struct DwSlideParams
     const int4* wcol;        // [K][C4 / 4]: per channel the window column's first four rows, one byte each
     const int4* wrow5;       // [K][C4 / 4]: 5 x 5 only, the fifth row's weight at the channel's own byte
     const int4* rec;         // [C4][2]
+    const int* usable;       // whether every record may be used; else (walk_general):
+    const int8_t* w;         // [K][K][C]
+    const int32_t* corr;     // [C4] bias less the zero point's share
+    const int32_t* mult;
+    const int8_t* shift;
+    int per_channel, out_zp;
+    int* status;
     int N, IH, IW, C, OH, OW, pad_t, pad_l;
     int c4, strips, row_groups, len;    // channel words, pieces of a row, groups of rows, outputs of a piece
     uint32_t fd_c4[2], fd_strips[2], fd_rg[2];
@@ -38,6 +48,33 @@ struct DwSlideParams
     uint32_t fill4;
     int clamp_lo, clamp_hi;
 };
+
+// Outputs [ox0, ox1) x `rows` rows of four channels, tap by tap, by apply_scale_32 with its checks.
+__device__ __noinline__ void walk_general(const DwSlideParams& p, int K, int S, int double_round, int n, int oy, int rows, int c, int ox0, int ox1)
+{
+    const int live = min(4, p.C - c), zp = (int)(int8_t)(p.fill4 & 0xffu);
+    bool bad       = false;
+    for (int y = oy; y < min(p.OH, oy + rows); y++)
+        for (int ox = ox0; ox < ox1; ox++)
+            for (int i = 0; i < live; i++)
+            {
+                int32_t acc = p.corr[c + i];
+                for (int k = 0; k < K * K; k++)
+                {
+                    const int iy = y * S - p.pad_t + k / K, ix = ox * S - p.pad_l + k % K;
+                    const bool inside = (unsigned)iy < (unsigned)p.IH && (unsigned)ix < (unsigned)p.IW;
+                    const int v = inside ? (int)p.in[(((int64_t)n * p.IH + iy) * p.IW + ix) * p.C + c + i] : zp;
+                    acc += v * (int)p.w[k * p.C + c + i];
+                }
+                const int at = p.per_channel ? c + i : 0;
+                int64_t z    = (int64_t)apply_scale_32_dev(acc, p.mult[at], p.shift[at], double_round != 0, bad) + p.out_zp;
+                bad |= z > 2147483647LL || z < -2147483648LL;
+                z = z < p.clamp_lo ? p.clamp_lo : z > p.clamp_hi ? p.clamp_hi : z;
+                p.out[(((int64_t)n * p.OH + y) * p.OW + ox) * p.C + c + i] = (int8_t)z;
+            }
+    if (bad)
+        atomicOr(p.status, TB200_DEV_UNPREDICTABLE);
+}
 
 template <int K, int S, bool ALIGNED, bool FIX>
 __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_constant__ DwSlideParams p)
@@ -53,6 +90,11 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
     const int c  = cw * 4;
     const int ox0 = strip * p.len, ox1 = min(p.OW, ox0 + p.len);
 
+    if (*p.usable == 0)
+    {
+        walk_general(p, K, S, FIX, n, oy, R, c, ox0, ox1);
+        return;
+    }
     int wc[K][4], w5[K == 5 ? K : 1][4];
 #pragma unroll
     for (int k = 0; k < K; k++)
@@ -200,7 +242,8 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
 // Weights [K][K][C] packed by window columns, RESCALE records; one thread per channel (of C rounded up to four).
 __global__ void depthwise_pack_kernel(const int8_t* __restrict__ w, const int32_t* __restrict__ bias, int bias_n, int C, int C4, int K, int32_t in_zp,
                                       const int32_t* __restrict__ mult, const int8_t* __restrict__ shift, int per_channel, int double_round,
-                                      int32_t out_zp, int32_t* __restrict__ wcol, int32_t* __restrict__ wrow5, int32_t* __restrict__ rec, int* all_ok)
+                                      int32_t out_zp, int32_t* __restrict__ wcol, int32_t* __restrict__ wrow5, int32_t* __restrict__ rec,
+                                      int32_t* __restrict__ corr, int* all_ok)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C4)
@@ -230,6 +273,7 @@ __global__ void depthwise_pack_kernel(const int8_t* __restrict__ w, const int32_
         rescale_rec_build(mult[per_channel ? c : 0], (int32_t)shift[per_channel ? c : 0], double_round, out_zp, b - in_zp * sum, vmax, r8);
         if (r8[7] == 0)
             *all_ok = 0;
+        corr[c] = (int32_t)((uint32_t)b - (uint32_t)in_zp * (uint32_t)sum);
     }
     for (int i = 0; i < 8; i++)
         rec[c * 8 + i] = r8[i];
@@ -238,7 +282,7 @@ __global__ void depthwise_pack_kernel(const int8_t* __restrict__ w, const int32_
 size_t pack_words(int C, int K)
 {
     const size_t C4 = (size_t)((C + 3) & ~3);
-    return C4 * (size_t)(K == 5 ? 2 * K : K) + C4 * 8;
+    return C4 * (size_t)(K == 5 ? 2 * K : K) + C4 * 9;    // weights, records, corrections
 }
 
 }    // namespace
@@ -266,10 +310,11 @@ tb200_status depthwise_slide_pack(tb200_ctx* ctx, const DepthwiseI8Problem& q, v
     int32_t* wcol = reinterpret_cast<int32_t*>(block);
     int32_t* five = wcol + C4 * q.K;
     int32_t* rec  = five + (q.K == 5 ? C4 * q.K : 0);
-    int* flag     = reinterpret_cast<int*>(rec + C4 * 8);
+    int32_t* corr = rec + C4 * 8;
+    int* flag     = reinterpret_cast<int*>(corr + C4);
     TB200_CUDA_CHECK(ctx, cudaMemsetAsync(flag, 1, sizeof(int), ctx->stream));
     depthwise_pack_kernel<<<(C4 + 127) / 128, 128, 0, ctx->stream>>>(q.w, q.bias, q.bias_n, q.C, C4, q.K, q.in_zp, q.mult, q.shift, q.per_channel,
-                                                                    q.double_round, q.out_zp, wcol, five, rec, flag);
+                                                                    q.double_round, q.out_zp, wcol, five, rec, corr, flag);
     return post_launch(ctx, "depthwise_pack");
 }
 
@@ -284,12 +329,15 @@ tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q,
     p.wcol   = reinterpret_cast<const int4*>(block);
     p.wrow5  = p.wcol + C4 / 4 * q.K;
     p.rec    = p.wrow5 + (q.K == 5 ? C4 / 4 * q.K : 0);
+    p.corr   = reinterpret_cast<const int32_t*>(p.rec + C4 * 2);
+    p.usable = reinterpret_cast<const int*>(p.corr + C4);
+    p.w = q.w; p.mult = q.mult; p.shift = q.shift; p.per_channel = q.per_channel; p.out_zp = q.out_zp; p.status = ctx->d_status;
     p.N = q.N; p.IH = q.IH; p.IW = q.IW; p.C = q.C; p.OH = q.OH; p.OW = q.OW; p.pad_t = q.pad_t; p.pad_l = q.pad_l;
     p.c4         = C4 / 4;
     const int R  = q.K == 3 && q.S == 1 ? 2 : 1;
     p.row_groups = (q.OH + R - 1) / R;
     // A piece's first K - S columns are fetched again by its neighbour: long pieces waste less, short ones make more
-    // threads.  The longest that still gives every SM two blocks of 256 threads' worth of work, at most 28.
+    // threads.  The longest that still makes 1 024 threads per SM (in blocks of 128), at most 28.
     const int64_t lines = (int64_t)q.N * p.row_groups * p.c4;
     const int64_t want  = (int64_t)ctx->num_sms * 1024;
     int strips = (int)std::min<int64_t>(std::max<int64_t>((want + lines - 1) / lines, (q.OW + 27) / 28), std::max(1, q.OW / 2));

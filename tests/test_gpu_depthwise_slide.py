@@ -67,3 +67,78 @@ def test_depthwise_slide(ctx, case):
         assert ctx.sync(check=False) == tb.Status.UNPREDICTABLE
     for t in (tx, tw, tbias, tm, ts, to):
         t.free()
+
+
+@pytest.mark.parametrize("C,K,stride", [(24, 3, 1), (21, 5, 2), (33, 3, 2)])
+def test_general_arithmetic_and_captured_graph(ctx, C, K, stride):
+    """Constants whose records are not usable from the first call on (the kernel's general arithmetic), and constants replaced
+    under a captured graph: usable, not usable, usable, out of the accepted range."""
+    r = util.rng(1950 + C)
+    p = K // 2
+    pad, IH, IW = [p, p, p, p], 31, 33
+    OH, OW = orc.conv_out_hw(IH, IW, K, K, pad, [stride] * 2, [1, 1])
+    N = -(-(1 << 20) // (OH * OW * C * K * K))
+    x = r.integers(-128, 128, size=(N, IH, IW, C), dtype=np.int8)
+    w = r.integers(-128, 128, size=(K, K, C, 1), dtype=np.int8)
+    b = r.integers(-1000, 1000, size=C).astype(np.int32)
+    acc = orc.depthwise_conv2d(x, w, b, pad, [stride] * 2, [1, 1], 9, 0, nthreads=8)
+    bits = int(np.abs(acc).max()).bit_length()
+    assert (1 << (bits - 1)) < K * K * 255 * 128 and np.abs(acc).max() >= 1 << (bits - 2)
+    good = util.rescale_params(r, C)
+    tight, low = ((np.full(C, 1 << 20, np.int32), np.full(C, bits + d, np.int8)) for d in (1, -1))
+    tx, tw, tbias, tm, ts = (ctx.from_numpy(v) for v in (x, w, b, *tight))
+    to = ctx.empty(tb.DType.INT8, acc.shape)
+    epi = tb.Epilogue(tb.RescaleAttr(tm, ts, 0, -5, True, "DOUBLE_ROUND", per_channel=True), (-128, 100))
+    call = lambda: ctx.depthwise_conv2d(tx, tw, tbias, to, pad, [stride] * 2, [1, 1], 9, 0, epi)
+
+    def check(params):
+        st, out = to.download(check=False)
+        est, exp = orc.rescale(acc, *params, True, True, "DOUBLE_ROUND", 0, -5, 32, 8)
+        assert est == orc.VALID and st == tb.Status.OK and np.array_equal(out, np.clip(exp, -128, 100))
+
+    call()
+    assert ctx.last_kernel() == "depthwise_slide_i8"
+    check(tight)
+    tm.upload(good[0]), ts.upload(good[1])
+    call()
+    check(good)
+    ctx.capture_begin()
+    call()
+    graph = ctx.capture_end()
+    for params in (good, tight, good):
+        tm.upload(params[0]), ts.upload(params[1])
+        ctx.graph_launch(graph)
+        check(params)
+    tm.upload(low[0]), ts.upload(low[1])
+    ctx.graph_launch(graph)
+    assert ctx.sync(check=False) == tb.Status.UNPREDICTABLE
+    ctx.graph_destroy(graph)
+    for t in (tx, tw, tbias, tm, ts, to):
+        t.free()
+
+
+def test_weights_that_an_operator_writes(ctx):
+    """Such weights are read where they are: no packing before every call, and never a packed copy that has gone stale."""
+    r = util.rng(1990)
+    N, C, K = 3, 24, 3
+    x = r.integers(-128, 128, size=(N, 57, 57, C), dtype=np.int8)
+    w32 = r.integers(-100, 100, size=(K, K, C, 1)).astype(np.int32)
+    mult, shift = util.rescale_params(r, C)
+    tx, tw32, tw, tbias, tm, ts = (ctx.from_numpy(v) for v in (x, w32, w32.astype(np.int8), np.zeros(C, np.int32), mult, shift))
+    one, two = ctx.from_numpy(np.full(1, 1 << 30, np.int32)), ctx.from_numpy(np.full(1, 30, np.int8))
+    to = ctx.empty(tb.DType.INT8, x.shape)
+    epi = tb.Epilogue(tb.RescaleAttr(tm, ts, 0, 0, True, "DOUBLE_ROUND", per_channel=True), (-128, 127))
+    for rep in range(3):
+        if rep:
+            w32 = r.integers(-100, 100, size=w32.shape).astype(np.int32)
+            tw32.upload(w32)
+            ctx.rescale(tw32, tb.RescaleAttr(one, two, 0, 0, True, "SINGLE_ROUND"), tw)
+        launches = ctx.launch_count()
+        ctx.depthwise_conv2d(tx, tw, tbias, to, [1] * 4, [1, 1], [1, 1], 0, 0, epi)
+        assert rep == 0 or ctx.launch_count() == launches + 1
+        acc = orc.depthwise_conv2d(x, w32.astype(np.int8), np.zeros(C, np.int32), [1] * 4, [1, 1], [1, 1], 0, 0, nthreads=8)
+        est, exp = orc.rescale(acc, mult, shift, True, True, "DOUBLE_ROUND", 0, 0, 32, 8)
+        st, out = to.download()
+        assert est == orc.VALID and st == tb.Status.OK and np.array_equal(out, exp)
+    for t in (tx, tw32, tw, tbias, tm, ts, one, two, to):
+        t.free()
