@@ -1423,8 +1423,9 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
     }
 
     // ---- fp32: tiled FFMA kernel (sgemm_f32.cu).  Its row table packs window origins into 16 bits and input offsets into 32.
-    // Padding is a zero-filled tap, which equals the reference's skipped tap only for finite weights: a padded layer whose
-    // weights are not known to be finite takes the kernel below.
+    // Padding is a zero-filled tap, which equals the reference's skipped tap only for finite weights.  The kernels mend the NaNs
+    // that other weights leave, one by one; a padded layer that is used again has its weights' verdict read by the host, and
+    // takes the kernel below, which skips taps, if they are not all finite.
     // Sums of at most 20 products, up to 6 M of them in all, stay with one thread per output (5x109x33x16 1x1 16 channels: 9.3
     // against 11.5 us; at 8x56x56x64 3x3 64 channels it is 60 times slower).
     const bool shallow = KH * KW * IC <= 20 && (int64_t)N * OH * OW * OC * KH * KW * IC <= 6000000;
@@ -1453,11 +1454,12 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
         if (e)
         {
             st = cache_use(ctx, e);
-            if (st == TB200_OK && padded)
+            if (st == TB200_OK && padded && e->used)
                 st = read_host_flag(ctx, e, flag_off);
             if (st != TB200_OK)
                 return st;
-            if (!padded || e->host_flag == 1)
+            e->used = true;
+            if (!padded || e->host_flag != 0)
                 block = e->block;
         }
         else if (!padded)
@@ -1478,6 +1480,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
             q.bias_n = bias->shape[0];
             q.pad_t = pad[0]; q.pad_l = pad[2]; q.sy = stride[0]; q.sx = stride[1]; q.dy = dilation[0]; q.dx = dilation[1];
             q.in_sn = input->stride[0]; q.in_sh = input->stride[1]; q.in_sw = input->stride[2];
+            q.padded    = padded;
             q.has_clamp = epi.has_clamp; q.clamp_lo = epi.clamp_lo_f; q.clamp_hi = epi.clamp_hi_f;
             return conv_f32_launch(ctx, q);
         }

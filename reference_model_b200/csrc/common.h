@@ -403,6 +403,7 @@ struct ConvF32Problem
     int N, IH, IW, IC, OH, OW, OC, KH, KW, bias_n;
     int pad_t, pad_l, sy, sx, dy, dx;
     int64_t in_sn, in_sh, in_sw;
+    int padded;    // some window may leave the image
     int has_clamp;
     float clamp_lo, clamp_hi;
 };

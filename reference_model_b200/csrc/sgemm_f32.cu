@@ -39,13 +39,37 @@ struct SgemmParams
     int tiles_m, tiles_n;
     int k_per_split;         // K range of one CTA of a cluster, a multiple of BK
     // CONV2D: A is gathered from an NHWC input
-    int IH, IW, IC, OH, OW, KW, pad_t, pad_l, sy, sx, dy, dx;
+    int IH, IW, IC, OH, OW, KH, KW, pad_t, pad_l, sy, sx, dy, dx;
     int in_sn, in_sh, in_sw;
+    int padded;              // some window may leave the image
     const float* bias;
     int bias_n;              // CONV2D bias length (OC or 1), 0 = none
     int has_clamp;
     float clamp_lo, clamp_hi;
 };
+
+// A tap outside the image is a zero that is multiplied like any other, where the reference skips it
+// (reference_model/src/ops/tensor_ops.cpp:828-873).  They differ where a weight is infinite or NaN: zero times it is NaN, and
+// only then.  A NaN of a window that leaves the image is summed again here, over the taps inside.
+__device__ __noinline__ float sum_inside(const SgemmParams& p, int m, int n)
+{
+    const int ox = m % p.OW, q = m / p.OW, oy = q % p.OH;
+    const int y0 = oy * p.sy - p.pad_t, x0 = ox * p.sx - p.pad_l;
+    if (y0 >= 0 && x0 >= 0 && y0 + (p.KH - 1) * p.dy < p.IH && x0 + (p.KW - 1) * p.dx < p.IW)
+        return __uint_as_float(0x7fffffffu);    // every tap is inside: the NaN stands
+    const float* const in = p.a + (int64_t)(q / p.OH) * p.in_sn;
+    float sum = 0.f;
+    for (int ky = 0; ky < p.KH; ky++)
+        for (int kx = 0; kx < p.KW; kx++)
+        {
+            const int y = y0 + ky * p.dy, x = x0 + kx * p.dx;
+            if ((unsigned)y >= (unsigned)p.IH || (unsigned)x >= (unsigned)p.IW)
+                continue;
+            for (int c = 0; c < p.IC; c++)
+                sum = fmaf(in[(int64_t)y * p.in_sh + (int64_t)x * p.in_sw + c], p.b[((int64_t)(ky * p.KW + kx) * p.IC + c) * p.ldb + n], sum);
+        }
+    return sum;
+}
 
 // asynchronous copy of RUN floats, or zero fill
 template <int RUN>
@@ -257,6 +281,16 @@ __global__ void __launch_bounds__(SgemmShape<BM, BN, TM, TN, ST>::kThreads, OCC)
         if (m >= p.M || n >= p.N)
             return;
         float f[4] = { v.x, v.y, v.z, v.w };
+        if (CONV && p.padded && (isnan(v.x) || isnan(v.y) || isnan(v.z) || isnan(v.w)))
+            for (int j = 0; j < 4; j++)
+            {
+                const float x = j == 0 ? f[0] : j == 1 ? f[1] : j == 2 ? f[2] : f[3];
+                if (isnan(x) && n + j < p.N)
+                {
+                    const float s = sum_inside(p, m, n + j);
+                    f[0] = j == 0 ? s : f[0]; f[1] = j == 1 ? s : f[1]; f[2] = j == 2 ? s : f[2]; f[3] = j == 3 ? s : f[3];
+                }
+            }
         if (CONV)
         {
 #pragma unroll
@@ -419,7 +453,7 @@ tb200_status launch_any(tb200_ctx* ctx, SgemmParams p, int batches, const SgemmP
 }
 
 // CONV2D weights [OC][K] -> [K][ldb] (ldb = OC rounded up to four; the pad columns are zero), and whether they are all
-// finite: a zero-filled tap outside the image would turn an infinite weight into NaN, where the reference skips the tap.
+// finite (see sum_inside(): layers whose weights are not are faster on a kernel that skips taps in the first place).
 __global__ void transpose_weights_f32_kernel(const float* __restrict__ w, float* __restrict__ wt, int OC, int K, int ldb, int* all_finite)
 {
     __shared__ float t[32][33];
@@ -480,7 +514,7 @@ tb200_status conv_f32_launch(tb200_ctx* ctx, const ConvF32Problem& q)
     memset(&p, 0, sizeof(p));
     p.a = q.in; p.b = q.wt; p.out = q.out;
     p.M = q.N * q.OH * q.OW; p.N = q.OC; p.K = q.KH * q.KW * q.IC; p.ldb = conv_f32_ldb(q.OC);
-    p.IH = q.IH; p.IW = q.IW; p.IC = q.IC; p.OH = q.OH; p.OW = q.OW; p.KW = q.KW;
+    p.IH = q.IH; p.IW = q.IW; p.IC = q.IC; p.OH = q.OH; p.OW = q.OW; p.KH = q.KH; p.KW = q.KW; p.padded = q.padded;
     p.pad_t = q.pad_t; p.pad_l = q.pad_l; p.sy = q.sy; p.sx = q.sx; p.dy = q.dy; p.dx = q.dx;
     p.in_sn = (int)q.in_sn; p.in_sh = (int)q.in_sh; p.in_sw = (int)q.in_sw;
     p.bias = q.bias; p.bias_n = q.bias_n;

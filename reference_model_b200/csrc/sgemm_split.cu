@@ -158,7 +158,8 @@ __device__ __forceinline__ float finish(const SplitParams& p, int n, float y)
 
 // 32 rows x 32 columns of the output with ordinary multiply-adds, K in order: a lane's row, column by column.  One warp, eight
 // K elements at a time through `st`: A as 32 rows of nine words (no bank conflicts), then B as eight rows of 32.  Per K element
-// a warp reads one word of A and eight broadcast quads of B for its 32 multiply-adds, as the FFMA kernel does.
+// a warp reads one word of A and eight broadcast quads of B for its 32 multiply-adds, as the FFMA kernel does.  Taps outside
+// the image are skipped, whatever their weight.
 // (40 x 256 x 4096 x 256, every block: 2.3 ms, where a row and sixteen columns at a time inside the pipeline took 25.)
 template <bool CONV>
 __device__ __noinline__ void plain_block(const SplitParams& p, int batch, int m0, int n0, float* st)
@@ -177,8 +178,10 @@ __device__ __noinline__ void plain_block(const SplitParams& p, int batch, int m0
         kx = tap - ky * p.KW;
     }
     float ra[8], rb[8];
+    uint32_t taps = 0, next_taps = 0;    // CONV: which of the piece's K elements lie inside the image, for this lane's row
     auto load = [&](int k) {
         const int y = ky * p.dy, x = kx * p.dx;
+        next_taps   = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++)
         {
@@ -186,7 +189,12 @@ __device__ __noinline__ void plain_block(const SplitParams& p, int batch, int m0
             if (CONV)
             {
                 const int2 o = make_int2(__shfl_sync(0xffffffffu, r.x, row), __shfl_sync(0xffffffffu, r.y, row));
-                ra[i]        = load1_if(A + (o.x + y * p.in_sh + x * p.in_sw + ic), k + kq < p.K && window_has(p, o, y, x));
+                const bool inside = k + kq < p.K && window_has(p, o, y, x);
+                ra[i]             = load1_if(A + (o.x + y * p.in_sh + x * p.in_sw + ic), inside);
+                // (lanes 8 rq + kq: byte rq of the ballot belongs to row rq + 4 i)
+                const uint32_t all = __ballot_sync(0xffffffffu, inside);
+                if (lane >> 2 == i)
+                    next_taps = all >> (8 * (lane & 3)) & 0xffu;
             }
             else
                 ra[i] = load1_if(A + (int64_t)(m0 + row) * p.K + k + kq, k + kq < p.K && m0 + row < p.M);
@@ -220,12 +228,15 @@ __device__ __noinline__ void plain_block(const SplitParams& p, int batch, int m0
             bs[i * 32 + lane]         = rb[i];
         }
         __syncwarp();
+        taps = next_taps;
         if (k + 8 < p.K)
             load(k + 8);
 #pragma unroll
         for (int i = 0; i < 8; i++)
         {
             const float x = as[lane * 9 + i];
+            if (CONV && !(taps >> i & 1))
+                continue;
 #pragma unroll
             for (int j = 0; j < 32; j += 4)
             {

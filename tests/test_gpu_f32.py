@@ -305,3 +305,46 @@ def test_split_bounded_waits_give_up(ctx, conv):
     assert st == tb.Status.OK and np.array_equal(out, exp)
     for t in tensors:
         t.free()
+
+
+@pytest.mark.parametrize("case", [(2, 9, 11, 8, 5), (2, 9, 11, 7, 6), (1, 20, 20, 300, 40), (32, 28, 28, 64, 128), (32, 28, 27, 33, 127)])
+def test_conv_f32_nonfinite_weights_under_padding(ctx, case):
+    """Infinite and NaN weights of a padded layer, from the first call on (no verdict is known to the host yet) and through an
+    upload under a captured graph: they reach only the pixels whose windows hold them.  The last two run on the tensor
+    cores, the third splits K over a cluster."""
+    N, IH, IW, IC, OC = case
+    r = util.rng(1030 + IC)
+    x, w = r.standard_normal((N, IH, IW, IC)).astype(np.float32), r.standard_normal((OC, 3, 3, IC)).astype(np.float32)
+    b = r.standard_normal(OC).astype(np.float32)
+    finite = w.copy()
+    w[0, 0, 0, 1], w[2, 2, 1, 0], w[OC - 1, 1, 2, IC - 1] = np.inf, np.nan, -np.inf
+    x[0, 4, 5, 2] = np.inf
+    args = ([1] * 4, [1, 1], [1, 1])
+    ref, bnd = (orc.conv2d(x, w, b, *args, mode="f64", bounds=f, nthreads=8) for f in (False, True))
+    ksb = orc.dot_product_ksb(9 * IC + 1, "fp32", "fp32")
+    tx, tbias, to = ctx.from_numpy(x), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, ref.shape)
+
+    def check():
+        st, out = to.download()
+        assert st == tb.Status.OK
+        assert np.array_equal(np.isnan(out), np.isnan(ref)) and np.array_equal(np.isinf(out), np.isinf(ref))
+        fin = np.isfinite(ref)
+        assert fin[..., [0, 2, OC - 1]].any()
+        ok, info = orc.verify_dot_product(out[fin], ref[fin], bnd[fin], ksb, out="fp32")
+        assert ok, info
+
+    tw = ctx.from_numpy(w)
+    ctx.conv2d(tx, tw, tbias, to, *args)
+    assert ctx.last_kernel() == "conv_f32"
+    check()
+    tw2 = ctx.from_numpy(finite)
+    ctx.conv2d(tx, tw2, tbias, to, *args)
+    ctx.capture_begin()
+    ctx.conv2d(tx, tw2, tbias, to, *args)
+    graph = ctx.capture_end()
+    tw2.upload(w)
+    ctx.graph_launch(graph)
+    check()
+    ctx.graph_destroy(graph)
+    for t in (tx, tw, tw2, tbias, to):
+        t.free()
