@@ -52,6 +52,13 @@ tb200_status ensure_scratch(tb200_ctx* ctx, size_t bytes)
     return TB200_OK;
 }
 
+// Whether ensure_scratch(bytes) can succeed as far as capturing goes: a path that only makes a call faster is left for one that
+// needs no scratch where it cannot.
+static bool scratch_ready(const tb200_ctx* ctx, size_t bytes)
+{
+    return !ctx->capturing || bytes <= ctx->scratch_bytes;
+}
+
 tb200_status post_launch(tb200_ctx* ctx, const char* kernel_name, int n_launches)
 {
     ctx->launches += (uint64_t)n_launches;
@@ -1386,39 +1393,42 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     e = cache_insert(ctx, key, std::move(ops), wr_bytes + tab_bytes, build);
                 }
             }
-            void* block = nullptr;
-            if (e)
+            if (e || scratch_ready(ctx, wr_bytes + tab_bytes))
             {
-                st = cache_use(ctx, e);
-                if (st != TB200_OK)
-                    return st;
-                block = e->block;
+                void* block = nullptr;
+                if (e)
+                {
+                    st = cache_use(ctx, e);
+                    if (st != TB200_OK)
+                        return st;
+                    block = e->block;
+                }
+                else
+                {
+                    st = ensure_scratch(ctx, wr_bytes + tab_bytes);
+                    if (st == TB200_OK)
+                        st = build(ctx, ctx->scratch);
+                    if (st != TB200_OK)
+                        return st;
+                    block = ctx->scratch;
+                }
+                uint8_t* tab = reinterpret_cast<uint8_t*>(block) + wr_bytes;
+                if (repack)
+                    q.b = block;
+                if (int_path)
+                {
+                    int32_t* corr = reinterpret_cast<int32_t*>(tab) + prefix_elems;
+                    q.corr        = corr;
+                    q.corr_stride = OCpad;
+                    q.mult_pad    = corr + OCpad;
+                    q.shift_pad   = reinterpret_cast<const int8_t*>(q.mult_pad + OCpad);
+                    q.rec         = has_rs ? reinterpret_cast<const int32_t*>(tab + rec_off) : nullptr;
+                    q.rec_ok      = reinterpret_cast<const int*>(tab + flag_off);
+                }
+                else
+                    q.bias_f_pad = reinterpret_cast<const float*>(tab);
+                return tc_any_launch(ctx, q);
             }
-            else
-            {
-                st = ensure_scratch(ctx, wr_bytes + tab_bytes);
-                if (st == TB200_OK)
-                    st = build(ctx, ctx->scratch);
-                if (st != TB200_OK)
-                    return st;
-                block = ctx->scratch;
-            }
-            uint8_t* tab = reinterpret_cast<uint8_t*>(block) + wr_bytes;
-            if (repack)
-                q.b = block;
-            if (int_path)
-            {
-                int32_t* corr = reinterpret_cast<int32_t*>(tab) + prefix_elems;
-                q.corr        = corr;
-                q.corr_stride = OCpad;
-                q.mult_pad    = corr + OCpad;
-                q.shift_pad   = reinterpret_cast<const int8_t*>(q.mult_pad + OCpad);
-                q.rec         = has_rs ? reinterpret_cast<const int32_t*>(tab + rec_off) : nullptr;
-                q.rec_ok      = reinterpret_cast<const int*>(tab + flag_off);
-            }
-            else
-                q.bias_f_pad = reinterpret_cast<const float*>(tab);
-            return tc_any_launch(ctx, q);
         }
     }
 
@@ -1462,7 +1472,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
             if (!padded || e->host_flag != 0)
                 block = e->block;
         }
-        else if (!padded)
+        else if (!padded && scratch_ready(ctx, flag_off + 64))
         {
             st = ensure_scratch(ctx, flag_off + 64);
             if (st == TB200_OK)

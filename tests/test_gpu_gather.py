@@ -274,3 +274,37 @@ def test_two_streams_share_the_chip():
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("kind", ["i8", "i8 rescale", "f16", "f32"])
+def test_capture_before_any_eager_call(kind):
+    """A convolution whose tables are neither built nor have room while capturing is captured all the same, on a kernel that needs
+    none."""
+    r = util.rng(2700)
+    N, H, IC, OC = 2, 14, 100, 70
+    with tb.Context(0) as c:
+        if kind[0] == "i":
+            x, w, b = util.conv_int8_case(r, N, H, H, IC, OC, 1, 1)
+            exp = orc.conv2d(x, w, b, [0] * 4, [1, 1], [1, 1], 5, 0, nthreads=8)
+        else:
+            x, w, b = (r.integers(-3, 4, s).astype(np.float32) for s in ((N, H, H, IC), (OC, 1, 1, IC), (OC,)))
+            exp = x @ w[:, 0, 0].T + b    # small whole numbers: exact
+            if kind == "f16":
+                x, w, b, exp = (v.astype(np.float16) for v in (x, w, b, exp))
+        tensors = [c.from_numpy(v) for v in (x, w, b)]
+        epi = None
+        if kind == "i8 rescale":
+            mult, shift = util.rescale_params(r, OC)
+            tensors += [c.from_numpy(mult), c.from_numpy(shift)]
+            epi = tb.Epilogue(tb.RescaleAttr(*tensors[3:], 0, 3, True, "DOUBLE_ROUND", per_channel=True), (-128, 127))
+            exp = np.clip(orc.rescale(exp, mult, shift, True, True, "DOUBLE_ROUND", 0, 3, 32, 8)[1], -128, 127)
+        to = c.empty({"i8": tb.DType.INT32, "i8 rescale": tb.DType.INT8, "f16": F16, "f32": F32}[kind], exp.shape)
+        c.capture_begin()
+        c.conv2d(*tensors[:3], to, [0] * 4, [1, 1], [1, 1], 5 if kind[0] == "i" else 0, 0, epi)
+        graph = c.capture_end()
+        c.graph_launch(graph)
+        st, out = to.download()
+        assert st == tb.Status.OK and np.array_equal(out, exp)
+        c.graph_destroy(graph)
+        for t in tensors + [to]:
+            t.free()
