@@ -1432,7 +1432,8 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
         }
     }
 
-    // ---- fp32: tiled FFMA kernel (sgemm_f32.cu).  Its row table packs window origins into 16 bits and input offsets into 32.
+    // ---- fp32: tiled FFMA kernel (sgemm_f32.cu).  Its row table packs window origins into 16 bits and input offsets into 32,
+    // and row numbers, past the end of the last tile too, are 32 bits.
     // Padding is a zero-filled tap, which equals the reference's skipped tap only for finite weights.  The kernels mend the NaNs
     // that other weights leave, one by one; a padded layer that is used again has its weights' verdict read by the host, and
     // takes the kernel below, which skips taps, if they are not all finite.
@@ -1440,7 +1441,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
     // against 11.5 us; at 8x56x56x64 3x3 64 channels it is 60 times slower).
     const bool shallow = KH * KW * IC <= 20 && (int64_t)N * OH * OW * OC * KH * KW * IC <= 6000000;
     if (input->dtype == TB200_FP32 && ctx->policy == 0 && !shallow && input->stride[3] == 1 && IH + pad[0] + pad[1] < 32768 &&
-        IW + pad[2] + pad[3] < 32768 && (int64_t)N * input->stride[0] < (1LL << 31))
+        IW + pad[2] + pad[3] < 32768 && (int64_t)N * input->stride[0] < (1LL << 31) && (int64_t)N * OH * OW < (1LL << 31) - 256)
     {
         const int K             = KH * KW * IC;
         const size_t flag_off   = (size_t)K * conv_f32_ldb(OC) * sizeof(float);

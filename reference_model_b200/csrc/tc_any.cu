@@ -1049,7 +1049,10 @@ bool any_layout(const TcProblem& q, int max_smem, int block_n, int splits, AnyPl
     k.es        = (int)dtype_size(q.in_dtype);
     k.conv      = matmul ? 0 : 1;
     k.run_bytes = q.IC * k.es;
-    k.M         = matmul ? q.OW : q.N * q.OH * q.OW;
+    const int64_t rows = matmul ? (int64_t)q.OW : (int64_t)q.N * q.OH * q.OW;
+    if (rows > 0x7fffffff - 2 * kRows)
+        return false;    // row numbers, past the end of the last tile too, are 32 bits
+    k.M         = (int)rows;
     k.N         = q.OC;
     const int64_t sw = matmul || !q.a_stride_w ? q.IC : q.a_stride_w, sh = matmul ? 0 : q.a_stride_h ? q.a_stride_h : sw * q.IW,
                   sn = matmul ? 0 : q.a_stride_n ? q.a_stride_n : sh * q.IH;

@@ -308,3 +308,23 @@ def test_capture_before_any_eager_call(kind):
         c.graph_destroy(graph)
         for t in tensors + [to]:
             t.free()
+
+
+def test_as_many_pixels_as_a_tensor_holds(ctx):
+    """2^31 - 8 output pixels: the last tile's rows would not have 32-bit numbers, another kernel takes the call."""
+    n = (1 << 31) - 8
+    x = np.frombuffer(util.rng(2800).bytes(n), np.int8).reshape(1, 1, n, 1)
+    w, b = np.array([77], np.int8).reshape(1, 1, 1, 1), np.array([-1234], np.int32)
+    mult, shift = np.array([1 << 30], np.int32), np.array([37], np.int8)
+    every = np.arange(256, dtype=np.uint8).view(np.int8)    # the result depends on the byte alone
+    lut = orc.rescale(every.astype(np.int32) * 77 - 1234, mult, shift, False, True, "SINGLE_ROUND", 0, 2, 32, 8)[1].astype(np.int8)
+    tensors = [ctx.from_numpy(v) for v in (x, w, b, mult, shift)]
+    to = ctx.empty(tb.DType.INT8, x.shape)
+    ctx.conv2d(*tensors[:3], to, [0] * 4, [1, 1], [1, 1], 0, 0, tb.Epilogue(tb.RescaleAttr(*tensors[3:], 0, 2, True, "SINGLE_ROUND"), None))
+    st, out = to.download()
+    assert st == tb.Status.OK
+    x, out = x.reshape(-1).view(np.uint8), out.reshape(-1)
+    for at in range(0, n, 1 << 27):
+        assert np.array_equal(out[at:at + (1 << 27)], lut[x[at:at + (1 << 27)]])
+    for t in tensors + [to]:
+        t.free()
