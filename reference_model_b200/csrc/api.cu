@@ -1302,10 +1302,17 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
         }
     }
 
-    // ---- channel runs that are no multiple of 32 bytes: gathering tensor-core kernel (tc_any.cu).  Not for up to 2^20
-    // multiply-adds in sums of at most 64: one thread per output finishes within the launch's own time there, and needs no
-    // tables and no tensor map (32x32x8 1x1 16 channels: 7.4 against 7.8 us a call, 19 against 49 us the first).
-    const bool tiny = (int64_t)KH * KW * IC <= 64 && (int64_t)N * OH * OW * OC * KH * KW * IC <= (1 << 20);
+    // ---- channel runs that are no multiple of 32 bytes: gathering tensor-core kernel (tc_any.cu).  Small layers stay with one
+    // thread per output, which has no tile to fill and needs no tables (a first call is 5 to 15 us dearer with them).  Device
+    // times of a call, one thread per output against the gathering kernel:
+    //   * int8 1x1 (four channels at a time): 28x28, 24 to 40 channels 2.9 against 6.4 us, 56x56, 24 to 40 3.8 / 6.6, 28x28, 100
+    //     to 100 5.2 / 6.8, 14x14, 200 to 70 5.0 / 7.7; beyond the line 3x56x56, 24 to 40 7.1 / 6.8, 28x28, 200 to 70 16 / 8.3;
+    //   * 16-bit and fp8: 56x56, 8 to 16 channels 2.2 / 3.7, 28x28, 24 to 40 2.8 / 3.7; beyond it 56x56, 24 to 40 4.4 / 3.9;
+    //   * windows of several taps are slower there at any size from 64 products on (14x14, 3x3, 12 to 24: 7.5 / 4.9).
+    const int64_t depth = (int64_t)KH * KW * IC, outs = (int64_t)N * OH * OW * OC;
+    const bool tiny = depth <= 64 && outs * depth <= (1 << 20) ? true
+                      : int_path ? KH * KW == 1 && depth <= 256 && OC <= 256 && outs <= (1 << 17) && outs * depth <= 12000000
+                                 : depth <= 48 && outs * depth <= 2500000;
     if (ctx->policy == 0 && !tiny && (!int_path || weight_zp == 0) && tc_rescale_ok && input->dtype != TB200_FP32 && input->stride[3] == 1 && IC > 0)
     {
         const int es       = (int)dtype_size(input->dtype);
@@ -1437,9 +1444,10 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
     // Padding is a zero-filled tap, which equals the reference's skipped tap only for finite weights.  The kernels mend the NaNs
     // that other weights leave, one by one; a padded layer that is used again has its weights' verdict read by the host, and
     // takes the kernel below, which skips taps, if they are not all finite.
-    // Sums of at most 20 products, up to 6 M of them in all, stay with one thread per output (5x109x33x16 1x1 16 channels: 9.3
-    // against 11.5 us; at 8x56x56x64 3x3 64 channels it is 60 times slower).
-    const bool shallow = KH * KW * IC <= 20 && (int64_t)N * OH * OW * OC * KH * KW * IC <= 6000000;
+    // Sums of at most 20 products, up to 6 M of them in all, stay with one thread per output (device times, 1x1: 8x56x56, 12 to 16
+    // channels 5.4 against 5.9 us, 3x56x56, 16 to 16 4.5 / 4.7, 8x56x56, 8 to 8 3.4 / 5.9; at 8x56x56x64 3x3 64 channels it is 60
+    // times slower).
+    const bool shallow = depth <= 20 && outs * depth <= 6000000;
     if (input->dtype == TB200_FP32 && ctx->policy == 0 && !shallow && input->stride[3] == 1 && IH + pad[0] + pad[1] < 32768 &&
         IW + pad[2] + pad[3] < 32768 && (int64_t)N * input->stride[0] < (1LL << 31) && (int64_t)N * OH * OW < (1LL << 31) - 256)
     {
@@ -2338,8 +2346,9 @@ extern "C" tb200_status tb200_depthwise_conv2d(tb200_ctx* ctx, const tb200_tenso
     d.in_zp = input_zp; d.w_zp = weight_zp; d.bias_n = bias->shape[0];
     fill_conv_dev(&d, epi);
     const int block = 256;
-    // int8 with RESCALE to int8: the sliding kernel, for at least 2^20 multiply-adds (below, the kernels after it finish within
-    // the launch's own time and need no tables: 9x42x9x107 3x3 stride 2 7.7 against 8.2 us a call)
+    // int8 with RESCALE to int8: the sliding kernel, for at least 2^20 multiply-adds.  Device times, kernels below against this:
+    // 56x56x144 3x3 10.5 against 4.0 us (first call 37 / 43), 28x28x240 5x5 17.4 / 4.3, 3x29x29x69 3x3 8.8 / 6.6.  Below the line
+    // channel counts that are no multiple of four gain nothing (28x28x75 3x3 5.1 / 5.5); the others would (8 to 10 / 2.5 to 3.1).
     if (int_path && M == 1 && ctx->policy == 0 && weight_zp == 0 && KH == KW && stride[0] == stride[1] && dilation[0] == 1 && dilation[1] == 1 &&
         epi.has_rescale && epi.rs.scale32 && epi.rs.rounding != TB200_INEXACT_ROUND && output->dtype == TB200_INT8 && !epi.rs.out_unsigned &&
         ctx->const_cache_on && numel(output) * KH * KW >= (1 << 20))
@@ -2559,9 +2568,12 @@ extern "C" tb200_status tb200_matmul(tb200_ctx* ctx, const tb200_tensor* a, cons
         // (the CTA-pair kernel takes K tails the single-CTA kernel does not)
         const bool ragged = !tc_gemm_pair_supported(q, ctx->num_sms) && (pad_b || !tc_gemm_supported(q, &why));
         // Ragged products of up to 2^23 multiply-adds in sums of at most 64 stay with one thread per output: most of a 128-byte
-        // chunk of K would be padding, and the call is its launch (bf16 4x338x16x363: 8.7 against 10.7 us, 1x133x47x152: 7.4
-        // against 8.9; beyond, 96x197x64x197 takes 72 us there and 23 us on the tensor cores).
-        const bool tiny = ragged && C <= 64 && (int64_t)N * H * W * C <= (1 << 23);
+        // chunk of K would be padding.  Device times of a call against the gathering kernel's: int8 4x338x16x363 7.2 / 9.7 us,
+        // 4x130x62x130 8.5 / 9.8; fp16 4x338x16x363 6.3 / 10.3, 4x130x62x130 5.3 / 7.7; beyond, fp16 4x338x30x363 is even and
+        // 96x197x64x197 takes 68 us there and 22 us on the tensor cores.  16-bit and fp8 sums of up to 160 with 65 to 256 columns
+        // do as well, up to 10 M: 4x130x100x130 7.3 / 9.0, 4x130x130x130 8.6 / 10.6; 4x130x200x130 12.1 / 10.3.
+        const int64_t products = (int64_t)N * H * W * C;
+        const bool tiny = ragged && ((C <= 64 && products <= (1 << 23)) || (!int_path && C <= 160 && W > 64 && W <= 256 && products <= 10000000));
         if (ragged && !tiny)
         {
             TcProblem g = q;
