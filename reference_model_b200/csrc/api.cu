@@ -1400,7 +1400,12 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     e = cache_insert(ctx, key, std::move(ops), wr_bytes + tab_bytes, build);
                 }
             }
-            if (e || scratch_ready(ctx, wr_bytes + tab_bytes))
+            // Weights that an operator writes, or that a caller stages, have their tables built on every call: 10 us for int8,
+            // 4 us for the others (27 M products of K = 216, int8: 13.3 us one thread per output, 17.7 here; 81 M 27.8 / 18.1;
+            // fp16 2 M of K = 108 7.6 / 9.4, 8 M 11.1 / 9.4).
+            const bool every_call = !use_cache || (e && e->unstable);
+            const bool worth      = !every_call || outs * depth > (int_path ? 40000000 : depth <= 128 ? 6000000 : 0);
+            if (worth && (e || scratch_ready(ctx, wr_bytes + tab_bytes)))
             {
                 void* block = nullptr;
                 if (e)
@@ -1470,7 +1475,10 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
         }
         const bool padded = pad[0] || pad[1] || pad[2] || pad[3];
         void* block       = nullptr;
-        if (e)
+        // (weights that an operator writes, or that a caller stages, are re-ordered on every call, which takes 4.5 us: 1.2 M
+        // products of K = 48 5.6 us one thread per output, 9 here; 4.8 M 12.8 / 9.1)
+        const bool worth = (use_cache && !(e && e->unstable)) || outs * depth > 4000000;
+        if (e && worth)
         {
             st = cache_use(ctx, e);
             if (st == TB200_OK && padded && e->used)
@@ -1481,7 +1489,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
             if (!padded || e->host_flag != 0)
                 block = e->block;
         }
-        else if (!padded && scratch_ready(ctx, flag_off + 64))
+        else if (worth && !padded && scratch_ready(ctx, flag_off + 64))
         {
             st = ensure_scratch(ctx, flag_off + 64);
             if (st == TB200_OK)

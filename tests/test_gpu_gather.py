@@ -276,6 +276,39 @@ def test_two_streams_share_the_chip():
     assert not errors, errors
 
 
+@pytest.mark.parametrize("kind,size", [("i8", 30), ("i8", 120), ("f16", 14), ("f16", 90), ("f32", 14), ("f32", 90)])
+def test_weights_that_an_operator_writes(ctx, kind, size):
+    """Their tables would be built on every call: small layers read the weights where they are, in one launch; larger ones build
+    them, and never use ones that have gone stale."""
+    r = util.rng(2650 + size)
+    IC, OC = 24, 40
+    dt = {"i8": tb.DType.INT8, "f16": F16, "f32": F32}[kind]
+    np_dt = {"i8": np.int8, "f16": np.float16, "f32": np.float32}[kind]
+    x = r.integers(-3, 4, (1, size, size, IC)).astype(np_dt)    # small whole numbers: exact in any type and order
+    tw = ctx.from_numpy(np.zeros((OC, 3, 3, IC), np_dt))
+    tx, tbias, to = ctx.from_numpy(x), ctx.from_numpy(np.zeros(OC, np.int32 if kind == "i8" else np_dt)), ctx.empty(
+        tb.DType.INT32 if kind == "i8" else dt, (1, size, size, OC))
+    source = [ctx.empty(dt, tw.shape), ctx.empty(dt, tw.shape)]
+    for rep in range(3):
+        w = r.integers(-1, 2, tw.shape).astype(np_dt)
+        if rep:    # CLAMP copies: its output is the weight tensor
+            source[rep - 1].upload(w)
+            ctx.clamp(source[rep - 1], tw, -100, 100)
+        else:
+            tw.upload(w)
+        launches = ctx.launch_count()
+        ctx.conv2d(tx, tw, tbias, to, [1] * 4, [1, 1], [1, 1])
+        if rep:
+            large = 9 * IC * OC * size * size > {"i8": 40000000, "f16": 0, "f32": 4000000}[kind]    # (fp16: sums of more than 128)
+            assert (ctx.last_kernel() == "conv2d_direct") == (not large) and (large or ctx.launch_count() == launches + 1)
+        xp = np.pad(x.astype(np.float64), ((0, 0), (1, 1), (1, 1), (0, 0)))
+        exp = sum(xp[:, ky:ky + size, kx:kx + size] @ w[:, ky, kx].astype(np.float64).T for ky in range(3) for kx in range(3))
+        st, out = to.download()
+        assert st == tb.Status.OK and np.array_equal(out.astype(np.float64), exp)
+    for t in [tx, tw, tbias, to] + source:
+        t.free()
+
+
 @pytest.mark.parametrize("kind", ["i8", "i8 rescale", "f16", "f32"])
 def test_capture_before_any_eager_call(kind):
     """A convolution whose tables are neither built nor have room while capturing is captured all the same, on a kernel that needs
