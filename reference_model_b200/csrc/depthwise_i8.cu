@@ -90,11 +90,7 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
     const int c  = cw * 4;
     const int ox0 = strip * p.len, ox1 = min(p.OW, ox0 + p.len);
 
-    if (*p.usable == 0)
-    {
-        walk_general(p, K, S, FIX, n, oy, R, c, ox0, ox1);
-        return;
-    }
+    const bool usable = *p.usable != 0;    // (asked below, behind the loads that a usable layer waits for as well)
     int wc[K][4], w5[K == 5 ? K : 1][4];
 #pragma unroll
     for (int k = 0; k < K; k++)
@@ -114,6 +110,12 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
     {
         ra[i] = __ldg(p.rec + (c + i) * 2);
         rb[i] = __ldg(reinterpret_cast<const int2*>(p.rec + (c + i) * 2 + 1));
+    }
+
+    if (!usable)
+    {
+        walk_general(p, K, S, FIX, n, oy, R, c, ox0, ox1);
+        return;
     }
 
     const int8_t* row[NR];

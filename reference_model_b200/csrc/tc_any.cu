@@ -186,6 +186,16 @@ __device__ __noinline__ float sum_inside(const AnyParams& p, int m, int col)
     return sum;
 }
 
+// The NaNs among sixteen neighbouring columns of one row, `mask`, by sum_inside().
+__device__ __noinline__ void mend_nans(const AnyParams& p, int m, int col, uint32_t mask, uint32_t* v)
+{
+    for (; mask; mask &= mask - 1)
+    {
+        const int at = __ffs((int)mask) - 1;
+        v[at]        = __float_as_uint(sum_inside(p, m, col + at));
+    }
+}
+
 // Sixteen neighbouring columns of one row: corrections, RESCALE or bias, CLAMP, packing.  w: the packed output bytes.
 enum : int
 {
@@ -193,6 +203,7 @@ enum : int
     ANY_RESCALE = 1,
     ANY_FLOAT   = 2,
     ANY_SUM32   = 3,    // floating-point operands, fp32 output
+    ANY_CONV    = 4,    // ANY_FLOAT of a CONV2D: NaNs of windows that leave the image are looked at (MATMUL would pay 3 % for it)
 };
 
 template <int EPI>
@@ -812,19 +823,22 @@ __global__ void __launch_bounds__(kThreads, EPI == ANY_SUM32 ? 1 : 2) tc_any_ker
     const int s_pitch = p.tiles_n == 1 ? ncols * p.out_es : (ncols * p.out_es + 7) & ~3;
     bool bad = false;
     auto finish = [&](int row, int c, uint32_t (&v)[16]) {
-        if (EPI == ANY_FLOAT && p.skip_nan)
+        if (EPI == ANY_CONV && p.skip_nan)
         {
             uint32_t nans = 0;
 #pragma unroll
             for (int i = 0; i < 16; i++)
                 nans |= (v[i] & 0x7fffffffu) > 0x7f800000u && c * 16 + i < ncols ? 1u << i : 0u;
-            for (; nans; nans &= nans - 1)
+            if (nans)
             {
-                const int at       = __ffs((int)nans) - 1;
-                const uint32_t sum = __float_as_uint(sum_inside(p, m0 + row, n0 + c * 16 + at));
+                uint32_t t[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++)
-                    v[i] = i == at ? sum : v[i];
+                    t[i] = v[i];
+                mend_nans(p, m0 + row, n0 + c * 16, nans, t);
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    v[i] = t[i];
             }
         }
         uint32_t w[16];
@@ -1251,14 +1265,15 @@ tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q)
     k.wait_limit = ctx->wait_limit_cycles;
     k.status     = ctx->d_status;
     const int al = plan.align == 16 ? 0 : plan.align == 8 ? 1 : plan.align == 4 ? 2 : 3;
-    const int variant = plan.sum32 ? ANY_SUM32 : q.epi;
-    static void (*const kernels[4][4])(const AnyParams) = {
+    const int variant = plan.sum32 ? ANY_SUM32 : q.epi == TC_EPI_FLOAT && !matmul ? ANY_CONV : q.epi;
+    static void (*const kernels[5][4])(const AnyParams) = {
         { tc_any_kernel<ANY_I32, 16>, tc_any_kernel<ANY_I32, 8>, tc_any_kernel<ANY_I32, 4>, tc_any_kernel<ANY_I32, 0> },
         { tc_any_kernel<ANY_RESCALE, 16>, tc_any_kernel<ANY_RESCALE, 8>, tc_any_kernel<ANY_RESCALE, 4>, tc_any_kernel<ANY_RESCALE, 0> },
         { tc_any_kernel<ANY_FLOAT, 16>, tc_any_kernel<ANY_FLOAT, 8>, tc_any_kernel<ANY_FLOAT, 4>, tc_any_kernel<ANY_FLOAT, 0> },
-        { tc_any_kernel<ANY_SUM32, 16>, tc_any_kernel<ANY_SUM32, 8>, tc_any_kernel<ANY_SUM32, 4>, tc_any_kernel<ANY_SUM32, 0> } };
+        { tc_any_kernel<ANY_SUM32, 16>, tc_any_kernel<ANY_SUM32, 8>, tc_any_kernel<ANY_SUM32, 4>, tc_any_kernel<ANY_SUM32, 0> },
+        { tc_any_kernel<ANY_CONV, 16>, tc_any_kernel<ANY_CONV, 8>, tc_any_kernel<ANY_CONV, 4>, tc_any_kernel<ANY_CONV, 0> } };
     void (*const kern)(const AnyParams) = kernels[variant][al];
-    const tb200_status st = raise_smem_limit(ctx, (plan.sum32 ? 56 : 20 + q.epi * 4) + al, reinterpret_cast<const void*>(kern), plan.smem_bytes);
+    const tb200_status st = raise_smem_limit(ctx, (variant >= ANY_SUM32 ? 56 - 4 * ANY_SUM32 : 20) + variant * 4 + al, reinterpret_cast<const void*>(kern), plan.smem_bytes);
     if (st != TB200_OK)
         return st;
     cudaLaunchConfig_t cfg;
