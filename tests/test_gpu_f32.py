@@ -1,6 +1,7 @@
 """fp32 MATMUL and CONV2D at the edges of the tiled FFMA kernel: row / column / K remainders of every tile size, K split
 over a cluster, unaligned rows, window shapes, strides, dilation, a view, infinite weights under padding; against the
-fp64 oracle under the DOT_PRODUCT rule."""
+fp64 oracle under the DOT_PRODUCT rule.  And on the tensor cores (three bf16 parts per operand): remainders, accuracy,
+operands that parts cannot carry, waits that give up."""
 import numpy as np
 import pytest
 
@@ -304,6 +305,46 @@ def test_split_bounded_waits_give_up(ctx, conv):
     st, out = tensors[-1].download()
     assert st == tb.Status.OK and np.array_equal(out, exp)
     for t in tensors:
+        t.free()
+
+
+@pytest.mark.parametrize("dil,stride,pad,IC,c0", [(1, [1, 1], [1, 1, 1, 1], 64, 4), (2, [1, 1], [2, 2, 2, 2], 64, 4), (2, [1, 2], [2, 2, 0, 2], 63, 0),
+                                                 (1, [1, 1], [0, 0, 0, 0], 61, 4)])
+def test_conv_f32_split_views(ctx, dil, stride, pad, IC, c0):
+    """A zero-copy view as the input of a layer that runs on the tensor cores, dilation, strides, an infinity and a NaN in it."""
+    r = util.rng(1050 + IC)
+    full, w = r.standard_normal((36, 31, 33, 68)).astype(np.float32), r.standard_normal((128, 3, 3, IC)).astype(np.float32)
+    full[5, 7, 8:10, 9], full[6, 20, 20:22, 20] = np.inf, np.nan
+    b = r.standard_normal(128).astype(np.float32)
+    x = full[2:, 1:30, 3:32, c0:c0 + IC]
+    OH, OW = orc.conv_out_hw(29, 29, 3, 3, pad, stride, [dil, dil])
+    tfull, tw, tbias, to = ctx.from_numpy(full), ctx.from_numpy(w), ctx.from_numpy(b), ctx.empty(tb.DType.FP32, (34, OH, OW, 128))
+    view = tfull.slice([2, 1, 3, c0], [34, 29, 29, IC])
+    call = lambda: ctx.conv2d(view, tw, tbias, to, pad, stride, [dil, dil])
+    call()
+    assert ctx.last_kernel() == "conv_f32"
+    st, out = to.download()
+    xp = np.pad(x.astype(np.float64), ((0, 0), (pad[0], pad[1]), (pad[2], pad[3]), (0, 0)))
+    ref, bound = np.zeros(out.shape) + b, np.zeros(out.shape) + np.abs(b)
+    with np.errstate(all="ignore"):
+        for ky in range(3):
+            for kx in range(3):
+                win = xp[:, ky * dil:ky * dil + (OH - 1) * stride[0] + 1:stride[0], kx * dil:kx * dil + (OW - 1) * stride[1] + 1:stride[1]]
+                wt = w[:, ky, kx].astype(np.float64).T
+                ref, bound = ref + win @ wt, bound + np.abs(win) @ np.abs(wt)
+        assert st == tb.Status.OK and np.array_equal(np.isnan(out), np.isnan(ref)) and np.array_equal(out[np.isinf(ref)], ref[np.isinf(ref)])
+        # blocks that hold such results are summed with multiply-adds in K order: K roundings
+        near = np.abs(out - ref) <= 9 * IC * 2.0 ** -24 * bound
+        assert np.isnan(out).any() and np.isinf(out).any() and near[np.isfinite(ref)].all()
+    # that it ran there: the multiply-add kernel has no waits to give up
+    ctx.set_wait_limit(1)
+    try:
+        call()
+        assert ctx.sync(check=False) == tb.Status.INTERNAL
+    finally:
+        ctx.set_wait_limit(4000000000)
+    view.free()
+    for t in (tfull, tw, tbias, to):
         t.free()
 
 

@@ -1,6 +1,7 @@
 """The gathering tensor-core kernel at the edges of its tiles: runs, rows and columns of every alignment, K shorter than a
-chunk and split over a cluster, one row, borders, views, both zero points, every element type, outputs that are no whole
-16-byte rows; integers bit for bit against the oracle, floats under the DOT_PRODUCT rule."""
+chunk and split over a cluster, one row, borders, views, strides, dilation, both zero points, every element type and pair of
+fp8 types, outputs that are no whole 16-byte rows, constants that change; integers bit for bit against the oracle, floats
+under the DOT_PRODUCT rule and against the kernel that rounds every multiply-add."""
 import threading
 
 import numpy as np
@@ -176,6 +177,89 @@ def test_conv_float(ctx, dt, name, case):
     st, out, kernel = run_conv_fp(ctx, x, w, b, *args, dt)
     ok, info = orc.verify_dot_product(out, ref, bnd, orc.dot_product_ksb(K * K * IC + 1, "fp32", name), out=name)
     assert kernel == "tc_gemm_any_f16" and st == tb.Status.OK and ok, (kernel, info)
+
+
+# parent [N, IH, IW, bytes of channels], view start and size (channels in elements), OC, KH, KW, stride, dilation, pad; what the
+# run and the pitches are multiples of: 16 bytes, 8, 4, less
+VIEWS = [((2, 13, 15, 64), (0, 1, 2), (2, 11, 12), 16, 48, 20, 3, 2, [1, 1], [2, 1], [2, 2, 1, 0]),
+         ((1, 19, 32, 48), (0, 0, 16), (1, 18, 15), 16, 24, 33, 2, 3, [1, 3], [1, 2], [0, 1, 2, 3]),
+         ((3, 10, 24, 44), (1, 0, 8), (2, 9, 16), 0, 20, 65, 3, 3, [3, 1], [1, 3], [1, 2, 3, 3]),
+         ((2, 12, 32, 46), (0, 2, 16), (2, 9, 16), 0, 22, 30, 2, 5, [2, 1], [1, 3], [1, 0, 5, 4])]
+
+
+@pytest.mark.parametrize("name", ["i8", "i8 rescale", "fp16", "bf16", "e4m3", "e5m2"])
+@pytest.mark.parametrize("case", range(len(VIEWS)))
+def test_conv_views(ctx, name, case):
+    """A zero-copy view as the input (pitches beyond the run), unequal strides, dilation and padding, every element type."""
+    (N0, H0, W0, cb), (n, y, x0), (N, IH, IW), cstart, run, OC, KH, KW, stride, dil, pad = VIEWS[case]
+    es = 2 if name in ("fp16", "bf16") else 1
+    C0, c0, IC = cb // es, cstart // es, run // es
+    r = util.rng(2900 + case)
+    oname = "bf16" if name == "bf16" else "fp16"
+    up = lambda v: ctx.from_numpy(util.to_bf16_bits(v), BF16) if name == "bf16" else ctx.from_numpy(v.astype(np.float16))
+    shapes, izp = ((N0, H0, W0, C0), (OC, KH, KW, IC)), 0
+    if name[0] == "i":
+        izp = -7
+        full, w = (r.integers(-128, 128, sh).astype(np.int8) for sh in shapes)
+        b = r.integers(-1000, 1000, OC).astype(np.int32)
+        tfull, tw, tbias = (ctx.from_numpy(v) for v in (full, w, b))
+    elif name[0] == "e":
+        cf, cw = (_fp8_codes(r, sh, name) for sh in shapes)
+        full, w, b = orc.fp8_to_f32(cf, name), orc.fp8_to_f32(cw, name), r.standard_normal(OC).astype(np.float16).astype(np.float32)
+        dt = tb.DType.FP8E4M3 if name == "e4m3" else tb.DType.FP8E5M2
+        tfull, tw, tbias = ctx.from_numpy(cf, dt), ctx.from_numpy(cw, dt), up(b)
+    else:
+        full, w, b = (orc.fptrunc(r.standard_normal(sh).astype(np.float32), name) for sh in shapes + ((OC,),))
+        tfull, tw, tbias = up(full), up(w), up(b)
+    view = tfull.slice([n, y, x0, c0], [N, IH, IW, IC])
+    x = np.ascontiguousarray(full[n:n + N, y:y + IH, x0:x0 + IW, c0:c0 + IC])
+    args, extra, epi = (pad, stride, dil), [], None
+    if name[0] == "i":
+        exp = orc.conv2d(x, w, b, *args, izp, 0, nthreads=8)
+        odt = tb.DType.INT32
+        if name == "i8 rescale":
+            mult, shift = util.rescale_params(r, OC)
+            extra, odt = [ctx.from_numpy(mult), ctx.from_numpy(shift)], tb.DType.INT8
+            epi = tb.Epilogue(tb.RescaleAttr(*extra, 0, 3, True, "DOUBLE_ROUND", per_channel=True), (-120, 110))
+            exp = np.clip(orc.rescale(exp, mult, shift, True, True, "DOUBLE_ROUND", 0, 3, 32, 8)[1], -120, 110)
+    else:
+        exp, bnd = (orc.conv2d(x, w, b, *args, mode="f64", bounds=f) for f in (False, True))
+        odt = BF16 if name == "bf16" else F16
+    to = ctx.empty(odt, exp.shape)
+    ctx.conv2d(view, tw, tbias, to, *args, izp, 0, epi)
+    assert ctx.last_kernel().startswith("tc_gemm_any"), ctx.last_kernel()
+    st, out = to.download()
+    assert st == tb.Status.OK
+    if name[0] == "i":
+        assert np.array_equal(out, exp)
+    else:
+        out = util.from_bf16_bits(out) if name == "bf16" else out.astype(np.float32)
+        ok, info = orc.verify_dot_product(out, exp, bnd, orc.dot_product_ksb(KH * KW * IC + 1, "fp32", oname), out=oname)
+        assert ok, info
+    view.free()
+    for t in [tfull, tw, tbias, to] + extra:
+        t.free()
+
+
+@pytest.mark.parametrize("fa,fb", [("e4m3", "e5m2"), ("e5m2", "e4m3"), ("e5m2", "e5m2")])
+@pytest.mark.parametrize("shape", [(3, 130, 90, 31), (2, 60, 177, 300), (1, 7, 2679, 72)])
+def test_matmul_fp8_pairs(ctx, fa, fb, shape):
+    N, H, C, W = shape
+    r = util.rng(2950 + C)
+    ca, cb = _fp8_codes(r, (N, H, C), fa), _fp8_codes(r, (N, C, W), fb)
+    a, b = orc.fp8_to_f32(ca, fa), orc.fp8_to_f32(cb, fb)
+    ref, bnd = orc.matmul(a, b, mode="f64"), orc.matmul(np.abs(a), np.abs(b), mode="f64")
+    dts = {"e4m3": tb.DType.FP8E4M3, "e5m2": tb.DType.FP8E5M2}
+    ta, tbb = ctx.from_numpy(ca, dts[fa]), ctx.from_numpy(cb, dts[fb])
+    for dt, oname in ((F16, "fp16"), (F32, "fp32")):
+        to = ctx.empty(dt, (N, H, W))
+        ctx.matmul(ta, tbb, to)
+        assert ctx.last_kernel() == "tc_gemm_any_f8"
+        st, out = to.download()
+        ok, info = orc.verify_dot_product(out.astype(np.float32), ref, bnd, orc.dot_product_ksb(C, "fp32", oname), out=oname)
+        assert st == tb.Status.OK and ok, info
+        to.free()
+    ta.free(), tbb.free()
 
 
 @pytest.mark.parametrize("name", ["fp16", "bf16", "e5m2"])
