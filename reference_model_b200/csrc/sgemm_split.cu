@@ -8,8 +8,9 @@
 // products not beside the small ones: per stage of 64 K elements one accumulator takes a0 b0 (products of 16 bits, whose sums
 // mostly fit 24), and another, over four stages, the five others (whose cut-off is 2^-8 of the result's).  Both are read back and
 // added to fp32 accumulators in registers, rounded to nearest.
-// Error against 64 bits, relative 2-norm, K = 320: normal operands 8.5e-8 (multiply-adds in K order 3.2e-7), positive ones
-// 4.1e-8 (2.7e-7), one product per sum 2.52e-8 (2.48e-8).
+// Error against 64 bits, relative 2-norm, K = 256 / 1024 / 4096: normal operands 8.0e-8 / 1.1e-7 / 1.8e-7 (multiply-adds in K
+// order 2.9e-7 / 5.7e-7 / 1.1e-6), positive ones 4.0e-8 / 7.7e-8 / 1.4e-7 (2.4e-7 / 4.8e-7 / 9.6e-7); one product per sum 2.52e-8
+// (2.48e-8).
 //
 // One persistent CTA per SM, 128 x 128 output tiles, sixteen warps:
 //   warps 0-7   add up stages (32 rows x 64 columns each, 64 accumulators per thread), finish and store the tile; the first
@@ -791,8 +792,8 @@ constexpr int kMinSplitK = 256;
 }    // namespace
 
 // Estimated SM cycles of the split kernel, 0 where it does not serve.
-// A stage measured 3 700 cycles, 4 600 with unaligned pairs, 5 000 - 6 500 where A is gathered (16x28x28x256 3x3 256
-// channels: 187 us, 79 TFLOP/s).
+// A stage measured 3 700 cycles, 4 500 with unaligned pairs, 4 500 - 5 600 where A is gathered (16x28x28x256 3x3 256
+// channels: 181 us, 82 TFLOP/s; 32x28x28x64 3x3 128 channels: 58 us, where FFMA takes 71).
 double sgemm_split_cost(const tb200_ctx* ctx, int64_t batches, int64_t M, int64_t N, int64_t K, bool conv)
 {
     const int64_t tiles = batches * ((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile);
