@@ -797,7 +797,7 @@ constexpr int kMinSplitK = 256;
 double sgemm_split_cost(const tb200_ctx* ctx, int64_t batches, int64_t M, int64_t N, int64_t K, bool conv)
 {
     const int64_t tiles = batches * ((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile);
-    if (K < kMinSplitK || tiles >= (1LL << 30) || (ctx->max_smem_optin > 0 && ctx->max_smem_optin < kSplitSmem + 256) || ctx->d_status == nullptr)
+    if (K < kMinSplitK || tiles >= (1LL << 30) || (ctx->max_smem_optin > 0 && ctx->max_smem_optin < kSplitSmem + 1024) || ctx->d_status == nullptr)
         return 0.0;
     const double rounds = (double)((tiles + ctx->num_sms - 1) / ctx->num_sms);
     const double stage  = conv ? 6200.0 : (K % 2 || N % 2) ? 4600.0 : 3700.0;

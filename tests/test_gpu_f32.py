@@ -389,3 +389,27 @@ def test_conv_f32_nonfinite_weights_under_padding(ctx, case):
     ctx.graph_destroy(graph)
     for t in (tx, tw, tw2, tbias, to):
         t.free()
+
+
+def test_split_more_tiles_than_slots(ctx):
+    """More tiles per CTA (129 on 148 SMs) than there are words for blocks to be computed again: tiles that share a word."""
+    torch = pytest.importorskip("torch")
+    N, late = 148 * 129, 5 + 148 * 128
+    gen = torch.Generator(device="cuda").manual_seed(83)
+    a, b = (torch.randn(N, *s, generator=gen, device="cuda") for s in ((128, 256), (256, 128)))
+    a[5, 3, 7], a[late, 70, 0], a[late + 1, 9] = float("nan"), float("inf"), 1e-30
+    b[late + 1] *= 1e-8
+    out = torch.empty((N, 128, 128), device="cuda")
+    torch.cuda.synchronize()
+    ta, tbb, to = (ctx.wrap(tb.DType.FP32, tuple(v.shape), v.data_ptr(), v) for v in (a, b, out))
+    ctx.matmul(ta, tbb, to)
+    ctx.sync()
+    for n in (0, 5, 6, late - 148, late, late + 1, N - 1):
+        x, y = a[n].double(), b[n].double()
+        ref, bound, got = x @ y, x.abs() @ y.abs(), out[n].double()
+        fin = torch.isfinite(ref)
+        assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(torch.isinf(got), torch.isinf(ref))
+        assert bool(((got - ref).abs() <= 256 * 2.0 ** -24 * bound + 256 * 2.0 ** -149)[fin].all())
+        assert bool(fin.all()) == (n not in (5, late))
+    for t in (ta, tbb, to):
+        t.free()
