@@ -321,6 +321,45 @@ def test_bounded_waits_give_up(ctx):
     assert st == tb.Status.OK and np.array_equal(out, exp)
 
 
+@pytest.mark.parametrize("kind", ["i8 split", "f16 split", "f16 to f32", "f16 to f32 split", "f16 to f32 unaligned", "f8 to f32"])
+def test_every_form_gives_up_and_recovers(ctx, kind):
+    """The shortest wait limit on each form of the kernel: clusters that meet after a role gave up, tensor memory given back early,
+    chunk sums read back.  It ends and reports (one call of twenty at least does not finish in time), and the same call is right
+    afterwards."""
+    N, H, C, W = {"i8 split": (1, 5, 3000, 300), "f16 split": (1, 64, 4000, 62), "f16 to f32": (40, 300, 2000, 61), "f16 to f32 split": (1, 64, 4000, 62),
+                  "f16 to f32 unaligned": (2, 130, 3001, 63), "f8 to f32": (2, 130, 3001, 63)}[kind]
+    r = util.rng(2450 + W)
+    to = ctx.empty(tb.DType.INT32 if kind[0] == "i" else F32 if "f32" in kind else F16, (N, H, W))
+    zp = (3, -2) if kind[0] == "i" else (0, 0)
+    a, b = (r.integers(-3, 4, size=s).astype(np.int8) for s in ((N, H, C), (N, C, W)))    # small whole numbers: exact
+    exp = (a.astype(np.float64) - zp[0]) @ (b.astype(np.float64) - zp[1])
+    if kind[0] == "i":
+        ta, tbb = ctx.from_numpy(a), ctx.from_numpy(b)
+    elif kind[:3] == "f16":
+        ta, tbb = ctx.from_numpy(a.astype(np.float16)), ctx.from_numpy(b.astype(np.float16))
+    else:
+        code = np.array([0, 0x38, 0x40, 0x44], np.uint8)    # E4M3 of 0, 1, 2, 3
+        ta, tbb = (ctx.from_numpy(code[np.abs(v)] | (v < 0).astype(np.uint8) << 7, tb.DType.FP8E4M3) for v in (a, b))
+    ctx.matmul(ta, tbb, to, *zp)
+    assert ctx.last_kernel().startswith("tc_gemm_any")
+    ctx.sync()
+    ctx.set_wait_limit(1)
+    try:
+        for _ in range(20):
+            ctx.matmul(ta, tbb, to, *zp)
+            st = ctx.sync(check=False)
+            if st == tb.Status.INTERNAL:
+                break
+    finally:
+        ctx.set_wait_limit(4000000000)
+    assert st == tb.Status.INTERNAL
+    ctx.matmul(ta, tbb, to, *zp)
+    st, out = to.download()
+    assert st == tb.Status.OK and np.array_equal(out.astype(np.float64), exp)
+    for t in (ta, tbb, to):
+        t.free()
+
+
 def test_two_streams_share_the_chip():
     """Products whose K is split over clusters, from two contexts (two streams) and two threads at once.  Their plans leave room
     for both on an SM in shared memory but not in tensor memory (512 and 64 columns and more): CTAs queue for columns, and
