@@ -322,6 +322,20 @@ extern "C"
                                               const tb200_rescale_attr* out_attr, int32_t has_clamp, int32_t clamp_min,
                                               int32_t clamp_max, tb200_tensor* output);
 
+    /* tb200_conv2d with a RESCALE epilogue to INT8, followed by the residual join of its result with `other`:
+     * RESCALE(conv_attr) of the convolution's result and RESCALE(other_attr) of `other` to INT32, ADD,
+     * RESCALE(out_attr) to INT8, CLAMP.  One kernel where the shapes and constants allow (tb200_last_kernel then names
+     * tc_conv_lean_i8_join): the result of the convolution, which has no other consumer, never reaches device memory.  Everything
+     * else runs tb200_conv2d into `output` and tb200_residual_add on it in place.  `other` has the output's shape and must
+     * not overlap it. */
+    TB200_API tb200_status tb200_conv2d_add(tb200_ctx* ctx, const tb200_tensor* input, const tb200_tensor* weight,
+                                            const tb200_tensor* bias, int32_t input_zp, int32_t weight_zp,
+                                            const int32_t pad[4], const int32_t stride[2], const int32_t dilation[2],
+                                            const tb200_epilogue* epilogue, const tb200_rescale_attr* conv_attr,
+                                            const tb200_tensor* other, const tb200_rescale_attr* other_attr,
+                                            const tb200_rescale_attr* out_attr, int32_t has_clamp, int32_t clamp_min,
+                                            int32_t clamp_max, tb200_tensor* output);
+
     /* MAX_POOL2D.  Replaces OpMaxPool2d<T>::eval (reference_model/src/ops/tensor_ops.cpp:1545-1641; checks :28-117).
      * kernel = {y,x}. */
     TB200_API tb200_status tb200_max_pool2d(tb200_ctx* ctx, const tb200_tensor* input, const int32_t kernel[2],

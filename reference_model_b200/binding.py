@@ -72,7 +72,7 @@ EXPORTS = [
     "tb200_timer_enable", "tb200_timer_read", "tb200_capture_begin", "tb200_capture_end", "tb200_graph_launch",
     "tb200_graph_destroy",
     "tb200_tensor_alloc", "tb200_tensor_wrap", "tb200_tensor_free", "tb200_tensor_upload", "tb200_tensor_download",
-    "tb200_tensor_data", "tb200_tensor_bytes", "tb200_tensor_slice", "tb200_tensor_reshape", "tb200_conv2d", "tb200_depthwise_conv2d", "tb200_conv2d_depthwise", "tb200_conv3d", "tb200_transpose_conv2d", "tb200_matmul",
+    "tb200_tensor_data", "tb200_tensor_bytes", "tb200_tensor_slice", "tb200_tensor_reshape", "tb200_conv2d", "tb200_depthwise_conv2d", "tb200_conv2d_depthwise", "tb200_conv2d_add", "tb200_conv3d", "tb200_transpose_conv2d", "tb200_matmul",
     "tb200_rescale", "tb200_clamp", "tb200_add", "tb200_residual_add", "tb200_max_pool2d", "tb200_avg_pool2d",
     "tb200_matmul_host", "tb200_set_kernel_policy", "tb200_last_kernel", "tb200_matmul_i8_noalloc",
     "tb200_npy_probe", "tb200_tensor_load_npy", "tb200_tensor_save_npy",
@@ -126,6 +126,9 @@ def load_library():
         "tb200_add": (i32, [vp, vp, vp, vp]),
         "tb200_residual_add": (i32, [vp, vp, ctypes.POINTER(_RescaleAttr), vp, ctypes.POINTER(_RescaleAttr),
                                      ctypes.POINTER(_RescaleAttr), i32, i32, i32, vp]),
+        "tb200_conv2d_add": (i32, [vp, vp, vp, vp, i32, i32, p_i32, p_i32, p_i32, ctypes.POINTER(_Epilogue),
+                                   ctypes.POINTER(_RescaleAttr), vp, ctypes.POINTER(_RescaleAttr),
+                                   ctypes.POINTER(_RescaleAttr), i32, i32, i32, vp]),
         "tb200_max_pool2d": (i32, [vp, vp, p_i32, p_i32, p_i32, vp]),
         "tb200_avg_pool2d": (i32, [vp, vp, p_i32, p_i32, p_i32, i32, i32, vp]),
         "tb200_matmul_host": (i32, [vp, i32, i32, vp, vp, i32, i32, i32, i32, i32, i32, vp]),
@@ -442,6 +445,15 @@ class Context:
             dw_w.handle, dw_bias.handle, _ivec(dw_pad), _ivec(dw_stride),
             ctypes.byref(dw_epilogue.c) if dw_epilogue else None, expanded.handle if expanded is not None else None,
             out.handle), check)
+
+    def conv2d_add(self, x, w, bias, out, pad, stride, dilation, input_zp, weight_zp, epilogue, conv_attr, other, other_attr,
+                   out_attr, clamp=None, check=True):
+        """CONV2D with a RESCALE epilogue, then the residual join of its result with `other` (conv2d + residual_add)."""
+        lo, hi = clamp if clamp is not None else (0, 0)
+        return self._check(self.lib.tb200_conv2d_add(
+            self.handle, x.handle, w.handle, bias.handle, int(input_zp), int(weight_zp), _ivec(pad), _ivec(stride),
+            _ivec(dilation), ctypes.byref(epilogue.c) if epilogue else None, ctypes.byref(conv_attr.c), other.handle,
+            ctypes.byref(other_attr.c), ctypes.byref(out_attr.c), int(clamp is not None), int(lo), int(hi), out.handle), check)
 
     def transpose_conv2d(self, x, w, bias, out, out_pad, stride, input_zp=0, weight_zp=0, epilogue=None, check=True):
         return self._check(self.lib.tb200_transpose_conv2d(self.handle, x.handle, w.handle, bias.handle,

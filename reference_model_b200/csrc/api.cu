@@ -17,7 +17,7 @@ namespace tb200
 
 tb200_status raise_smem_limit(tb200_ctx* ctx, int bit, const void* kernel, int bytes)
 {
-    if (ctx->smem_attr_set & (1ull << bit))
+    if (ctx->smem_attr_set.test((size_t)bit))
         return TB200_OK;
     // a context that knows its device's limit raises the kernel to it once; a bare one (the allocation-free entry
     // point's stack object) asks for what this launch needs, every time
@@ -31,7 +31,7 @@ tb200_status raise_smem_limit(tb200_ctx* ctx, int bit, const void* kernel, int b
     }
     TB200_CUDA_CHECK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, want));
     if (ctx->max_smem_optin > 0)
-        ctx->smem_attr_set |= 1ull << bit;
+        ctx->smem_attr_set.set((size_t)bit);
     return TB200_OK;
 }
 
@@ -807,6 +807,16 @@ struct ConvOutView
 };
 static const tb200_status kNeedsDenseOutput = (tb200_status)-77;
 
+// A residual join to run on the convolution's int8 results before they are stored (tb200_conv2d_add).  conv2d_impl answers
+// kNeedsSeparateJoin, before the convolution is launched, where the kernel it would take has no such form.
+struct ConvJoin
+{
+    const int32_t* block;    // residual_record_kernel
+    const void* other;
+    int double_round, lo, hi;
+};
+static const tb200_status kNeedsSeparateJoin = (tb200_status)-78;
+
 // The word a builder left at `offset` of a cache entry's block (e.g. "every column's lean RESCALE record is usable"),
 // read back once per build: a copy and a stream synchronisation at the first use of the entry, nothing afterwards.
 // An entry that is rebuilt on every use, or that is first met while capturing, stays unread: the caller then takes
@@ -825,7 +835,8 @@ static tb200_status read_host_flag(tb200_ctx* ctx, Prepared* e, size_t offset)
 static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const tb200_tensor* weight,
                                 const tb200_tensor* bias, int32_t input_zp, int32_t weight_zp, const int32_t pad[4],
                                 const int32_t stride[2], const int32_t dilation[2], const tb200_epilogue* epilogue,
-                                tb200_tensor* output, const ConvOutView* view, bool dry_run, bool use_cache)
+                                tb200_tensor* output, const ConvOutView* view, bool dry_run, bool use_cache,
+                                const ConvJoin* join = nullptr)
 {
     if (!ctx)
         return TB200_ERROR;
@@ -914,18 +925,51 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
             {
                 const bool padded  = pad[0] || pad[1] || pad[2] || pad[3];
                 const bool classes = input_zp != 0 && padded;
-                const size_t ncls  = classes ? (size_t)(KH + 1) * (KH + 1) * (KW + 1) * (KW + 1) : 1;
-                // block: prefix | corr | mult_pad | shift_pad
-                // block: prefix | corr | mult_pad | shift_pad | records of the lean RESCALE form | border deltas
-                const size_t prefix_elems = ((size_t)(KH + 1) * (KW + 1) * OC + 3) & ~(size_t)3;
-                const size_t corr_elems   = ncls * OCpad;
-                const size_t rec_off      = ((prefix_elems + corr_elems + OCpad) * sizeof(int32_t) + OCpad + 63) & ~(size_t)63;
-                const bool want_rec       = epi.has_rescale;
-                const size_t delta_off    = rec_off + (want_rec ? (size_t)OCpad * 8 * sizeof(int32_t) : 0);
-                const size_t flag_off     = delta_off + ((want_rec && classes) ? corr_elems * sizeof(int32_t) : 0);
-                const size_t bytes        = flag_off + 64;
-                if (bytes <= ((size_t)64 << 20))
-                {
+                // the lean form packs with int8 saturation: it serves RESCALEs to signed int8 only
+                const bool want_rec = epi.has_rescale;
+                const bool lean_out = want_rec && output->dtype == TB200_INT8 && !epi.rs.out_unsigned;
+                const tb200_status kNextForm = (tb200_status)-79;
+                // The problem with E output pixels of a row side by side in the channel dimension (E = 1: as it is).
+                // kNextForm: nothing launched but tables, this E does not serve.
+                auto run = [&](const int E) -> tb200_status {
+                    TcProblem qe  = q;
+                    const bool flat = E > 1 && KH == 1 && KW == 1;    // 1x1: E pixels are one row of E * IC values
+                    const int OCe = E * OC, KWe = E > 1 ? KW + (E - 1) * stride[1] : KW;
+                    const int OCpad = (OCe + 255) / 256 * 256;
+                    if (flat)
+                    {
+                        qe.N = 1; qe.IH = qe.OH = 1; qe.IW = qe.OW = N * OH * OW / E; qe.IC = E * IC;
+                        qe.a_stride_w = qe.a_stride_h = qe.a_stride_n = 0;
+                    }
+                    else
+                    {
+                        qe.OW = OW / E; qe.KW = KWe; qe.stride_x = E * stride[1];
+                    }
+                    qe.OC = OCe;
+                    const size_t ncls  = classes ? (size_t)(KH + 1) * (KH + 1) * (KWe + 1) * (KWe + 1) : 1;
+                    // block: weights embedded for E pixels | prefix | corr | mult_pad | shift_pad | records of the lean RESCALE
+                    // form | border deltas | verdict
+                    const size_t emb          = E > 1 ? ((size_t)OCe * KH * KWe * IC + 255) & ~(size_t)255 : 0;
+                    const size_t prefix_elems = ((size_t)(KH + 1) * (KWe + 1) * OCe + 3) & ~(size_t)3;
+                    const size_t corr_elems   = ncls * OCpad;
+                    const size_t rec_off      = (emb + (prefix_elems + corr_elems + OCpad) * sizeof(int32_t) + OCpad + 63) & ~(size_t)63;
+                    const size_t delta_off    = rec_off + (want_rec ? (size_t)OCpad * 8 * sizeof(int32_t) : 0);
+                    const size_t flag_off     = delta_off + ((want_rec && classes) ? corr_elems * sizeof(int32_t) : 0);
+                    const size_t bytes        = flag_off + 64;
+                    if (bytes > ((size_t)64 << 20))
+                        return kNextForm;
+                    if (E > 1)
+                    {
+                        // would the kernel take it?  (any aligned address stands for the block)
+                        const int32_t* some = reinterpret_cast<const int32_t*>(static_cast<uintptr_t>(256));
+                        qe.b = some; qe.rec = some; qe.delta = some; qe.lean_ok = 1; qe.corr_classes = classes ? 1 : 0;
+                        if (join)
+                        {
+                            qe.join = some; qe.res = join->other;
+                        }
+                        if (!conv_chan_supported(ctx, qe))
+                            return kNextForm;
+                    }
                     if (dry_run)
                         return TB200_OK;
                     const int8_t* wp   = reinterpret_cast<const int8_t*>(weight->data);
@@ -933,21 +977,23 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     const int32_t* mp  = epi.has_rescale ? reinterpret_cast<const int32_t*>(epi.rs.mult) : nullptr;
                     const int8_t* sp   = epi.has_rescale ? epi.rs.shift : nullptr;
                     const int bias_n = bias->shape[0], per_ch = epi.rs.per_channel, has_rs = epi.has_rescale ? 1 : 0;
-                    const int cls_i = classes ? 1 : 0;
+                    const int cls_i = classes ? 1 : 0, sx = stride[1];
                     const int dr_i  = epi.has_rescale && epi.rs.rounding == TB200_DOUBLE_ROUND ? 1 : 0;
                     const int32_t ozp_i = epi.has_rescale ? (int32_t)epi.rs.out_zp_ext : 0;
-                    auto build = [=](tb200_ctx* c, void* block) -> tb200_status {
-                        int32_t* prefix   = reinterpret_cast<int32_t*>(block);
+                    auto build = [=](tb200_ctx* c, void* blk) -> tb200_status {
+                        uint8_t* block    = reinterpret_cast<uint8_t*>(blk);
+                        int32_t* prefix   = reinterpret_cast<int32_t*>(block + emb);
                         int32_t* corr     = prefix + prefix_elems;
                         int32_t* mult_pad = corr + corr_elems;
                         int8_t* shift_pad = reinterpret_cast<int8_t*>(mult_pad + OCpad);
-                        int32_t* rec      = want_rec ? reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(block) + rec_off) : nullptr;
-                        int32_t* delta    = (want_rec && cls_i) ? reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(block) + delta_off) : nullptr;
-                        int* all_ok       = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(block) + flag_off);
+                        int32_t* rec      = want_rec ? reinterpret_cast<int32_t*>(block + rec_off) : nullptr;
+                        int32_t* delta    = (want_rec && cls_i) ? reinterpret_cast<int32_t*>(block + delta_off) : nullptr;
+                        int* all_ok       = reinterpret_cast<int*>(block + flag_off);
                         TB200_CUDA_CHECK(c, cudaMemsetAsync(all_ok, want_rec ? 1 : 0, sizeof(int), c->stream));
                         conv_epilogue_tables_kernel<<<(OCpad * 32 + 127) / 128, 128, 0, c->stream>>>(
-                            wp, bp, bias_n, OC, OCpad, KH, KW, IC, input_zp, cls_i, mp, sp, per_ch, prefix, corr,
-                            has_rs ? mult_pad : nullptr, shift_pad, rec, delta, dr_i, ozp_i, all_ok);
+                            wp, bp, bias_n, OCe, OCpad, KH, KWe, IC, input_zp, cls_i, mp, sp, per_ch, prefix, corr,
+                            has_rs ? mult_pad : nullptr, shift_pad, rec, delta, dr_i, ozp_i, all_ok, E, KW, sx,
+                            E > 1 ? reinterpret_cast<int8_t*>(block) : nullptr);
                         return post_launch(c, "conv_epilogue_tables");
                     };
                     void* block = nullptr;
@@ -960,6 +1006,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                         key_add(&key, OC); key_add(&key, KH); key_add(&key, KW); key_add(&key, IC); key_add(&key, bias_n);
                         key_add(&key, input_zp); key_add(&key, per_ch); key_add(&key, has_rs); key_add(&key, cls_i);
                         key_add(&key, dr_i); key_add(&key, ozp_i);
+                        key_add(&key, E); key_add(&key, E > 1 ? sx : 0);
                         e = cache_find(ctx, key);
                         if (!e)
                         {
@@ -973,44 +1020,65 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                             e = cache_insert(ctx, key, std::move(ops), bytes, build);
                         }
                     }
+                    // (a verdict that cannot be read now: no reason to fill the block)
+                    if (E > 1 && (!e || e->unstable || (ctx->capturing && e->host_flag < 0)))
+                        return kNextForm;
                     bool lean_ok = false;
                     if (e)
                     {
-                        st = cache_use(ctx, e);
-                        if (st != TB200_OK)
-                            return st;
-                        block = e->block;
-                        st    = read_host_flag(ctx, e, flag_off);
-                        if (st != TB200_OK)
-                            return st;
+                        tb200_status est = cache_use(ctx, e);
+                        if (est == TB200_OK)
+                            est = read_host_flag(ctx, e, flag_off);
+                        if (est != TB200_OK)
+                            return est;
+                        block   = e->block;
                         lean_ok = e->host_flag == 1;
                     }
-                    else
+                    if (E > 1 && !lean_ok)
+                        return kNextForm;
+                    if (!e)
                     {
-                        st = ensure_scratch(ctx, bytes);
-                        if (st != TB200_OK)
-                            return st;
-                        st = build(ctx, ctx->scratch);
-                        if (st != TB200_OK)
-                            return st;
+                        tb200_status est = ensure_scratch(ctx, bytes);
+                        if (est == TB200_OK)
+                            est = build(ctx, ctx->scratch);
+                        if (est != TB200_OK)
+                            return est;
                         block = ctx->scratch;
                     }
-                    q.lean_ok         = lean_ok ? 1 : 0;
-                    int32_t* corr     = reinterpret_cast<int32_t*>(block) + prefix_elems;
+                    uint8_t* bytes_at = reinterpret_cast<uint8_t*>(block);
+                    if (E > 1)
+                        qe.b = block;
+                    qe.lean_ok        = lean_ok ? 1 : 0;
+                    int32_t* corr     = reinterpret_cast<int32_t*>(bytes_at + emb) + prefix_elems;
                     int32_t* mult_pad = corr + corr_elems;
-                    q.corr         = corr;
-                    q.corr_stride  = OCpad;
-                    q.corr_classes = cls_i;
-                    q.mult_pad     = mult_pad;
-                    q.shift_pad    = reinterpret_cast<int8_t*>(mult_pad + OCpad);
-                    // the lean form packs with int8 saturation: it serves RESCALEs to signed int8 only
-                    const bool lean_out = want_rec && output->dtype == TB200_INT8 && !epi.rs.out_unsigned;
-                    q.rec   = lean_out ? reinterpret_cast<const int32_t*>(reinterpret_cast<const uint8_t*>(block) + rec_off) : nullptr;
-                    q.delta = (lean_out && classes)
-                                  ? reinterpret_cast<const int32_t*>(reinterpret_cast<const uint8_t*>(block) + delta_off)
-                                  : nullptr;
-                    return tc_gemm_launch(ctx, q);
-                }
+                    qe.corr         = corr;
+                    qe.corr_stride  = OCpad;
+                    qe.corr_classes = cls_i;
+                    qe.mult_pad     = mult_pad;
+                    qe.shift_pad    = reinterpret_cast<int8_t*>(mult_pad + OCpad);
+                    qe.rec   = lean_out ? reinterpret_cast<const int32_t*>(bytes_at + rec_off) : nullptr;
+                    qe.delta = (lean_out && classes) ? reinterpret_cast<const int32_t*>(bytes_at + delta_off) : nullptr;
+                    if (join)
+                    {
+                        qe.join = join->block; qe.res = join->other;
+                        qe.join_double = join->double_round; qe.join_lo = join->lo; qe.join_hi = join->hi;
+                        if (!conv_chan_supported(ctx, qe))
+                            return kNeedsSeparateJoin;
+                    }
+                    return tc_gemm_launch(ctx, qe);
+                };
+                // At most 64 channels leave half of conv_chan_kernel's 128 rows empty: two pixels side by side fill them, at
+                // (KW + stride) / KW times the products (which the empty rows would have cost twice over).  Batch 256 at 56x56, 64
+                // to 64: 1x1 37 -> 25 us, 3x3 93 -> 61.  Small problems are a chain of latencies, which the longer products
+                // lengthen: 1x1 on 2x16x10x384 4.8 us against 4.2, 3x3 on 8x18x43x128 7.4 / 6.7, on 14x34x79x32 (9 282 pixels) 7.6 / 8.4.
+                const bool one = KH == 1 && KW == 1 && stride[0] == 1 && stride[1] == 1 && !padded && input->contiguous;
+                const bool two = lean_out && !view && use_cache && ctx->const_cache_on && OC == 64 && (int64_t)N * OH * OW >= 8192 && dilation[1] == 1 &&
+                                 (one ? (int64_t)N * OH * OW % 2 == 0 && (int64_t)N * OH * OW < (1 << 30) : OW % 2 == 0 && !(KH == 1 && KW == 1));
+                st = two ? run(2) : kNextForm;
+                if (st == kNextForm)
+                    st = run(1);
+                if (st != kNextForm)
+                    return st;
             }
             else
             {
@@ -1065,6 +1133,8 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
 
     if (view || dry_run)
         return kNeedsDenseOutput;
+    if (join)
+        return kNeedsSeparateJoin;
 
     // ---- few-channel int8 convolutions with a horizontal stride of 2 (the RGB stem), parity-split form: four bytes per
     // pixel and one padded copy per parity of the output column make the KW taps a 32-byte window at a 16-byte pitch,
@@ -2952,6 +3022,61 @@ extern "C" tb200_status tb200_add(tb200_ctx* ctx, const tb200_tensor* a, const t
     return post_launch(ctx, "add");
 }
 
+// Per-tensor legs with 32-bit scales and exact rounding, on signed tensors: what the tabulated and fused joins take
+static bool residual_simple(const tb200_ctx* ctx, const tb200_rescale_attr* a, const tb200_rescale_attr* b, const tb200_rescale_attr* o)
+{
+    return !a->per_channel && !b->per_channel && !o->per_channel && a->scale32 && b->scale32 && o->scale32 &&
+           a->rounding_mode != TB200_INEXACT_ROUND && b->rounding_mode != TB200_INEXACT_ROUND &&
+           o->rounding_mode != TB200_INEXACT_ROUND && !a->input_unsigned && !b->input_unsigned && !o->output_unsigned && ctx->policy == 0;
+}
+
+static ResidualFast residual_fast_args(const tb200_rescale_attr* a, const tb200_rescale_attr* b, const tb200_rescale_attr* o,
+                                       int32_t has_clamp, int32_t clamp_min, int32_t clamp_max)
+{
+    ResidualFast f;
+    auto leg = [](const tb200_rescale_attr* at) {
+        ResidualLeg l;
+        l.mult         = reinterpret_cast<const int32_t*>(at->multiplier->data);
+        l.shift        = reinterpret_cast<const int8_t*>(at->shift->data);
+        l.zp_in        = (int32_t)(int8_t)at->input_zp;
+        l.zp_out       = (int32_t)(int8_t)at->output_zp;
+        l.double_round = at->rounding_mode == TB200_DOUBLE_ROUND;
+        return l;
+    };
+    f.a = leg(a);
+    f.b = leg(b);
+    f.o = leg(o);
+    f.o.zp_in = 0;    // INT32 input of the last leg has no zero point (checked by make_rescale_dev)
+    // clip to int8, then CLAMP: one clip to [lo, hi]
+    f.lo = has_clamp ? std::min(std::max(-128, clamp_min), clamp_max) : -128;
+    f.hi = has_clamp ? std::min(std::max(127, clamp_min), clamp_max) : 127;
+    return f;
+}
+
+// What a block built from the join's three RESCALEs depends on, as cache key and operand ranges
+static void residual_key(std::string* key, int kind, const ResidualFast& f)
+{
+    key_add(key, kind);
+    for (const ResidualLeg* l : { &f.a, &f.b, &f.o })
+    {
+        key_add(key, l->mult); key_add(key, l->shift);
+        key_add(key, l->zp_in); key_add(key, l->zp_out); key_add(key, l->double_round);
+    }
+    key_add(key, f.lo); key_add(key, f.hi);
+}
+
+static std::vector<std::pair<const char*, size_t>> residual_operands(const tb200_rescale_attr* a, const tb200_rescale_attr* b,
+                                                                     const tb200_rescale_attr* o)
+{
+    std::vector<std::pair<const char*, size_t>> ops;
+    for (const tb200_rescale_attr* at : { a, b, o })
+    {
+        ops.push_back({ reinterpret_cast<const char*>(at->multiplier->data), at->multiplier->bytes });
+        ops.push_back({ reinterpret_cast<const char*>(at->shift->data), at->shift->bytes });
+    }
+    return ops;
+}
+
 extern "C" tb200_status tb200_residual_add(tb200_ctx* ctx, const tb200_tensor* a, const tb200_rescale_attr* a_attr,
                                            const tb200_tensor* b, const tb200_rescale_attr* b_attr,
                                            const tb200_rescale_attr* out_attr, int32_t has_clamp, int32_t clamp_min,
@@ -2987,29 +3112,9 @@ extern "C" tb200_status tb200_residual_add(tb200_ctx* ctx, const tb200_tensor* a
                            reinterpret_cast<uintptr_t>(output->data)) & 15) == 0;
     const bool pc = a_attr->per_channel || b_attr->per_channel || out_attr->per_channel;
     const int block = 256;
-    const bool simple = !pc && a_attr->scale32 && b_attr->scale32 && out_attr->scale32 &&
-                        a_attr->rounding_mode != TB200_INEXACT_ROUND && b_attr->rounding_mode != TB200_INEXACT_ROUND &&
-                        out_attr->rounding_mode != TB200_INEXACT_ROUND && !a_attr->input_unsigned &&
-                        !b_attr->input_unsigned && !out_attr->output_unsigned && ctx->policy == 0;
-    if (simple && aligned && n % 16 == 0)
+    if (residual_simple(ctx, a_attr, b_attr, out_attr) && aligned && n % 16 == 0)
     {
-        ResidualFast f;
-        auto leg = [](const tb200_rescale_attr* at) {
-            ResidualLeg l;
-            l.mult         = reinterpret_cast<const int32_t*>(at->multiplier->data);
-            l.shift        = reinterpret_cast<const int8_t*>(at->shift->data);
-            l.zp_in        = (int32_t)(int8_t)at->input_zp;
-            l.zp_out       = (int32_t)(int8_t)at->output_zp;
-            l.double_round = at->rounding_mode == TB200_DOUBLE_ROUND;
-            return l;
-        };
-        f.a = leg(a_attr);
-        f.b = leg(b_attr);
-        f.o = leg(out_attr);
-        f.o.zp_in = 0;    // INT32 input of the last leg has no zero point (checked above)
-        // clip to int8, then CLAMP: one clip to [lo, hi]
-        f.lo = has_clamp ? std::min(std::max(-128, clamp_min), clamp_max) : -128;
-        f.hi = has_clamp ? std::min(std::max(127, clamp_min), clamp_max) : 127;
+        const ResidualFast f = residual_fast_args(a_attr, b_attr, out_attr, has_clamp, clamp_min, clamp_max);
         // Large joins pay for tabulating all 65536 byte pairs first (two launches, one lookup per element after that)
         if (n >= ((int64_t)1 << 22))
         {
@@ -3024,24 +3129,10 @@ extern "C" tb200_status tb200_residual_add(tb200_ctx* ctx, const tb200_tensor* a
             if (ctx->const_cache_on)
             {
                 std::string key;
-                key_add(&key, (int)3);
-                for (const ResidualLeg* l : { &f.a, &f.b, &f.o })
-                {
-                    key_add(&key, l->mult); key_add(&key, l->shift);
-                    key_add(&key, l->zp_in); key_add(&key, l->zp_out); key_add(&key, l->double_round);
-                }
-                key_add(&key, f.lo); key_add(&key, f.hi);
+                residual_key(&key, 3, f);
                 e = cache_find(ctx, key);
                 if (!e)
-                {
-                    std::vector<std::pair<const char*, size_t>> ops;
-                    for (const tb200_rescale_attr* at : { a_attr, b_attr, out_attr })
-                    {
-                        ops.push_back({ reinterpret_cast<const char*>(at->multiplier->data), at->multiplier->bytes });
-                        ops.push_back({ reinterpret_cast<const char*>(at->shift->data), at->shift->bytes });
-                    }
-                    e = cache_insert(ctx, key, std::move(ops), kTableSmem, build);
-                }
+                    e = cache_insert(ctx, key, residual_operands(a_attr, b_attr, out_attr), kTableSmem, build);
             }
             uint8_t* table = nullptr;
             if (e)
@@ -3125,6 +3216,70 @@ extern "C" tb200_status tb200_residual_add(tb200_ctx* ctx, const tb200_tensor* a
             reinterpret_cast<const int8_t*>(a->data), reinterpret_cast<const int8_t*>(b->data),
             reinterpret_cast<int8_t*>(output->data), n, C, r, ctx->d_status);
     return post_launch(ctx, "residual_add_i8");
+}
+
+extern "C" tb200_status tb200_conv2d_add(tb200_ctx* ctx, const tb200_tensor* input, const tb200_tensor* weight,
+                                         const tb200_tensor* bias, int32_t input_zp, int32_t weight_zp, const int32_t pad[4],
+                                         const int32_t stride[2], const int32_t dilation[2], const tb200_epilogue* epilogue,
+                                         const tb200_rescale_attr* conv_attr, const tb200_tensor* other,
+                                         const tb200_rescale_attr* other_attr, const tb200_rescale_attr* out_attr,
+                                         int32_t has_clamp, int32_t clamp_min, int32_t clamp_max, tb200_tensor* output)
+{
+    if (!ctx)
+        return TB200_ERROR;
+    TB200_ENTER(ctx);
+    TB200_ERROR_IF(ctx, !output || !other || !conv_attr || !other_attr || !out_attr, "conv2d_add: null operand");
+    TB200_ERROR_IF(ctx, !all_contiguous({ other, output }), "%s: zero-copy views are accepted only as the CONV2D input; this operand must be contiguous", "conv2d_add");
+    TB200_ERROR_IF(ctx, !same_shape(other, output), "residual_add: operand shapes differ");
+    TB200_ERROR_IF(ctx, other->dtype != TB200_INT8 || output->dtype != TB200_INT8, "residual_add: INT8 tensors only");
+    TB200_ERROR_IF(ctx, has_clamp && clamp_max < clamp_min, "OpClamp: max smaller than min");
+    const int C = output->rank > 0 ? output->shape[output->rank - 1] : 1;
+    RescaleDev rs;
+    tb200_status st = make_rescale_dev(ctx, conv_attr, TB200_INT8, TB200_INT32, C, &rs);
+    if (st == TB200_OK)
+        st = make_rescale_dev(ctx, other_attr, TB200_INT8, TB200_INT32, C, &rs);
+    if (st == TB200_OK)
+        st = make_rescale_dev(ctx, out_attr, TB200_INT32, TB200_INT8, C, &rs);
+    if (st != TB200_OK)
+        return st;
+    // the output holds the convolution's results first where the two run one after the other
+    const char* lo = reinterpret_cast<const char*>(output->data);
+    const char* ot = reinterpret_cast<const char*>(other->data);
+    TB200_ERROR_IF(ctx, ot < lo + output->bytes && lo < ot + other->bytes, "conv2d_add: the output must not overlap the other operand");
+    if (residual_simple(ctx, conv_attr, other_attr, out_attr) && ctx->const_cache_on)
+    {
+        const ResidualFast f = residual_fast_args(conv_attr, other_attr, out_attr, has_clamp, clamp_min, clamp_max);
+        auto build = [=](tb200_ctx* c, void* block) -> tb200_status {
+            residual_record_kernel<<<1, 256, 0, c->stream>>>(f, reinterpret_cast<int32_t*>(block));
+            return post_launch(c, "residual_record");
+        };
+        std::string key;
+        residual_key(&key, 12, f);
+        Prepared* e = cache_find(ctx, key);
+        if (!e)
+            e = cache_insert(ctx, key, residual_operands(conv_attr, other_attr, out_attr), kJoinWords * sizeof(int32_t), build);
+        if (e)
+        {
+            st = cache_use(ctx, e);
+            if (st == TB200_OK)
+                st = read_host_flag(ctx, e, kJoinUsable * sizeof(int32_t));
+            if (st != TB200_OK)
+                return st;
+            // a record that is not usable runs in the kernel's general form, which is slower than two kernels: only where
+            // constants change under a captured graph
+            if (e->host_flag == 1)
+            {
+                const ConvJoin j = { reinterpret_cast<const int32_t*>(e->block), other->data, f.o.double_round, f.lo, f.hi };
+                st = conv2d_impl(ctx, input, weight, bias, input_zp, weight_zp, pad, stride, dilation, epilogue, output, nullptr, false, true, &j);
+                if (st != kNeedsSeparateJoin)
+                    return st;
+            }
+        }
+    }
+    st = conv2d_impl(ctx, input, weight, bias, input_zp, weight_zp, pad, stride, dilation, epilogue, output, nullptr, false, true);
+    if (st != TB200_OK)
+        return st;
+    return tb200_residual_add(ctx, output, conv_attr, other, other_attr, out_attr, has_clamp, clamp_min, clamp_max, output);
 }
 
 // =================================================================================================== pools

@@ -1,5 +1,6 @@
 // Shared host-side definitions of the tb200 library: context, tensor handle, status helpers.
 #pragma once
+#include <bitset>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -97,7 +98,7 @@ struct tb200_ctx
     int join_stream      = 1;    // large table joins through the bulk-copy ring kernel (join_stream.cuh)
     int launch_overlap   = 1;    // launch the kernels that support it with programmatic stream serialization
     int max_pairs[3]     = { 0, 0, 0 };    // resident CTA pairs of the three CTA-pair kernels on this device, 0 = not asked yet
-    uint64_t smem_attr_set = 0;            // bit per kernel whose dynamic shared-memory limit has been raised on this device
+    std::bitset<128> smem_attr_set;        // bit per kernel whose dynamic shared-memory limit has been raised on this device
     // output gather across GPUs (dist.cu): an NCCL communicator created by tb200_comm_init or handed in by the host
     void* comm           = nullptr;
     bool comm_owned      = false;
@@ -322,6 +323,11 @@ struct TcProblem
     // tc_conv_lean_kernel only: the batch dimension is (image, parity of the output column): batch index 2 n + p holds
     // the output columns 2 ox' + p of image n; out_ow_real is the true output width (OW is the per-parity width)
     int xpar, out_ow_real;
+    // conv_chan_kernel only: residual join behind the RESCALE.  join: block of kJoinWords words, res: the other operand, a
+    // dense int8 tensor of the output's shape; join_lo / join_hi: clip range of the join's result
+    const int32_t* join;
+    const void* res;
+    int join_double, join_lo, join_hi;
     int double_round;
     int32_t out_zp;
     int32_t clamp_lo, clamp_hi;    // also the dtype range
@@ -348,6 +354,19 @@ void* tensor_map_encode_fn();
 // interior pixels (q.a_fill is what taps outside the image read).
 bool tc_any_supported(const tb200_ctx* ctx, const TcProblem& q);
 tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q);
+
+// int8 CONV2D + RESCALE with channels on the accumulator rows (conv_chan.cu), q.lean_ok problems; with q.join the residual join
+// RESCALE, RESCALE, ADD, RESCALE, CLAMP runs on the results before they are stored
+bool conv_chan_supported(const tb200_ctx* ctx, const TcProblem& q);
+tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q);
+// Words of the block behind q.join (residual_record_kernel): with both legs exact multiples of their operand, sum * pk + c is
+// one dp2a of (convolution result, other operand) with the two 16-bit coefficients, followed by rescale_rec_apply's second
+// half; the rest serves joins where that does not hold (usable == 0)
+enum : int
+{
+    kJoinCoef = 0, kJoinC, kJoinM, kJoinSh, kJoinRlo, kJoinRhi, kJoinUsable, kJoinOutMult, kJoinOutShift, kJoinOutZp, kJoinOutDouble,
+    kJoinLutA = 16, kJoinLutB = 272, kJoinBadA = 528, kJoinBadB = 784, kJoinWords = 1040
+};
 
 // int8 MATMUL on CTA pairs (tc_gemm_pair.cu): large MN-major-B problems with int32 output; tc_gemm_launch routes to it
 bool tc_gemm_pair_supported(const TcProblem& p, int num_sms);

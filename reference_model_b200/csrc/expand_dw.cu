@@ -635,7 +635,7 @@ tb200_status expand_dw_launch(tb200_ctx* ctx, const ExpandDwProblem& q)
                               : reinterpret_cast<const void*>(&expand_dw_kernel<__half>);
     const XdLayout lay = xd_layout(q, kXdStages);
     const int attr_bit = bf16 ? 13 : 12;
-    if (!(ctx->smem_attr_set & (1u << attr_bit)))    // several CTAs of this size per SM need the largest shared-memory carve-out
+    if (!ctx->smem_attr_set.test((size_t)attr_bit))    // several CTAs of this size per SM need the largest shared-memory carve-out
         TB200_CUDA_CHECK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     tb200_status st = raise_smem_limit(ctx, attr_bit, kernel, lay.smem_bytes);
     if (st != TB200_OK)

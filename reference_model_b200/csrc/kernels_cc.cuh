@@ -347,6 +347,63 @@ __global__ void __launch_bounds__(256) residual_add_i8_fast_kernel(const int8_t*
         atomicOr(status, TB200_DEV_UNPREDICTABLE);
 }
 
+// Record of a residual join that runs inside the convolution that makes its first operand (conv_chan.cu).  The legs to INT32
+// have 256 values each; where both are exact multiples (k * q + constant, as every power-of-two scale is) the sum is one
+// dp2a of the two bytes and the RESCALE back to int8 takes the lean form with the sum's static bound.  The tables serve the
+// kernel where that does not hold.  One block of 256 threads.
+__global__ void __launch_bounds__(256) residual_record_kernel(ResidualFast r, int32_t* __restrict__ block)
+{
+    __shared__ int32_t lut[2][256];
+    const int i = threadIdx.x;
+    bool fits   = true;
+    for (int leg = 0; leg < 2; leg++)
+    {
+        int32_t vlim;
+        const Scale32Fast c = make_scale32_fast(leg == 0 ? r.a : r.b, &vlim);
+        const int32_t x     = i - 128 - c.zp_in;
+        bool ov             = (x > vlim) || (x < ~vlim);
+        const int32_t y     = scale32_fast(x, c, ov);
+        lut[leg][i]         = y;
+        block[(leg ? kJoinLutB : kJoinLutA) + i] = y;
+        block[(leg ? kJoinBadB : kJoinBadA) + i] = ov ? 1 : 0;
+        fits = fits && !ov;
+    }
+    __syncthreads();
+    int64_t k[2];
+    for (int leg = 0; leg < 2; leg++)
+    {
+        k[leg] = (int64_t)lut[leg][1] - lut[leg][0];
+        fits   = fits && (int64_t)lut[leg][i] == (int64_t)lut[leg][0] + k[leg] * i;
+    }
+    const bool linear = __syncthreads_and(fits) != 0;
+    if (i != 0)
+        return;
+    const int32_t m = __ldg(r.o.mult), sh = (int32_t)__ldg(r.o.shift);
+    const int64_t c0 = (int64_t)lut[0][0] + lut[1][0] + 128 * (k[0] + k[1]);
+    int64_t vmax = 0;
+    for (int e = 0; e < 4; e++)
+    {
+        const int64_t t = c0 + k[0] * (e & 1 ? 127 : -128) + k[1] * (e & 2 ? 127 : -128);
+        vmax = t < 0 ? (-t > vmax ? -t : vmax) : (t > vmax ? t : vmax);
+    }
+    bool ok = linear && vmax < ((int64_t)1 << 31);
+    int32_t rec[8];
+    rescale_rec_build(m, sh, r.o.double_round, r.o.zp_out, ok ? (int32_t)c0 : 0, vmax, rec);
+    const int64_t ca = k[0] * rec[1], cb = k[1] * rec[1];    // 16-bit coefficients
+    ok = ok && rec[7] == 1 && ca >= -32768 && ca <= 32767 && cb >= -32768 && cb <= 32767;
+    block[kJoinCoef]   = ok ? (int32_t)(((uint32_t)ca & 0xffffu) | ((uint32_t)cb << 16)) : 0;
+    block[kJoinC]      = rec[2];
+    block[kJoinM]      = rec[0];
+    block[kJoinSh]     = rec[3];
+    block[kJoinRlo]    = rec[4];
+    block[kJoinRhi]    = rec[5];
+    block[kJoinUsable] = ok ? 1 : 0;
+    block[kJoinOutMult]   = m;
+    block[kJoinOutShift]  = sh;
+    block[kJoinOutZp]     = r.o.zp_out;
+    block[kJoinOutDouble] = r.o.double_round;
+}
+
 // Residual join through one table.  With per-tensor parameters the whole RESCALE, RESCALE, ADD, RESCALE, CLAMP chain is
 // a function of the two input bytes alone.  residual_table_kernel evaluates it for all 65536 byte pairs (with every
 // REQUIRE verdict as one bit per pair), and residual_add_i8_table_kernel keeps the table in shared memory and spends one
@@ -1677,14 +1734,17 @@ __global__ void __launch_bounds__(256) matmul_col_corr_kernel(const int8_t* __re
 // rescale_rec_build) and, for padded layers with an input zero point, `delta`: per class of clipped tap rectangle the
 // difference between that class's correction row and the interior one (all taps in scope), which border pixels add
 // to their accumulators before the common arithmetic.  `all_ok`, preset to non-zero by the caller, is cleared when some
-// column's record is unusable.
+// column's record is unusable.  With E > 1 the OC rows are E blocks of OC / E channels, block e for the e-th of E pixels side by
+// side: the filter of KW0 taps sits e * step taps into a window of KW, zeros elsewhere, and is written to `embedded`
+// ([OC][KH][KW][IC]) in the same pass.
 __global__ void conv_epilogue_tables_kernel(const int8_t* __restrict__ w, const int32_t* __restrict__ bias, int bias_n,
                                             int OC, int OCpad, int KH, int KW, int IC, int32_t in_zp, int classes,
                                             const int32_t* __restrict__ mult, const int8_t* __restrict__ shift,
                                             int per_channel, int32_t* __restrict__ prefix, int32_t* __restrict__ corr,
                                             int32_t* __restrict__ mult_pad, int8_t* __restrict__ shift_pad,
                                             int32_t* __restrict__ rec = nullptr, int32_t* __restrict__ delta = nullptr,
-                                            int double_round = 0, int32_t out_zp = 0, int* __restrict__ all_ok = nullptr)
+                                            int double_round = 0, int32_t out_zp = 0, int* __restrict__ all_ok = nullptr,
+                                            int E = 1, int KW0 = 0, int step = 0, int8_t* __restrict__ embedded = nullptr)
 {
     // One warp per output channel: lanes split the channel run of each tap (128-bit loads), the warp-reduced tap
     // sums become 2-D prefix sums kept in registers by lane 0 .. and mirrored to `prefix` for the class loop, which
@@ -1713,15 +1773,31 @@ __global__ void conv_epilogue_tables_kernel(const int8_t* __restrict__ w, const 
         return;
     }
     int32_t* P = prefix + (int64_t)oc * H1 * W1;    // this channel's (KH+1) x (KW+1) prefix sums
+    // E > 1: row oc is channel src's filter of KW0 taps, `first` taps into a window of KW; the row is written as well
+    const int src   = E > 1 ? oc % (OC / E) : oc;
+    const int first = E > 1 ? oc / (OC / E) * step : 0;
+    const int taps0 = E > 1 ? KW0 : KW;
     for (int ky = 0; ky <= KH; ky++)
         for (int kx = 0; kx <= KW; kx++)
         {
             int32_t v = 0;
             if (ky > 0 && kx > 0)
             {
-                const int8_t* wp = w + (((int64_t)oc * KH + (ky - 1)) * KW + (kx - 1)) * IC;
+                const int k      = kx - 1 - first;
+                const bool tap   = k >= 0 && k < taps0;
+                const int8_t* wp = w + (((int64_t)src * KH + (ky - 1)) * taps0 + (tap ? k : 0)) * IC;
                 int32_t s        = 0;
-                if ((IC & 15) == 0)
+                if (embedded)
+                {
+                    // (whole 32-byte channel runs)
+                    int4* row = reinterpret_cast<int4*>(embedded + (((int64_t)oc * KH + (ky - 1)) * KW + (kx - 1)) * IC);
+                    for (int i = lane; i < IC / 16; i += 32)
+                        row[i] = tap ? __ldg(reinterpret_cast<const int4*>(wp) + i) : make_int4(0, 0, 0, 0);
+                }
+                if (!tap)
+                {
+                }
+                else if ((IC & 15) == 0)
                 {
                     for (int ic = lane * 16; ic < IC; ic += 512)
                     {
@@ -1749,7 +1825,7 @@ __global__ void conv_epilogue_tables_kernel(const int8_t* __restrict__ w, const 
             }
         }
     __syncwarp();
-    const int32_t b = bias[bias_n == 1 ? 0 : oc];
+    const int32_t b = bias[bias_n == 1 ? 0 : src];
     const int32_t corr_interior = b - in_zp * P[KH * W1 + KW];    // every tap in scope
     if (!classes)
     {
@@ -1771,15 +1847,15 @@ __global__ void conv_epilogue_tables_kernel(const int8_t* __restrict__ w, const 
     }
     if (mult_pad && lane == 0)
     {
-        mult_pad[oc]  = mult[per_channel ? oc : 0];
-        shift_pad[oc] = shift[per_channel ? oc : 0];
+        mult_pad[oc]  = mult[per_channel ? src : 0];
+        shift_pad[oc] = shift[per_channel ? src : 0];
     }
     if (rec && lane == 0)
     {
         // largest magnitude bias + accumulator can reach: every tap at full scale |x - zp| <= 255, |w| <= 128
         const int64_t vmax = (int64_t)KH * KW * IC * 255 * 128 + (b < 0 ? -(int64_t)b : (int64_t)b);
         int32_t r8[8];
-        rescale_rec_build(mult[per_channel ? oc : 0], (int32_t)shift[per_channel ? oc : 0], double_round, out_zp,
+        rescale_rec_build(mult[per_channel ? src : 0], (int32_t)shift[per_channel ? src : 0], double_round, out_zp,
                           corr_interior, vmax, r8);
 #pragma unroll
         for (int i = 0; i < 8; i++)
