@@ -291,6 +291,35 @@ def fuse(graph):
     return steps
 
 
+def fuse_joins(graph, steps):
+    """Second pass over fuse()'s steps: a residual join moves into the int8 convolution that makes one of its operands, when
+    nothing else reads that operand and the other one is there by then (the later of two convolutions takes it).  Returns the
+    new steps and {tensor that no longer reaches device memory: its CONV_RESCALE_CLAMP step}."""
+    cons = graph.consumers()
+    last = lambda step: [o for o in (step[1] if isinstance(step[1], tuple) else (step[1],)) if o is not None][-1]
+    where = {last(step).outputs[0]: i for i, step in enumerate(steps)}
+    out, inside = list(steps), {}
+    for i, (kind, p) in enumerate(steps):
+        if kind != "RESIDUAL_JOIN":
+            continue
+        ra, rb, add, ro, c = p
+        best = None
+        for mine, leg, other in ((ra.inputs[0], ra, rb), (rb.inputs[0], rb, ra)):
+            j = where.get(mine)
+            if j is None or steps[j][0] != "CONV_RESCALE_CLAMP" or steps[j][1][0].kind != "CONV2D" or mine == other.inputs[0]:
+                continue
+            if cons.get(mine, []) != [leg] or mine in graph.outputs or where.get(other.inputs[0], -1) > j:
+                continue
+            if best is None or j > best[0]:
+                best = (j, mine, leg, other)
+        if best is None:
+            continue
+        j, mine, leg, other = best
+        out[j], out[i] = ("CONV_JOIN", steps[j][1] + (leg, other, add, ro, c)), None
+        inside[mine] = steps[j]
+    return [s for s in out if s is not None], inside
+
+
 # ------------------------------------------------------------------------------------------------ device runner
 class DeviceRunner:
     """Evaluates a Graph on one tb200 context.  Constants are uploaded once (they are CONST node outputs in the
@@ -303,7 +332,7 @@ class DeviceRunner:
         self.t = dict(external or {})
         for name_, arr in graph.consts.items():
             self.t[name_] = ctx.from_numpy(arr, graph.meta[name_][0])
-        self.steps = fuse(graph) if fused else [(op.kind, op) for op in graph.ops]
+        self.steps, self._inside = fuse_joins(graph, fuse(graph)) if fused else ([(op.kind, op) for op in graph.ops], {})
         produced = set()
         for kind, payload in self.steps:
             ops = payload if isinstance(payload, tuple) else (payload,)
@@ -364,6 +393,14 @@ class DeviceRunner:
                 ctx.residual_add(t[ra.inputs[0]], self._rescale_attr(ra), t[rb.inputs[0]], self._rescale_attr(rb),
                                  self._rescale_attr(ro), t[out],
                                  (c.attr["min_val"], c.attr["max_val"]) if c else None)
+            elif kind == "CONV_JOIN":
+                conv, r, c, leg, other, add, ro, cj = p
+                epi = tb.Epilogue(self._rescale_attr(r), (c.attr["min_val"], c.attr["max_val"]) if c else None)
+                a = conv.attr
+                ctx.conv2d_add(t[conv.inputs[0]], t[conv.inputs[1]], t[conv.inputs[2]], t[(cj or ro).outputs[0]], a["pad"],
+                               a["stride"], a["dilation"], a["input_zp"], a["weight_zp"], epi, self._rescale_attr(leg),
+                               t[other.inputs[0]], self._rescale_attr(other), self._rescale_attr(ro),
+                               (cj.attr["min_val"], cj.attr["max_val"]) if cj else None)
             elif kind == "CONV_DW":
                 conv, c1, dw, c2 = p
                 e1 = tb.Epilogue(None, (c1.attr["min_val"], c1.attr["max_val"])) if c1 else None
@@ -447,6 +484,11 @@ class DeviceRunner:
             self.captured = self.ctx.capture_end()
 
     def output(self, name_=None):
+        if name_ in self._inside and name_ not in self.t:
+            # a result that stays inside a fused step: its operator on its own, on the inputs of the last evaluation
+            self.t[name_] = self.ctx.empty(*self.graph.meta[name_])
+        if name_ in self._inside:
+            self._eval([self._inside[name_]])
         st, out = self.t[name_ or self.graph.outputs[0]].download()
         return st, out
 
