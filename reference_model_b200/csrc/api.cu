@@ -813,7 +813,7 @@ struct ConvJoin
 {
     const int32_t* block;    // residual_record_kernel
     const void* other;
-    int double_round, lo, hi;
+    int f32, lo, hi;
 };
 static const tb200_status kNeedsSeparateJoin = (tb200_status)-78;
 
@@ -828,7 +828,7 @@ static tb200_status read_host_flag(tb200_ctx* ctx, Prepared* e, size_t offset)
     TB200_CUDA_CHECK(ctx, cudaMemcpyAsync(ctx->h_status, reinterpret_cast<const uint8_t*>(e->block) + offset, sizeof(int),
                                           cudaMemcpyDeviceToHost, ctx->stream));
     TB200_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-    e->host_flag = *ctx->h_status != 0 ? 1 : 0;
+    e->host_flag = *ctx->h_status == 0 ? 0 : *ctx->h_status == 0x01010101 ? 2 : 1;
     return TB200_OK;
 }
 
@@ -1032,7 +1032,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                         if (est != TB200_OK)
                             return est;
                         block   = e->block;
-                        lean_ok = e->host_flag == 1;
+                        lean_ok = e->host_flag >= 1;
                     }
                     if (E > 1 && !lean_ok)
                         return kNextForm;
@@ -1061,7 +1061,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     if (join)
                     {
                         qe.join = join->block; qe.res = join->other;
-                        qe.join_double = join->double_round; qe.join_lo = join->lo; qe.join_hi = join->hi;
+                        qe.join_f32 = join->f32; qe.join_lo = join->lo; qe.join_hi = join->hi;
                         if (!conv_chan_supported(ctx, qe))
                             return kNeedsSeparateJoin;
                     }
@@ -1224,7 +1224,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                 q.mult_pad    = mult_pad;
                 q.shift_pad   = reinterpret_cast<int8_t*>(mult_pad + OCpad);
                 q.rec         = reinterpret_cast<const int32_t*>(wr + wr_bytes + rec_off);
-                q.lean_ok     = e->host_flag == 1 ? 1 : 0;
+                q.lean_ok     = e->host_flag >= 1 ? 1 : 0;
                 // the scratch address enters the plan only as a pointer: any 16-byte aligned value serves the dry run
                 q.a = ctx->scratch ? ctx->scratch : reinterpret_cast<const void*>(static_cast<uintptr_t>(256));
                 if (q.lean_ok && tc_gemm_lean_supported(ctx, q))
@@ -1345,7 +1345,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     st = cache_use(ctx, e);
                     if (st == TB200_OK)
                         st = read_host_flag(ctx, e, wr_bytes + flag_off);
-                    q.lean_ok = e->host_flag == 1 ? 1 : 0;
+                    q.lean_ok = e->host_flag >= 1 ? 1 : 0;
                 }
                 else
                     st = build(ctx, wr);
@@ -3267,9 +3267,9 @@ extern "C" tb200_status tb200_conv2d_add(tb200_ctx* ctx, const tb200_tensor* inp
                 return st;
             // a record that is not usable runs in the kernel's general form, which is slower than two kernels: only where
             // constants change under a captured graph
-            if (e->host_flag == 1)
+            if (e->host_flag >= 1)
             {
-                const ConvJoin j = { reinterpret_cast<const int32_t*>(e->block), other->data, f.o.double_round, f.lo, f.hi };
+                const ConvJoin j = { reinterpret_cast<const int32_t*>(e->block), other->data, e->host_flag == 2 ? 1 : 0, f.lo, f.hi };
                 st = conv2d_impl(ctx, input, weight, bias, input_zp, weight_zp, pad, stride, dilation, epilogue, output, nullptr, false, true, &j);
                 if (st != kNeedsSeparateJoin)
                     return st;

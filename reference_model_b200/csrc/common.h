@@ -57,7 +57,8 @@ struct Prepared
     size_t bytes  = 0;
     bool valid    = false;    // the block holds what the operands' current contents give
     bool unstable = false;    // an operator wrote into an operand: rebuild before every use
-    int host_flag = -1;       // a verdict the builder left in the block and the host has read back (-1: not read yet)
+    int host_flag = -1;       // a verdict the builder left in the block and the host has read back (-1: not read yet): 0 no, 2 for
+                              // 0x01010101, 1 for any other word
     bool used     = false;    // a kernel that reads the verdict itself has run on the block
     uint64_t last_use = 0;
     // enqueues, on the context's stream, the kernels that fill `block` from the operands
@@ -327,7 +328,7 @@ struct TcProblem
     // dense int8 tensor of the output's shape; join_lo / join_hi: clip range of the join's result
     const int32_t* join;
     const void* res;
-    int join_double, join_lo, join_hi;
+    int join_f32, join_lo, join_hi;
     int double_round;
     int32_t out_zp;
     int32_t clamp_lo, clamp_hi;    // also the dtype range
@@ -359,9 +360,10 @@ tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q);
 // RESCALE, RESCALE, ADD, RESCALE, CLAMP runs on the results before they are stored
 bool conv_chan_supported(const tb200_ctx* ctx, const TcProblem& q);
 tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q);
-// Words of the block behind q.join (residual_record_kernel): with both legs exact multiples of their operand, sum * pk + c is
+// Words of the block behind q.join (residual_record_kernel): with both legs exact multiples of their operand, the sum is
 // one dp2a of (convolution result, other operand) with the two 16-bit coefficients, followed by rescale_rec_apply's second
-// half; the rest serves joins where that does not hold (usable == 0)
+// half (usable == 1; sum and constant are scaled by pk) or by join_f32_apply (usable == 0x01010101: M, Sh and Rlo are its
+// S, d and base, and C holds its 0x4B400000); the rest serves joins where neither holds (usable == 0)
 enum : int
 {
     kJoinCoef = 0, kJoinC, kJoinM, kJoinSh, kJoinRlo, kJoinRhi, kJoinUsable, kJoinOutMult, kJoinOutShift, kJoinOutZp, kJoinOutDouble,

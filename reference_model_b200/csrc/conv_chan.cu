@@ -75,33 +75,42 @@ __device__ __forceinline__ uint32_t chan_pack4(int a, int b, int c, int d)
     return r;
 }
 
-// A join whose record is not usable (a leg that is no multiple of its operand, constants out of range): the four pairs
-// of a word through the tabulated legs and the exact arithmetic, REQUIRE conditions reported.
-__device__ __noinline__ uint32_t chan_join_general(uint32_t qa, uint32_t qb, const int32_t* blk, int lo, int hi, int* status)
+// A join whose record is not usable (constants uploaded under a captured graph): the pairs of four words through the tabulated
+// legs and the exact arithmetic, REQUIRE conditions reported for the words of `real`.  Reads the other operand from the slot and
+// stores the results there.
+__device__ __noinline__ void chan_join_general(uint32_t dst, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, const int32_t* blk, int lo, int hi,
+                                               uint32_t real, int* status)
 {
     const int32_t m = blk[kJoinOutMult], sh = blk[kJoinOutShift], zp = blk[kJoinOutZp];
     const bool dr = blk[kJoinOutDouble] != 0;
-    uint32_t w    = 0;
-    bool bad      = false;
-    for (int j = 0; j < 4; j++)
+    bool any      = false;
+    for (int q = 0; q < 4; q++)
     {
-        const int ia = (int)((qa >> (8 * j)) & 0xffu) ^ 0x80, ib = (int)((qb >> (8 * j)) & 0xffu) ^ 0x80;
-        const int32_t ya = blk[kJoinLutA + ia], yb = blk[kJoinLutB + ib];
-        bad = bad || blk[kJoinBadA + ia] != 0 || blk[kJoinBadB + ib] != 0;
-        const int32_t sum = (int32_t)((uint32_t)ya + (uint32_t)yb);
-        bad = bad || ((ya ^ sum) & (yb ^ sum)) < 0;
-        const int64_t r = (int64_t)apply_scale_32_dev(sum, m, sh, dr, bad) + zp;
-        bad = bad || r > 2147483647LL || r < -2147483648LL;
-        const int32_t z = min(max((int32_t)r, lo), hi);
-        w |= (uint32_t)(z & 0xff) << (8 * j);
+        const uint32_t qa = q == 0 ? w0 : q == 1 ? w1 : q == 2 ? w2 : w3;
+        uint32_t qb, w = 0;
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(qb) : "r"(dst + (uint32_t)q * 128u));
+        bool bad = false;
+        for (int j = 0; j < 4; j++)
+        {
+            const int ia = (int)((qa >> (8 * j)) & 0xffu) ^ 0x80, ib = (int)((qb >> (8 * j)) & 0xffu) ^ 0x80;
+            const int32_t ya = blk[kJoinLutA + ia], yb = blk[kJoinLutB + ib];
+            bad = bad || blk[kJoinBadA + ia] != 0 || blk[kJoinBadB + ib] != 0;
+            const int32_t sum = (int32_t)((uint32_t)ya + (uint32_t)yb);
+            bad = bad || ((ya ^ sum) & (yb ^ sum)) < 0;
+            const int64_t r = (int64_t)apply_scale_32_dev(sum, m, sh, dr, bad) + zp;
+            bad = bad || r > 2147483647LL || r < -2147483648LL;
+            const int32_t z = min(max((int32_t)r, lo), hi);
+            w |= (uint32_t)(z & 0xff) << (8 * j);
+        }
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (uint32_t)q * 128u), "r"(w) : "memory");
+        any = any || (bad && (real >> q & 1u));
     }
-    if (bad && status != nullptr)
+    if (any)
         atomicOr(status, TB200_DEV_UNPREDICTABLE);
-    return w;
 }
 
 // CLASSES: padding with a non-zero input zero point, border pixels add what their clipped window leaves out.  FIX: the
-// RESCALE has double_round.  JOIN: 0 none, 1 residual join whose RESCALE to int8 has no double_round, 2 with it.
+// RESCALE has double_round.  JOIN: 0 none, 1 residual join in integers, 2 in single precision.
 template <bool CLASSES, bool FIX, int JOIN>
 __global__ void __launch_bounds__(kChanThreads, 1) conv_chan_kernel(const __grid_constant__ ChanParams p)
 {
@@ -332,8 +341,10 @@ __global__ void __launch_bounds__(kChanThreads, 1) conv_chan_kernel(const __grid
             jsh   = p.join[kJoinSh];
             jrlo  = p.join[kJoinRlo];
             jrhi  = p.join[kJoinRhi];
-            jusable = p.join[kJoinUsable] != 0;
+            // (the coefficients of the two forms differ)
+            jusable = JOIN == 2 ? p.join[kJoinUsable] == 0x01010101 : p.join[kJoinUsable] == 1;
         }
+        const int32_t jfix = JOIN && p.join[kJoinOutDouble] ? -1 : 0;
         int cur_cb = -1;
         bool ok    = true;
         int tile   = (int)blockIdx.x;
@@ -466,11 +477,20 @@ __global__ void __launch_bounds__(kChanThreads, 1) conv_chan_kernel(const __grid
                     }
                     if (JOIN)
                     {
+                        if (!jusable)
+                        {
+                            // (pixels and channels past the end hold no operands: whatever they give is not stored and says nothing)
+                            uint32_t real = 0;
+                            for (int q = 0; q < 4; q++)
+                                if (pb * p.px + group * cols + c0 + 4 * q + t < p.pixels && cb * 128 + quarter * 32 + (lane & ~3) < p.OC)
+                                    real |= 1u << q;
+                            chan_join_general(dst, w[0], w[1], w[2], w[3], p.join, p.join_lo, p.join_hi, real, p.status);
+                            return;
+                        }
                         uint32_t r[4];
 #pragma unroll
                         for (int q = 0; q < 4; q++)
                             asm volatile("ld.shared.b32 %0, [%1];" : "=r"(r[q]) : "r"(dst + (uint32_t)q * 128u));
-                        if (jusable)
                         {
 #pragma unroll
                             for (int q = 0; q < 4; q++)
@@ -484,11 +504,13 @@ __global__ void __launch_bounds__(kChanThreads, 1) conv_chan_kernel(const __grid
 #pragma unroll
                                 for (int e = 0; e < 4; e++)
                                 {
-                                    const int64_t P = (int64_t)s[e] * (int64_t)jm + (int64_t)(((uint64_t)(uint32_t)jrhi << 32) | (uint32_t)jrlo);
-                                    int32_t hi      = (int32_t)(P >> 32);
                                     if (JOIN == 2)
-                                        hi += s[e] >> 31;
-                                    z[e] = hi >> jsh;
+                                        z[e] = join_f32_apply(s[e], __int_as_float(jm), __int_as_float(jsh), __int_as_float(jrlo));
+                                    else
+                                    {
+                                        const int64_t P = (int64_t)s[e] * (int64_t)jm + (int64_t)(((uint64_t)(uint32_t)jrhi << 32) | (uint32_t)jrlo);
+                                        z[e] = ((int32_t)(P >> 32) + ((s[e] >> 31) & jfix)) >> jsh;
+                                    }
                                 }
                                 w[q] = chan_pack4(z[0], z[1], z[2], z[3]);
                             }
@@ -497,27 +519,6 @@ __global__ void __launch_bounds__(kChanThreads, 1) conv_chan_kernel(const __grid
 #pragma unroll
                                 for (int q = 0; q < 4; q++)
                                     w[q] = __vmins4(__vmaxs4(w[q], jlo4), jhi4);
-                            }
-                        }
-                        else
-                        {
-#pragma unroll 1
-                            for (int q = 0; q < 4; q++)
-                            {
-                                // (selected with constant indices: an array indexed at run time would live in local memory)
-                                const uint32_t wq = q == 0 ? w[0] : q == 1 ? w[1] : q == 2 ? w[2] : w[3];
-                                const uint32_t rq = q == 0 ? r[0] : q == 1 ? r[1] : q == 2 ? r[2] : r[3];
-                                // (pixels and channels past the end hold no operands: whatever they give is not stored and says nothing)
-                                const bool real   = pb * p.px + group * cols + c0 + 4 * q + t < p.pixels && cb * 128 + quarter * 32 + (lane & ~3) < p.OC;
-                                const uint32_t o  = chan_join_general(wq, rq, p.join, p.join_lo, p.join_hi, real ? p.status : nullptr);
-                                if (q == 0)
-                                    w[0] = o;
-                                else if (q == 1)
-                                    w[1] = o;
-                                else if (q == 2)
-                                    w[2] = o;
-                                else
-                                    w[3] = o;
                             }
                         }
                     }
@@ -846,7 +847,7 @@ tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q)
           { conv_chan_kernel<false, true, 0>, conv_chan_kernel<false, true, 1>, conv_chan_kernel<false, true, 2> } },
         { { conv_chan_kernel<true, false, 0>, conv_chan_kernel<true, false, 1>, conv_chan_kernel<true, false, 2> },
           { conv_chan_kernel<true, true, 0>, conv_chan_kernel<true, true, 1>, conv_chan_kernel<true, true, 2> } } };
-    const int ci = q.corr_classes ? 1 : 0, fi = q.double_round ? 1 : 0, ji = q.join ? (q.join_double ? 2 : 1) : 0;
+    const int ci = q.corr_classes ? 1 : 0, fi = q.double_round ? 1 : 0, ji = q.join ? (q.join_f32 ? 2 : 1) : 0;
     const Kern kern = kerns[ci][fi][ji];
     const tb200_status ast = raise_smem_limit(ctx, 64 + (ci * 2 + fi) * 3 + ji, reinterpret_cast<const void*>(kern), plan.smem_bytes);
     if (ast != TB200_OK)

@@ -349,8 +349,9 @@ __global__ void __launch_bounds__(256) residual_add_i8_fast_kernel(const int8_t*
 
 // Record of a residual join that runs inside the convolution that makes its first operand (conv_chan.cu).  The legs to INT32
 // have 256 values each; where both are exact multiples (k * q + constant, as every power-of-two scale is) the sum is one
-// dp2a of the two bytes and the RESCALE back to int8 takes the lean form with the sum's static bound.  The tables serve the
-// kernel where that does not hold.  One block of 256 threads.
+// dp2a of the two bytes and the RESCALE back to int8 takes the lean form with the sum's static bound, or single precision where
+// every sum there is comes out the same (kJoinUsable 1 or 0x01010101; 0 is neither).  The tables serve the kernel where that
+// does not hold.  One block of 256 threads.
 __global__ void __launch_bounds__(256) residual_record_kernel(ResidualFast r, int32_t* __restrict__ block)
 {
     __shared__ int32_t lut[2][256];
@@ -376,8 +377,6 @@ __global__ void __launch_bounds__(256) residual_record_kernel(ResidualFast r, in
         fits   = fits && (int64_t)lut[leg][i] == (int64_t)lut[leg][0] + k[leg] * i;
     }
     const bool linear = __syncthreads_and(fits) != 0;
-    if (i != 0)
-        return;
     const int32_t m = __ldg(r.o.mult), sh = (int32_t)__ldg(r.o.shift);
     const int64_t c0 = (int64_t)lut[0][0] + lut[1][0] + 128 * (k[0] + k[1]);
     int64_t vmax = 0;
@@ -389,15 +388,48 @@ __global__ void __launch_bounds__(256) residual_record_kernel(ResidualFast r, in
     bool ok = linear && vmax < ((int64_t)1 << 31);
     int32_t rec[8];
     rescale_rec_build(m, sh, r.o.double_round, r.o.zp_out, ok ? (int32_t)c0 : 0, vmax, rec);
-    const int64_t ca = k[0] * rec[1], cb = k[1] * rec[1];    // 16-bit coefficients
+    // a leg of the other's power of two is taken in units of the smaller one: t = c0 + g * n
+    const int64_t ka = k[0] < 0 ? -k[0] : k[0], kb = k[1] < 0 ? -k[1] : k[1];
+    const bool single = ok && rec[7] == 1 && ka <= 32767 && kb <= 32767;
+    bool f32 = single && ka > 0 && kb > 0 && (ka % kb == 0 || kb % ka == 0);
+    const int64_t g = ka < kb ? ka : kb, reach = f32 ? 128 * (ka / g + kb / g) : 0;    // |n| <= reach
+    f32             = f32 && reach <= 4096;
+    // single precision for the sum: checked against the exact arithmetic for every sum there is
+    const int32_t s32   = sh < 2 ? 2 : sh > 62 ? 62 : sh;
+    const float S       = (float)((double)m * __hiloint2double((1023 - s32) << 20, 0));    // m * 2^-shift
+    const float dr      = r.o.double_round && s32 > 31 ? __int_as_float((127 + 30 - s32) << 23) : 0.0f;
+    const float base    = 12582912.0f + (float)r.o.zp_out;
+    f32                 = f32 && vmax < (1 << 22);
+    bool same[3]        = { f32, f32, f32 };
+    for (int64_t n = -reach + i; n <= reach && f32; n += 256)
+    {
+        const int32_t t = (int32_t)(c0 + g * n);
+        if (t > vmax || t < -vmax)
+            continue;
+        bool bad        = false;
+        const int32_t z = apply_scale_32_dev(t, m, sh, r.o.double_round != 0, bad) + r.o.zp_out;
+        for (int c = 0; c < 3; c++)
+        {
+            const int32_t y = join_f32_apply(t + 0x4B400000, S, c == 0 ? 0.0f : c == 1 ? dr : -dr, base);
+            same[c]         = same[c] && (bad || min(max(z, -128), 127) == min(max(y, -128), 127));
+        }
+    }
+    int form = -1;
+    for (int c = 2; c >= 0; c--)
+        if (__syncthreads_and(same[c]))
+            form = c;
+    f32 = form >= 0;
+    if (i != 0)
+        return;
+    const int64_t ca = f32 ? k[0] : k[0] * rec[1], cb = f32 ? k[1] : k[1] * rec[1];    // 16-bit coefficients
     ok = ok && rec[7] == 1 && ca >= -32768 && ca <= 32767 && cb >= -32768 && cb <= 32767;
     block[kJoinCoef]   = ok ? (int32_t)(((uint32_t)ca & 0xffffu) | ((uint32_t)cb << 16)) : 0;
-    block[kJoinC]      = rec[2];
-    block[kJoinM]      = rec[0];
-    block[kJoinSh]     = rec[3];
-    block[kJoinRlo]    = rec[4];
+    block[kJoinC]      = f32 ? (int32_t)c0 + 0x4B400000 : rec[2];
+    block[kJoinM]      = f32 ? __float_as_int(S) : rec[0];
+    block[kJoinSh]     = f32 ? __float_as_int(form == 0 ? 0.0f : form == 1 ? dr : -dr) : rec[3];
+    block[kJoinRlo]    = f32 ? __float_as_int(base) : rec[4];
     block[kJoinRhi]    = rec[5];
-    block[kJoinUsable] = ok ? 1 : 0;
+    block[kJoinUsable] = !ok ? 0 : f32 ? 0x01010101 : 1;
     block[kJoinOutMult]   = m;
     block[kJoinOutShift]  = sh;
     block[kJoinOutZp]     = r.o.zp_out;

@@ -140,6 +140,16 @@ __host__ __device__ __forceinline__ int32_t rescale_rec_apply(int32_t acc, int32
     return hi >> sh;
 }
 
+// The sum of a residual join to its int8 result before saturation, in single precision.  `bits` is the sum t, |t| < 2^22, plus
+// 0x4B400000, which read as a float is 1.5 * 2^23 + t; S = m * 2^-shift, `base` is 1.5 * 2^23 + out_zp and d one of 0,
+// +-2^(30-shift) (double rounding adds it by the sign of t; few sums come so close to a tie that it matters).
+// residual_record_kernel uses it only where all sums there are come out as in the exact arithmetic.
+__device__ __forceinline__ int32_t join_f32_apply(int32_t bits, float S, float d, float base)
+{
+    const float t = __fadd_rn(__int_as_float(bits), -12582912.0f);
+    return __float_as_int(__fadd_rn(__fmaf_rn(t, S, d), base)) - 0x4B400000;
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // Unsigned division by an invariant d >= 1 as a multiply-high and shifts, exact for every 32-bit dividend:
 // l = ceil(log2 d), m = floor(2^32 (2^l - d) / d) + 1, q = (t + ((n - t) >> 1)) >> (l - 1) with t = high word of m * n;
