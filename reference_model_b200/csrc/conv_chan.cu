@@ -61,8 +61,12 @@ struct ChanParams
     const int32_t* delta;              // [classes][corr_stride] class row minus interior row
     int corr_stride;
     int clamp_lo, clamp_hi;
-    const int32_t* join;               // ChanJoinBlock
+    const int32_t* join;               // block of kJoinWords words, or null
     int join_lo, join_hi;
+    // conv_split_kernel
+    int split, chunks_per_cta, red_off, double_round;
+    int8_t* out;
+    const int8_t* res;
     long long wait_limit;
     int* status;
 };
@@ -75,6 +79,17 @@ __device__ __forceinline__ uint32_t chan_pack4(int a, int b, int c, int d)
     return r;
 }
 
+// One pair of a join through the tabulated legs (indexes: byte ^ 0x80) and the exact arithmetic
+__device__ __forceinline__ int32_t chan_join_general_one(const int32_t* blk, int ia, int ib, int32_t m, int32_t sh, int32_t zp, int lo, int hi, bool& bad)
+{
+    const int32_t ya = blk[kJoinLutA + ia], yb = blk[kJoinLutB + ib];
+    const int32_t sum = (int32_t)((uint32_t)ya + (uint32_t)yb);
+    bad = bad || blk[kJoinBadA + ia] != 0 || blk[kJoinBadB + ib] != 0 || ((ya ^ sum) & (yb ^ sum)) < 0;
+    const int64_t r = (int64_t)apply_scale_32_dev(sum, m, sh, blk[kJoinOutDouble] != 0, bad) + zp;
+    bad = bad || r > 2147483647LL || r < -2147483648LL;
+    return min(max((int32_t)r, lo), hi);
+}
+
 // A join whose record is not usable (constants uploaded under a captured graph): the pairs of four words through the tabulated
 // legs and the exact arithmetic, REQUIRE conditions reported for the words of `real`.  Reads the other operand from the slot and
 // stores the results there.
@@ -82,8 +97,7 @@ __device__ __noinline__ void chan_join_general(uint32_t dst, uint32_t w0, uint32
                                                uint32_t real, int* status)
 {
     const int32_t m = blk[kJoinOutMult], sh = blk[kJoinOutShift], zp = blk[kJoinOutZp];
-    const bool dr = blk[kJoinOutDouble] != 0;
-    bool any      = false;
+    bool any = false;
     for (int q = 0; q < 4; q++)
     {
         const uint32_t qa = q == 0 ? w0 : q == 1 ? w1 : q == 2 ? w2 : w3;
@@ -92,14 +106,7 @@ __device__ __noinline__ void chan_join_general(uint32_t dst, uint32_t w0, uint32
         bool bad = false;
         for (int j = 0; j < 4; j++)
         {
-            const int ia = (int)((qa >> (8 * j)) & 0xffu) ^ 0x80, ib = (int)((qb >> (8 * j)) & 0xffu) ^ 0x80;
-            const int32_t ya = blk[kJoinLutA + ia], yb = blk[kJoinLutB + ib];
-            bad = bad || blk[kJoinBadA + ia] != 0 || blk[kJoinBadB + ib] != 0;
-            const int32_t sum = (int32_t)((uint32_t)ya + (uint32_t)yb);
-            bad = bad || ((ya ^ sum) & (yb ^ sum)) < 0;
-            const int64_t r = (int64_t)apply_scale_32_dev(sum, m, sh, dr, bad) + zp;
-            bad = bad || r > 2147483647LL || r < -2147483648LL;
-            const int32_t z = min(max((int32_t)r, lo), hi);
+            const int32_t z = chan_join_general_one(blk, (int)((qa >> (8 * j)) & 0xffu) ^ 0x80, (int)((qb >> (8 * j)) & 0xffu) ^ 0x80, m, sh, zp, lo, hi, bad);
             w |= (uint32_t)(z & 0xff) << (8 * j);
         }
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (uint32_t)q * 128u), "r"(w) : "memory");
@@ -107,6 +114,74 @@ __device__ __noinline__ void chan_join_general(uint32_t dst, uint32_t w0, uint32
     }
     if (any)
         atomicOr(status, TB200_DEV_UNPREDICTABLE);
+}
+
+// One word of the same where nothing is held in registers for it (conv_split_kernel): four results of the convolution with
+// the four of the other operand.
+__device__ __forceinline__ uint32_t chan_join_word(uint32_t w, uint32_t r, const int32_t* blk, int lo, int hi, int* status)
+{
+    const int usable = __ldg(blk + kJoinUsable);
+    if (usable == 0)
+    {
+        const int32_t m = blk[kJoinOutMult], sh = blk[kJoinOutShift], zp = blk[kJoinOutZp];
+        uint32_t o      = 0;
+        bool bad        = false;
+        for (int j = 0; j < 4; j++)
+        {
+            const int32_t z = chan_join_general_one(blk, (int)((w >> (8 * j)) & 0xffu) ^ 0x80, (int)((r >> (8 * j)) & 0xffu) ^ 0x80, m, sh, zp, lo, hi, bad);
+            o |= (uint32_t)(z & 0xff) << (8 * j);
+        }
+        if (bad && status != nullptr)
+            atomicOr(status, TB200_DEV_UNPREDICTABLE);
+        return o;
+    }
+    const int4 c0 = __ldg(reinterpret_cast<const int4*>(blk));        // coefficients, constant, m or S, shift or d
+    const int2 c1 = __ldg(reinterpret_cast<const int2*>(blk + 4));    // R, or base
+    const uint32_t i01 = __byte_perm(w, r, 0x5140), i23 = __byte_perm(w, r, 0x7362);
+    int32_t s[4], z[4];
+    asm("dp2a.lo.s32.s32 %0, %1, %2, %3;" : "=r"(s[0]) : "r"(c0.x), "r"(i01), "r"(c0.y));
+    asm("dp2a.hi.s32.s32 %0, %1, %2, %3;" : "=r"(s[1]) : "r"(c0.x), "r"(i01), "r"(c0.y));
+    asm("dp2a.lo.s32.s32 %0, %1, %2, %3;" : "=r"(s[2]) : "r"(c0.x), "r"(i23), "r"(c0.y));
+    asm("dp2a.hi.s32.s32 %0, %1, %2, %3;" : "=r"(s[3]) : "r"(c0.x), "r"(i23), "r"(c0.y));
+    const bool fix = __ldg(blk + kJoinOutDouble) != 0;
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+    {
+        if (usable == 0x01010101)
+            z[e] = join_f32_apply(s[e], __int_as_float(c0.z), __int_as_float(c0.w), __int_as_float(c1.x));
+        else
+        {
+            const int64_t P = (int64_t)s[e] * (int64_t)c0.z + (int64_t)(((uint64_t)(uint32_t)c1.y << 32) | (uint32_t)c1.x);
+            z[e] = ((int32_t)(P >> 32) + (fix ? s[e] >> 31 : 0)) >> c0.w;
+        }
+    }
+    w = chan_pack4(z[0], z[1], z[2], z[3]);
+    if (lo > -128 || hi < 127)
+        w = __vmins4(__vmaxs4(w, (uint32_t)(lo & 0xff) * 0x01010101u), (uint32_t)(hi & 0xff) * 0x01010101u);
+    return w;
+}
+
+// The class of a pixel's clipped window (the rectangle of filter taps inside the image); *border: it is clipped.
+__device__ __forceinline__ int chan_border_class(const ChanParams& p, int oy, int ox, bool* border)
+{
+    const int iy0 = oy * p.stride_y - p.pad_t, ix0 = ox * p.stride_x - p.pad_l;
+    *border = iy0 < 0 || ix0 < 0 || iy0 + (p.KH - 1) * p.dil_y >= p.IH || ix0 + (p.KW - 1) * p.dil_x >= p.IW;
+    if (!*border)
+        return 0;
+    int ky_lo = 0, ky_hi = p.KH, kx_lo = 0, kx_hi = p.KW;
+    if (iy0 < 0)
+        ky_lo = (-iy0 + p.dil_y - 1) / p.dil_y;
+    if (ix0 < 0)
+        kx_lo = (-ix0 + p.dil_x - 1) / p.dil_x;
+    if (iy0 + (p.KH - 1) * p.dil_y >= p.IH)
+        ky_hi = iy0 >= p.IH ? 0 : (p.IH - 1 - iy0) / p.dil_y + 1;
+    if (ix0 + (p.KW - 1) * p.dil_x >= p.IW)
+        kx_hi = ix0 >= p.IW ? 0 : (p.IW - 1 - ix0) / p.dil_x + 1;
+    ky_lo = min(ky_lo, p.KH);
+    kx_lo = min(kx_lo, p.KW);
+    ky_hi = max(ky_hi, ky_lo);
+    kx_hi = max(kx_hi, kx_lo);
+    return ((ky_lo * (p.KH + 1) + ky_hi) * (p.KW + 1) + kx_lo) * (p.KW + 1) + kx_hi;
 }
 
 // CLASSES: padding with a non-zero input zero point, border pixels add what their clipped window leaves out.  FIX: the
@@ -386,25 +461,8 @@ __global__ void __launch_bounds__(kChanThreads, 1) conv_chan_kernel(const __grid
                     const int n   = (int)fastdiv_apply((uint32_t)pix, p.fd_ohow);
                     const int r   = pix - n * (p.OH * p.OW);
                     const int oy  = (int)fastdiv_apply((uint32_t)r, p.fd_ow);
-                    const int iy0 = oy * p.stride_y - p.pad_t, ix0 = (r - oy * p.OW) * p.stride_x - p.pad_l;
-                    const bool b  = iy0 < 0 || ix0 < 0 || iy0 + (p.KH - 1) * p.dil_y >= p.IH || ix0 + (p.KW - 1) * p.dil_x >= p.IW;
-                    if (b)
-                    {
-                        int ky_lo = 0, ky_hi = p.KH, kx_lo = 0, kx_hi = p.KW;
-                        if (iy0 < 0)
-                            ky_lo = (-iy0 + p.dil_y - 1) / p.dil_y;
-                        if (ix0 < 0)
-                            kx_lo = (-ix0 + p.dil_x - 1) / p.dil_x;
-                        if (iy0 + (p.KH - 1) * p.dil_y >= p.IH)
-                            ky_hi = iy0 >= p.IH ? 0 : (p.IH - 1 - iy0) / p.dil_y + 1;
-                        if (ix0 + (p.KW - 1) * p.dil_x >= p.IW)
-                            kx_hi = ix0 >= p.IW ? 0 : (p.IW - 1 - ix0) / p.dil_x + 1;
-                        ky_lo = min(ky_lo, p.KH);
-                        kx_lo = min(kx_lo, p.KW);
-                        ky_hi = max(ky_hi, ky_lo);
-                        kx_hi = max(kx_hi, kx_lo);
-                        cls[k] = ((ky_lo * (p.KH + 1) + ky_hi) * (p.KW + 1) + kx_lo) * (p.KW + 1) + kx_hi;
-                    }
+                    bool b;
+                    cls[k] = chan_border_class(p, oy, r - oy * p.OW, &b);
                     border[k] = __ballot_sync(0xffffffffu, b);
                 }
             }
@@ -624,6 +682,315 @@ __global__ void __launch_bounds__(kChanThreads, 1) conv_chan_kernel(const __grid
     }
 }
 
+// ------------------------------------------------------------------------------------------------ small problems
+// The same product where there are fewer tiles than SMs: a chain of latencies, in which the load and the multiplication of
+// a whole K by one SM were the longest link (3x3 512 to 512 on one 7x7 map: 590 KB and 144 MMAs in 8 CTAs, 13 of 14 us).
+// A cluster of S CTAs shares a tile of 128 channels by PX pixels: each multiplies its part of K, hands every other
+// one the columns that one owns (PX / S of them, written to its shared memory) and finishes its own columns.  All
+// chunks of a CTA are in flight at once, the weights before the predecessor in the stream has finished.  192 threads and at most
+// half of an SM's shared memory, so that two grids fit an SM and the successor's set-up hides behind this one.
+// One 128-thread epilogue; results are stored from registers, four channels of a pixel per thread.
+// Tensor memory is given back before the CTAs meet: none holds columns that a cluster on another stream waits for.
+constexpr int kSplitThreads   = 192;
+constexpr int kSplitMaxChunks = 16;
+
+template <int PX>
+__global__ void __launch_bounds__(kSplitThreads, 2) conv_split_kernel(const __grid_constant__ ChanParams p)
+{
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bar_full[kSplitMaxChunks];
+    __shared__ __align__(8) uint64_t bar_acc, bar_drain;
+    __shared__ uint32_t tmem_base_holder;
+    __shared__ int abort_flag;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t s_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+    const int S      = p.split;
+    const int rank   = S > 1 ? (int)ptx::cluster_ctarank() : 0;
+    const int tile   = (int)blockIdx.x / S;
+    const int pb     = (int)fastdiv_apply((uint32_t)tile, p.fd_cbs), cb = tile - pb * p.cbs;
+    const int p0     = pb * PX;
+    const int first  = rank * p.chunks_per_cta;
+    const int chunks = max(0, min(p.chunks_per_cta, p.total_chunks - first));
+
+    if (S > 1)
+        ptx::cluster_arrive();    // this CTA has started: waited for before its shared memory is written to
+    if (threadIdx.x == 0)
+    {
+        for (int c = 0; c < chunks; c++)
+            ptx::mbar_init(ptx::smem_u32(&bar_full[c]), 1);
+        ptx::mbar_init(ptx::smem_u32(&bar_acc), 1);
+        ptx::mbar_init(ptx::smem_u32(&bar_drain), 1);
+        abort_flag = 0;
+        ptx::fence_barrier_init();
+        ptx::prefetch_tmap(&p.tmW);
+        ptx::prefetch_tmap(&p.tmX);
+    }
+    if (warp == 1)
+    {
+        ptx::tmem_alloc(ptx::smem_u32(&tmem_base_holder), (uint32_t)p.tmem_cols);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    ptx::tc_fence_after_sync();
+    const uint32_t tmem_base = tmem_base_holder;
+    // (behind the allocation: a successor may take what is left of this SM's tensor memory)
+    if (threadIdx.x == 0)
+        ptx::dep_launch_trigger();
+
+    const int quarter = warp & 3, t = lane & 3;
+    const int own     = PX / S;                   // columns of the tile that this CTA finishes
+    const int col0    = rank * own;
+    const int ch4     = cb * 128 + quarter * 32 + (lane & ~3);    // this thread's four channels after the transposition
+    const int64_t at0 = (int64_t)(p0 + col0 + t) * p.OC + ch4;    // ... of column col0 + t
+    uint32_t v[PX];
+    uint32_t res[PX / 4];
+    int cls[2]         = { 0, 0 };
+    uint32_t border[2] = { 0, 0 };
+    int32_t rm = 0, rpk = 0, rcpk = 0, rsh = 0, rlo = 0, rhi = 0;
+    const int ch = cb * 128 + quarter * 32 + lane;
+    bool ok      = true;
+
+    if (warp == 0)
+    {
+        if (lane == 0)
+        {
+            for (int c = 0; c < chunks; c++)
+            {
+                const uint32_t full = ptx::smem_u32(&bar_full[c]);
+                ptx::mbar_arrive_expect_tx(full, (uint32_t)((PX + 128) * p.chunk));
+                ptx::tma_load_3d(s_base + (uint32_t)(c * p.stage_bytes + p.x_chunk_bytes), &p.tmW, full, (first + c) * p.chunk, cb * 128, 0);
+            }
+            ptx::dep_launch_wait();
+            int n0 = 0, y0 = 0, x0 = 0;
+            if (p.im2col)
+            {
+                n0           = (int)fastdiv_apply((uint32_t)p0, p.fd_ohow);
+                const int r  = p0 - n0 * (p.OH * p.OW);
+                const int oy = (int)fastdiv_apply((uint32_t)r, p.fd_ow);
+                y0           = oy * p.stride_y - p.pad_t;
+                x0           = (r - oy * p.OW) * p.stride_x - p.pad_l;
+            }
+            const int tap = first / p.chunks_per_tap;
+            int cc = first - tap * p.chunks_per_tap, ky = tap / p.KW, kx = tap - ky * p.KW;
+            for (int c = 0; c < chunks; c++)
+            {
+                const uint32_t full = ptx::smem_u32(&bar_full[c]), dst = s_base + (uint32_t)(c * p.stage_bytes);
+                if (p.im2col)
+                    ptx::tma_load_im2col_4d(dst, &p.tmX, full, cc * p.chunk, x0, y0, n0, (uint16_t)(kx * p.dil_x), (uint16_t)(ky * p.dil_y));
+                else
+                    ptx::tma_load_2d(dst, &p.tmX, full, cc * p.chunk, p0);
+                if (++cc == p.chunks_per_tap)
+                {
+                    cc = 0;
+                    if (++kx == p.KW)
+                    {
+                        kx = 0;
+                        ky++;
+                    }
+                }
+            }
+        }
+    }
+    else if (warp == 1)
+    {
+        if (lane == 0)
+        {
+            uint32_t accum = 0;
+            for (int c = 0; c < chunks; c++)
+            {
+                if (!ptx::mbar_wait_bounded(ptx::smem_u32(&bar_full[c]), 0u, p.wait_limit))
+                {
+                    ok = false;
+                    break;
+                }
+                ptx::tc_fence_after_sync();
+                const uint32_t sx = s_base + (uint32_t)(c * p.stage_bytes);
+                ptx::mma_i8_ss_chunk(tmem_base, ptx::smem_desc(p.desc_hi, sx + (uint32_t)p.x_chunk_bytes), ptx::smem_desc(p.desc_hi, sx), p.idesc, accum,
+                                     p.mmas);
+                accum = 1;
+            }
+            if (ok && chunks > 0)
+                ptx::mma_commit(ptx::smem_u32(&bar_acc));
+            if (!ok)
+                atomicExch(&abort_flag, 1);
+        }
+    }
+    else
+    {
+        // constants, and what does not depend on the product, while it is on its way
+        const int4 r0 = __ldg(reinterpret_cast<const int4*>(p.rec + (int64_t)ch * 8));
+        const int2 r1 = __ldg(reinterpret_cast<const int2*>(p.rec + (int64_t)ch * 8 + 4));
+        rm = r0.x; rpk = r0.y; rcpk = r0.z; rsh = r0.w; rlo = r1.x; rhi = r1.y;
+        if (p.delta != nullptr)
+        {
+#pragma unroll
+            for (int k = 0; k < (PX > 32 ? 2 : 1); k++)
+            {
+                const int pix = p0 + col0 + k * 32 + lane;
+                const int n   = (int)fastdiv_apply((uint32_t)pix, p.fd_ohow);
+                const int r   = pix - n * (p.OH * p.OW);
+                const int oy  = (int)fastdiv_apply((uint32_t)r, p.fd_ow);
+                bool b;
+                cls[k]    = chan_border_class(p, oy, r - oy * p.OW, &b);
+                border[k] = __ballot_sync(0xffffffffu, b);
+            }
+        }
+        ptx::dep_launch_wait();    // the other operand of a join is the predecessor's; the output may still be read by it
+        if (p.join != nullptr)
+        {
+#pragma unroll
+            for (int q = 0; q < PX / 4; q++)
+                if (4 * q < own)
+                    res[q] = p0 + col0 + 4 * q + t < p.pixels && ch4 < p.OC
+                                 ? __ldcg(reinterpret_cast<const unsigned int*>(p.res + at0 + (int64_t)(4 * q) * p.OC))
+                                 : 0u;
+        }
+        if (chunks > 0)
+        {
+            ok = ptx::mbar_wait_bounded(ptx::smem_u32(&bar_acc), 0u, p.wait_limit);
+            ok = __all_sync(0xffffffffu, ok);
+        }
+        if (ok && chunks > 0)
+        {
+            ptx::tc_fence_after_sync();
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+            for (int c = 0; c < PX; c += 16)
+            {
+                uint32_t x[16];
+                ptx::tmem_ld_32x32b_x16(taddr + (uint32_t)c, x);
+                ptx::tmem_ld_wait_x16(x);
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    v[c + j] = x[j];
+            }
+        }
+        else
+        {
+#pragma unroll
+            for (int c = 0; c < PX; c++)
+                v[c] = 0;
+        }
+        if (!ok && lane == 0)
+            atomicExch(&abort_flag, 1);
+    }
+
+    // ---------------------------------------------------------------------- tensor memory goes back before the CTAs meet
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    const bool aborted = abort_flag != 0;
+    if (aborted)
+    {
+        if (threadIdx.x == 0)
+        {
+            atomicOr(p.status, TB200_DEV_TIMEOUT);
+            // let copies that may still be in flight land before the CTA's shared memory is released
+            for (int c = 0; c < chunks; c++)
+                ptx::mbar_wait_bounded(ptx::smem_u32(&bar_full[c]), 0u, 2000000LL);
+        }
+        if (warp == 1 && lane == 0)
+        {
+            ptx::mma_commit(ptx::smem_u32(&bar_drain));
+            ptx::mbar_wait_bounded(ptx::smem_u32(&bar_drain), 0u, 40000000LL);
+        }
+        __syncthreads();
+    }
+    if (warp == 1)
+    {
+        ptx::tc_fence_after_sync();
+        ptx::tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
+    }
+
+    // ---------------------------------------------------------------------- columns to their owners
+    const uint32_t s_red = s_base + (uint32_t)p.red_off;    // [source rank][own columns][128 channels]
+    if (S > 1)
+    {
+        ptx::cluster_wait();
+        if (warp >= 2)
+        {
+            const uint32_t mine = s_red + (uint32_t)(rank * own) * 512u + (uint32_t)(quarter * 32 + lane) * 4u;
+#pragma unroll
+            for (int c = 0; c < PX; c++)
+            {
+                const int d = c >> (__ffs(own) - 1);    // (own is a power of two of at least 4)
+                ptx::st_shared_cluster(ptx::map_to_cta(mine + (uint32_t)(c & (own - 1)) * 512u, (uint32_t)d), v[c]);
+            }
+        }
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+    }
+    if (warp < 2 || aborted)
+        return;
+
+    // ---------------------------------------------------------------------- RESCALE, join, store
+    const uint32_t sel1 = t < 2 ? 0x5410u : 0x3276u, sel2 = (t & 1) ? 0x3715u : 0x6240u;
+    const bool narrow  = p.clamp_lo > -128 || p.clamp_hi < 127;
+    const uint32_t lo4 = (uint32_t)(p.clamp_lo & 0xff) * 0x01010101u, hi4 = (uint32_t)(p.clamp_hi & 0xff) * 0x01010101u;
+    auto emit = [&](int q, int32_t(&x)[4], uint32_t other) {
+        if (p.delta != nullptr)
+        {
+            const uint32_t bm = (q >= 8 ? border[1] : border[0]) >> ((4 * q) & 31) & 15u;
+            if (bm != 0)
+            {
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                {
+                    const int cj = __shfl_sync(0xffffffffu, q >= 8 ? cls[1] : cls[0], (4 * q + e) & 31);
+                    if (bm >> e & 1u)
+                        x[e] += __ldg(p.delta + (int64_t)cj * p.corr_stride + ch);
+                }
+            }
+        }
+        int32_t z[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            z[e] = p.double_round ? rescale_rec_apply(x[e], rm, rpk, rcpk, rsh, rlo, rhi, true)
+                                  : rescale_rec_apply(x[e], rm, rpk, rcpk, rsh, rlo, rhi, false);
+        uint32_t w = chan_pack4(z[0], z[1], z[2], z[3]);
+        uint32_t y = __shfl_xor_sync(0xffffffffu, w, 2);
+        w          = __byte_perm(w, y, sel1);
+        y          = __shfl_xor_sync(0xffffffffu, w, 1);
+        w          = __byte_perm(w, y, sel2);
+        if (narrow)
+            w = __vmins4(__vmaxs4(w, lo4), hi4);
+        const bool real = p0 + col0 + 4 * q + t < p.pixels && ch4 < p.OC;
+        if (p.join != nullptr)
+            w = chan_join_word(w, other, p.join, p.join_lo, p.join_hi, real ? p.status : nullptr);
+        if (real)
+            *reinterpret_cast<uint32_t*>(p.out + at0 + (int64_t)(4 * q) * p.OC) = w;
+    };
+    if (S == 1)
+    {
+#pragma unroll
+        for (int q = 0; q < PX / 4; q++)
+        {
+            int32_t x[4] = { (int32_t)v[4 * q], (int32_t)v[4 * q + 1], (int32_t)v[4 * q + 2], (int32_t)v[4 * q + 3] };
+            emit(q, x, res[q]);
+        }
+    }
+    else
+    {
+        const uint32_t mine = s_red + (uint32_t)(quarter * 32 + lane) * 4u;
+#pragma unroll
+        for (int q = 0; q < PX / 8; q++)
+            if (4 * q < own)
+            {
+                int32_t x[4] = { 0, 0, 0, 0 };
+                for (int r = 0; r < S; r++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                    {
+                        int32_t y;
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(y) : "r"(mine + (uint32_t)(r * own + 4 * q + e) * 512u));
+                        x[e] += y;
+                    }
+                emit(q, x, res[q]);
+            }
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ planning
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -654,6 +1021,16 @@ struct ChanPlan
     CUtensorMapSwizzle swz;
 };
 
+// SM cycles of a small problem on conv_split_kernel, in the measure of chan_plan's estimates (fitted to device times of layers on
+// one and two images): a chunk costs its MMAs, an exchange the columns that a CTA hands out and finishes; 0: not worth trying.
+double split_cost(int px, int S, int chunks, int mmas)
+{
+    const double chunk = 130.0 * mmas + 50;
+    if (px == 32)
+        return chunks * chunk + (S == 2 ? 4800 : 3600);
+    return S == 8 ? chunks * chunk + 5600 : S == 4 ? chunks * chunk + 6600 : 0;
+}
+
 bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
 {
     if (q.epi != TC_EPI_RESCALE || !q.lean_ok || q.rec == nullptr || q.b_mn_major || q.in_dtype != TB200_INT8 ||
@@ -665,16 +1042,6 @@ bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
     if (q.clamp_lo < -128 || q.clamp_hi > 127 || q.clamp_lo > q.clamp_hi || q.out_zp < -128 || q.out_zp > 127)
         return false;
     if (q.corr_classes && q.delta == nullptr)
-        return false;
-    // Channel blocks less than three quarters full leave rows of the product and threads of the epilogue idle: 160 channels on
-    // 21x102x13x96 7.6 us against 6.6 with a pixel per thread, 32 channels 3x3 on 13x32x12x32 8.5 against 5.9; 192 channels 3x3 on
-    // 8x26x10x192 10.4 against 13.5.  Where the products are long they are what counts, and there this kernel needs fewer of
-    // them: 64 channels 3x3 on 10x42x43x512 19.8 against 25.6, 32 channels on 5x43x64x512 19.5 / 24.9, but 5x11x24x192 10.3 / 8.9.
-    // A residual join pays for itself at any width.
-    if (!q.join && q.OC * 4 < (q.OC + 127) / 128 * 128 * 3 && (int64_t)q.KH * q.KW * q.IC < 3072)
-        return false;
-    // Windows over 32-byte pieces, loaded again for each of many channel blocks: 512 channels 3x3 on 24x34x49x96 23.7 / 19.9.
-    if (!q.join && q.KH * q.KW > 1 && q.IC % 64 != 0 && q.OC >= 512)
         return false;
     const int64_t pixels = (int64_t)q.N * q.OH * q.OW;
     if (pixels >= (1LL << 30))
@@ -772,10 +1139,47 @@ bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
                     plan->smem_bytes = 1024 + staging + w_bytes + stages * ksub * per_chunk;
                 }
             }
+    // One tile per cluster of S CTAs, where that fills one wave at most (conv_split_kernel).
+    for (int px = 64; px >= 32; px >>= 1)
+        for (int S = 1; S <= 8 && px / S >= 4 && S <= k.total_chunks; S *= 2)
+        {
+            const int64_t tiles = (pixels + px - 1) / px * k.cbs;
+            const int cpc       = (k.total_chunks + S - 1) / S;
+            const int stage     = (px + 128) * swz;
+            const int smem      = 1024 + cpc * stage + (S > 1 ? px * 512 : 0);
+            // one wave: clusters of 8 and 4 leave SMs of a GPC over when a CTA fills its SM
+            const int room = smem <= 110 * 1024 || S == 1 ? ctx->num_sms : ctx->num_sms * (S == 8 ? 3 : 4) / (S == 8 ? 4 : 5);
+            if (tiles * S > room || cpc > kSplitMaxChunks || smem > budget)
+                continue;
+            const double cost = split_cost(px, S, cpc, k.mmas);
+            if (cost > 0 && (best == 0 || cost < best))
+            {
+                best             = cost;
+                k.split          = S;
+                k.chunks_per_cta = cpc;
+                k.px             = px;
+                k.x_chunk_bytes  = px * swz;
+                k.stage_bytes    = stage;
+                k.red_off        = cpc * stage;
+                k.tiles          = (int)tiles;
+                plan->grid       = (int)tiles * S;
+                plan->smem_bytes = smem;
+            }
+        }
     if (best == 0)
         return false;
+    // Channel blocks less than three quarters full leave rows of the product and threads of the epilogue idle: 160 channels on
+    // 21x102x13x96 7.6 us against 6.6 with a pixel per thread, 32 channels 3x3 on 13x32x12x32 8.5 against 5.9; 192 channels 3x3 on
+    // 8x26x10x192 10.4 against 13.5.  Where the products are long they are what counts, and there this kernel needs fewer of
+    // them: 64 channels 3x3 on 10x42x43x512 19.8 against 25.6, 32 channels on 5x43x64x512 19.5 / 24.9, but 5x11x24x192 10.3 / 8.9.
+    // A residual join pays for itself at any width.
+    if (!k.split && !q.join && q.OC * 4 < (q.OC + 127) / 128 * 128 * 3 && (int64_t)q.KH * q.KW * q.IC < 3072)
+        return false;
+    // Windows over 32-byte pieces, loaded again for each of many channel blocks: 512 channels 3x3 on 24x34x49x96 23.7 / 19.9.
+    if (!k.split && !q.join && q.KH * q.KW > 1 && q.IC % 64 != 0 && q.OC >= 512)
+        return false;
     k.idesc     = ptx::make_idesc(2u, 1u, 1u, 0u, 0u, 128u, (uint32_t)k.px);
-    k.tmem_cols = 2 * k.px;
+    k.tmem_cols = k.split ? k.px : 2 * k.px;
     fastdiv_make((uint32_t)(q.OH * q.OW), k.fd_ohow);
     fastdiv_make((uint32_t)q.OW, k.fd_ow);
     fastdiv_make((uint32_t)k.cbs, k.fd_cbs);
@@ -829,9 +1233,9 @@ tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q)
         r = enc(&k.tmW, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(q.b), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, plan.swz,
                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
-    if (r == CUDA_SUCCESS)
+    if (r == CUDA_SUCCESS && !k.split)
         r = matrix(&k.tmO, q.out, pixels, (cuuint64_t)q.OC, 32, (cuuint32_t)k.px / 4, CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (r == CUDA_SUCCESS && q.join)
+    if (r == CUDA_SUCCESS && !k.split && q.join)
         r = matrix(&k.tmR, q.res, pixels, (cuuint64_t)q.OC, 32, (cuuint32_t)k.px / 4, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (r != CUDA_SUCCESS)
         return fail(ctx, TB200_INTERNAL, "tensor map rejected (CUresult %d)", (int)r);
@@ -840,8 +1244,39 @@ tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q)
     k.join = q.join; k.join_lo = q.join_lo; k.join_hi = q.join_hi;
     k.wait_limit = ctx->wait_limit_cycles;
     k.status     = ctx->d_status;
+    k.double_round = q.double_round;
+    k.out          = reinterpret_cast<int8_t*>(q.out);
+    k.res          = reinterpret_cast<const int8_t*>(q.res);
+    if (!q.corr_classes)
+        k.delta = nullptr;
 
     typedef void (*Kern)(const ChanParams);
+    if (k.split)
+    {
+        const Kern kern        = k.px == 64 ? conv_split_kernel<64> : conv_split_kernel<32>;
+        const tb200_status ast = raise_smem_limit(ctx, 76 + (k.px == 64 ? 1 : 0), reinterpret_cast<const void*>(kern), plan.smem_bytes);
+        if (ast != TB200_OK)
+            return ast;
+        timer_begin(ctx);
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim          = dim3((unsigned)plan.grid);
+        cfg.blockDim         = dim3((unsigned)kSplitThreads);
+        cfg.dynamicSmemBytes = (size_t)plan.smem_bytes;
+        cfg.stream           = ctx->stream;
+        cudaLaunchAttribute at[2];
+        at[0].id               = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)k.split;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        at[1].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs    = at;
+        cfg.numAttrs = ctx->launch_overlap ? 2 : 1;
+        cudaLaunchKernelEx(&cfg, kern, k);
+        timer_end(ctx);
+        return post_launch(ctx, q.join ? "tc_conv_lean_i8_join" : "tc_conv_lean_i8");
+    }
     static const Kern kerns[2][2][3] = {
         { { conv_chan_kernel<false, false, 0>, conv_chan_kernel<false, false, 1>, conv_chan_kernel<false, false, 2> },
           { conv_chan_kernel<false, true, 0>, conv_chan_kernel<false, true, 1>, conv_chan_kernel<false, true, 2> } },

@@ -394,6 +394,23 @@ __device__ __forceinline__ void cluster_sync()
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The two halves of it: nothing another CTA of the cluster may touch before it has started, or read before it is written, comes
+// between them.
+__device__ __forceinline__ void cluster_arrive()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void cluster_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void st_shared_cluster(uint32_t cluster_addr, uint32_t v)
+{
+    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+}
+
 // shared::cluster address of the same shared-memory location in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank)
 {

@@ -49,6 +49,13 @@ CASES = [
     (2, 17, 19, 32, 192, (3, 3), [1, 1, 1, 1], [2, 1], [1, 1], -128),       # a stride per axis
     (5, 7, 7, 512, 512, (3, 3), [1, 1, 1, 1], [1, 1], [1, 1], -128),        # long K
     (9, 14, 14, 256, 288, (3, 3), [1, 1, 1, 1], [1, 1], [1, 1], 100),
+    # few tiles: K split over clusters
+    (1, 28, 28, 128, 128, (3, 3), [1, 1, 1, 1], [1, 1], [1, 1], -128),      # nine chunks over four CTAs, the last without any
+    (1, 7, 7, 2048, 512, (1, 1), [0, 0, 0, 0], [1, 1], [1, 1], 11),         # over eight
+    (1, 10, 20, 96, 32, (3, 3), [1, 1, 1, 1], [1, 1], [1, 1], -128),        # 27 short chunks, a quarter of a channel block
+    (1, 12, 11, 64, 384, (5, 5), [2, 2, 2, 2], [1, 1], [1, 1], -128),
+    (2, 13, 17, 256, 192, (3, 3), [1, 1, 1, 1], [2, 2], [1, 1], 64),
+    (1, 31, 19, 384, 32, (3, 3), [1, 1, 1, 1], [1, 1], [1, 1], -1),
 ]
 
 
@@ -115,7 +122,8 @@ JOINS = [
 ]
 
 
-@pytest.mark.parametrize("shape", [(1, 6, 6, 32, 128, 1), (30, 64, 64, 32, 128, 1), (5, 48, 50, 64, 64, 3), (3, 9, 9, 64, 96, 3), (40, 7, 7, 512, 512, 1)])
+@pytest.mark.parametrize("shape", [(1, 6, 6, 32, 128, 1), (30, 64, 64, 32, 128, 1), (5, 48, 50, 64, 64, 3), (3, 9, 9, 64, 96, 3), (40, 7, 7, 512, 512, 1),
+                                   (1, 7, 7, 512, 512, 3), (1, 14, 14, 256, 320, 1), (1, 28, 26, 96, 96, 3)])
 @pytest.mark.parametrize("join", JOINS)
 def test_join_against_oracle(ctx, shape, join):
     n, h, w, ic, oc, k = shape
@@ -174,4 +182,28 @@ def test_join_follows_constants_under_a_captured_graph(ctx):
     # the output may not overlap the other operand
     assert ctx.conv2d_add(ts[0], ts[1], ts[2], to, [0] * 4, [1, 1], [1, 1], -128, 0, epi, at[0], to, at[1], ao, check=False) == tb.Status.ERROR
     for t in ts + cs + [to]:
+        t.free()
+
+
+def test_split_form_gives_up_and_recovers(ctx):
+    """A wait limit far below the latency of a load from memory: every CTA of the clusters leaves, the call reports
+    TB200_INTERNAL and the next one is exact."""
+    _, x, wt, b, mult, shift = _operands(5, 1, 7, 7, 512, 512, 3, 3)
+    exp = _conv(x, wt, b, mult, shift, [1] * 4, [1, 1], [1, 1], -128, "DOUBLE_ROUND", -128, 127)
+    ts = [ctx.from_numpy(v) for v in (x, wt, b, mult, shift)]
+    to = ctx.empty(I8, exp.shape)
+    epi = tb.Epilogue(tb.RescaleAttr(ts[3], ts[4], 0, -3, True, "DOUBLE_ROUND", per_channel=True), (-128, 127))
+    run = lambda: ctx.conv2d(ts[0], ts[1], ts[2], to, [1] * 4, [1, 1], [1, 1], -128, 0, epi)
+    run()
+    assert ctx.sync() == tb.Status.OK
+    ctx.set_wait_limit(100)
+    try:
+        run()
+        assert ctx.sync(check=False) == tb.Status.INTERNAL
+    finally:
+        ctx.set_wait_limit(4000000000)
+    run()
+    st, out = to.download()
+    assert st == tb.Status.OK and np.array_equal(out.astype(np.int32), exp)
+    for t in ts + [to]:
         t.free()
