@@ -14,9 +14,12 @@
 //     cost 20 registers).  The kernel reads that verdict itself, so no call waits for it and a captured graph follows
 //     constants that are replaced under it.
 // Channel counts that are no multiple of four read each word as two aligned ones.
-// 32 x 56 x 56 x 144, 3 x 3: 20 us on the device, where the sixteen-channels-per-thread kernel with the general RESCALE takes 119.
-// What bounds it: the latency of the loads, used as soon as they are asked for (issue slots 34 % busy), and 1.4 waves of blocks.
+// 32 x 56 x 56 x 144, 3 x 3: 18.4 us per call with operands that come from DRAM, 16.6 from L2 (24.5 and 20.0 where each load was
+// used as soon as it was asked for and a row's pieces were made without regard to the waves of blocks);
+// 32 x 57 x 57 x 144 stride 2 14.3 -> 9.2, 16 x 28 x 28 x 240 5 x 5 stride 2 9.9 -> 5.3.  What bounds it: 17 instructions per
+// output of four channels and row, issued in 40 % of the slots by the 14 warps per SM that registers and pieces leave.
 #include <algorithm>
+#include <cmath>
 #include <cuda_runtime.h>
 
 #include "common.h"
@@ -104,6 +107,16 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
             w5[K == 5 ? k : 0][0] = u.x; w5[K == 5 ? k : 0][1] = u.y; w5[K == 5 ? k : 0][2] = u.z; w5[K == 5 ? k : 0][3] = u.w;
         }
     }
+    // the second row's weights, kept (the compiler would shift them again for every output)
+    int wd[R == 2 ? K : 1][4];
+    if (R == 2)
+    {
+#pragma unroll
+        for (int k = 0; k < K; k++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                asm volatile("shl.b32 %0, %1, 8;" : "=r"(wd[R == 2 ? k : 0][i]) : "r"(wc[k][i]));
+    }
     int4 ra[4];
     int2 rb[4];
 #pragma unroll
@@ -119,6 +132,9 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
         return;
     }
 
+    // Rows and columns outside the image are the zero point.  An aligned word's load is predicated and leaves a register that
+    // holds it already: a select after the load would wait for the load where it is asked for.
+    const int8_t* const img = p.in + (int64_t)n * p.IH * p.IW * p.C + c;
     const int8_t* row[NR];
     bool row_in[NR];
 #pragma unroll
@@ -126,30 +142,37 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
     {
         const int y = oy * S - p.pad_t + r;
         row_in[r]   = (unsigned)y < (unsigned)p.IH;
-        row[r]      = p.in + ((int64_t)n * p.IH + (row_in[r] ? y : 0)) * p.IW * p.C + c;
+        row[r]      = img + (int64_t)(row_in[r] ? y : 0) * p.IW * p.C;
     }
-    auto fetch = [&](int r, int x) -> uint32_t {
-        if (!row_in[r] || (unsigned)x >= (unsigned)p.IW)
-            return p.fill4;
-        const int8_t* a = row[r] + x * p.C;
-        if (ALIGNED)
-            return *reinterpret_cast<const uint32_t*>(a);
-        const int sh      = (int)(reinterpret_cast<uintptr_t>(a) & 3);
-        const int8_t* lo  = a - sh;
-        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(lo);
-        const uint32_t w1 = sh && lo + 4 < p.in_end ? *reinterpret_cast<const uint32_t*>(lo + 4) : 0u;
-        return __funnelshift_r(w0, w1, 8 * sh);
+    auto fetch_column = [&](int x, uint32_t(&a)[NR]) {
+        const bool in = (unsigned)x < (unsigned)p.IW;
+        const int xo  = ALIGNED ? x * p.C : min(max(x, 0), p.IW - 1) * p.C;
+#pragma unroll
+        for (int r = 0; r < NR; r++)
+        {
+            const int8_t* at = row[r] + xo;
+            if (ALIGNED)
+            {
+                uint32_t v = p.fill4;
+                asm("{\n\t.reg .pred in;\n\tsetp.ne.s32 in, %2, 0;\n\t@in ld.global.nc.b32 %0, [%1];\n\t}" : "+r"(v) : "l"(at), "r"((int)(in && row_in[r])));
+                a[r] = v;
+            }
+            else
+            {
+                const int sh      = (int)(reinterpret_cast<uintptr_t>(at) & 3);
+                const int8_t* lo  = at - sh;
+                const uint32_t w0 = *reinterpret_cast<const uint32_t*>(lo);
+                const uint32_t w1 = sh && lo + 4 < p.in_end ? *reinterpret_cast<const uint32_t*>(lo + 4) : 0u;
+                a[r] = in && row_in[r] ? __funnelshift_r(w0, w1, 8 * sh) : p.fill4;
+            }
+        }
     };
     // column x of the window's rows: t[0..3] one word per channel (rows 0..3), t[4] the fifth row's four channels
     struct Column
     {
         uint32_t t[K == 5 ? 5 : 4];
     };
-    auto column = [&](int x, Column& q) {
-        uint32_t a[NR];
-#pragma unroll
-        for (int r = 0; r < NR; r++)
-            a[r] = fetch(r, x);
+    auto column = [&](const uint32_t(&a)[NR], Column& q) {
         const uint32_t lo01 = __byte_perm(a[0], a[1], 0x5140), hi01 = __byte_perm(a[0], a[1], 0x7362);
         if (NR == 3)
         {
@@ -173,9 +196,10 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
     };
     const bool narrow  = p.clamp_lo > -128 || p.clamp_hi < 127;
     const uint32_t lo4 = (uint32_t)(p.clamp_lo & 0xff) * 0x01010101u, hi4 = (uint32_t)(p.clamp_hi & 0xff) * 0x01010101u;
-    int8_t* const o0   = p.out + (((int64_t)n * p.OH + oy) * p.OW) * p.C + c;
+    int8_t* o0         = p.out + (((int64_t)n * p.OH + oy) * p.OW + ox0) * p.C + c;
+    const int64_t o_row = (int64_t)p.OW * p.C;
     const bool two     = R == 2 && oy + 1 < p.OH;
-    auto emit = [&](int ox, const int (&acc)[4], int rr) {
+    auto emit = [&](int8_t* o, const int (&acc)[4]) {
         uint32_t w;
         int z[4];
 #pragma unroll
@@ -185,7 +209,6 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
         asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(z[1]), "r"(z[0]), "r"(w));
         if (narrow)
             w = __vmins4(__vmaxs4(w, lo4), hi4);
-        int8_t* o = o0 + (rr * p.OW + ox) * p.C;
         if (ALIGNED)
             *reinterpret_cast<uint32_t*>(o) = w;
         else
@@ -197,13 +220,21 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
         }
     };
 
-    // The last K columns, as a ring whose positions are compile-time constants: the loop over x is unrolled K times.
+    // The last K columns, as a ring whose positions are compile-time constants: the loop over x is unrolled K times.  An
+    // output's new columns are asked for K outputs before they are used.
     Column q[K];
+    uint32_t raw[K * S][NR], head[K - S][NR];
     int x = ox0 * S - p.pad_l;
 #pragma unroll
     for (int k = 0; k < K - S; k++)
-        column(x + k, q[k]);
+        fetch_column(x + k, head[k]);
     x += K - S;
+#pragma unroll
+    for (int k = 0; k < K * S; k++)
+        fetch_column(x + k, raw[k]);
+#pragma unroll
+    for (int k = 0; k < K - S; k++)
+        column(head[k], q[k]);
     for (int ox = ox0; ox < ox1; ox += K)
     {
 #pragma unroll
@@ -214,7 +245,13 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
                 // ring position of window column k at output ox + u: (u S + k) mod K
 #pragma unroll
                 for (int s = 0; s < S; s++)
-                    column(x + u * S + s, q[(u * S + K - S + s) % K]);
+                    column(raw[u * S + s], q[(u * S + K - S + s) % K]);
+                if (ox + u + K < ox1)
+                {
+#pragma unroll
+                    for (int s = 0; s < S; s++)
+                        fetch_column(x + (u + K) * S + s, raw[u * S + s]);
+                }
                 int acc[4], acc2[4];
 #pragma unroll
                 for (int i = 0; i < 4; i++)
@@ -230,12 +267,13 @@ __global__ void __launch_bounds__(128) depthwise_slide_i8_kernel(const __grid_co
                         if (K == 5)
                             acc[i] = __dp4a((int)w.t[K == 5 ? 4 : 0], w5[K == 5 ? k : 0][i], acc[i]);
                         if (R == 2)
-                            acc2[i] = __dp4a((int)w.t[i], wc[k][i] << 8, acc2[i]);
+                            acc2[i] = __dp4a((int)w.t[i], wd[R == 2 ? k : 0][i], acc2[i]);
                     }
                 }
-                emit(ox + u, acc, 0);
+                emit(o0, acc);
                 if (two)
-                    emit(ox + u, acc2, 1);
+                    emit(o0 + o_row, acc2);
+                o0 += p.C;
             }
         }
         x += K * S;
@@ -339,13 +377,47 @@ tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q,
     p.c4         = C4 / 4;
     const int R  = q.K == 3 && q.S == 1 ? 2 : 1;
     p.row_groups = (q.OH + R - 1) / R;
-    // A piece's first K - S columns are fetched again by its neighbour: long pieces waste less, short ones make more
-    // threads.  The longest that still makes 1 024 threads per SM (in blocks of 128), at most 28.
+    const bool al = q.C % 4 == 0 && ((reinterpret_cast<uintptr_t>(q.in) | reinterpret_cast<uintptr_t>(q.out)) & 3) == 0;
+    typedef void (*Kern)(const DwSlideParams);
+    static const Kern kerns[16] = {
+#define TB200_DW(KK, SS)                                                                                                     \
+    depthwise_slide_i8_kernel<KK, SS, false, false>, depthwise_slide_i8_kernel<KK, SS, false, true>,                         \
+        depthwise_slide_i8_kernel<KK, SS, true, false>, depthwise_slide_i8_kernel<KK, SS, true, true>
+        TB200_DW(3, 1), TB200_DW(3, 2), TB200_DW(5, 1), TB200_DW(5, 2)
+#undef TB200_DW
+    };
+    const int which = (q.K == 5 ? 8 : 0) + (q.S == 2 ? 4 : 0) + (al ? 2 : 0) + (q.double_round ? 1 : 0);
+    if (ctx->dw_blocks[which] == 0)
+    {
+        int occ = 0;
+        TB200_CUDA_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kerns[which], 128, 0));
+        ctx->dw_blocks[which] = std::max(1, occ);
+    }
+    // Pieces of a row: a thread is a chain of columns, so a call takes a chain's length times the waves of blocks, or the time its
+    // instructions take where that is longer.  SM cycles: 350 per column of a 3 x 3 chain, 600 of a 5 x 5
+    // one, 1500 to 2500 for the first output; 5 per 32 outputs.  32 x 56 x 56 x 144, 3 x 3, by outputs per piece: 56 24.3 us, 28
+    // and 14 18.4, 19, 12 and 8 20.5, 5 26.6.
     const int64_t lines = (int64_t)q.N * p.row_groups * p.c4;
-    const int64_t want  = (int64_t)ctx->num_sms * 1024;
-    int strips = (int)std::min<int64_t>(std::max<int64_t>((want + lines - 1) / lines, (q.OW + 27) / 28), std::max(1, q.OW / 2));
-    p.len      = (q.OW + strips - 1) / strips;
-    p.strips   = (q.OW + p.len - 1) / p.len;
+    const double room   = (double)ctx->num_sms * ctx->dw_blocks[which];
+    double best         = 0;
+    for (int strips = 1, last = 0; strips <= std::max(1, q.OW / 2); strips++)
+    {
+        const int len = (q.OW + strips - 1) / strips;
+        if (len == last)
+            continue;
+        last = len;
+        const int64_t threads = lines * ((q.OW + len - 1) / len);
+        const double waves    = std::max(1.0, std::ceil((double)((threads + 127) / 128) / room));
+        const double chain    = q.K == 3 ? (len + 3 - q.S) * 350.0 + 2500 : (len + 5 - q.S) * 600.0 + 1500;
+        const double work     = (double)threads / 32 / ctx->num_sms * (len + 3) * R * 4 * 5;
+        const double cost     = std::max(waves * chain, work);
+        if (best == 0 || cost < best * 0.99)
+        {
+            best     = cost;
+            p.len    = len;
+            p.strips = (q.OW + len - 1) / len;
+        }
+    }
     fastdiv_make((uint32_t)p.c4, p.fd_c4);
     fastdiv_make((uint32_t)p.strips, p.fd_strips);
     fastdiv_make((uint32_t)p.row_groups, p.fd_rg);
@@ -353,21 +425,7 @@ tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q,
     p.fill4    = (uint32_t)(q.in_zp & 0xff) * 0x01010101u;
     p.clamp_lo = q.clamp_lo;
     p.clamp_hi = q.clamp_hi;
-    const bool al = q.C % 4 == 0 && ((reinterpret_cast<uintptr_t>(q.in) | reinterpret_cast<uintptr_t>(q.out)) & 3) == 0;
-    const int grid = (p.total + 127) / 128;
-#define TB200_DW(KK, SS)                                                                                                     \
-    if (q.K == KK && q.S == SS)                                                                                              \
-    {                                                                                                                        \
-        if (al && q.double_round) depthwise_slide_i8_kernel<KK, SS, true, true><<<grid, 128, 0, ctx->stream>>>(p);           \
-        else if (al) depthwise_slide_i8_kernel<KK, SS, true, false><<<grid, 128, 0, ctx->stream>>>(p);                       \
-        else if (q.double_round) depthwise_slide_i8_kernel<KK, SS, false, true><<<grid, 128, 0, ctx->stream>>>(p);           \
-        else depthwise_slide_i8_kernel<KK, SS, false, false><<<grid, 128, 0, ctx->stream>>>(p);                              \
-    }
-    TB200_DW(3, 1)
-    TB200_DW(3, 2)
-    TB200_DW(5, 1)
-    TB200_DW(5, 2)
-#undef TB200_DW
+    kerns[which]<<<(p.total + 127) / 128, 128, 0, ctx->stream>>>(p);
     return post_launch(ctx, name);
 }
 
