@@ -6,8 +6,8 @@
 //   * a channel's RESCALE record is six registers of the thread that owns it.  With a pixel per thread every output read
 //     its record from shared memory, and those reads and the scattered 32-byte stores were what the kernel waited for
 //     (LSU pipe: 5 wavefronts per 32 outputs);
-//   * pixels are columns, and the number of columns is free: 256, 128 or 64 per tile, whichever fills the SMs;
-//   * results leave through shared memory ([pixel][channel], 128-byte swizzle) and one bulk tensor store per tile.
+//   * pixels are columns, and the number of columns is free: 256, 192, 128 or 64 per tile, whichever fills the SMs;
+//   * results leave through shared memory, a slot of [pixel][32 channels] per warp, by a tensor store that the warp issues itself.
 // The bytes of four pixels are transposed between the four threads of a quad (two shuffles and two byte permutes per four
 // outputs) into words of four channels of one pixel.  A residual join works on those words: its other operand's tile
 // is loaded into the slot the result will be written to.
@@ -17,8 +17,9 @@
 // across rows and images, zero outside the image (which is the padding), so no tile works on rows that are cut off.
 //
 // Roles (576 threads, one CTA per SM): warp 0 lane 0 issues the loads, warp 1 lane 0 the MMAs, warps 2..17 are the
-// epilogue: quarter warp % 4 of the TMEM lanes, four groups of four warps, each with a quarter of a tile's pixels, slots, barrier and
-// stores of its own (one barrier for all sixteen warps kept them in step, waiting for the same thing at the same time).  Two accumulators alternate.  Weights stay
+// epilogue: quarter warp % 4 of the TMEM lanes, four groups of four warps, each with a quarter of a tile's pixels.  No warp waits for
+// another: each has slots, stores and residual loads of its own (64 to 256 channels on 256x56x56: 98.7 us with a barrier for all
+// sixteen, which kept them in step, 86.9 with one per group, 84).  Two accumulators alternate.  Weights stay
 // in shared memory when the K extent of a channel block fits beside the ring (the grid is then a multiple of the channel blocks
 // and a CTA keeps its block).  Every wait is bounded (p.wait_limit); a wait that gives up sets TB200_DEV_TIMEOUT, the roles
 // leave their loops, copies and MMAs in flight are waited for, tensor memory is freed.
@@ -45,7 +46,7 @@ struct ChanParams
 {
     CUtensorMap tmW, tmX, tmO, tmR;
     int tiles, cbs;                    // tile = pixel block * cbs + channel block
-    int px;                            // pixels per tile: 256, 128 or 64
+    int px;                            // pixels per tile: 256, 192, 128 or 64
     int pixels, OC;
     int im2col;
     uint32_t fd_ohow[2], fd_ow[2], fd_cbs[2];
@@ -1086,11 +1087,12 @@ bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
     const int budget = (ctx->max_smem_optin > 0 ? ctx->max_smem_optin : 232448) - 2048;
 
     // Pixels per tile, where the weights live, slots and stages: the smallest estimate of a first tile from its loads
-    // to its store, and the longest of MMAs, epilogue and loads for every further round.  SM cycles: an MMA of 128 channels by 256 / 128 / 64 pixels and 32
-    // bytes of K 171 / 107 / 104, a commit 60; the loads of all SMs together bring 50 bytes per cycle to each, and no
-    // more than what is in flight (the ring less the stage in use) per 2900 cycles of latency.
+    // to its store, and the longest of MMAs, epilogue and loads for every further round.  SM cycles: an MMA of 128 channels by 256 / 192 / 128 / 64 pixels and
+    // 32 bytes of K 171 / 139 / 107 / 104, a commit 60; loads bring 50 bytes per cycle to an SM, 32 when all SMs load (3x3 512 to
+    // 512 on 256x7x7: 8.9 TB/s in tiles of 128 and of 240 pixels alike), and no more than what is in flight (the ring less the
+    // stage in use) per 2900 cycles of latency.
     double best = 0;
-    for (int px = 256; px >= 64; px >>= 1)
+    for (const int px : { 256, 192, 128, 64 })
         for (int res = 1; res >= 0; res--)
             for (int slots = q.join ? 3 : 2; slots >= (q.join ? 2 : 1); slots--)
             {
@@ -1114,8 +1116,8 @@ bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
                 while (ksub > 1 && avail / (ksub * per_chunk) < 3)
                     ksub--;
                 const int stages = std::min(kChanMaxStages, avail / (ksub * per_chunk));
-                const double rate = std::min(50.0, (double)(stages - 1) * ksub * per_chunk / 2900.0);
-                const double mma  = (double)k.total_chunks * k.mmas * (px == 256 ? 171 : px == 128 ? 107 : 104) +
+                const double rate = std::min(std::min(50.0, 32.0 * ctx->num_sms / grid), (double)(stages - 1) * ksub * per_chunk / 2900.0);
+                const double mma  = (double)k.total_chunks * k.mmas * (px == 256 ? 171 : px == 192 ? 139 : px == 128 ? 107 : 104) +
                                    60.0 * ((k.total_chunks + ksub - 1) / ksub + 1);
                 const double epi  = px * (q.join ? 26.0 : 14.7) + 500;
                 const double load = (double)k.total_chunks * per_chunk / rate + (q.join ? px * 128 / 50.0 : 0.0);
@@ -1179,7 +1181,7 @@ bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
     if (!k.split && !q.join && q.KH * q.KW > 1 && q.IC % 64 != 0 && q.OC >= 512)
         return false;
     k.idesc     = ptx::make_idesc(2u, 1u, 1u, 0u, 0u, 128u, (uint32_t)k.px);
-    k.tmem_cols = k.split ? k.px : 2 * k.px;
+    k.tmem_cols = k.split ? k.px : k.px == 192 ? 512 : 2 * k.px;
     fastdiv_make((uint32_t)(q.OH * q.OW), k.fd_ohow);
     fastdiv_make((uint32_t)q.OW, k.fd_ow);
     fastdiv_make((uint32_t)k.cbs, k.fd_cbs);

@@ -123,7 +123,7 @@ JOINS = [
 
 
 @pytest.mark.parametrize("shape", [(1, 6, 6, 32, 128, 1), (30, 64, 64, 32, 128, 1), (5, 48, 50, 64, 64, 3), (3, 9, 9, 64, 96, 3), (40, 7, 7, 512, 512, 1),
-                                   (1, 7, 7, 512, 512, 3), (1, 14, 14, 256, 320, 1), (1, 28, 26, 96, 96, 3)])
+                                   (1, 7, 7, 512, 512, 3), (1, 14, 14, 256, 320, 1), (1, 28, 26, 96, 96, 3), (31, 14, 14, 256, 1024, 1)])
 @pytest.mark.parametrize("join", JOINS)
 def test_join_against_oracle(ctx, shape, join):
     n, h, w, ic, oc, k = shape
