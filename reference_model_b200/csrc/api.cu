@@ -3383,7 +3383,12 @@ extern "C" tb200_status tb200_avg_pool2d(tb200_ctx* ctx, const tb200_tensor* inp
     switch (input->dtype)
     {
         case TB200_INT8:
-            if (p.C % 4 == 0 && ctx->policy == 0 &&
+            if (p.C % 4 == 0 && ctx->policy == 0 && p.ky * p.kx >= 16 &&
+                ((reinterpret_cast<uintptr_t>(input->data) | reinterpret_cast<uintptr_t>(output->data)) & 3) == 0)
+                avg_pool_i8x4_shared_kernel<<<(int)std::min<int64_t>((n / 4 + 31) / 32, (int64_t)ctx->num_sms * 8), 256, 0, ctx->stream>>>(
+                    reinterpret_cast<const int8_t*>(input->data), reinterpret_cast<int8_t*>(output->data), p, input_zp, output_zp,
+                    -128, 127, ctx->d_status);
+            else if (p.C % 4 == 0 && ctx->policy == 0 &&
                 ((reinterpret_cast<uintptr_t>(input->data) | reinterpret_cast<uintptr_t>(output->data)) & 3) == 0)
                 avg_pool_i8x4_kernel<<<grid_for(ctx, n / 4, block), block, 0, ctx->stream>>>(
                     reinterpret_cast<const int8_t*>(input->data), reinterpret_cast<int8_t*>(output->data), p, input_zp, output_zp,

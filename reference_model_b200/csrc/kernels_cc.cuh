@@ -866,6 +866,88 @@ __global__ void avg_pool_int_kernel(const T* __restrict__ in, T* __restrict__ ou
         atomicOr(status, TB200_DEV_UNPREDICTABLE);
 }
 
+// The int8 case with large windows (the global average pool at the end of a ResNet-shaped graph): eight threads share an output's
+// taps.  A block is 32 channel words x 8 shares; a thread's loads of a 7 x 7 window are all in flight at once, where one thread per
+// word took seven rounds of them, in two blocks for one image of 2048 channels (11 us).
+__global__ void __launch_bounds__(256) avg_pool_i8x4_shared_kernel(const int8_t* __restrict__ in, int8_t* __restrict__ out, PoolDev p, int32_t in_zp,
+                                                                   int32_t out_zp, int32_t qmin, int32_t qmax, int* status)
+{
+    __shared__ int32_t part[8][4][32];
+    const int cv        = p.C / 4;
+    const int64_t total = (int64_t)p.N * p.OH * p.OW * cv;
+    const int lane = threadIdx.x & 31, share = threadIdx.x >> 5;
+    for (int64_t i0 = (int64_t)blockIdx.x * 32; i0 < total; i0 += (int64_t)gridDim.x * 32)
+    {
+        const int64_t i = i0 + lane;
+        int32_t acc[4]  = { 0, 0, 0, 0 };
+        int count       = 0;
+        if (i < total)
+        {
+            const int c4 = (int)(i % cv) * 4;
+            int64_t r    = i / cv;
+            const int ox = (int)(r % p.OW);
+            r /= p.OW;
+            const int oy = (int)(r % p.OH);
+            const int n  = (int)(r / p.OH);
+            const int y0 = oy * p.sy - p.pad_t, x0 = ox * p.sx - p.pad_l;
+            const int ya = max(y0, 0), yb = min(y0 + p.ky, p.IH), xa = max(x0, 0), xb = min(x0 + p.kx, p.IW);
+            const int nx = xb - xa;
+            count        = yb > ya && nx > 0 ? (yb - ya) * nx : 0;
+            const int8_t* base = in + (((int64_t)n * p.IH + ya) * p.IW + xa) * p.C + c4;
+            for (int t0 = share; t0 < count; t0 += 64)
+            {
+                uint32_t w[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                {
+                    const int t = t0 + 8 * j, ky = t / nx, kx = t - ky * nx;
+                    w[j] = t < count ? __ldg(reinterpret_cast<const uint32_t*>(base + ((int64_t)ky * p.IW + kx) * p.C)) : 0u;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                {
+                    acc[0] += (int32_t)(int8_t)(w[j] & 0xff);
+                    acc[1] += (int32_t)(int8_t)((w[j] >> 8) & 0xff);
+                    acc[2] += (int32_t)(int8_t)((w[j] >> 16) & 0xff);
+                    acc[3] += (int32_t)(int8_t)(w[j] >> 24);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            part[share][j][lane] = acc[j];
+        __syncthreads();
+        if (share == 0 && i < total)
+        {
+            int32_t mult, shift;
+            reciprocal_scale_dev(count, mult, shift);
+            uint32_t packed = 0;
+            bool bad        = false;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+            {
+                int32_t s = (int32_t)((uint32_t)-count * (uint32_t)in_zp);
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    s += part[q][j][lane];
+                bool b    = false;
+                int32_t v = apply_scale_32_dev(s, mult, shift, false, b);
+                if (b)
+                    v = 0;
+                bad |= b;
+                v = (int32_t)((uint32_t)v + (uint32_t)out_zp);
+                v = v > qmin ? v : qmin;
+                v = v < qmax ? v : qmax;
+                packed |= ((uint32_t)v & 0xffu) << (8 * j);
+            }
+            reinterpret_cast<uint32_t*>(out)[i] = packed;
+            if (bad)
+                atomicOr(status, TB200_DEV_UNPREDICTABLE);
+        }
+        __syncthreads();
+    }
+}
+
 // The int8 case with four channels per thread (one 32-bit load per tap and thread, 128 bytes per warp): the global
 // average pool at the end of a ResNet-shaped graph reads 49 taps per output and was bound by one-byte loads.
 __global__ void avg_pool_i8x4_kernel(const int8_t* __restrict__ in, int8_t* __restrict__ out, PoolDev p, int32_t in_zp,

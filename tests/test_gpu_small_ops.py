@@ -1,4 +1,5 @@
-"""MATMUL with up to four rows (matmul_rows.cu), at the sizes where it can go wrong, against the oracle."""
+"""MATMUL with up to four rows (matmul_rows.cu) and AVG_POOL2D whose windows are shared between threads, at the sizes where they
+can go wrong, against the oracle."""
 import numpy as np
 import pytest
 
@@ -72,3 +73,17 @@ def test_matmul_rows_keeps_infinities_apart(ctx):
     assert np.array_equal(out[0], exp, equal_nan=True)
     for t in (ta, tbb, to):
         t.free()
+
+
+@pytest.mark.parametrize("case", [((1, 7, 7, 2048), [7, 7], [0] * 4, [1, 1]), ((3, 9, 8, 36), [5, 4], [2, 2, 1, 1], [2, 1]),
+                                  ((2, 20, 17, 4), [16, 9], [3, 3, 4, 4], [2, 2]), ((1, 33, 33, 8), [33, 33], [0] * 4, [1, 1])])
+def test_avg_pool_shared_windows(ctx, case):
+    shape, kernel, pad, stride = case
+    x = util.rng(3200 + shape[3]).integers(-128, 128, size=shape).astype(np.int8)
+    st, exp = orc.avg_pool2d(x, kernel, pad, stride, -7, 11)
+    assert st == orc.VALID
+    tx, to = ctx.from_numpy(x), ctx.empty(tb.DType.INT8, exp.shape)
+    ctx.avg_pool2d(tx, to, kernel, pad, stride, -7, 11)
+    st, out = to.download()
+    assert st == tb.Status.OK and np.array_equal(out.astype(np.int32), exp)
+    tx.free(), to.free()
