@@ -360,7 +360,7 @@ tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q);
 // int8 CONV2D + RESCALE with channels on the accumulator rows (conv_chan.cu), q.lean_ok problems; with q.join the residual join
 // RESCALE, RESCALE, ADD, RESCALE, CLAMP runs on the results before they are stored
 bool conv_chan_supported(const tb200_ctx* ctx, const TcProblem& q);
-tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q);
+tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q, bool* taken);    // not taken: nothing done
 // Words of the block behind q.join (residual_record_kernel): with both legs exact multiples of their operand, the sum is
 // one dp2a of (convolution result, other operand) with the two 16-bit coefficients, followed by rescale_rec_apply's second
 // half (usable == 1; sum and constant are scaled by pk) or by join_f32_apply (usable == 0x01010101: M, Sh and Rlo are its

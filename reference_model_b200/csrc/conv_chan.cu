@@ -1196,11 +1196,12 @@ bool conv_chan_supported(const tb200_ctx* ctx, const TcProblem& q)
     return chan_plan(ctx, q, &plan);
 }
 
-tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q)
+tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q, bool* taken)
 {
     ChanPlan plan;
-    if (!chan_plan(ctx, q, &plan))
-        return fail(ctx, TB200_ERROR, "conv_chan: shape not supported");
+    *taken = chan_plan(ctx, q, &plan);
+    if (!*taken)
+        return TB200_OK;
     PFN_encodeTiled enc = reinterpret_cast<PFN_encodeTiled>(tensor_map_encode_fn());
     if (!enc)
         return fail(ctx, TB200_INTERNAL, "cuTensorMapEncodeTiled is not available from the driver");

@@ -2197,6 +2197,64 @@ __global__ void pad_expand_parity_i8_kernel(const int8_t* __restrict__ in, int8_
     }
 }
 
+// Few-channel input, four bytes per pixel: xp[n][y][x] = padded pixel (y, x), the input zero point outside the image.  Four pixels
+// per thread; three channels (12 contiguous bytes) as words, by byte otherwise and at the image's edges.  64 bytes read and
+// written per 4 pixels and image row: 256 x 224 x 224 x 3 is 38 MB in, 54 MB out.
+__global__ void __launch_bounds__(256) pad_expand_i8x4_kernel(const int8_t* __restrict__ in, int8_t* __restrict__ xp, int64_t rows, int IH, int IW, int IC, int Hp,
+                                                              int wq4, int pad_t, int pad_l, int32_t zp)
+{
+    const int64_t total = rows * wq4;
+    const uint32_t zp4  = (uint32_t)(zp & 0xff) * 0x01010101u;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
+    {
+        const int64_t r = i / wq4;
+        const int x0 = (int)(i - r * wq4) * 4 - pad_l;
+        const int64_t n = r / Hp;
+        const int y     = (int)(r - n * Hp) - pad_t;
+        uint32_t v[4]   = { zp4, zp4, zp4, zp4 };
+        if ((unsigned)y < (unsigned)IH && x0 > -4 && x0 < IW)
+        {
+            const int8_t* src = in + ((n * IH + y) * IW + x0) * IC;
+            if (IC == 3 && x0 >= 0 && x0 + 4 <= IW)
+            {
+                // the aligned words around 12 bytes; the fourth only where some of them lie in it
+                const int sh       = (int)(reinterpret_cast<uintptr_t>(src) & 3);
+                const uint32_t* at = reinterpret_cast<const uint32_t*>(src - sh);
+                const uint32_t w0 = __ldg(at), w1 = __ldg(at + 1), w2 = __ldg(at + 2), w3 = sh ? __ldg(at + 3) : 0u;
+                const uint32_t a = __funnelshift_r(w0, w1, 8 * sh), b = __funnelshift_r(w1, w2, 8 * sh), c = __funnelshift_r(w2, w3, 8 * sh);
+                v[0] = __byte_perm(a, zp4, 0x4210);
+                v[1] = __byte_perm(__byte_perm(a, b, 0x0543), zp4, 0x4210);
+                v[2] = __byte_perm(__byte_perm(b, c, 0x0432), zp4, 0x4210);
+                v[3] = __byte_perm(c >> 8, zp4, 0x4210);
+            }
+            else
+                for (int j = 0; j < 4; j++)
+                    if ((unsigned)(x0 + j) < (unsigned)IW)
+                        for (int c = 0; c < IC; c++)
+                            v[j] = (v[j] & ~(0xffu << (8 * c))) | ((uint32_t)(uint8_t)src[j * IC + c] << (8 * c));
+        }
+        *reinterpret_cast<uint4*>(xp + i * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// weights OHWI [OC][KH][KW][IC] -> [E * OC][KH][64], element ((kx + e * step) * 4 + c) of row e * OC + oc = w[oc][ky][kx][c], rest 0;
+// and `plain` [OC][KH][KW * 4] for the epilogue's tables
+__global__ void embed_weights_smallc_kernel(const int8_t* __restrict__ w, int8_t* __restrict__ wr, int8_t* __restrict__ plain, int OC, int KH, int KW, int IC,
+                                            int E, int step)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= E * OC * KH * 64)
+        return;
+    const int k = i % 64, r = i / 64;
+    const int ky = r % KH, row = r / KH;
+    const int oc = row % OC, kx = k / 4 - row / OC * step, c = k % 4;
+    const bool tap = kx >= 0 && kx < KW;
+    const int8_t v = tap && c < IC ? w[((oc * KH + ky) * KW + kx) * IC + c] : (int8_t)0;
+    wr[i]          = v;
+    if (tap && row < OC)
+        plain[((oc * KH + ky) * KW + kx) * 4 + c] = v;
+}
+
 // weights OHWI [OC][KH][KW][IC] -> [OC][KH][win] with win >= KW*Cp, element (kx*Cp + c) = w[oc][ky][kx][c], rest 0
 __global__ void repack_weights_smallc_kernel(const int8_t* __restrict__ w, int8_t* __restrict__ wr, int OC, int KH, int KW,
                                              int IC, int Cp, int win)

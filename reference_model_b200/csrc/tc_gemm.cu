@@ -1585,8 +1585,10 @@ tb200_status tc_gemm_launch(tb200_ctx* ctx, const TcProblem& q)
 {
     if (tc_gemm_pair_supported(q, ctx->num_sms))
         return tc_gemm_pair_launch(ctx, q);
-    if (conv_chan_supported(ctx, q))
-        return conv_chan_launch(ctx, q);
+    bool taken              = false;
+    const tb200_status chan = conv_chan_launch(ctx, q, &taken);
+    if (taken)
+        return chan;
     TcPlan plan;
     plan.lean = false;
     std::string why;

@@ -87,3 +87,38 @@ def test_avg_pool_shared_windows(ctx, case):
     st, out = to.download()
     assert st == tb.Status.OK and np.array_equal(out.astype(np.int32), exp)
     tx.free(), to.free()
+
+
+@pytest.mark.parametrize("case", [
+    # N, H, W, IC, OC, KH, KW, stride, pad, in_zp, shift
+    (1, 224, 224, 3, 64, 7, 7, 2, (3, 2, 3, 2), -128, 33),      # two pixels of a row side by side
+    (3, 113, 116, 3, 64, 3, 3, 2, (0, 0, 0, 1), 5, 33),         # windows up to the last byte of a row
+    (5, 131, 132, 3, 32, 3, 3, 2, (1, 1, 1, 0), -128, 33),      # four
+    (2, 77, 72, 4, 32, 5, 5, 1, (2, 2, 2, 2), 0, 33),
+    (1, 96, 100, 1, 32, 3, 2, 1, (1, 1, 1, 0), 17, 33),
+    (3, 90, 512, 2, 64, 2, 12, 4, (0, 0, 4, 4), -128, 33),
+    (2, 128, 129, 3, 64, 7, 7, 2, (3, 2, 3, 3), 9, 33),         # an odd number of columns: another form
+    (1, 224, 224, 3, 64, 7, 7, 2, (3, 2, 3, 2), -128, 20),      # records that are not usable: another form
+])
+def test_few_channels_side_by_side(ctx, case):
+    N, H, W, IC, OC, KH, KW, s, pad, izp, sh = case
+    r = util.rng(3100 + W + OC + sh)
+    x, w, b = util.conv_int8_case(r, N, H, W, IC, OC, KH, KW, bias_range=1 << 12)
+    mult, shift = util.rescale_params(r, OC)
+    shift = np.maximum(shift, 33).astype(np.int8) if sh >= 33 else np.full(OC, sh, np.int8)
+    if sh < 33:
+        mult = (mult >> 12).astype(np.int32)
+    acc = orc.conv2d(x, w, b, list(pad), [s, s], [1, 1], izp, 0, nthreads=orc.num_procs())
+    est, q = orc.rescale(acc, mult, shift, True, True, "SINGLE_ROUND", 0, -3, 32, 8)
+    exp = np.clip(q, -120, 119)
+    ts = [ctx.from_numpy(v) for v in (x, w, b, mult, shift)]
+    to = ctx.empty(tb.DType.INT8, exp.shape)
+    epi = tb.Epilogue(tb.RescaleAttr(ts[3], ts[4], 0, -3, True, "SINGLE_ROUND", per_channel=True), (-120, 119))
+    for _ in range(2):
+        to.upload(np.full(exp.shape, 55, np.int8))
+        ctx.conv2d(ts[0], ts[1], ts[2], to, list(pad), [s, s], [1, 1], izp, 0, epi)
+        st, out = to.download()
+        assert (st == tb.Status.OK) == (est == orc.VALID)
+        assert est != orc.VALID or np.array_equal(out.astype(np.int32), exp)
+    for t in ts + [to]:
+        t.free()
