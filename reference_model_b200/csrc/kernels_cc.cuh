@@ -2198,8 +2198,8 @@ __global__ void pad_expand_parity_i8_kernel(const int8_t* __restrict__ in, int8_
 }
 
 // Few-channel input, four bytes per pixel: xp[n][y][x] = padded pixel (y, x), the input zero point outside the image.  Four pixels
-// per thread; three channels (12 contiguous bytes) as words, by byte otherwise and at the image's edges.  64 bytes read and
-// written per 4 pixels and image row: 256 x 224 x 224 x 3 is 38 MB in, 54 MB out.
+// per thread; three channels (12 contiguous bytes) as words, by byte otherwise and at the image's edges.  Memory bounds
+// it: 256 x 224 x 224 x 3 is 38 MB in, 54 MB out, half of what a copy per output parity writes.
 __global__ void __launch_bounds__(256) pad_expand_i8x4_kernel(const int8_t* __restrict__ in, int8_t* __restrict__ xp, int64_t rows, int IH, int IW, int IC, int Hp,
                                                               int wq4, int pad_t, int pad_l, int32_t zp)
 {
