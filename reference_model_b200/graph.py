@@ -291,9 +291,10 @@ def fuse(graph):
     return steps
 
 
-def fuse_joins(graph, steps):
+def fuse_joins(graph, steps, external=()):
     """Second pass over fuse()'s steps: a residual join moves into the int8 convolution that makes one of its operands, when
-    nothing else reads that operand and the other one is there by then (the later of two convolutions takes it).  Returns the
+    nothing else reads that operand and the other one is there by then (the later of two convolutions takes it).  `external`
+    names the tensors that the caller owns: they are written by every evaluation, so none stays inside a step.  Returns the
     new steps and {tensor that no longer reaches device memory: its CONV_RESCALE_CLAMP step}."""
     cons = graph.consumers()
     last = lambda step: [o for o in (step[1] if isinstance(step[1], tuple) else (step[1],)) if o is not None][-1]
@@ -308,7 +309,7 @@ def fuse_joins(graph, steps):
             j = where.get(mine)
             if j is None or steps[j][0] != "CONV_RESCALE_CLAMP" or steps[j][1][0].kind != "CONV2D" or mine == other.inputs[0]:
                 continue
-            if cons.get(mine, []) != [leg] or mine in graph.outputs or where.get(other.inputs[0], -1) > j:
+            if cons.get(mine, []) != [leg] or mine in graph.outputs or mine in external or where.get(other.inputs[0], -1) > j:
                 continue
             if best is None or j > best[0]:
                 best = (j, mine, leg, other)
@@ -330,9 +331,9 @@ class DeviceRunner:
         collective reads)."""
         self.ctx, self.graph = ctx, graph
         self.t = dict(external or {})
+        self.steps, self._inside = fuse_joins(graph, fuse(graph), set(self.t)) if fused else ([(op.kind, op) for op in graph.ops], {})
         for name_, arr in graph.consts.items():
             self.t[name_] = ctx.from_numpy(arr, graph.meta[name_][0])
-        self.steps, self._inside = fuse_joins(graph, fuse(graph)) if fused else ([(op.kind, op) for op in graph.ops], {})
         produced = set()
         for kind, payload in self.steps:
             ops = payload if isinstance(payload, tuple) else (payload,)

@@ -1,0 +1,122 @@
+"""The graph runner around residual joins that run inside a convolution (fuse_joins, CONV_JOIN), without a GPU: a context
+whose operators are the oracle's, on host arrays."""
+import numpy as np
+import pytest
+
+import reference_model_b200 as tb
+from oracle import graph_eval
+from oracle import oracle as orc
+from reference_model_b200 import graph as G
+
+I8, I32 = tb.DType.INT8, tb.DType.INT32
+
+
+class _Tensor:
+    def __init__(self, ctx, dtype, shape):
+        self.ctx, self.a = ctx, np.full(shape, 77, {I8: np.int8, I32: np.int32}[tb.DType(dtype)])
+        self.written = 0
+
+    def upload(self, array):
+        self.a[...] = array
+        self.ctx.writes += 1
+        self.written = self.ctx.writes
+
+    def download(self, check=True):
+        return tb.Status.OK, self.a.copy()
+
+
+class _Context:
+    """Results are written into the output's array at once, as a kernel would."""
+
+    def __init__(self):
+        self.kinds, self.writes = [], 0
+
+    def empty(self, dtype, shape):
+        return _Tensor(self, dtype, shape)
+
+    def from_numpy(self, array, dtype=None):
+        t = _Tensor(self, I8 if array.dtype == np.int8 else I32, array.shape)
+        t.upload(array)
+        return t
+
+    def conv2d(self, x, w, b, out, pad, stride, dil, izp, wzp, epi):
+        self.kinds.append("conv2d")
+        acc = orc.conv2d(x.a, w.a, b.a, pad, stride, dil, izp, wzp, nthreads=4)
+        rs, (lo, hi) = epi
+        out.a[...] = np.clip(orc.rescale(acc, rs[0].a, rs[1].a, *rs[2:], 32, 8)[1], lo, hi)
+
+    def residual_add(self, a, ra, b, rb, ro, out, clamp):
+        self.kinds.append("residual_add")
+        leg = lambda t, r: orc.rescale(t.a, r[0].a, r[1].a, *r[2:], 8, 32)[1]
+        s = orc.add(leg(a, ra), leg(b, rb))[1]
+        out.a[...] = np.clip(orc.rescale(s, ro[0].a, ro[1].a, *ro[2:], 32, 8)[1], *clamp)
+
+    def conv2d_add(self, x, w, b, out, pad, stride, dil, izp, wzp, epi, leg, other, other_leg, ro, clamp):
+        t = _Tensor(self, I8, out.a.shape)
+        self.conv2d(x, w, b, t, pad, stride, dil, izp, wzp, epi)
+        self.residual_add(t, leg, other, other_leg, ro, out, clamp)
+        self.kinds[-2:] = ["conv2d_add"]
+
+
+@pytest.fixture()
+def ctx(monkeypatch):
+    monkeypatch.setattr(G.tb, "Epilogue", lambda rescale, clamp: (rescale, clamp))
+    monkeypatch.setattr(G.tb, "RescaleAttr", lambda m, s, izp, ozp, scale32, rounding, per_channel, iu, ou: (m, s, per_channel, scale32, rounding, izp, ozp))
+    return _Context()
+
+
+class _Net:
+    """A graph of 8-channel 5x5 convolutions and joins, by name."""
+
+    def __init__(self, inputs=("x",)):
+        self.g, self.r = G.Graph(), np.random.default_rng(5)
+        for name in inputs:
+            self.g.inputs.append(self.g.tensor(name, I8, (1, 5, 5, 8)))
+
+    def conv(self, x, y):
+        g, r = self.g, self.r
+        w, b = g.const(y + "_w", r.integers(-127, 128, (8, 1, 1, 8)).astype(np.int8)), g.const(y + "_b", np.zeros(8, np.int32))
+        m, s = g.const(y + "_m", np.array([1 << 30], np.int32)), g.const(y + "_s", np.array([38], np.int8))
+        acc, q = g.tensor(y + "_acc", I32, (1, 5, 5, 8)), g.tensor(y + "_q", I8, (1, 5, 5, 8))
+        g.add("CONV2D", [x, w, b], [acc], pad=[0] * 4, stride=[1, 1], dilation=[1, 1], input_zp=0, weight_zp=0)
+        g.add("RESCALE", [acc, m, s], [q], input_zp=0, output_zp=0, scale32=True, rounding="SINGLE_ROUND", per_channel=False)
+        g.add("CLAMP", [q], [g.tensor(y, I8, (1, 5, 5, 8))], min_val=-128, max_val=127)
+
+    def join(self, a, b, y):
+        g = self.g
+        t = lambda k, dt: g.tensor(y + k, dt, (1, 5, 5, 8))
+        c = lambda k, m, s: [g.const(y + k + "m", np.array([m], np.int32)), g.const(y + k + "s", np.array([s], np.int8))]
+        rs = dict(input_zp=0, output_zp=0, scale32=True, rounding="SINGLE_ROUND", per_channel=False)
+        g.add("RESCALE", [a] + c("a", 1 << 30, 30), [t("_a", I32)], **rs)
+        g.add("RESCALE", [b] + c("b", 1 << 30, 30), [t("_b", I32)], **rs)
+        g.add("ADD", [y + "_a", y + "_b"], [t("_sum", I32)])
+        g.add("RESCALE", [y + "_sum"] + c("o", 1 << 30, 31), [t("_q", I8)], **rs)
+        g.add("CLAMP", [y + "_q"], [t("", I8)], min_val=-128, max_val=127)
+
+    def image(self, k=0):
+        return np.random.default_rng(100 + k).integers(-128, 128, (1, 5, 5, 8)).astype(np.int8)
+
+
+def _block(outputs=("y",)):
+    """x -> stem -> (a -> b) + stem -> y: the block of a residual network."""
+    n = _Net()
+    n.conv("x", "stem")
+    n.conv("stem", "a")
+    n.conv("a", "b")
+    n.join("b", "stem", "y")
+    n.g.outputs += list(outputs)
+    return n
+
+
+def _ref(n, x):
+    return graph_eval.evaluate(n.g, {"x": x}, nthreads=4)[1]
+
+
+def test_a_buffer_of_the_caller_is_written_by_every_evaluation(ctx):
+    n, mine = _block(), ctx.empty(I8, (1, 5, 5, 8))
+    run = G.DeviceRunner(ctx, n.g, external={"b": mine})
+    for k in range(2):
+        run.set_input(n.image(k))
+        run.run()
+        ref = _ref(n, n.image(k))
+        assert np.array_equal(mine.a, ref["b"]) and np.array_equal(run.output()[1], ref["y"])
