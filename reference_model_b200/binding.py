@@ -228,6 +228,7 @@ class Tensor:
     def __init__(self, ctx, dtype, shape, handle, keepalive=None):
         self.ctx, self.dtype, self.shape, self.handle = ctx, DType(dtype), tuple(int(s) for s in shape), handle
         self._keepalive = keepalive
+        self.written = 0    # the context's count of uploads at the last one into this tensor
 
     @property
     def nbytes(self):
@@ -241,6 +242,8 @@ class Tensor:
         arr = np.ascontiguousarray(array)
         if arr.nbytes != self.nbytes:
             raise ValueError("upload of %d bytes into a tensor of %d bytes" % (arr.nbytes, self.nbytes))
+        self.ctx.writes += 1
+        self.written = self.ctx.writes
         return self.ctx._check(load_library().tb200_tensor_upload(self.ctx.handle, self.handle,
                                                                   arr.ctypes.data_as(ctypes.c_void_p), arr.nbytes))
 
@@ -286,6 +289,7 @@ class Context:
             raise Tb200Error(st, "tb200_ctx_create failed (is a CUDA device present?)")
         self.handle = h
         self.device = device
+        self.writes = 0
 
     def close(self):
         if self.handle is not None:

@@ -294,9 +294,17 @@ def fuse(graph):
 def fuse_joins(graph, steps, external=()):
     """Second pass over fuse()'s steps: a residual join moves into the int8 convolution that makes one of its operands, when
     nothing else reads that operand and the other one is there by then (the later of two convolutions takes it).  `external`
-    names the tensors that the caller owns: they are written by every evaluation, so none stays inside a step.  Returns the
-    new steps and {tensor that no longer reaches device memory: its CONV_RESCALE_CLAMP step}."""
+    names the tensors that the caller owns: they are written by every evaluation, so none stays inside a step.  Nor does a
+    tensor made from what the caller writes between evaluations (graph inputs and `external`, or a view of them): when it is
+    asked for later, its convolution runs again on operands that only an evaluation writes.  Returns the new steps and {tensor
+    that no longer reaches device memory: its CONV_RESCALE_CLAMP step}."""
     cons = graph.consumers()
+    producer = {o: op for op in graph.ops for o in op.outputs}
+
+    def callers(name):
+        while name in producer and producer[name].kind in ("SLICE", "RESHAPE", "IDENTITY") and name not in external:
+            name = producer[name].inputs[0]
+        return name in external or name in graph.inputs
     last = lambda step: [o for o in (step[1] if isinstance(step[1], tuple) else (step[1],)) if o is not None][-1]
     where = {last(step).outputs[0]: i for i, step in enumerate(steps)}
     out, inside = list(steps), {}
@@ -311,6 +319,8 @@ def fuse_joins(graph, steps, external=()):
                 continue
             if cons.get(mine, []) != [leg] or mine in graph.outputs or mine in external or where.get(other.inputs[0], -1) > j:
                 continue
+            if callers(steps[j][1][0].inputs[0]):
+                continue
             if best is None or j > best[0]:
                 best = (j, mine, leg, other)
         if best is None:
@@ -322,6 +332,17 @@ def fuse_joins(graph, steps, external=()):
 
 
 # ------------------------------------------------------------------------------------------------ device runner
+class _Tensors(dict):
+    """name -> Tensor; what stays inside a fused step is made when it is asked for."""
+
+    def __init__(self, make, items):
+        super().__init__(items)
+        self._make = make
+
+    def __missing__(self, name):
+        return self._make(name)
+
+
 class DeviceRunner:
     """Evaluates a Graph on one tb200 context.  Constants are uploaded once (they are CONST node outputs in the
     reference, decoded at graph initialisation); activations are allocated once and reused across runs."""
@@ -330,7 +351,8 @@ class DeviceRunner:
         """external: optional name -> Tensor for tensors the caller owns (e.g. an output wrapped over a buffer that a
         collective reads)."""
         self.ctx, self.graph = ctx, graph
-        self.t = dict(external or {})
+        self.t = _Tensors(self._inside_tensor, external or {})
+        self._late, self._seen = {}, 0
         self.steps, self._inside = fuse_joins(graph, fuse(graph), set(self.t)) if fused else ([(op.kind, op) for op in graph.ops], {})
         for name_, arr in graph.consts.items():
             self.t[name_] = ctx.from_numpy(arr, graph.meta[name_][0])
@@ -368,8 +390,28 @@ class DeviceRunner:
             rows.append((step[0], last.outputs[0], self.ctx.last_kernel(), (t1 - t0) * 1e3))
         return rows
 
+    def _inside_tensor(self, name):
+        """A result that stays inside a fused step: its operator on its own, on what the last evaluation left."""
+        if name not in self._inside:
+            raise KeyError(name)
+        step = self._inside[name]
+        for o in (step[1][0], step[1][1]):
+            for c in o.inputs[1:]:
+                if self.t[c].written > self._seen:
+                    raise RuntimeError("%s was replaced after the last evaluation, which did not keep %s" % (c, name))
+        if name not in self._late:
+            self._late[name] = self.ctx.empty(*self.graph.meta[name])
+        self.t[name] = self._late[name]
+        try:
+            self._eval([step])
+        finally:
+            del self.t[name]    # made again at the next request: the next evaluation does not write it
+        return self._late[name]
+
     def _eval(self, steps=None):
         ctx, t = self.ctx, self.t
+        if steps is None:
+            self._seen = ctx.writes
         for kind, p in (self.steps if steps is None else steps):
             if kind == "CONV_RESCALE_CLAMP":
                 conv, r, c = p
@@ -469,6 +511,7 @@ class DeviceRunner:
     def run(self):
         """Evaluates the graph once (eagerly, or by replaying the captured CUDA graph)."""
         if self.captured is not None:
+            self._seen = self.ctx.writes
             self.ctx.graph_launch(self.captured)
         else:
             self._eval()
@@ -485,11 +528,6 @@ class DeviceRunner:
             self.captured = self.ctx.capture_end()
 
     def output(self, name_=None):
-        if name_ in self._inside and name_ not in self.t:
-            # a result that stays inside a fused step: its operator on its own, on the inputs of the last evaluation
-            self.t[name_] = self.ctx.empty(*self.graph.meta[name_])
-        if name_ in self._inside:
-            self._eval([self._inside[name_]])
         st, out = self.t[name_ or self.graph.outputs[0]].download()
         return st, out
 

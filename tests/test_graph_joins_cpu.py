@@ -120,3 +120,48 @@ def test_a_buffer_of_the_caller_is_written_by_every_evaluation(ctx):
         run.run()
         ref = _ref(n, n.image(k))
         assert np.array_equal(mine.a, ref["b"]) and np.array_equal(run.output()[1], ref["y"])
+
+
+def test_a_result_inside_a_step_is_that_of_the_last_evaluation(ctx):
+    n = _block()
+    run = G.DeviceRunner(ctx, n.g)
+    assert [k for k, _ in run.steps] == ["CONV_RESCALE_CLAMP"] * 2 + ["CONV_JOIN"]
+    run.set_input(n.image(0))
+    run.run()
+    ref = _ref(n, n.image(0))
+    run.set_input(n.image(1))    # the next image is there already
+    for name in ("b", "a", "stem", "y"):
+        assert np.array_equal(run.output(name)[1], ref[name]), name
+        assert np.array_equal(run.t[name].download()[1], ref[name]), name
+    run.run()
+    ref = _ref(n, n.image(1))
+    assert np.array_equal(run.t["b"].download()[1], ref["b"]) and np.array_equal(run.output("b")[1], ref["b"])
+    assert "b" not in run.t    # nothing that the next evaluation would leave as it is
+    with pytest.raises(KeyError):
+        run.t["b_q"]
+    # its weights are others now: what it was cannot be made again, and it says so
+    run.t["b_w"].upload(np.zeros((8, 1, 1, 8), np.int8))
+    with pytest.raises(RuntimeError):
+        run.output("b")
+    run.run()
+    assert np.array_equal(run.output("b")[1], np.zeros((1, 5, 5, 8), np.int8))
+
+
+@pytest.mark.parametrize("view", [False, True])
+def test_a_convolution_of_the_graphs_input_keeps_its_result(ctx, view):
+    """... as an evaluation made it, whatever the caller has uploaded since."""
+    n = _Net(("x", "z"))
+    src = "x"
+    if view:
+        src = n.g.tensor("v", I8, (1, 5, 5, 8))
+        n.g.add("IDENTITY", ["x"], [src])
+    n.conv(src, "a")
+    n.join("a", "z", "y")
+    n.g.outputs.append("y")
+    run = G.DeviceRunner(ctx, n.g)
+    z = n.image(9)
+    run.set_input(n.image(0), "x"), run.set_input(z, "z")
+    run.run()
+    ref = graph_eval.evaluate(n.g, {"x": n.image(0), "z": z}, nthreads=4)[1]
+    run.set_input(n.image(1), "x")
+    assert np.array_equal(run.output("a")[1], ref["a"]) and np.array_equal(run.output()[1], ref["y"])
