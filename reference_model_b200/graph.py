@@ -296,15 +296,20 @@ def fuse_joins(graph, steps, external=()):
     nothing else reads that operand and the other one is there by then (the later of two convolutions takes it).  `external`
     names the tensors that the caller owns: they are written by every evaluation, so none stays inside a step.  Nor does a
     tensor made from what the caller writes between evaluations (graph inputs and `external`, or a view of them): when it is
-    asked for later, its convolution runs again on operands that only an evaluation writes.  Returns the new steps and {tensor
-    that no longer reaches device memory: its CONV_RESCALE_CLAMP step}."""
+    asked for later, its convolution runs again on operands that only an evaluation writes.  A join into a tensor of the caller
+    stays where it is while others of the caller's are read that late, for they may be the same memory (a join in place).
+    Returns the new steps and {tensor that no longer reaches device memory: its CONV_RESCALE_CLAMP step}."""
     cons = graph.consumers()
     producer = {o: op for op in graph.ops for o in op.outputs}
 
-    def callers(name):
+    def base(name):    # whose memory it is
         while name in producer and producer[name].kind in ("SLICE", "RESHAPE", "IDENTITY") and name not in external:
             name = producer[name].inputs[0]
-        return name in external or name in graph.inputs
+        return name
+
+    def reads(step):    # its activations
+        return [t for o in (step[1] if isinstance(step[1], tuple) else (step[1],)) if o is not None
+                for t in o.inputs if t in producer or t in graph.inputs]
     last = lambda step: [o for o in (step[1] if isinstance(step[1], tuple) else (step[1],)) if o is not None][-1]
     where = {last(step).outputs[0]: i for i, step in enumerate(steps)}
     out, inside = list(steps), {}
@@ -319,7 +324,9 @@ def fuse_joins(graph, steps, external=()):
                 continue
             if cons.get(mine, []) != [leg] or mine in graph.outputs or mine in external or where.get(other.inputs[0], -1) > j:
                 continue
-            if callers(steps[j][1][0].inputs[0]):
+            if base(steps[j][1][0].inputs[0]) in set(graph.inputs) | set(external):
+                continue
+            if (c or ro).outputs[0] in external and any(base(t) in external for s in steps[j:i + 1] for t in reads(s)):
                 continue
             if best is None or j > best[0]:
                 best = (j, mine, leg, other)

@@ -165,3 +165,34 @@ def test_a_convolution_of_the_graphs_input_keeps_its_result(ctx, view):
     ref = graph_eval.evaluate(n.g, {"x": n.image(0), "z": z}, nthreads=4)[1]
     run.set_input(n.image(1), "x")
     assert np.array_equal(run.output("a")[1], ref["a"]) and np.array_equal(run.output()[1], ref["y"])
+
+
+def test_joins_in_place_on_memory_of_the_caller(ctx):
+    """The join's result over its other operand, or over what a step between the convolution and the join reads."""
+    n = _Net(("x", "z"))
+    n.conv("x", "a")
+    n.conv("a", "b")
+    n.join("b", "z", "y")
+    n.g.outputs.append("y")
+    buf = ctx.empty(I8, (1, 5, 5, 8))
+    ref = graph_eval.evaluate(n.g, {"x": n.image(0), "z": n.image(1)}, nthreads=4)[1]
+    run = G.DeviceRunner(ctx, n.g, external={"z": buf, "y": buf})
+    assert "CONV_JOIN" not in [k for k, _ in run.steps]    # tb200_conv2d_add refuses an output over the other operand
+    run.set_input(n.image(0), "x"), run.set_input(n.image(1), "z")
+    run.run()
+    assert np.array_equal(buf.a, ref["y"])
+
+    n = _Net(("x", "z"))
+    n.conv("x", "a")
+    n.conv("a", "b")
+    n.conv("z", "late")
+    n.join("b", "a", "y")
+    n.g.outputs += ["y", "late"]
+    ref = graph_eval.evaluate(n.g, {"x": n.image(0), "z": n.image(1)}, nthreads=4)[1]
+    run = G.DeviceRunner(ctx, n.g, external={"z": buf, "y": buf})
+    run.set_input(n.image(0), "x"), run.set_input(n.image(1), "z")
+    run.run()
+    assert np.array_equal(run.output("late")[1], ref["late"]) and np.array_equal(buf.a, ref["y"])
+    # an output of the caller's that meets none of its other tensors is no obstacle
+    run = G.DeviceRunner(ctx, _block().g, external={"y": buf, "x": ctx.empty(I8, (1, 5, 5, 8))})
+    assert "CONV_JOIN" in [k for k, _ in run.steps]
