@@ -363,6 +363,8 @@ extern "C" tb200_status tb200_ctx_destroy(tb200_ctx* ctx)
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     tb200_comm_destroy(ctx);
+    for (tb200_graph* g : ctx->graphs)
+        g->owner = nullptr;
     for (auto& e : ctx->prepared)
         if (e->block)
             cudaFree(e->block);
@@ -457,6 +459,7 @@ extern "C" tb200_status tb200_capture_begin(tb200_ctx* ctx)
     TB200_ERROR_IF(ctx, ctx->timing, "disable the kernel timer before capturing");
     TB200_CUDA_CHECK(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     ctx->capturing = true;
+    ctx->capture_swaps.clear();
     return TB200_OK;
 }
 
@@ -487,6 +490,9 @@ extern "C" tb200_status tb200_capture_end(tb200_ctx* ctx, tb200_graph** out)
     }
     tg->graph = g;
     tg->exec  = exec;
+    tg->swaps.swap(ctx->capture_swaps);
+    tg->owner = ctx;
+    ctx->graphs.push_back(tg);
     ctx->live_graphs++;
     size_t n  = 0;
     if (cudaGraphGetNodes(g, nullptr, &n) == cudaSuccess)
@@ -502,6 +508,8 @@ extern "C" tb200_status tb200_graph_launch(tb200_ctx* ctx, tb200_graph* graph)
     TB200_ENTER(ctx);
     TB200_ERROR_IF(ctx, !graph || !graph->exec, "null graph");
     TB200_ERROR_IF(ctx, ctx->capturing, "a captured graph cannot be launched while capturing");
+    for (const ReplaySwap& s : graph->swaps)
+        TB200_ERROR_IF(ctx, s.stuck, "constants uploaded under this graph need another kernel for one of its convolutions: capture it again");
     TB200_CUDA_CHECK(ctx, cudaGraphLaunch(graph->exec, ctx->stream));
     ctx->launches += graph->launches;
     ctx->last_kernel = "cuda_graph_replay";
@@ -518,6 +526,8 @@ extern "C" tb200_status tb200_graph_destroy(tb200_ctx* ctx, tb200_graph* graph)
         cudaGraphExecDestroy(graph->exec);
     if (graph->graph)
         cudaGraphDestroy(graph->graph);
+    if (tb200_ctx* o = graph->owner)
+        o->graphs.erase(std::remove(o->graphs.begin(), o->graphs.end(), graph), o->graphs.end());
     delete graph;
     if (ctx && ctx->live_graphs > 0 && --ctx->live_graphs == 0)
     {
@@ -962,7 +972,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     {
                         // would the kernel take it?  (any aligned address stands for the block)
                         const int32_t* some = reinterpret_cast<const int32_t*>(static_cast<uintptr_t>(256));
-                        qe.b = some; qe.rec = some; qe.delta = some; qe.lean_ok = 1; qe.corr_classes = classes ? 1 : 0;
+                        qe.b = some; qe.rec = some; qe.rec_ok = some; qe.delta = some; qe.lean_ok = 1; qe.corr_classes = classes ? 1 : 0;
                         if (join)
                         {
                             qe.join = some; qe.res = join->other;
@@ -1056,7 +1066,8 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     qe.corr_classes = cls_i;
                     qe.mult_pad     = mult_pad;
                     qe.shift_pad    = reinterpret_cast<int8_t*>(mult_pad + OCpad);
-                    qe.rec   = lean_out ? reinterpret_cast<const int32_t*>(bytes_at + rec_off) : nullptr;
+                    qe.rec    = lean_out ? reinterpret_cast<const int32_t*>(bytes_at + rec_off) : nullptr;
+                    qe.rec_ok = reinterpret_cast<const int*>(bytes_at + flag_off);
                     qe.delta = (lean_out && classes) ? reinterpret_cast<const int32_t*>(bytes_at + delta_off) : nullptr;
                     if (join)
                     {
@@ -1228,6 +1239,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     q.mult_pad    = corr + OCpad;
                     q.shift_pad   = reinterpret_cast<int8_t*>(corr + 2 * OCpad);
                     q.rec         = reinterpret_cast<const int32_t*>(bytes_at + rec_off);
+                    q.rec_ok      = reinterpret_cast<const int*>(bytes_at + flag_off);
                     pad_expand_i8x4_kernel<<<grid_for(ctx, (int64_t)N * Hp * (Wp / 4), 256), 256, 0, ctx->stream>>>(
                         reinterpret_cast<const int8_t*>(input->data), xp, (int64_t)N * Hp, IH, IW, IC, Hp, Wp / 4, pad[0], pad[2], input_zp);
                     st = post_launch(ctx, "conv_window_relayout", 1);
@@ -1330,6 +1342,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                 q.mult_pad    = mult_pad;
                 q.shift_pad   = reinterpret_cast<int8_t*>(mult_pad + OCpad);
                 q.rec         = reinterpret_cast<const int32_t*>(wr + wr_bytes + rec_off);
+                q.rec_ok      = reinterpret_cast<const int*>(wr + wr_bytes + flag_off);
                 q.lean_ok     = e->host_flag >= 1 ? 1 : 0;
                 // the scratch address enters the plan only as a pointer: any 16-byte aligned value serves the dry run
                 q.a = ctx->scratch ? ctx->scratch : reinterpret_cast<const void*>(static_cast<uintptr_t>(256));
@@ -1470,6 +1483,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                 q.shift_pad   = reinterpret_cast<int8_t*>(mult_pad + OCpad);
                 if (has_rs && output->dtype == TB200_INT8 && !epi.rs.out_unsigned)
                     q.rec = reinterpret_cast<const int32_t*>(wr + wr_bytes + rec_off);
+                q.rec_ok = reinterpret_cast<const int*>(wr + wr_bytes + flag_off);
                 st = tc_gemm_launch(ctx, q);
                 // a driver that refuses the overlapping-window tensor map sends this shape to the CUDA-core kernel
                 if (!(st == TB200_INTERNAL && ctx->err.find("rejected") != std::string::npos))

@@ -35,11 +35,44 @@ enum : int
     TB200_DEV_TIMEOUT       = 2,    // a bounded pipeline wait gave up (internal error)
 };
 
+namespace tb200
+{
+// One int8 CONV2D + RESCALE (+ residual join) to int8 as conv_general_kernel evaluates it (replay.cu); the fields are those of
+// TcProblem
+struct ConvGeneral
+{
+    const int8_t *a, *w;
+    int64_t a_stride_w, a_stride_h, a_stride_n;
+    int N, OH, OW, OC, IH, IW, IC, KH, KW, pad_t, pad_l, stride_y, stride_x, dil_y, dil_x, xpar, out_ow;
+    const int32_t* corr;
+    int corr_stride, classes;
+    const int32_t* mult;
+    const int8_t* shift;
+    int double_round, out_zp, clamp_lo, clamp_hi;
+    const int32_t* join;
+    const int8_t* res;
+    int join_lo, join_hi;
+    int8_t* out;
+    int* status;
+};
+
+// A captured launch that runs on lean RESCALE records, and what stands in for it while they are not usable
+struct ReplaySwap
+{
+    cudaGraphNode_t node = nullptr;
+    const int* verdict   = nullptr;    // device word in the block of the records
+    bool swapped = false, stuck = false;
+    ConvGeneral general;
+};
+}    // namespace tb200
+
 struct tb200_graph
 {
     cudaGraph_t graph    = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint64_t launches    = 0;    // kernels recorded
+    std::vector<tb200::ReplaySwap> swaps;
+    tb200_ctx* owner     = nullptr;    // the context that lists it, while that lives
 };
 
 namespace tb200
@@ -90,6 +123,8 @@ struct tb200_ctx
     // Captured graphs hold raw addresses of the blocks above: while any is alive a block that would have to move is
     // refused (TB200_ERROR) and blocks of dropped cache entries are parked in `retired` instead of being freed.
     int live_graphs      = 0;
+    std::vector<tb200_graph*> graphs;                  // those that are alive
+    std::vector<tb200::ReplaySwap> capture_swaps;      // of the capture in progress
     std::vector<void*> retired;
     // every bounded device-side wait gives up after this many SM clock cycles (about two seconds by default)
     long long wait_limit_cycles = 4000000000LL;
@@ -249,6 +284,10 @@ tb200_status cache_note_upload(tb200_ctx* ctx, const void* ptr, size_t bytes);
 // [ptr, ptr + bytes) is being released: entries derived from it are dropped.
 void cache_note_free(tb200_ctx* ctx, const void* ptr, size_t bytes);
 void cache_clear(tb200_ctx* ctx);
+// Captured launches on lean records (replay.cu): one has just been recorded; a block of records has been rebuilt under live graphs.
+struct TcProblem;
+void replay_note_launch(tb200_ctx* ctx, const TcProblem& q);
+tb200_status replay_follow(tb200_ctx* ctx, const void* block, size_t bytes);
 // Frees a device block now, or parks it until the context goes while a captured graph may still hold its address.
 void release_block(tb200_ctx* ctx, void* block);
 
@@ -319,7 +358,7 @@ struct TcProblem
     const int32_t* mult_pad;     // TC_EPI_RESCALE: multipliers / shifts expanded per column and padded to corr_stride
     const int8_t* shift_pad;
     const int32_t* rec;          // optional: [corr_stride][8] prepared records of the lean RESCALE form (rescale_rec_build)
-    const int* rec_ok;           // gathering kernel, with rec: device word, whether every record is usable
+    const int* rec_ok;           // gathering kernel and lean_ok problems, with rec: device word, whether every record is usable
     const int32_t* delta;        // optional, with corr_classes: [classes][corr_stride] class row minus interior row
     int lean_ok;                 // the host knows every column's record is usable: tc_conv_lean_kernel may run
     // tc_conv_lean_kernel only: the batch dimension is (image, parity of the output column): batch index 2 n + p holds

@@ -124,9 +124,11 @@ tb200_status cache_note_upload(tb200_ctx* ctx, const void* ptr, size_t bytes)
     for (auto& e : ctx->prepared)
         if (overlaps(*e, lo, bytes))
         {
-            const tb200_status st = e->rebuild(ctx, e->block);
-            e->valid              = st == TB200_OK;
-            e->host_flag          = -1;
+            tb200_status st = e->rebuild(ctx, e->block);
+            e->valid        = st == TB200_OK;
+            e->host_flag    = -1;
+            if (st == TB200_OK && ctx->live_graphs > 0)
+                st = replay_follow(ctx, e->block, e->bytes);
             if (st != TB200_OK)
                 return st;
         }

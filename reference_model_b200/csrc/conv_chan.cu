@@ -83,12 +83,8 @@ __device__ __forceinline__ uint32_t chan_pack4(int a, int b, int c, int d)
 // One pair of a join through the tabulated legs (indexes: byte ^ 0x80) and the exact arithmetic
 __device__ __forceinline__ int32_t chan_join_general_one(const int32_t* blk, int ia, int ib, int32_t m, int32_t sh, int32_t zp, int lo, int hi, bool& bad)
 {
-    const int32_t ya = blk[kJoinLutA + ia], yb = blk[kJoinLutB + ib];
-    const int32_t sum = (int32_t)((uint32_t)ya + (uint32_t)yb);
-    bad = bad || blk[kJoinBadA + ia] != 0 || blk[kJoinBadB + ib] != 0 || ((ya ^ sum) & (yb ^ sum)) < 0;
-    const int64_t r = (int64_t)apply_scale_32_dev(sum, m, sh, blk[kJoinOutDouble] != 0, bad) + zp;
-    bad = bad || r > 2147483647LL || r < -2147483648LL;
-    return min(max((int32_t)r, lo), hi);
+    bad = bad || blk[kJoinBadA + ia] != 0 || blk[kJoinBadB + ib] != 0;
+    return join_general(blk[kJoinLutA + ia], blk[kJoinLutB + ib], m, sh, blk[kJoinOutDouble] != 0, zp, lo, hi, bad);
 }
 
 // A join whose record is not usable (constants uploaded under a captured graph): the pairs of four words through the tabulated
@@ -1034,7 +1030,7 @@ double split_cost(int px, int S, int chunks, int mmas)
 
 bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
 {
-    if (q.epi != TC_EPI_RESCALE || !q.lean_ok || q.rec == nullptr || q.b_mn_major || q.in_dtype != TB200_INT8 ||
+    if (q.epi != TC_EPI_RESCALE || !q.lean_ok || q.rec == nullptr || q.rec_ok == nullptr || q.b_mn_major || q.in_dtype != TB200_INT8 ||
         q.out_dtype != TB200_INT8 || q.out_sy != 0 || q.xpar || q.tile_begin != 0 || q.tile_end != 0)
         return false;
     if (q.OC % 32 != 0 || q.IC % 32 != 0 || ((reinterpret_cast<uintptr_t>(q.out) | reinterpret_cast<uintptr_t>(q.a) |

@@ -140,6 +140,25 @@ __host__ __device__ __forceinline__ int32_t rescale_rec_apply(int32_t acc, int32
     return hi >> sh;
 }
 
+// One accumulator (correction added) through the RESCALE itself to an int8 result clipped to [lo, hi]: where a lean record is not
+// usable
+__host__ __device__ __forceinline__ int32_t rescale_general(int32_t t, int32_t m, int32_t shift, bool double_round, int32_t out_zp, int32_t lo, int32_t hi,
+                                                            bool& bad)
+{
+    const int64_t z = (int64_t)apply_scale_32_dev(t, m, shift, double_round, bad) + out_zp;
+    bad |= z < -((int64_t)1 << 31) || z >= ((int64_t)1 << 31);
+    return (int32_t)(z < lo ? lo : z > hi ? hi : z);
+}
+
+// The sum of a residual join's two INT32 legs to its int8 result clipped to [lo, hi], likewise
+__host__ __device__ __forceinline__ int32_t join_general(int32_t ya, int32_t yb, int32_t m, int32_t shift, bool double_round, int32_t out_zp, int32_t lo,
+                                                         int32_t hi, bool& bad)
+{
+    const int32_t sum = (int32_t)((uint32_t)ya + (uint32_t)yb);
+    bad               = bad || ((ya ^ sum) & (yb ^ sum)) < 0;
+    return rescale_general(sum, m, shift, double_round, out_zp, lo, hi, bad);
+}
+
 // The sum of a residual join to its int8 result before saturation, in single precision.  `bits` is the sum t, |t| < 2^22, plus
 // 0x4B400000, which read as a float is 1.5 * 2^23 + t; S = m * 2^-shift, `base` is 1.5 * 2^23 + out_zp and d one of 0,
 // +-2^(30-shift) (double rounding adds it by the sign of t; few sums come so close to a tie that it matters).

@@ -1405,7 +1405,7 @@ bool make_lean_plan(const TcProblem& q, int num_sms, int max_smem_optin, TcPlan*
 {
     if (diag_env_int("TB200_TC_LEAN", 1) == 0)
         return false;
-    if (q.epi != TC_EPI_RESCALE || !q.lean_ok || q.rec == nullptr || q.b_mn_major || q.in_dtype != TB200_INT8 ||
+    if (q.epi != TC_EPI_RESCALE || !q.lean_ok || q.rec == nullptr || q.rec_ok == nullptr || q.b_mn_major || q.in_dtype != TB200_INT8 ||
         q.out_dtype != TB200_INT8 || q.out_sy != 0 || q.tile_begin != 0 || q.tile_end != 0)
         return false;
     if ((q.OC % 32) != 0 || (reinterpret_cast<uintptr_t>(q.out) & 31) != 0)
@@ -1588,7 +1588,11 @@ tb200_status tc_gemm_launch(tb200_ctx* ctx, const TcProblem& q)
     bool taken              = false;
     const tb200_status chan = conv_chan_launch(ctx, q, &taken);
     if (taken)
+    {
+        if (chan == TB200_OK)
+            replay_note_launch(ctx, q);
         return chan;
+    }
     TcPlan plan;
     plan.lean = false;
     std::string why;
@@ -1676,7 +1680,9 @@ tb200_status tc_gemm_launch(tb200_ctx* ctx, const TcProblem& q)
         }
         timer_end(ctx);
         const tb200_status lst = post_launch(ctx, "tc_conv_lean_i8");
-        if (lst != TB200_OK)
+        if (lst == TB200_OK)
+            replay_note_launch(ctx, q);
+        else
         {
             // say what the launch asked for: the usual cause is a build whose register or shared-memory use grew
             cudaFuncAttributes fa;

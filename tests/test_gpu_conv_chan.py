@@ -207,3 +207,72 @@ def test_split_form_gives_up_and_recovers(ctx):
     assert st == tb.Status.OK and np.array_equal(out.astype(np.int32), exp)
     for t in ts + [to]:
         t.free()
+
+
+# ------------------------------------------------------------------------------------------------ constants under a captured graph
+REPLACED = [
+    # n, h, w, ic, oc, (kh, kw), pad, stride, zero point, join behind it
+    (30, 64, 64, 32, 128, (1, 1), [0, 0, 0, 0], [1, 1], 3, False),
+    (9, 14, 14, 256, 288, (3, 3), [1, 1, 1, 1], [1, 1], 100, False),      # border classes
+    (7, 38, 40, 96, 64, (3, 3), [1, 1, 1, 1], [1, 1], -128, False),       # two pixels side by side
+    (1, 28, 28, 128, 128, (3, 3), [1, 1, 1, 1], [1, 1], -128, False),     # K split over clusters
+    (5, 7, 7, 512, 512, (3, 3), [1, 1, 1, 1], [1, 1], -128, False),
+    (16, 30, 30, 64, 160, (3, 3), [1, 1, 1, 1], [1, 1], -128, False),     # a pixel per thread
+    (16, 30, 31, 64, 160, (1, 1), [0, 0, 0, 0], [1, 1], 5, False),
+    (1, 224, 224, 3, 64, (7, 7), [3, 2, 3, 2], [2, 2], -128, False),      # few channels, pixels side by side
+    (2, 128, 129, 3, 64, (7, 7), [3, 2, 3, 3], [2, 2], 9, False),         # ... an odd number of columns
+    (30, 64, 64, 32, 128, (1, 1), [0, 0, 0, 0], [1, 1], 3, True),
+    (31, 14, 14, 256, 1024, (1, 1), [0, 0, 0, 0], [1, 1], -128, True),
+    (6, 31, 30, 96, 96, (3, 3), [1, 1, 1, 1], [1, 1], -128, True),
+    (1, 14, 14, 256, 320, (1, 1), [0, 0, 0, 0], [1, 1], -128, True),
+]
+
+
+@pytest.mark.parametrize("rounding", ["SINGLE_ROUND", "DOUBLE_ROUND"])
+@pytest.mark.parametrize("case", REPLACED)
+def test_records_follow_constants_under_a_captured_graph(ctx, case, rounding):
+    """Multipliers and shifts uploaded under a captured graph: usable records, ones that are not (the RESCALE accepts every value
+    there is, but not every value its K could make), a REQUIRE that fails, and back."""
+    n, h, w, ic, oc, (kh, kw), pad, stride, zp, join = case
+    r, x, wt, b, mult, shift = _operands(n * h + oc, n, h, w, ic, oc, kh, kw)
+    acc = orc.conv2d(x, wt, b, pad, stride, [1, 1], zp, 0, nthreads=orc.num_procs())
+    bits = int(np.abs(acc).max()).bit_length()
+    # |acc| < 2^bits, so shift bits + 1 is accepted; the record of a K that reaches 2^(bits + 1) is not usable
+    assert kh * kw * ic * 255 * 128 >= 1 << (bits + 1)
+    good = (mult, shift)
+    tight, low = ((np.full(oc, 1 << 20, np.int32), np.full(oc, bits + d, np.int8)) for d in (1, -1))
+    ts = [ctx.from_numpy(v) for v in (x, wt, b, mult, shift)]
+    other = r.integers(-128, 128, size=acc.shape).astype(np.int8)
+    outp, lo, hi = (1700000001, 41, -128), -100, 90
+    cs = [ctx.from_numpy(other)]
+    cs += [ctx.from_numpy(np.array([v], dt)) for m, s, _ in LINEAR + (outp,) for v, dt in ((m, np.int32), (s, np.int8))]
+    legs = [tb.RescaleAttr(cs[2 * i + 1], cs[2 * i + 2], LINEAR[i][2], 0) for i in range(2)]
+    back = tb.RescaleAttr(cs[5], cs[6], 0, outp[2], rounding="DOUBLE_ROUND")
+    to  = ctx.empty(I8, acc.shape)
+    epi = tb.Epilogue(tb.RescaleAttr(ts[3], ts[4], 0, -3, True, rounding, per_channel=True), (lo, hi))
+    if join:
+        run = lambda: ctx.conv2d_add(ts[0], ts[1], ts[2], to, pad, stride, [1, 1], zp, 0, epi, legs[0], cs[0], legs[1], back)
+    else:
+        run = lambda: ctx.conv2d(ts[0], ts[1], ts[2], to, pad, stride, [1, 1], zp, 0, epi)
+    run()
+    assert ctx.sync() == tb.Status.OK and ctx.last_kernel() == "tc_conv_lean_i8" + ("_join" if join else "")
+    ctx.capture_begin()
+    run()
+    g = ctx.capture_end()
+    for params in (good, tight, low, good):
+        ts[3].upload(params[0]), ts[4].upload(params[1])
+        to.upload(np.full(acc.shape, 55, np.int8))
+        ctx.graph_launch(g)
+        st, out = to.download(check=False)
+        est, q = orc.rescale(acc, *params, True, True, rounding, 0, -3, 32, 8)
+        assert (est == orc.VALID) == (params is not low)
+        if params is low:
+            assert st == tb.Status.UNPREDICTABLE
+            continue
+        exp = np.clip(q, lo, hi)
+        if join:
+            est, exp = _join(exp.astype(np.int8), other, LINEAR, outp, "DOUBLE_ROUND", -128, 127)
+        assert st == tb.Status.OK and np.array_equal(out.astype(np.int32), exp)
+    ctx.graph_destroy(g)
+    for t in ts + cs + [to]:
+        t.free()
