@@ -122,3 +122,25 @@ def test_few_channels_side_by_side(ctx, case):
         assert est != orc.VALID or np.array_equal(out.astype(np.int32), exp)
     for t in ts + [to]:
         t.free()
+
+
+@pytest.mark.parametrize("H", [1, 4])
+@pytest.mark.parametrize("name", ["fp16", "bf16"])
+def test_matmul_rows_long_sums(ctx, name, H):
+    """K = 4000 in one block per column (as many batches as fill the SMs).  Sums of 16 products, 31 of those per warp, eight
+    warps: with unit roundoff u the rounding errors' root mean square is u / sqrt(3) * sqrt((248 * 136 + 8 * 496 * 16 + 36 *
+    500) / 4000) = 1.85e-7 of the result's, less for mantissas above one; a running sum over 500 gives 5.5e-7 by the same rule,
+    sums of 64 by the tensor core 1.8e-7."""
+    N, C, W = 160, 4000, 100
+    r = util.rng(3400 + H)
+    a, b = (orc.fptrunc(r.standard_normal(s).astype(np.float32), name) for s in ((N, H, C), (N, C, W)))
+    up = lambda v: ctx.from_numpy(v.astype(np.float16)) if name == "fp16" else ctx.from_numpy(util.to_bf16_bits(v), BF16)
+    ta, tbb, to = up(a), up(b), ctx.empty(F32, (N, H, W))
+    ctx.matmul(ta, tbb, to)
+    assert ctx.last_kernel() == "matmul_rows_f16"
+    st, out = to.download()
+    ref = np.matmul(a.astype(np.float64), b.astype(np.float64))
+    err = np.sqrt(np.mean((out - ref) ** 2) / np.mean(ref ** 2))
+    assert st == tb.Status.OK and err < 1.85e-7, err
+    for t in (ta, tbb, to):
+        t.free()
