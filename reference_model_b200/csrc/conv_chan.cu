@@ -834,14 +834,15 @@ __global__ void __launch_bounds__(kSplitThreads, 2) conv_split_kernel(const __gr
                 border[k] = __ballot_sync(0xffffffffu, b);
             }
         }
-        ptx::dep_launch_wait();    // the other operand of a join is the predecessor's; the output may still be read by it
+        // the other operand of a join is the predecessor's (an ordinary load, which stays behind this); the output may still be read by it
+        ptx::dep_launch_wait();
         if (p.join != nullptr)
         {
 #pragma unroll
             for (int q = 0; q < PX / 4; q++)
                 if (4 * q < own)
                     res[q] = p0 + col0 + 4 * q + t < p.pixels && ch4 < p.OC
-                                 ? __ldcg(reinterpret_cast<const unsigned int*>(p.res + at0 + (int64_t)(4 * q) * p.OC))
+                                 ? *reinterpret_cast<const uint32_t*>(p.res + at0 + (int64_t)(4 * q) * p.OC)
                                  : 0u;
         }
         if (chunks > 0)

@@ -144,3 +144,45 @@ def test_matmul_rows_long_sums(ctx, name, H):
     assert st == tb.Status.OK and err < 1.85e-7, err
     for t in (ta, tbb, to):
         t.free()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_matmul_rows_read_what_the_launch_before_wrote(ctx, captured):
+    """A chain of products with permutations, each launch overlapping the tail of the one whose result it reads (as B in the
+    last one): exact for every input."""
+    r, C, steps = util.rng(3500), 512, 24
+    ps = [r.permutation(C) for _ in range(4)]
+    ms = []
+    for p in ps:
+        m = np.zeros((1, C, C), np.float16)
+        m[0, p, np.arange(C)] = 1.0
+        ms.append(ctx.from_numpy(m))
+    xs, last = [ctx.empty(F16, (1, 4, C)) for _ in range(2)], ctx.empty(F32, (1, 1, 4))
+    one = ctx.from_numpy(np.ones((1, 1, C), np.float16))
+
+    def chain():
+        for i in range(steps):
+            ctx.matmul(xs[i % 2], ms[i % 4], xs[1 - i % 2])
+            assert ctx.last_kernel() == "matmul_rows_f16"
+        ctx.matmul(one, column, last)
+
+    column = xs[steps % 2].reshape([1, C, 4])
+    chain()
+    if captured:
+        ctx.capture_begin()
+        chain()
+        g = ctx.capture_end()
+    for k in range(8):
+        x = r.integers(-8, 8, size=(1, 4, C)).astype(np.float16)
+        xs[0].upload(x)
+        ctx.graph_launch(g) if captured else chain()
+        exp = x
+        for i in range(steps):
+            exp = exp[:, :, ps[i % 4]]
+        assert np.array_equal(xs[steps % 2].download()[1], exp)
+        assert np.array_equal(last.download()[1][0, 0], exp.reshape(C, 4).astype(np.float32).sum(0))
+    if captured:
+        ctx.graph_destroy(g)
+    column.free()
+    for t in ms + xs + [one, last]:
+        t.free()
