@@ -135,6 +135,7 @@ struct tb200_ctx
     int launch_overlap   = 1;    // launch the kernels that support it with programmatic stream serialization
     int max_pairs[3]     = { 0, 0, 0 };    // resident CTA pairs of the three CTA-pair kernels on this device, 0 = not asked yet
     int dw_blocks[16]    = {};             // resident blocks per SM of the sliding depthwise kernels, 0 = not asked yet
+    int rows_blocks[12]  = {};             // ... of the kernels for MATMUL with up to four rows
     std::bitset<128> smem_attr_set;        // bit per kernel whose dynamic shared-memory limit has been raised on this device
     // output gather across GPUs (dist.cu): an NCCL communicator created by tb200_comm_init or handed in by the host
     void* comm           = nullptr;

@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(kRowsThreads) matmul_rows_i8_kernel(const __gr
 {
     __shared__ int32_t part[kRowsWarps][H + 1][kRowsCols];
     __shared__ int32_t sum[H + 1][kRowsCols];
-    __shared__ int32_t row_sum[H];
+    constexpr int P = kRowsWarps / H;    // warps that share out a row of A
+    __shared__ int32_t row_part[H][P];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = p.splits > 1 ? (int)ptx::cluster_ctarank() : 0;
     const int col0 = (int)(blockIdx.x / (unsigned)p.splits) * kRowsCols, col = col0 + lane * 4;
@@ -110,6 +111,18 @@ __global__ void __launch_bounds__(kRowsThreads) matmul_rows_i8_kernel(const __gr
     if (tid == 0)
         ptx::dep_launch_trigger();
     ptx::dep_launch_wait();
+    // sums of A's rows over all of K, for B's zero point: the first words are asked for here and added up behind the loop (a warp
+    // each behind it added a latency per 128 elements: 2x3x500x3168 7.7 us, 7.0 so)
+    const bool summing = p.b_zp != 0 && warp < H * P;
+    const int sum_k = (warp / H * 32 + lane) * 4, sum_step = P * 128;
+    uint32_t row_words[4] = { 0, 0, 0, 0 };
+    if (summing)
+    {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (sum_k + j * sum_step < p.C)
+                row_words[j] = rows_load(A + (int64_t)(warp % H) * p.C + sum_k + j * sum_step);
+    }
     int32_t acc[H + 1][4];
 #pragma unroll
     for (int h = 0; h <= H; h++)
@@ -147,17 +160,19 @@ __global__ void __launch_bounds__(kRowsThreads) matmul_rows_i8_kernel(const __gr
             }
         }
     }
-    // sums of A's rows, a warp each, over all of K
-    if (warp < H)
+    if (summing)
     {
         int32_t s = 0;
-        for (int k = lane * 4; k < p.C; k += 128)
-            s = __dp4a((int)rows_load(A + (int64_t)warp * p.C + k), 0x01010101, s);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            s = __dp4a((int)row_words[j], 0x01010101, s);
+        for (int k = sum_k + 4 * sum_step; k < p.C; k += sum_step)
+            s = __dp4a((int)rows_load(A + (int64_t)(warp % H) * p.C + k), 0x01010101, s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
             s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0)
-            row_sum[warp] = s;
+            row_part[warp % H][warp / H] = s;
     }
     // all sums of a column meet in shared memory again (the warps' parts have been added up by then)
     int32_t* const out = reinterpret_cast<int32_t*>(p.out) + (int64_t)blockIdx.y * H * p.W;
@@ -168,9 +183,16 @@ __global__ void __launch_bounds__(kRowsThreads) matmul_rows_i8_kernel(const __gr
     for (int e = tid; e < H * own; e += kRowsThreads)
     {
         const int h = e / own, c = rank * own + e % own;
+        int32_t row_sum = 0;
+        if (p.b_zp != 0)
+        {
+#pragma unroll
+            for (int j = 0; j < P; j++)
+                row_sum += row_part[h][j];
+        }
         if (col0 + c < p.W)
             out[(int64_t)h * p.W + col0 + c] =
-                (int32_t)((uint32_t)cs[h * kRowsCols + c] - (uint32_t)p.a_zp * (uint32_t)cs[H * kRowsCols + c] - (uint32_t)p.b_zp * (uint32_t)row_sum[h] +
+                (int32_t)((uint32_t)cs[h * kRowsCols + c] - (uint32_t)p.a_zp * (uint32_t)cs[H * kRowsCols + c] - (uint32_t)p.b_zp * (uint32_t)row_sum +
                           (uint32_t)p.C * (uint32_t)(p.a_zp * p.b_zp));
     }
 }
@@ -282,10 +304,11 @@ typedef void (*RowsKern)(const RowsParams);
 }    // namespace
 
 // Whole words of both operands; K deep enough to share out.  65 535 batches are a grid's limit.  Per call, against the tensor core's
-// tiles (us): int8 1x1x2048x1000 5.5 / 9.3, 1x4x256x64 3.9 / 13.2, 32x3x1024x512 10.3 / 17.4, 1x4x8192x8192 31 / 45, 1000x4x256x256
-// 24 / 39; fp16 1x1x2048x1000 3.7 / 23.1, 1x4x256x64 3.1 / 6.4, 8x2x4096x1024 16.4 / 40.5, 1x4x8192x8192 33 / 76, 1000x1x256x64
-// 8.7 / 14.6, but 1000x4x256x256 36 / 31: with more than eight blocks per SM the tiles' own loads keep memory busy, and several
-// rows of 16-bit elements cost a conversion and a multiply-add each.
+// tiles (us): int8 1x1x2048x1000 5.3 / 9.5, 1x4x256x64 4.0 / 16.3, 32x3x1024x512 7.5 / 23.9, 1x4x8192x8192 23 / 51, 1000x4x256x256
+// 25 / 45; fp16 1x1x2048x1000 4.5 / 24.6, 1x4x256x64 3.8 / 8.2, 8x2x4096x1024 17.1 / 42.1, 1x4x8192x8192 35 / 78, 1000x1x256x64
+// 8.3 / 16.4, but 1000x4x256x256 36 / 31: with more than eight blocks per SM the tiles' own loads keep memory busy, and several
+// rows of 16-bit elements cost a conversion and a multiply-add each.  Over 460 shapes the time is 0.56 of the tiles'; they are faster
+// in some with about a block per SM: int8 16x1x488x880 8.2 / 6.7, fp16 34x2x3208x416 27.9 / 19.5 (but 13x2x2848x944 13.9 / 27.8).
 bool matmul_rows_supported(tb200_dtype dt, const void* a, const void* b, int N, int H, int C, int W)
 {
     const uintptr_t al = dt == TB200_INT8 ? 3 : 7;
@@ -305,10 +328,22 @@ tb200_status matmul_rows_launch(tb200_ctx* ctx, tb200_dtype dt, const void* a, c
     RowsParams p;
     p.a = a; p.b = b; p.out = out; p.C = C; p.W = W; p.a_zp = a_zp; p.b_zp = b_zp;
     p.out_f32 = out_dt == TB200_FP32 ? 1 : 0;
-    // K over a cluster while that leaves a block 128 rows and the grid below one block per SM
+    const int type      = dt == TB200_INT8 ? 0 : dt == TB200_FP16 ? 1 : 2;
+    const RowsKern kern = kerns[type][H - 1];
+    int& resident       = ctx->rows_blocks[type * 4 + H - 1];
+    if (resident == 0)
+    {
+        int occ = 0;
+        TB200_CUDA_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kRowsThreads, 0));
+        resident = std::max(1, occ);
+    }
+    // K over a cluster while that leaves a block 128 rows and the grid is below one block per SM, or still fits the SMs at once: it is
+    // the bytes in flight that a grid of one or two blocks per SM lacks (int8, up to one block per SM, so, and the tensor core's tiles, us:
+    // 4x1x2228x1840 16.8 / 11.1 / 10.6, 34x4x1248x288 15.0 / 10.8 / 10.5, 7x3x788x2000 11.1 / 7.5 / 8.3, 1x4x8192x8192 37 / 23 / 51).
     const int64_t blocks = (int64_t)((W + kRowsCols - 1) / kRowsCols) * N;
     p.splits = 1;
-    while (p.splits < 8 && C / (2 * p.splits) >= 128 && blocks * p.splits < ctx->num_sms)
+    while (p.splits < 8 && C / (2 * p.splits) >= 128 &&
+           (blocks * p.splits < ctx->num_sms || blocks * p.splits * 2 <= (int64_t)resident * ctx->num_sms))
         p.splits *= 2;
     p.k_per_cta = ((C + p.splits - 1) / p.splits + 3) & ~3;
     cudaLaunchConfig_t cfg;
@@ -325,7 +360,7 @@ tb200_status matmul_rows_launch(tb200_ctx* ctx, tb200_dtype dt, const void* a, c
     cfg.attrs    = at;
     cfg.numAttrs = ctx->launch_overlap ? 2 : 1;
     timer_begin(ctx);
-    cudaLaunchKernelEx(&cfg, kerns[dt == TB200_INT8 ? 0 : dt == TB200_FP16 ? 1 : 2][H - 1], p);
+    cudaLaunchKernelEx(&cfg, kern, p);
     timer_end(ctx);
     return post_launch(ctx, dt == TB200_INT8 ? "matmul_rows_i8" : "matmul_rows_f16");
 }

@@ -186,3 +186,18 @@ def test_matmul_rows_read_what_the_launch_before_wrote(ctx, captured):
     column.free()
     for t in ms + xs + [one, last]:
         t.free()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 8196, 132), (2, 2, 4100, 12), (1, 3, 1540, 260), (1, 4, 2052, 64), (300, 4, 256, 128)])
+def test_matmul_rows_sums_of_a(ctx, shape):
+    """B's zero point alone: the sums of A's rows, shared out among warps, with words behind the ones that are asked for first."""
+    N, H, C, W = shape
+    r = util.rng(3600 + C)
+    a, b = r.integers(-128, 128, size=(N, H, C)).astype(np.int8), r.integers(-128, 128, size=(N, C, W)).astype(np.int8)
+    ta, tbb, to = ctx.from_numpy(a), ctx.from_numpy(b), ctx.empty(tb.DType.INT32, (N, H, W))
+    ctx.matmul(ta, tbb, to, 0, 77)
+    assert ctx.last_kernel() == "matmul_rows_i8"
+    st, out = to.download()
+    assert st == tb.Status.OK and np.array_equal(out, orc.matmul(a, b, 0, 77, nthreads=8))
+    for t in (ta, tbb, to):
+        t.free()
