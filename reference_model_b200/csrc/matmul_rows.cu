@@ -303,7 +303,8 @@ typedef void (*RowsKern)(const RowsParams);
 
 }    // namespace
 
-// Whole words of both operands; K deep enough to share out.  65 535 batches are a grid's limit.  Per call, against the tensor core's
+// Whole words of both operands; K deep enough to share out, and no more rows than the kernels' 32-bit indexes (which step past the
+// last one) reach.  65 535 batches are a grid's limit.  Per call, against the tensor core's
 // tiles (us): int8 1x1x2048x1000 5.3 / 9.5, 1x4x256x64 4.0 / 16.3, 32x3x1024x512 7.5 / 23.9, 1x4x8192x8192 23 / 51, 1000x4x256x256
 // 25 / 45; fp16 1x1x2048x1000 4.5 / 24.6, 1x4x256x64 3.8 / 8.2, 8x2x4096x1024 17.1 / 42.1, 1x4x8192x8192 35 / 78, 1000x1x256x64
 // 8.3 / 16.4, but 1000x4x256x256 36 / 31: with more than eight blocks per SM the tiles' own loads keep memory busy, and several
@@ -312,7 +313,7 @@ typedef void (*RowsKern)(const RowsParams);
 bool matmul_rows_supported(tb200_dtype dt, const void* a, const void* b, int N, int H, int C, int W)
 {
     const uintptr_t al = dt == TB200_INT8 ? 3 : 7;
-    return (dt == TB200_INT8 || dt == TB200_FP16 || dt == TB200_BF16) && H >= 1 && H <= 4 && C >= 256 && W >= 4 && C % 4 == 0 && W % 4 == 0 && N <= 65535 &&
+    return (dt == TB200_INT8 || dt == TB200_FP16 || dt == TB200_BF16) && H >= 1 && H <= 4 && C >= 256 && C <= (1 << 30) && W >= 4 && C % 4 == 0 && W % 4 == 0 && N <= 65535 &&
            !(dt != TB200_INT8 && H > 1 && C % 8 == 0 && W % 8 == 0 && (int64_t)N * ((W + kRowsCols - 1) / kRowsCols) > 8 * 148) &&
            ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & al) == 0;
 }
