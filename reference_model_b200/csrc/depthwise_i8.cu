@@ -19,7 +19,6 @@
 // 32 x 57 x 57 x 144 stride 2 14.3 -> 9.2, 16 x 28 x 28 x 240 5 x 5 stride 2 9.9 -> 5.3.  What bounds it: 17 instructions per
 // output of four channels and row, issued in 40 % of the slots by the 14 warps per SM that registers and pieces leave.
 #include <algorithm>
-#include <cmath>
 #include <cuda_runtime.h>
 
 #include "common.h"
@@ -359,6 +358,37 @@ tb200_status depthwise_slide_pack(tb200_ctx* ctx, const DepthwiseI8Problem& q, v
     return post_launch(ctx, "depthwise_pack");
 }
 
+// Pieces of a row: a thread is a chain of columns, so a call takes a chain's length times the waves of blocks, or the time its
+// instructions take where that is longer.  SM cycles: 350 per column of a 3 x 3 chain, 600 of a 5 x 5
+// one, 1500 to 2500 for the first output; 5 per 32 outputs.  32 x 56 x 56 x 144, 3 x 3, by outputs per piece: 56 24.3 us, 28
+// and 14 18.4, 19, 12 and 8 20.5, 5 26.6.  Tried is each piece count that gives another length; on rows of more than 256 outputs a
+// quarter more pieces at a time, some twenty counts (all of them took the host 5 us for 4801 outputs).  Returns how many.
+static int dw_pieces(int64_t lines, int OW, int K, int S, int R, int num_sms, int blocks_per_sm, int* best_len, int* best_strips)
+{
+    const int64_t room = (int64_t)num_sms * blocks_per_sm;
+    double best        = 0;
+    int tried          = 0;
+    for (int strips = std::max(1, OW / 256), next; strips <= std::max(1, OW / 2); strips = next, tried++)
+    {
+        const int len = (OW + strips - 1) / strips;
+        next          = len > 1 ? (OW + len - 2) / (len - 1) : OW + 1;
+        if (OW > 256)
+            next = std::max(next, strips + strips / 4);
+        const int64_t threads = lines * ((OW + len - 1) / len);
+        const double waves    = (double)((threads + 128 * room - 1) / (128 * room));
+        const double chain    = K == 3 ? (len + 3 - S) * 350.0 + 2500 : (len + 5 - S) * 600.0 + 1500;
+        const double work     = (double)threads / 32 / num_sms * (len + 3) * R * 4 * 5;
+        const double cost     = std::max(waves * chain, work);
+        if (best == 0 || cost < best * 0.99)
+        {
+            best         = cost;
+            *best_len    = len;
+            *best_strips = (OW + len - 1) / len;
+        }
+    }
+    return tried;
+}
+
 tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q, const void* block, const char* name)
 {
     const int C4 = (q.C + 3) & ~3;
@@ -393,35 +423,11 @@ tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q,
         TB200_CUDA_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kerns[which], 128, 0));
         ctx->dw_blocks[which] = std::max(1, occ);
     }
-    // Pieces of a row: a thread is a chain of columns, so a call takes a chain's length times the waves of blocks, or the time its
-    // instructions take where that is longer.  SM cycles: 350 per column of a 3 x 3 chain, 600 of a 5 x 5
-    // one, 1500 to 2500 for the first output; 5 per 32 outputs.  32 x 56 x 56 x 144, 3 x 3, by outputs per piece: 56 24.3 us, 28
-    // and 14 18.4, 19, 12 and 8 20.5, 5 26.6.
-    const int64_t lines = (int64_t)q.N * p.row_groups * p.c4;
-    const double room   = (double)ctx->num_sms * ctx->dw_blocks[which];
-    double best         = 0;
-    for (int strips = 1, last = 0; strips <= std::max(1, q.OW / 2); strips++)
-    {
-        const int len = (q.OW + strips - 1) / strips;
-        if (len == last)
-            continue;
-        last = len;
-        const int64_t threads = lines * ((q.OW + len - 1) / len);
-        const double waves    = std::max(1.0, std::ceil((double)((threads + 127) / 128) / room));
-        const double chain    = q.K == 3 ? (len + 3 - q.S) * 350.0 + 2500 : (len + 5 - q.S) * 600.0 + 1500;
-        const double work     = (double)threads / 32 / ctx->num_sms * (len + 3) * R * 4 * 5;
-        const double cost     = std::max(waves * chain, work);
-        if (best == 0 || cost < best * 0.99)
-        {
-            best     = cost;
-            p.len    = len;
-            p.strips = (q.OW + len - 1) / len;
-        }
-    }
+    dw_pieces((int64_t)q.N * p.row_groups * p.c4, q.OW, q.K, q.S, R, ctx->num_sms, ctx->dw_blocks[which], &p.len, &p.strips);
     fastdiv_make((uint32_t)p.c4, p.fd_c4);
     fastdiv_make((uint32_t)p.strips, p.fd_strips);
     fastdiv_make((uint32_t)p.row_groups, p.fd_rg);
-    p.total    = (int)(lines * p.strips);
+    p.total    = (int)((int64_t)q.N * p.row_groups * p.c4 * p.strips);
     p.fill4    = (uint32_t)(q.in_zp & 0xff) * 0x01010101u;
     p.clamp_lo = q.clamp_lo;
     p.clamp_hi = q.clamp_hi;
