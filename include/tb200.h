@@ -411,6 +411,10 @@ extern "C"
     TB200_API int tb200_set_kernel_policy(tb200_ctx* ctx, int policy);
     /* Name of the kernel family the last operator call used ("tc_gemm_i8", "direct_conv", ...). */
     TB200_API const char* tb200_last_kernel(const tb200_ctx* ctx);
+    /* The form that call took where the family has several ("conv_chan 256 pixels, 3 slots", "conv_split 32 pixels, K over 4",
+     * "lean", "lean halo", each followed by ", 2 side by side" where output pixels of a row share a row of the product);
+     * tb200_last_kernel's name elsewhere.  For tests and diagnosis; valid until the next call. */
+    TB200_API const char* tb200_last_form(tb200_ctx* ctx);
 
 #ifdef __cplusplus
 }

@@ -74,7 +74,7 @@ EXPORTS = [
     "tb200_tensor_alloc", "tb200_tensor_wrap", "tb200_tensor_free", "tb200_tensor_upload", "tb200_tensor_download",
     "tb200_tensor_data", "tb200_tensor_bytes", "tb200_tensor_slice", "tb200_tensor_reshape", "tb200_conv2d", "tb200_depthwise_conv2d", "tb200_conv2d_depthwise", "tb200_conv2d_add", "tb200_conv3d", "tb200_transpose_conv2d", "tb200_matmul",
     "tb200_rescale", "tb200_clamp", "tb200_add", "tb200_residual_add", "tb200_max_pool2d", "tb200_avg_pool2d",
-    "tb200_matmul_host", "tb200_set_kernel_policy", "tb200_last_kernel", "tb200_matmul_i8_noalloc",
+    "tb200_matmul_host", "tb200_set_kernel_policy", "tb200_last_kernel", "tb200_last_form", "tb200_matmul_i8_noalloc",
     "tb200_npy_probe", "tb200_tensor_load_npy", "tb200_tensor_save_npy",
     "tb200_set_wait_limit", "tb200_set_shared_gpu", "tb200_set_launch_overlap", "tb200_const_cache_control", "tb200_const_cache_entries",
     "tb200_comm_unique_id", "tb200_comm_init", "tb200_comm_attach", "tb200_comm_destroy", "tb200_comm_rank",
@@ -140,6 +140,7 @@ def load_library():
         "tb200_tensor_save_npy": (i32, [vp, vp, cp]),
         "tb200_set_kernel_policy": (ctypes.c_int, [vp, ctypes.c_int]),
         "tb200_last_kernel": (cp, [vp]),
+        "tb200_last_form": (cp, [vp]),
         "tb200_set_wait_limit": (i32, [vp, ctypes.c_uint64]),
         "tb200_set_shared_gpu": (i32, [vp, i32]),
         "tb200_set_launch_overlap": (i32, [vp, i32]),
@@ -307,6 +308,9 @@ class Context:
 
     def last_kernel(self):
         return self.lib.tb200_last_kernel(self.handle).decode()
+
+    def last_form(self):
+        return self.lib.tb200_last_form(self.handle).decode()
 
     def launch_count(self):
         return int(self.lib.tb200_launch_count(self.handle))

@@ -63,6 +63,7 @@ tb200_status post_launch(tb200_ctx* ctx, const char* kernel_name, int n_launches
 {
     ctx->launches += (uint64_t)n_launches;
     ctx->last_kernel = kernel_name;
+    ctx->form        = tb200_ctx::Form();
     cudaError_t e    = cudaGetLastError();
     if (e != cudaSuccess)
         return fail(ctx, TB200_INTERNAL, "launch of %s failed: %s", kernel_name, cudaGetErrorString(e));
@@ -604,6 +605,23 @@ extern "C" const char* tb200_last_kernel(const tb200_ctx* ctx)
     return ctx ? ctx->last_kernel : "none";
 }
 
+extern "C" const char* tb200_last_form(tb200_ctx* ctx)
+{
+    if (!ctx || !ctx->form.name)
+        return tb200_last_kernel(ctx);
+    const tb200_ctx::Form& f = ctx->form;
+    int at = snprintf(ctx->form_text, sizeof(ctx->form_text), "%s", f.name);
+    if (f.pixels)
+        at += snprintf(ctx->form_text + at, sizeof(ctx->form_text) - at, " %d pixels", f.pixels);
+    if (f.slots)
+        at += snprintf(ctx->form_text + at, sizeof(ctx->form_text) - at, ", %d slots", f.slots);
+    if (f.split)
+        at += snprintf(ctx->form_text + at, sizeof(ctx->form_text) - at, ", K over %d", f.split);
+    if (f.side > 1)
+        snprintf(ctx->form_text + at, sizeof(ctx->form_text) - at, ", %d side by side", f.side);
+    return ctx->form_text;
+}
+
 extern "C" tb200_status tb200_sync(tb200_ctx* ctx)
 {
     if (!ctx)
@@ -1076,7 +1094,9 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                         if (!conv_chan_supported(ctx, qe))
                             return kNeedsSeparateJoin;
                     }
-                    return tc_gemm_launch(ctx, qe);
+                    const tb200_status lst = tc_gemm_launch(ctx, qe);
+                    ctx->form.side         = E;
+                    return lst;
                 };
                 // At most 64 channels leave half of conv_chan_kernel's 128 rows empty: two pixels side by side fill them, at
                 // (KW + stride) / KW times the products (which the empty rows would have cost twice over).  Batch 256 at 56x56, 64
@@ -1245,7 +1265,8 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     st = post_launch(ctx, "conv_window_relayout", 1);
                     if (st != TB200_OK)
                         return st;
-                    st = tc_gemm_launch(ctx, q);
+                    st             = tc_gemm_launch(ctx, q);
+                    ctx->form.side = E;
                     // a driver that refuses the overlapping-window tensor map sends this shape to the forms below
                     if (!(st == TB200_INTERNAL && ctx->err.find("rejected") != std::string::npos))
                         return st;

@@ -146,6 +146,13 @@ struct tb200_ctx
     uint64_t cache_clock = 0;
     std::vector<std::unique_ptr<tb200::Prepared>> prepared;
     const char* last_kernel = "none";
+    // the form of it (tb200_last_form); post_launch clears it, a launch with several forms sets it behind that
+    struct Form
+    {
+        const char* name = nullptr;
+        int pixels = 0, slots = 0, split = 0, side = 1;
+    } form;
+    char form_text[96] = {};
     std::string err;
     // host-buffer pipeline of tb200_matmul_host: copy streams, events and two sets of device staging buffers
     struct HostPipe

@@ -1275,7 +1275,9 @@ tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q, bool* taken)
         cfg.numAttrs = ctx->launch_overlap ? 2 : 1;
         cudaLaunchKernelEx(&cfg, kern, k);
         timer_end(ctx);
-        return post_launch(ctx, q.join ? "tc_conv_lean_i8_join" : "tc_conv_lean_i8");
+        const tb200_status st = post_launch(ctx, q.join ? "tc_conv_lean_i8_join" : "tc_conv_lean_i8");
+        ctx->form             = { "conv_split", k.px, 0, k.split, 1 };
+        return st;
     }
     static const Kern kerns[2][2][3] = {
         { { conv_chan_kernel<false, false, 0>, conv_chan_kernel<false, false, 1>, conv_chan_kernel<false, false, 2> },
@@ -1301,7 +1303,9 @@ tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q, bool* taken)
     cfg.numAttrs = ctx->launch_overlap ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kern, k);
     timer_end(ctx);
-    return post_launch(ctx, q.join ? "tc_conv_lean_i8_join" : "tc_conv_lean_i8");
+    const tb200_status st = post_launch(ctx, q.join ? "tc_conv_lean_i8_join" : "tc_conv_lean_i8");
+    ctx->form             = { "conv_chan", k.px, k.slots, 0, 1 };
+    return st;
 }
 
 }    // namespace tb200

@@ -1680,6 +1680,7 @@ tb200_status tc_gemm_launch(tb200_ctx* ctx, const TcProblem& q)
         }
         timer_end(ctx);
         const tb200_status lst = post_launch(ctx, "tc_conv_lean_i8");
+        ctx->form.name         = k.lean_halo ? "lean halo" : k.lean_xpar ? "lean, a copy per parity" : "lean";
         if (lst == TB200_OK)
             replay_note_launch(ctx, q);
         else
