@@ -3521,16 +3521,23 @@ extern "C" tb200_status tb200_avg_pool2d(tb200_ctx* ctx, const tb200_tensor* inp
     cache_note_write(ctx, output->data, output->bytes);
     const int block = 256;
     const int grid  = grid_for(ctx, n, block);
+    bool words       = false;
+    const char* form = nullptr;
     switch (input->dtype)
     {
         case TB200_INT8:
-            if (p.C % 4 == 0 && ctx->policy == 0 && p.ky * p.kx >= 16 &&
-                ((reinterpret_cast<uintptr_t>(input->data) | reinterpret_cast<uintptr_t>(output->data)) & 3) == 0)
+            // A share of an output's taps per thread pays while one thread per output word leaves the chip idle: below 256 words per
+            // SM 0.65 to 1.0 of the time (6x17x17x136 8x8 10.3 -> 6.7 us, 39 outputs of 5x5x80 8x8 10.8 -> 8.2), above 1.2 to 3.1 times
+            // (44 of 3x3x432 5x5 8.8 / 10.3, 63 of 12x12x1184 4x4 114 / 356).
+            words = p.C % 4 == 0 && ctx->policy == 0 && ((reinterpret_cast<uintptr_t>(input->data) | reinterpret_cast<uintptr_t>(output->data)) & 3) == 0;
+            if (words && p.ky * p.kx >= 16 && n / 4 <= (int64_t)ctx->num_sms * 256)
+            {
+                form = "avg_pool2d, taps shared";
                 avg_pool_i8x4_shared_kernel<<<(int)std::min<int64_t>((n / 4 + 31) / 32, (int64_t)ctx->num_sms * 8), 256, 0, ctx->stream>>>(
                     reinterpret_cast<const int8_t*>(input->data), reinterpret_cast<int8_t*>(output->data), p, input_zp, output_zp,
                     -128, 127, ctx->d_status);
-            else if (p.C % 4 == 0 && ctx->policy == 0 &&
-                ((reinterpret_cast<uintptr_t>(input->data) | reinterpret_cast<uintptr_t>(output->data)) & 3) == 0)
+            }
+            else if (words)
                 avg_pool_i8x4_kernel<<<grid_for(ctx, n / 4, block), block, 0, ctx->stream>>>(
                     reinterpret_cast<const int8_t*>(input->data), reinterpret_cast<int8_t*>(output->data), p, input_zp, output_zp,
                     -128, 127, ctx->d_status);
@@ -3552,7 +3559,9 @@ extern "C" tb200_status tb200_avg_pool2d(tb200_ctx* ctx, const tb200_tensor* inp
         default:
             return fail(ctx, TB200_ERROR, "OpAvgPool2d: unsupported dtype %d", (int)input->dtype);
     }
-    return post_launch(ctx, "avg_pool2d");
+    st             = post_launch(ctx, "avg_pool2d");
+    ctx->form.name = form;
+    return st;
 }
 
 // =================================================================================================== host buffers

@@ -201,3 +201,21 @@ def test_matmul_rows_sums_of_a(ctx, shape):
     assert st == tb.Status.OK and np.array_equal(out, orc.matmul(a, b, 0, 77, nthreads=8))
     for t in (ta, tbb, to):
         t.free()
+
+
+@pytest.mark.parametrize("shape,kernel,stride,form", [
+    ((63, 26, 26, 84), [4, 4], [2, 2], "avg_pool2d"),                       # 190 512 words of outputs
+    ((37, 9, 9, 164), [5, 5], [2, 2], "avg_pool2d, taps shared"),           # 13 653
+    ((40, 7, 7, 2048), [7, 7], [1, 1], "avg_pool2d, taps shared"),          # a classifier's pool
+    ((80, 7, 7, 2048), [7, 7], [1, 1], "avg_pool2d"),
+])
+def test_avg_pool_shares_taps_where_outputs_are_few(ctx, shape, kernel, stride, form):
+    x = util.rng(3700 + shape[3]).integers(-128, 128, size=shape).astype(np.int8)
+    st, exp = orc.avg_pool2d(x, kernel, [0] * 4, stride, -7, 11)
+    assert st == orc.VALID
+    tx, to = ctx.from_numpy(x), ctx.empty(tb.DType.INT8, exp.shape)
+    ctx.avg_pool2d(tx, to, kernel, [0] * 4, stride, -7, 11)
+    assert ctx.last_form() == form
+    st, out = to.download()
+    assert st == tb.Status.OK and np.array_equal(out.astype(np.int32), exp)
+    tx.free(), to.free()
