@@ -1101,10 +1101,12 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                 // At most 64 channels leave half of conv_chan_kernel's 128 rows empty: two pixels side by side fill them, at
                 // (KW + stride) / KW times the products (which the empty rows would have cost twice over).  Batch 256 at 56x56, 64
                 // to 64: 1x1 37 -> 25 us, 3x3 93 -> 61.  Small problems are a chain of latencies, which the longer products
-                // lengthen: 1x1 on 2x16x10x384 4.8 us against 4.2, 3x3 on 8x18x43x128 7.4 / 6.7, on 14x34x79x32 (9 282 pixels) 7.6 / 8.4.
+                // lengthen, and a 1x1 convolution of many channels is bound by its loads: 1x1 on 2x16x10x384 4.8 us against 4.2, on 106 920
+                // pixels of 512 14.6 / 11.1, 191 406 of 256 12.9 / 13.6; 3x3 on 8 288 pixels of 192 11.8 / 9.6,
+                // 11 232 14.1 / 9.8, 11 008 of 64 7.0 / 6.7, 9 728 of 160 15.3 / 12.6, but 16 500 of 96 11.3 / 13.5.
                 const bool one = KH == 1 && KW == 1 && stride[0] == 1 && stride[1] == 1 && !padded && input->contiguous;
-                const bool two = lean_out && !view && use_cache && ctx->const_cache_on && OC == 64 && (int64_t)N * OH * OW >= 8192 && dilation[1] == 1 &&
-                                 (one ? (int64_t)N * OH * OW % 2 == 0 && (int64_t)N * OH * OW < (1 << 30) : OW % 2 == 0 && !(KH == 1 && KW == 1));
+                const bool two = lean_out && !view && use_cache && ctx->const_cache_on && OC == 64 && (int64_t)N * OH * OW >= (one ? 8192 : 96 * ctx->num_sms) && dilation[1] == 1 &&
+                                 (one ? IC <= 256 && (int64_t)N * OH * OW % 2 == 0 && (int64_t)N * OH * OW < (1 << 30) : OW % 2 == 0 && !(KH == 1 && KW == 1));
                 st = two ? run(2) : kNextForm;
                 if (st == kNextForm)
                     st = run(1);

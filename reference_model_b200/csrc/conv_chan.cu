@@ -1169,13 +1169,18 @@ bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
         return false;
     // Channel blocks less than three quarters full leave rows of the product and threads of the epilogue idle: 160 channels on
     // 21x102x13x96 7.6 us against 6.6 with a pixel per thread, 32 channels 3x3 on 13x32x12x32 8.5 against 5.9; 192 channels 3x3 on
-    // 8x26x10x192 10.4 against 13.5.  Where the products are long they are what counts, and there this kernel needs fewer of
-    // them: 64 channels 3x3 on 10x42x43x512 19.8 against 25.6, 32 channels on 5x43x64x512 19.5 / 24.9, but 5x11x24x192 10.3 / 8.9.
+    // 8x26x10x192 10.4 against 13.5.  Where the products are long and the pixels many they are what counts, and there this kernel
+    // needs fewer of them (K, pixels, us here / with a pixel per thread): 64 channels 3200, 14 850 15.0 / 19.6, 4320, 26 884 35.7 / 91.5,
+    // 3744, 25 688 31.7 / 42.3, but 3456, 12 312 15.9 / 12.6, 4608, 13 392 18.7 / 14.6, 4320, 9 085 31.1 / 26.0; 32 channels 4000, 61 950
+    // 92 / 125, 4800, 16 302 26.3 / 32.9, but 3456, 27 360 27.0 / 20.2, 3168, 81 576 116 / 85, 4000, 6 912 42.9 / 24.0.
     // A residual join pays for itself at any width.
-    if (!k.split && !q.join && q.OC * 4 < (q.OC + 127) / 128 * 128 * 3 && (int64_t)q.KH * q.KW * q.IC < 3072)
+    const int rows = (q.OC + 127) / 128 * 128;
+    if (!k.split && !q.join && q.OC * 4 < rows * 3 &&
+        ((int64_t)q.KH * q.KW * q.IC < (q.OC * 4 <= rows ? 4000 : 3072) || pixels < 96 * (int64_t)ctx->num_sms))
         return false;
-    // Windows over 32-byte pieces, loaded again for each of many channel blocks: 512 channels 3x3 on 24x34x49x96 23.7 / 19.9.
-    if (!k.split && !q.join && q.KH * q.KW > 1 && q.IC % 64 != 0 && q.OC >= 512)
+    // Windows over 32-byte pieces, loaded again for each of several channel blocks: 512 channels 3x3 on 24x34x49x96 23.7 / 19.9, 256
+    // 5x5 on 22x18x50x32 25.9 / 18.9, 448 3x3 on 54x11x18x32 16.4 / 12.0, 416 5x5 on 9x64x25x96 41.3 / 38.4.
+    if (!k.split && !q.join && q.KH * q.KW > 1 && q.IC % 64 != 0 && q.OC >= 256)
         return false;
     k.idesc     = ptx::make_idesc(2u, 1u, 1u, 0u, 0u, 128u, (uint32_t)k.px);
     k.tmem_cols = k.split ? k.px : k.px == 192 ? 512 : 2 * k.px;

@@ -214,7 +214,7 @@ REPLACED = [
     # n, h, w, ic, oc, (kh, kw), pad, stride, zero point, join behind it
     (30, 64, 64, 32, 128, (1, 1), [0, 0, 0, 0], [1, 1], 3, False),
     (9, 14, 14, 256, 288, (3, 3), [1, 1, 1, 1], [1, 1], 100, False),      # border classes
-    (7, 38, 40, 96, 64, (3, 3), [1, 1, 1, 1], [1, 1], -128, False),       # two pixels side by side
+    (11, 38, 40, 96, 64, (3, 3), [1, 1, 1, 1], [1, 1], -128, False),      # two pixels side by side
     (1, 28, 28, 128, 128, (3, 3), [1, 1, 1, 1], [1, 1], -128, False),     # K split over clusters
     (5, 7, 7, 512, 512, (3, 3), [1, 1, 1, 1], [1, 1], -128, False),
     (16, 30, 30, 64, 160, (3, 3), [1, 1, 1, 1], [1, 1], -128, False),     # a pixel per thread
