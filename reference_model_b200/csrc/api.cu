@@ -1029,6 +1029,7 @@ static tb200_status conv2d_impl(tb200_ctx* ctx, const tb200_tensor* input, const
                     if (use_cache && ctx->const_cache_on)
                     {
                         std::string key;
+                        key.reserve(160);
                         key_add(&key, (int)0);
                         key_add(&key, wp); key_add(&key, bp); key_add(&key, mp); key_add(&key, sp);
                         key_add(&key, OC); key_add(&key, KH); key_add(&key, KW); key_add(&key, IC); key_add(&key, bias_n);

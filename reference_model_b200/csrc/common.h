@@ -99,6 +99,44 @@ struct Prepared
 };
 }    // namespace tb200
 
+namespace tb200
+{
+// What a launch works out from sizes alone, kept for the next launch of the same sizes: 64 slots, a newer one takes the place of
+// an older one.  Three words of sizes are the key; contents and addresses play no part.
+template <typename V>
+struct SizeMemo
+{
+    struct Slot
+    {
+        int64_t key[3] = { -1, -1, -1 };
+        V value;
+    } slots[64];
+    Slot& at(int64_t a, int64_t b, int64_t c, bool* known)
+    {
+        const uint64_t h = (uint64_t)a * 0x9E3779B97F4A7C15ull ^ (uint64_t)b * 0xC2B2AE3D27D4EB4Full ^ (uint64_t)c * 0x165667B19E3779F9ull;
+        Slot& s          = slots[h >> 58];
+        *known           = s.key[0] == a && s.key[1] == b && s.key[2] == c;
+        if (!*known)
+        {
+            s.key[0] = a;
+            s.key[1] = b;
+            s.key[2] = c;
+        }
+        return s;
+    }
+};
+
+// conv_chan.cu: which kernel a problem of these sizes runs on, and its layout
+struct ChanChoice
+{
+    int taken, px, resident, slots, ksub, num_stages, x_chunk_bytes, stage_bytes, tiles, w_off, ring_off, split, chunks_per_cta, red_off, grid, smem_bytes;
+};
+struct DwPieces
+{
+    int len, strips;
+};
+}    // namespace tb200
+
 struct tb200_ctx
 {
     int device           = 0;
@@ -134,6 +172,8 @@ struct tb200_ctx
     int join_stream      = 1;    // large table joins through the bulk-copy ring kernel (join_stream.cuh)
     int launch_overlap   = 1;    // launch the kernels that support it with programmatic stream serialization
     int max_pairs[3]     = { 0, 0, 0 };    // resident CTA pairs of the three CTA-pair kernels on this device, 0 = not asked yet
+    std::unique_ptr<tb200::SizeMemo<tb200::ChanChoice>> chan_memo;    // made at the first call that looks
+    std::unique_ptr<tb200::SizeMemo<tb200::DwPieces>> dw_memo;
     int dw_blocks[16]    = {};             // resident blocks per SM of the sliding depthwise kernels, 0 = not asked yet
     int rows_blocks[12]  = {};             // ... of the kernels for MATMUL with up to four rows
     std::bitset<128> smem_attr_set;        // bit per kernel whose dynamic shared-memory limit has been raised on this device
@@ -406,7 +446,7 @@ tb200_status tc_any_launch(tb200_ctx* ctx, const TcProblem& q);
 
 // int8 CONV2D + RESCALE with channels on the accumulator rows (conv_chan.cu), q.lean_ok problems; with q.join the residual join
 // RESCALE, RESCALE, ADD, RESCALE, CLAMP runs on the results before they are stored
-bool conv_chan_supported(const tb200_ctx* ctx, const TcProblem& q);
+bool conv_chan_supported(tb200_ctx* ctx, const TcProblem& q);
 tb200_status conv_chan_launch(tb200_ctx* ctx, const TcProblem& q, bool* taken);    // not taken: nothing done
 // Words of the block behind q.join (residual_record_kernel): with both legs exact multiples of their operand, the sum is
 // one dp2a of (convolution result, other operand) with the two 16-bit coefficients, followed by rescale_rec_apply's second

@@ -1029,7 +1029,119 @@ double split_cost(int px, int S, int chunks, int mmas)
     return S == 8 ? chunks * chunk + 5600 : S == 4 ? chunks * chunk + 6600 : 0;
 }
 
-bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
+// Which kernel takes a problem of these sizes, if any, and in which layout: a function of the sizes alone.
+ChanChoice chan_choose(int num_sms, int max_smem, int64_t pixels, int OC, int IC, int KH, int KW, bool join)
+{
+    ChanChoice c;
+    memset(&c, 0, sizeof(c));
+    const int swz = IC % 128 == 0 ? 128 : IC % 64 == 0 ? 64 : 32, mmas = swz / 32, w_chunk_bytes = 128 * swz;
+    const int total_chunks = KH * KW * (IC / swz), cbs = (OC + 127) / 128;
+    const int budget = (max_smem > 0 ? max_smem : 232448) - 2048;
+
+    // Pixels per tile, where the weights live, slots and stages: the smallest estimate of a first tile from its loads
+    // to its store, and the longest of MMAs, epilogue and loads for every further round.  SM cycles: an MMA of 128 channels by 256 / 192 / 128 / 64 pixels and
+    // 32 bytes of K 171 / 139 / 107 / 104, a commit 60; loads bring 50 bytes per cycle to an SM, 32 when all SMs load (3x3 512 to
+    // 512 on 256x7x7: 8.9 TB/s in tiles of 128 and of 240 pixels alike), and no more than what is in flight (the ring less the
+    // stage in use) per 2900 cycles of latency.
+    double best = 0;
+    for (const int px : { 256, 192, 128, 64 })
+        for (int res = 1; res >= 0; res--)
+            for (int slots = join ? 3 : 2; slots >= (join ? 2 : 1); slots--)
+            {
+                const int64_t pbs = (pixels + px - 1) / px, tiles = pbs * cbs;
+                if (tiles >= (1LL << 30))
+                    continue;
+                const int staging = slots * px * 128;
+                const int w_bytes = res ? total_chunks * w_chunk_bytes : 0;
+                int grid = (int)std::min<int64_t>(tiles, num_sms);
+                if (res)
+                {
+                    if (cbs > num_sms || w_bytes > budget)
+                        continue;
+                    grid = (int)std::min<int64_t>(tiles, (int64_t)num_sms / cbs * cbs);
+                }
+                const int per_chunk = px * swz + (res ? 0 : w_chunk_bytes);
+                const int avail     = budget - 1024 - staging - w_bytes;
+                if (avail < 2 * per_chunk)
+                    continue;
+                int ksub = std::max(1, std::min(total_chunks, 48 * 1024 / per_chunk));
+                while (ksub > 1 && avail / (ksub * per_chunk) < 3)
+                    ksub--;
+                const int stages = std::min(kChanMaxStages, avail / (ksub * per_chunk));
+                const double rate = std::min(std::min(50.0, 32.0 * num_sms / grid), (double)(stages - 1) * ksub * per_chunk / 2900.0);
+                const double mma  = (double)total_chunks * mmas * (px == 256 ? 171 : px == 192 ? 139 : px == 128 ? 107 : 104) +
+                                   60.0 * ((total_chunks + ksub - 1) / ksub + 1);
+                const double epi  = px * (join ? 26.0 : 14.7) + 500;
+                const double load = (double)total_chunks * per_chunk / rate + (join ? px * 128 / 50.0 : 0.0);
+                const int64_t rounds = (tiles + grid - 1) / grid;
+                const bool few       = slots == (join ? 2 : 1);    // the store, or the residual's load, is not overlapped
+                const double cost = 1200 + std::max(mma, load + w_bytes / 50.0) + epi + (double)(rounds - 1) * (std::max(mma, std::max(epi, load)) + (few ? 300 : 0));
+                if (best == 0 || cost < best * 0.98)
+                {
+                    best            = cost;
+                    c.px            = px;
+                    c.resident      = res;
+                    c.slots         = slots;
+                    c.ksub          = ksub;
+                    c.num_stages    = stages;
+                    c.x_chunk_bytes = px * swz;
+                    c.stage_bytes   = ksub * per_chunk;
+                    c.tiles         = (int)tiles;
+                    c.w_off         = staging;
+                    c.ring_off      = staging + w_bytes;
+                    c.grid      = grid;
+                    c.smem_bytes = 1024 + staging + w_bytes + stages * ksub * per_chunk;
+                }
+            }
+    // One tile per cluster of S CTAs, where that fills one wave at most (conv_split_kernel).
+    for (int px = 64; px >= 32; px >>= 1)
+        for (int S = 1; S <= 8 && px / S >= 4 && S <= total_chunks; S *= 2)
+        {
+            const int64_t tiles = (pixels + px - 1) / px * cbs;
+            const int cpc       = (total_chunks + S - 1) / S;
+            const int stage     = (px + 128) * swz;
+            const int smem      = 1024 + cpc * stage + (S > 1 ? px * 512 : 0);
+            // one wave: clusters of 8 and 4 leave SMs of a GPC over when a CTA fills its SM
+            const int room = smem <= 110 * 1024 || S == 1 ? num_sms : num_sms * (S == 8 ? 3 : 4) / (S == 8 ? 4 : 5);
+            if (tiles * S > room || cpc > kSplitMaxChunks || smem > budget)
+                continue;
+            const double cost = split_cost(px, S, cpc, mmas);
+            if (cost > 0 && (best == 0 || cost < best))
+            {
+                best             = cost;
+                c.split          = S;
+                c.chunks_per_cta = cpc;
+                c.px             = px;
+                c.x_chunk_bytes  = px * swz;
+                c.stage_bytes    = stage;
+                c.red_off        = cpc * stage;
+                c.tiles          = (int)tiles;
+                c.grid       = (int)tiles * S;
+                c.smem_bytes = smem;
+            }
+        }
+    if (best == 0)
+        return c;
+    // Channel blocks less than three quarters full leave rows of the product and threads of the epilogue idle: 160 channels on
+    // 21x102x13x96 7.6 us against 6.6 with a pixel per thread, 32 channels 3x3 on 13x32x12x32 8.5 against 5.9; 192 channels 3x3 on
+    // 8x26x10x192 10.4 against 13.5.  Where the products are long and the pixels many they are what counts, and there this kernel
+    // needs fewer of them (K, pixels, us here / with a pixel per thread): 64 channels 3200, 14 850 15.0 / 19.6, 4320, 26 884 35.7 / 91.5,
+    // 3744, 25 688 31.7 / 42.3, but 3456, 12 312 15.9 / 12.6, 4608, 13 392 18.7 / 14.6, 4320, 9 085 31.1 / 26.0; 32 channels 4000, 61 950
+    // 92 / 125, 4800, 16 302 26.3 / 32.9, but 3456, 27 360 27.0 / 20.2, 3168, 81 576 116 / 85, 4000, 6 912 42.9 / 24.0.
+    // A residual join pays for itself at any width.
+    const int rows = (OC + 127) / 128 * 128;
+    if (!c.split && !join && OC * 4 < rows * 3 &&
+        ((int64_t)KH * KW * IC < (OC * 4 <= rows ? 4000 : 3072) || pixels < 96 * (int64_t)num_sms))
+        return c;
+    // Windows over 32-byte pieces, loaded again for each of several channel blocks: 512 channels 3x3 on 24x34x49x96 23.7 / 19.9, 256
+    // 5x5 on 22x18x50x32 25.9 / 18.9, 448 3x3 on 54x11x18x32 16.4 / 12.0, 416 5x5 on 9x64x25x96 41.3 / 38.4.
+    if (!c.split && !join && KH * KW > 1 && IC % 64 != 0 && OC >= 256)
+        return c;
+    c.taken = 1;
+    return c;
+}
+
+bool chan_plan(tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
 {
     if (q.epi != TC_EPI_RESCALE || !q.lean_ok || q.rec == nullptr || q.rec_ok == nullptr || q.b_mn_major || q.in_dtype != TB200_INT8 ||
         q.out_dtype != TB200_INT8 || q.out_sy != 0 || q.xpar || q.tile_begin != 0 || q.tile_end != 0)
@@ -1081,107 +1193,19 @@ bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
     k.cbs            = (q.OC + 127) / 128;
     k.w_chunk_bytes  = 128 * swz;
     k.desc_hi        = ptx::make_smem_desc_hi(16, 8 * swz, swz == 128 ? 2u : swz == 64 ? 4u : 6u);
-    const int budget = (ctx->max_smem_optin > 0 ? ctx->max_smem_optin : 232448) - 2048;
-
-    // Pixels per tile, where the weights live, slots and stages: the smallest estimate of a first tile from its loads
-    // to its store, and the longest of MMAs, epilogue and loads for every further round.  SM cycles: an MMA of 128 channels by 256 / 192 / 128 / 64 pixels and
-    // 32 bytes of K 171 / 139 / 107 / 104, a commit 60; loads bring 50 bytes per cycle to an SM, 32 when all SMs load (3x3 512 to
-    // 512 on 256x7x7: 8.9 TB/s in tiles of 128 and of 240 pixels alike), and no more than what is in flight (the ring less the
-    // stage in use) per 2900 cycles of latency.
-    double best = 0;
-    for (const int px : { 256, 192, 128, 64 })
-        for (int res = 1; res >= 0; res--)
-            for (int slots = q.join ? 3 : 2; slots >= (q.join ? 2 : 1); slots--)
-            {
-                const int64_t pbs = (pixels + px - 1) / px, tiles = pbs * k.cbs;
-                if (tiles >= (1LL << 30))
-                    continue;
-                const int staging = slots * px * 128;
-                const int w_bytes = res ? k.total_chunks * k.w_chunk_bytes : 0;
-                int grid = (int)std::min<int64_t>(tiles, ctx->num_sms);
-                if (res)
-                {
-                    if (k.cbs > ctx->num_sms || w_bytes > budget)
-                        continue;
-                    grid = (int)std::min<int64_t>(tiles, (int64_t)ctx->num_sms / k.cbs * k.cbs);
-                }
-                const int per_chunk = px * swz + (res ? 0 : k.w_chunk_bytes);
-                const int avail     = budget - 1024 - staging - w_bytes;
-                if (avail < 2 * per_chunk)
-                    continue;
-                int ksub = std::max(1, std::min(k.total_chunks, 48 * 1024 / per_chunk));
-                while (ksub > 1 && avail / (ksub * per_chunk) < 3)
-                    ksub--;
-                const int stages = std::min(kChanMaxStages, avail / (ksub * per_chunk));
-                const double rate = std::min(std::min(50.0, 32.0 * ctx->num_sms / grid), (double)(stages - 1) * ksub * per_chunk / 2900.0);
-                const double mma  = (double)k.total_chunks * k.mmas * (px == 256 ? 171 : px == 192 ? 139 : px == 128 ? 107 : 104) +
-                                   60.0 * ((k.total_chunks + ksub - 1) / ksub + 1);
-                const double epi  = px * (q.join ? 26.0 : 14.7) + 500;
-                const double load = (double)k.total_chunks * per_chunk / rate + (q.join ? px * 128 / 50.0 : 0.0);
-                const int64_t rounds = (tiles + grid - 1) / grid;
-                const bool few       = slots == (q.join ? 2 : 1);    // the store, or the residual's load, is not overlapped
-                const double cost = 1200 + std::max(mma, load + w_bytes / 50.0) + epi + (double)(rounds - 1) * (std::max(mma, std::max(epi, load)) + (few ? 300 : 0));
-                if (best == 0 || cost < best * 0.98)
-                {
-                    best            = cost;
-                    k.px            = px;
-                    k.resident      = res;
-                    k.slots         = slots;
-                    k.ksub          = ksub;
-                    k.num_stages    = stages;
-                    k.x_chunk_bytes = px * swz;
-                    k.stage_bytes   = ksub * per_chunk;
-                    k.tiles         = (int)tiles;
-                    k.w_off         = staging;
-                    k.ring_off      = staging + w_bytes;
-                    plan->grid      = grid;
-                    plan->smem_bytes = 1024 + staging + w_bytes + stages * ksub * per_chunk;
-                }
-            }
-    // One tile per cluster of S CTAs, where that fills one wave at most (conv_split_kernel).
-    for (int px = 64; px >= 32; px >>= 1)
-        for (int S = 1; S <= 8 && px / S >= 4 && S <= k.total_chunks; S *= 2)
-        {
-            const int64_t tiles = (pixels + px - 1) / px * k.cbs;
-            const int cpc       = (k.total_chunks + S - 1) / S;
-            const int stage     = (px + 128) * swz;
-            const int smem      = 1024 + cpc * stage + (S > 1 ? px * 512 : 0);
-            // one wave: clusters of 8 and 4 leave SMs of a GPC over when a CTA fills its SM
-            const int room = smem <= 110 * 1024 || S == 1 ? ctx->num_sms : ctx->num_sms * (S == 8 ? 3 : 4) / (S == 8 ? 4 : 5);
-            if (tiles * S > room || cpc > kSplitMaxChunks || smem > budget)
-                continue;
-            const double cost = split_cost(px, S, cpc, k.mmas);
-            if (cost > 0 && (best == 0 || cost < best))
-            {
-                best             = cost;
-                k.split          = S;
-                k.chunks_per_cta = cpc;
-                k.px             = px;
-                k.x_chunk_bytes  = px * swz;
-                k.stage_bytes    = stage;
-                k.red_off        = cpc * stage;
-                k.tiles          = (int)tiles;
-                plan->grid       = (int)tiles * S;
-                plan->smem_bytes = smem;
-            }
-        }
-    if (best == 0)
+    bool known = false;
+    if (!ctx->chan_memo)
+        ctx->chan_memo.reset(new SizeMemo<ChanChoice>());
+    auto& memo = ctx->chan_memo->at(pixels, (int64_t)q.OC << 32 | q.IC, (int64_t)q.KH << 32 | q.KW << 1 | (q.join ? 1 : 0), &known);
+    if (!known)
+        memo.value = chan_choose(ctx->num_sms, ctx->max_smem_optin, pixels, q.OC, q.IC, q.KH, q.KW, q.join != nullptr);
+    const ChanChoice& c = memo.value;
+    if (!c.taken)
         return false;
-    // Channel blocks less than three quarters full leave rows of the product and threads of the epilogue idle: 160 channels on
-    // 21x102x13x96 7.6 us against 6.6 with a pixel per thread, 32 channels 3x3 on 13x32x12x32 8.5 against 5.9; 192 channels 3x3 on
-    // 8x26x10x192 10.4 against 13.5.  Where the products are long and the pixels many they are what counts, and there this kernel
-    // needs fewer of them (K, pixels, us here / with a pixel per thread): 64 channels 3200, 14 850 15.0 / 19.6, 4320, 26 884 35.7 / 91.5,
-    // 3744, 25 688 31.7 / 42.3, but 3456, 12 312 15.9 / 12.6, 4608, 13 392 18.7 / 14.6, 4320, 9 085 31.1 / 26.0; 32 channels 4000, 61 950
-    // 92 / 125, 4800, 16 302 26.3 / 32.9, but 3456, 27 360 27.0 / 20.2, 3168, 81 576 116 / 85, 4000, 6 912 42.9 / 24.0.
-    // A residual join pays for itself at any width.
-    const int rows = (q.OC + 127) / 128 * 128;
-    if (!k.split && !q.join && q.OC * 4 < rows * 3 &&
-        ((int64_t)q.KH * q.KW * q.IC < (q.OC * 4 <= rows ? 4000 : 3072) || pixels < 96 * (int64_t)ctx->num_sms))
-        return false;
-    // Windows over 32-byte pieces, loaded again for each of several channel blocks: 512 channels 3x3 on 24x34x49x96 23.7 / 19.9, 256
-    // 5x5 on 22x18x50x32 25.9 / 18.9, 448 3x3 on 54x11x18x32 16.4 / 12.0, 416 5x5 on 9x64x25x96 41.3 / 38.4.
-    if (!k.split && !q.join && q.KH * q.KW > 1 && q.IC % 64 != 0 && q.OC >= 256)
-        return false;
+    k.px = c.px; k.resident = c.resident; k.slots = c.slots; k.ksub = c.ksub; k.num_stages = c.num_stages;
+    k.x_chunk_bytes = c.x_chunk_bytes; k.stage_bytes = c.stage_bytes; k.tiles = c.tiles; k.w_off = c.w_off; k.ring_off = c.ring_off;
+    k.split = c.split; k.chunks_per_cta = c.chunks_per_cta; k.red_off = c.red_off;
+    plan->grid = c.grid; plan->smem_bytes = c.smem_bytes;
     k.idesc     = ptx::make_idesc(2u, 1u, 1u, 0u, 0u, 128u, (uint32_t)k.px);
     k.tmem_cols = k.split ? k.px : k.px == 192 ? 512 : 2 * k.px;
     fastdiv_make((uint32_t)(q.OH * q.OW), k.fd_ohow);
@@ -1192,7 +1216,7 @@ bool chan_plan(const tb200_ctx* ctx, const TcProblem& q, ChanPlan* plan)
 
 }    // namespace
 
-bool conv_chan_supported(const tb200_ctx* ctx, const TcProblem& q)
+bool conv_chan_supported(tb200_ctx* ctx, const TcProblem& q)
 {
     ChanPlan plan;
     return chan_plan(ctx, q, &plan);

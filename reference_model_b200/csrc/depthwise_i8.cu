@@ -432,11 +432,19 @@ tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q,
         TB200_CUDA_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kerns[which], 128, 0));
         ctx->dw_blocks[which] = std::max(1, occ);
     }
-    dw_pieces((int64_t)q.N * p.row_groups * p.c4, q.OW, q.K, q.S, R, ctx->num_sms, ctx->dw_blocks[which], &p.len, &p.strips);
+    const int64_t lines = (int64_t)q.N * p.row_groups * p.c4;
+    bool known          = false;
+    if (!ctx->dw_memo)
+        ctx->dw_memo.reset(new SizeMemo<DwPieces>());
+    auto& memo = ctx->dw_memo->at(lines, q.OW, which, &known);
+    if (!known)
+        dw_pieces(lines, q.OW, q.K, q.S, R, ctx->num_sms, ctx->dw_blocks[which], &memo.value.len, &memo.value.strips);
+    p.len    = memo.value.len;
+    p.strips = memo.value.strips;
     fastdiv_make((uint32_t)p.c4, p.fd_c4);
     fastdiv_make((uint32_t)p.strips, p.fd_strips);
     fastdiv_make((uint32_t)p.row_groups, p.fd_rg);
-    p.total    = (int)((int64_t)q.N * p.row_groups * p.c4 * p.strips);
+    p.total    = (int)(lines * p.strips);
     p.fill4    = (uint32_t)(q.in_zp & 0xff) * 0x01010101u;
     p.clamp_lo = q.clamp_lo;
     p.clamp_hi = q.clamp_hi;

@@ -29,3 +29,9 @@ def test_row_matmuls_stay_inside_32_bit_indexes(tmp_path):
 def test_depthwise_pieces_are_found_in_few_steps(tmp_path):
     rc, out = _run(tmp_path, "depthwise_pieces_check")
     assert rc == 0 and "wrong=0" in out, out
+
+
+@pytest.mark.skipif(NVCC is None, reason="needs nvcc")
+def test_channel_row_layouts(tmp_path):
+    rc, out = _run(tmp_path, "conv_chan_check")
+    assert rc == 0 and "wrong=0" in out, out
