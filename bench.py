@@ -398,6 +398,24 @@ def run_matmul(args, rank, local_rank, world, barrier, all_max):
 # ---------------------------------------------------------------------------------------------------------------------
 # The whole int8 ResNet-50-shaped TOSA graph, batch 256 split by N over the ranks, logits gathered behind the C ABI.
 # ---------------------------------------------------------------------------------------------------------------------
+def activation_bytes(g, steps):
+    """Activation traffic with fused epilogues: every tensor a device step reads or writes, once."""
+    total = 0
+    for kind, payload in steps:
+        ops = [o for o in (payload if isinstance(payload, tuple) else (payload,)) if o is not None]
+        if kind in ("SLICE", "RESHAPE"):
+            continue
+        names = {ops[0].inputs[0], ops[-1].outputs[0]}
+        if kind == "RESIDUAL_JOIN":
+            names.add(payload[1].inputs[0])
+        elif kind == "CONV_JOIN":
+            names.add(payload[4].inputs[0])    # the other operand of the join inside the convolution
+        for name in names:
+            dt, shape = g.meta[name]
+            total += int(np.prod(shape)) * (4 if dt.name == "INT32" else 1)
+    return total
+
+
 def run_graph(args, rank, local_rank, world, barrier, all_max, all_min, exchange_bytes):
     import torch
     import reference_model_b200 as tb
@@ -485,18 +503,7 @@ def run_graph(args, rank, local_rank, world, barrier, all_max, all_min, exchange
     peaks = measured_peaks()
     img_s = total * args.steps / (ms * 1e-3)
     macs = g.macs() / nb
-    # activation traffic with fused epilogues: every tensor a device step reads or writes, once
-    act_bytes = 0
-    for kind, payload in run.steps:
-        ops = [o for o in (payload if isinstance(payload, tuple) else (payload,)) if o is not None]
-        if kind in ("SLICE", "RESHAPE"):
-            continue
-        names = {ops[0].inputs[0], ops[-1].outputs[0]}
-        if kind == "RESIDUAL_JOIN":
-            names.add(ops[1].inputs[0])
-        for nme in names:
-            dt, shape = g.meta[nme]
-            act_bytes += int(np.prod(shape)) * (4 if dt == tb.DType.INT32 else 1)
+    act_bytes = activation_bytes(g, run.steps)
     weight_bytes = sum(int(a.nbytes) for a in g.consts.values())
     bytes_per_step = (act_bytes + weight_bytes) * world
     tops = 2.0 * macs * total * args.steps / (ms * 1e-3) / 1e12

@@ -196,3 +196,14 @@ def test_joins_in_place_on_memory_of_the_caller(ctx):
     # an output of the caller's that meets none of its other tensors is no obstacle
     run = G.DeviceRunner(ctx, _block().g, external={"y": buf, "x": ctx.empty(I8, (1, 5, 5, 8))})
     assert "CONV_JOIN" in [k for k, _ in run.steps]
+
+
+def test_bench_counts_the_other_operand_of_a_join_inside_a_convolution():
+    import bench
+    g = G.resnet50_int8(1, image=96)
+    fused, inside = G.fuse_joins(g, G.fuse(g))
+    apart = [s for s in G.fuse(g)]
+    size = lambda n: int(np.prod(g.meta[n][1]))
+    # a join inside saves writing the convolution's result and reading it again, and nothing else
+    assert len(inside) == 16
+    assert bench.activation_bytes(g, apart) - bench.activation_bytes(g, fused) == 2 * sum(size(n) for n in inside)
