@@ -2763,7 +2763,7 @@ extern "C" tb200_status tb200_matmul(tb200_ctx* ctx, const tb200_tensor* a, cons
             return sgemm_f32_launch(ctx, reinterpret_cast<const float*>(a->data), reinterpret_cast<const float*>(b->data),
                                     reinterpret_cast<float*>(output->data), N, H, C, W);
     }
-    else if (ctx->policy == 0 && a->dtype == b->dtype && matmul_rows_supported(a->dtype, a->data, b->data, N, H, C, W))
+    else if (ctx->policy == 0 && a->dtype == b->dtype && matmul_rows_supported(a->dtype, a->data, b->data, N, H, C, W, ctx->num_sms))
         return matmul_rows_launch(ctx, a->dtype, a->data, b->data, output->data, output->dtype, N, H, C, W, a_zp, b_zp);
     else if (ctx->policy == 0)
     {

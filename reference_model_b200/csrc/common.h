@@ -499,7 +499,7 @@ tb200_status depthwise_slide_pack(tb200_ctx* ctx, const DepthwiseI8Problem& q, v
 tb200_status depthwise_slide_launch(tb200_ctx* ctx, const DepthwiseI8Problem& q, const void* block, const char* name);
 
 // MATMUL of int8 (int32 out) and 16-bit operands with up to four rows (matmul_rows.cu)
-bool matmul_rows_supported(tb200_dtype dt, const void* a, const void* b, int N, int H, int C, int W);
+bool matmul_rows_supported(tb200_dtype dt, const void* a, const void* b, int N, int H, int C, int W, int num_sms);
 tb200_status matmul_rows_launch(tb200_ctx* ctx, tb200_dtype dt, const void* a, const void* b, void* out, tb200_dtype out_dt, int N, int H, int C, int W,
                                 int32_t a_zp, int32_t b_zp);
 

@@ -1074,7 +1074,10 @@ ChanChoice chan_choose(int num_sms, int max_smem, int64_t pixels, int OC, int IC
                 const double epi  = px * (join ? 26.0 : 14.7) + 500;
                 const double load = (double)total_chunks * per_chunk / rate + (join ? px * 128 / 50.0 : 0.0);
                 const int64_t rounds = (tiles + grid - 1) / grid;
-                const bool few       = slots == (join ? 2 : 1);    // the store, or the residual's load, is not overlapped
+                // the store, or the residual's load, is not overlapped.  (With a join two slots take as long as three where the tile is the
+                // same, 256 channels 3x3 on 128x14x14x256 24.4 / 24.3 us, 512 on 256x7x7x512 37.9 / 38.0, and less where they make room
+                // for a larger one, 128 on 128x28x28x128 24.9 / 27.5.)
+                const bool few       = slots == (join ? 2 : 1);
                 const double cost = 1200 + std::max(mma, load + w_bytes / 50.0) + epi + (double)(rounds - 1) * (std::max(mma, std::max(epi, load)) + (few ? 300 : 0));
                 if (best == 0 || cost < best * 0.98)
                 {

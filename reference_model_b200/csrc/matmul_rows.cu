@@ -310,11 +310,11 @@ typedef void (*RowsKern)(const RowsParams);
 // 8.3 / 16.4, but 1000x4x256x256 36 / 31: with more than eight blocks per SM the tiles' own loads keep memory busy, and several
 // rows of 16-bit elements cost a conversion and a multiply-add each.  Over 460 shapes the time is 0.56 of the tiles'; they are faster
 // in some with about a block per SM: int8 16x1x488x880 8.2 / 6.7, fp16 34x2x3208x416 27.9 / 19.5 (but 13x2x2848x944 13.9 / 27.8).
-bool matmul_rows_supported(tb200_dtype dt, const void* a, const void* b, int N, int H, int C, int W)
+bool matmul_rows_supported(tb200_dtype dt, const void* a, const void* b, int N, int H, int C, int W, int num_sms)
 {
     const uintptr_t al = dt == TB200_INT8 ? 3 : 7;
     return (dt == TB200_INT8 || dt == TB200_FP16 || dt == TB200_BF16) && H >= 1 && H <= 4 && C >= 256 && C <= (1 << 30) && W >= 4 && C % 4 == 0 && W % 4 == 0 && N <= 65535 &&
-           !(dt != TB200_INT8 && H > 1 && C % 8 == 0 && W % 8 == 0 && (int64_t)N * ((W + kRowsCols - 1) / kRowsCols) > 8 * 148) &&
+           !(dt != TB200_INT8 && H > 1 && C % 8 == 0 && W % 8 == 0 && (int64_t)N * ((W + kRowsCols - 1) / kRowsCols) > 8 * (int64_t)num_sms) &&
            ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & al) == 0;
 }
 

@@ -19,7 +19,7 @@ int main()
     for (tb200_dtype dt : { TB200_INT8, TB200_FP16, TB200_BF16 })
         for (long long c : { 256LL, 4096LL, 1LL << 20, (1LL << 30) - 4, 1LL << 30, (1LL << 30) + 4, (1LL << 31) - 1024, (1LL << 31) - 4 })
         {
-            if (!matmul_rows_supported(dt, p, p, 1, 1, (int)c, 4))
+            if (!matmul_rows_supported(dt, p, p, 1, 1, (int)c, 4, 148))
                 continue;
             taken++;
             for (int splits = 1; splits <= 8; splits *= 2)

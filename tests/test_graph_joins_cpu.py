@@ -207,3 +207,84 @@ def test_bench_counts_the_other_operand_of_a_join_inside_a_convolution():
     # a join inside saves writing the convolution's result and reading it again, and nothing else
     assert len(inside) == 16
     assert bench.activation_bytes(g, apart) - bench.activation_bytes(g, fused) == 2 * sum(size(n) for n in inside)
+
+
+def _kinds(n):
+    return [k for k, _ in G.fuse_joins(n.g, G.fuse(n.g))[0]]
+
+
+def _runs_right(ctx, n, inputs=("x",)):
+    """Every tensor that the runner can name is that of the oracle."""
+    x = {name: n.image(k) for k, name in enumerate(inputs)}
+    run = G.DeviceRunner(ctx, n.g)
+    for name, a in x.items():
+        run.set_input(a, name)
+    run.run()
+    ref = graph_eval.evaluate(n.g, x, nthreads=4)[1]
+    for name in n.g.meta:
+        if name in run.t or name in run._inside:
+            assert np.array_equal(run.output(name)[1], ref[name]), name
+
+
+def test_the_later_of_two_convolutions_takes_the_join(ctx):
+    n = _Net()
+    n.conv("x", "in")
+    n.conv("in", "a")
+    n.conv("in", "b")
+    n.join("a", "b", "y")    # b is there last
+    n.g.outputs.append("y")
+    steps, inside = G.fuse_joins(n.g, G.fuse(n.g))
+    assert [k for k, _ in steps] == ["CONV_RESCALE_CLAMP"] * 2 + ["CONV_JOIN"] and list(inside) == ["b"]
+    _runs_right(ctx, n)
+    n = _Net()
+    n.conv("x", "in")
+    n.conv("in", "a")
+    n.conv("in", "b")
+    n.join("b", "a", "y")    # ... as the first operand
+    n.g.outputs.append("y")
+    assert list(G.fuse_joins(n.g, G.fuse(n.g))[1]) == ["b"]
+    _runs_right(ctx, n)
+
+
+def test_an_operand_that_is_made_later_is_waited_for(ctx):
+    """Only the convolution that is there first has no other reader: it cannot take what is not there yet."""
+    n = _Net()
+    n.conv("x", "in")
+    n.conv("in", "a")
+    n.conv("in", "b")
+    n.conv("b", "c")         # a second reader of b
+    n.join("a", "b", "y")
+    n.join("y", "c", "z")    # c is there before y is
+    n.g.outputs.append("z")
+    kinds = _kinds(n)
+    assert kinds.count("RESIDUAL_JOIN") == 2 and "CONV_JOIN" not in kinds
+    _runs_right(ctx, n)
+
+
+@pytest.mark.parametrize("why", ["graph output", "second reader", "same tensor"])
+def test_results_that_others_read_stay_outside(ctx, why):
+    n = _Net()
+    n.conv("x", "in")
+    n.conv("in", "a")
+    n.join("a", "a" if why == "same tensor" else "in", "y")
+    n.g.outputs.append("y")
+    if why == "graph output":
+        n.g.outputs.append("a")
+    elif why == "second reader":
+        n.conv("a", "c")
+        n.g.outputs.append("c")
+    assert "CONV_JOIN" not in _kinds(n)
+    _runs_right(ctx, n)
+
+
+def test_a_chain_of_blocks(ctx):
+    """Joins over joins, as a network has them: the result of one is the other operand of the next."""
+    n = _Net()
+    n.conv("x", "s0")
+    for i in range(3):
+        n.conv("s%d" % i, "a%d" % i)
+        n.conv("a%d" % i, "b%d" % i)
+        n.join("b%d" % i, "s%d" % i, "s%d" % (i + 1))
+    n.g.outputs.append("s3")
+    assert _kinds(n).count("CONV_JOIN") == 3
+    _runs_right(ctx, n)
