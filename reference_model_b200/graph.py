@@ -18,6 +18,8 @@ outputs are allocated before a node runs.  Two things are added for the device:
 (the exact-division rule, reference_model/src/ops/tensor_ops.cpp:203-223), SLICE to an odd size in front of the
 stride-2 1x1 shortcut convolutions, INT32-only ADD for the residual joins (reference_model/src/ops/op_factory.cpp:189-195).
 """
+import weakref
+
 import numpy as np
 
 from . import binding as tb
@@ -340,14 +342,15 @@ def fuse_joins(graph, steps, external=()):
 
 # ------------------------------------------------------------------------------------------------ device runner
 class _Tensors(dict):
-    """name -> Tensor; what stays inside a fused step is made when it is asked for."""
+    """name -> Tensor; what stays inside a fused step is made when it is asked for.  (The runner owns this, not the other way
+    round: its graph's arrays go with its last reference.)"""
 
-    def __init__(self, make, items):
+    def __init__(self, runner, items):
         super().__init__(items)
-        self._make = make
+        self._runner = weakref.ref(runner)
 
     def __missing__(self, name):
-        return self._make(name)
+        return self._runner()._inside_tensor(name)
 
 
 class DeviceRunner:
@@ -358,7 +361,7 @@ class DeviceRunner:
         """external: optional name -> Tensor for tensors the caller owns (e.g. an output wrapped over a buffer that a
         collective reads)."""
         self.ctx, self.graph = ctx, graph
-        self.t = _Tensors(self._inside_tensor, external or {})
+        self.t = _Tensors(self, external or {})
         self._late, self._seen = {}, 0
         self.steps, self._inside = fuse_joins(graph, fuse(graph), set(self.t)) if fused else ([(op.kind, op) for op in graph.ops], {})
         for name_, arr in graph.consts.items():

@@ -288,3 +288,18 @@ def test_a_chain_of_blocks(ctx):
     n.g.outputs.append("s3")
     assert _kinds(n).count("CONV_JOIN") == 3
     _runs_right(ctx, n)
+
+
+def test_a_runner_goes_with_its_last_reference(ctx):
+    """... and its graph's arrays with it, not at the garbage collector's next look."""
+    import gc
+    import weakref
+    gc.disable()
+    try:
+        n = _block()
+        run = G.DeviceRunner(ctx, n.g)
+        ref = weakref.ref(run)
+        del run
+        assert ref() is None
+    finally:
+        gc.enable()
