@@ -1019,7 +1019,7 @@ struct ChanPlan
     CUtensorMapSwizzle swz;
 };
 
-// SM cycles of a small problem on conv_split_kernel, in the measure of chan_plan's estimates (fitted to device times of layers on
+// SM cycles of a small problem on conv_split_kernel, in the measure of chan_choose's estimates (fitted to device times of layers on
 // one and two images): a chunk costs its MMAs, an exchange the columns that a CTA hands out and finishes; 0: not worth trying.
 double split_cost(int px, int S, int chunks, int mmas)
 {
